@@ -322,7 +322,9 @@ __device__ __forceinline__ void spread_pair_body(const YgArgs& a, int u0, const 
         if (ok) s = ldg4(srow + static_cast<size_t>(xp) * a.cy + yb);
         if (paired && ok) q = ldg4(mrow + static_cast<size_t>(a.nx - 1 - xp) * a.cy + yb);
         if (ATT) {
-          const float4 m = sample4(mu, tb[tap_slot<R>(c)], yb, yok);
+          // the branch: the predicated form leaves too few registers beside the
+          // two transmissions (128^3 x 120: 0.298 ms a launch, predicated 0.349)
+          const float4 m = sample4_branch(mu, tb[tap_slot<R>(c)], yb, yok);
           if constexpr (KAHAN) {
             float4 cc = scomp[k * 32 * kW + threadIdx.x];
             kahan_add4p(Tc[k], cc, m);
