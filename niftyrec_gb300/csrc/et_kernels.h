@@ -60,6 +60,7 @@ struct YgArgs {
   int row0 = 0;                   // first row of the window (multiple of 4)
   int out_lo = 0, out_hi = 1 << 30;  // valid output rows of the window, relative to row0
   int cs = 0;                     // column stride of the backprojector's scratch
+  int lanes = 32;                 // lanes per column of the window's tile kernels (32, 16, 8)
   const CamGeom* geom = nullptr;  // device [ncam]
   const float* act = nullptr;     // [nz][nx][cy] (bfloat16 data when storage == kStorageBF16)
   const float* mu = nullptr;      // [nz][nx][cy] or null (same storage as act)
@@ -170,6 +171,8 @@ struct BatchStepDesc {
   YgArgs proj;
   int nwin = 0;
   int win[kMaxWindows][4] = {};  // row0, rows, lo, hi (as the launchers' windows)
+  int lanes[kMaxWindows] = {};   // lanes per column and x-tiles of each window
+  int tiles[kMaxWindows] = {};
   const float* counts = nullptr;   // subset counts, column layout
   float* act = nullptr;            // activity (column layout; proj.act), written by the update
   float* num = nullptr;            // backprojected ratio
@@ -194,6 +197,9 @@ struct BatchElems {
 // PSF); writes 4 ints per window (row0, rows, lo, hi), returns the count or
 // -1 if more than max_windows.
 int yg_row_windows(int ny, int psf_k, int* out, int max_windows);
+// Lanes per column the tile kernels take for a window of `rows` rows of nx
+// columns, and the x-tiles that gives.
+void yg_window_lanes(int rows, int nx, int* lanes, int* tiles);
 // Persistent projector over all selected volumes: clusters take work items
 // from the counter (zeroed by the caller) until none are left.  Volumes of
 // one launch share psf_k and whether they have mu; max_nz sizes the PSF table.

@@ -667,6 +667,7 @@ int nrgb_batch_create(void** out_batch, void* const* plans, int n_plans, void* s
         delete b;
         return kErrParameters;
       }
+      for (int w = 0; w < d.nwin; ++w) yg_window_lanes(d.win[w][1], pb.nx, &d.lanes[w], &d.tiles[w]);
       d.counts = b->counts[v] + plane * c0;
       d.act = b->act[v];
       d.num = p->osem_num;
@@ -780,9 +781,10 @@ int nrgb_batch_osem_step(void* batch, int step, int iterations, float epsilon, v
       const Plan& p = *b->plans[v];
       if (sub[v] < 0 || p.proj.psf_k != kinds[k].first || (p.has_att ? 1 : 0) != kinds[k].second) continue;
       const BatchStepDesc& d = b->h_desc[b->desc_base[v] + sub[v]];
-      const int ntile = (d.proj.nx + 31) / 32;
+      int ntile = 0;
+      for (int w = 0; w < d.nwin; ++w) ntile += d.tiles[w];
       sel.desc[sel.n] = b->desc_base[v] + sub[v];
-      sel.begin[sel.n + 1] = sel.begin[sel.n] + d.nwin * d.proj.ncam * ntile;
+      sel.begin[sel.n + 1] = sel.begin[sel.n] + d.proj.ncam * ntile;
       ++sel.n;
       max_nz = std::max(max_nz, d.proj.nz);
     }

@@ -1,0 +1,11 @@
+// Exact-transpose spread kernels for PSF radii 0 and 1.
+#include "et_yg_spread_kernels.cuh"
+
+namespace nrgb {
+
+template int launch_spread_R<0, true>(const YgArgs& a, int c0, int gcount, cudaStream_t st);
+template int launch_spread_pair_R<0, true>(const YgArgs& a, int u0, int gcount, cudaStream_t st);
+template int launch_spread_R<1, true>(const YgArgs& a, int c0, int gcount, cudaStream_t st);
+template int launch_spread_pair_R<1, true>(const YgArgs& a, int u0, int gcount, cudaStream_t st);
+
+}  // namespace nrgb

@@ -1,0 +1,11 @@
+// Exact-transpose spread kernels for PSF radii 4 and 5.
+#include "et_yg_spread_kernels.cuh"
+
+namespace nrgb {
+
+template int launch_spread_R<4, true>(const YgArgs& a, int c0, int gcount, cudaStream_t st);
+template int launch_spread_pair_R<4, true>(const YgArgs& a, int u0, int gcount, cudaStream_t st);
+template int launch_spread_R<5, true>(const YgArgs& a, int c0, int gcount, cudaStream_t st);
+template int launch_spread_pair_R<5, true>(const YgArgs& a, int u0, int gcount, cudaStream_t st);
+
+}  // namespace nrgb

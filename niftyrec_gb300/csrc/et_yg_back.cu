@@ -4,6 +4,13 @@
 #include "et_yg_device.cuh"
 
 namespace nrgb {
+
+// et_yg_spread_kernels.cuh
+template <int R, bool ADJ>
+int launch_spread_R(const YgArgs& a, int c0, int gcount, cudaStream_t st);
+template <int R, bool ADJ>
+int launch_spread_pair_R(const YgArgs& a, int u0, int gcount, cudaStream_t st);
+
 namespace {
 
 // ------------------------------------------------ backprojector: slab carry
@@ -12,18 +19,19 @@ namespace {
 // from; carry[c][a.bslabs][x][y] = the whole column's sum.  One block row per
 // camera c, or with a.units per unit (its first camera c; a mirror camera's
 // transmissions are c's read from the other end); one warp per depth slab.
-template <class V>
+// L lanes per column: a warp walks 32 / L times kCarryCols columns.
+template <class V, int L>
 __global__ void __launch_bounds__(32 * kSlabsB) k_mu_carry_yg(const YgArgs a, int u0) {
-  constexpr int C = kCarryCols;
+  constexpr int C = kCarryCols, GW = 32 / L;
   constexpr bool KAHAN = StorageTraits<V>::kKahan;
   const V* __restrict__ mu = reinterpret_cast<const V*>(a.mu) + a.row0;
-  __shared__ Tap s_tap[kSlabsB][C];
+  __shared__ Tap s_tap[kSlabsB][GW][C];
   __shared__ float4 s_sum[kSlabsB][C][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nchunk = (a.nx + C - 1) / C;
+  const int warp = threadIdx.x >> 5, wlane = threadIdx.x & 31, sub = wlane / L, lane = wlane % L;
+  const int nchunk = (a.nx + C * GW - 1) / (C * GW);
   const int unit = u0 + blockIdx.x / nchunk;
   const int cam = a.units ? a.units[unit].x : unit;
-  const int x0 = (blockIdx.x % nchunk) * C;
+  const int x0 = ((blockIdx.x % nchunk) * GW + sub) * C;
   const int yb = lane * 4;
   const bool yok = lane_rows_ok(a, yb);
   const CamRows cr = cam_rows(a.geom[cam].fwd);
@@ -39,15 +47,15 @@ __global__ void __launch_bounds__(32 * kSlabsB) k_mu_carry_yg(const YgArgs a, in
   for (int z = zbeg; z < zend; ++z) {
     if (lane < C) {
       const int xp = x0 + lane;
-      s_tap[warp][lane] = make_tap(xp, z, cr.m00, cr.m02, cr.m03, cr.m20, cr.m22, cr.m23, a.nx, a.nz, a.cy, xp < a.nx);
+      s_tap[warp][sub][lane] = make_tap(xp, z, cr.m00, cr.m02, cr.m03, cr.m20, cr.m22, cr.m23, a.nx, a.nz, a.cy, xp < a.nx);
     }
     __syncwarp();
 #pragma unroll
-    for (int i = 0; i < C; ++i) depth_add4<KAHAN>(S[i], cS[i], sample4(mu, s_tap[warp][i], yb, yok));
+    for (int i = 0; i < C; ++i) depth_add4<KAHAN>(S[i], cS[i], sample4(mu, s_tap[warp][sub][i], yb, yok));
     __syncwarp();
   }
 #pragma unroll
-  for (int i = 0; i < C; ++i) s_sum[warp][i][lane] = depth_value4<KAHAN>(S[i], cS[i]);
+  for (int i = 0; i < C; ++i) s_sum[warp][i][wlane] = depth_value4<KAHAN>(S[i], cS[i]);
   __syncthreads();
   if (!yok || !lane_writes(a, yb)) return;
 #pragma unroll
@@ -55,358 +63,14 @@ __global__ void __launch_bounds__(32 * kSlabsB) k_mu_carry_yg(const YgArgs a, in
     const int x = x0 + i;
     if (x >= a.nx) continue;
     float4 pre = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = 0; s < warp; ++s) add4(pre, s_sum[s][i][lane]);
+    for (int s = 0; s < warp; ++s) add4(pre, s_sum[s][i][wlane]);
     float* dst = a.slab_T + ((static_cast<size_t>(cam) * slots + warp) * a.nx + x) * a.cy + a.row0 + yb;
     *reinterpret_cast<float4*>(dst) = pre;
     if (warp == nsl - 1) {  // the column total, one slot further
-      add4(pre, s_sum[warp][i][lane]);
+      add4(pre, s_sum[warp][i][wlane]);
       *reinterpret_cast<float4*>(dst + static_cast<size_t>(a.nx) * a.cy) = pre;
     }
   }
-}
-
-// ---------------------------------------- backprojector: spread + PSF
-// temp[g][z][x][y] = PSF_z( s(x', y) * exp(-T_z(x', y)) ) for camera c0+g,
-// T inclusive (emission-lib/_et_line_backproject_attenuated.cpp:24-34), PSF
-// as in the projector.  CTA = (camera, x-tile, depth slab); every sampled
-// column starts its transmission from the slab carry.
-// ADJ: the exact transpose of the projector instead (not in the reference):
-// the PSF taps are flipped (correlation) and each output column is scattered
-// with the projector's own bilinear weights into the accumulator a.out
-// (vector reductions; all cameras in one launch, no scratch), or, with
-// a.det, written to the group scratch like the reference form for the
-// transposed gather k_tgather_yg (a fixed summation order).
-// CTAS: CTAs per SM the kernel is compiled for (3 where three tiles fit in
-// shared memory, for the float32 reference spread; else 2).
-// PTAB: the separated PSF comes from the kernel-parameter table `ptab`
-// ([nz][2K]) instead of a shared-memory copy of the slab's planes.
-template <int R, bool PSF, bool ATT, bool ADJ, class V, bool PTAB>
-__device__ __forceinline__ void spread_body(const YgArgs& a, int c0, const float* ptab) {
-  using TS = TileShape<R>;
-  constexpr bool KAHAN = StorageTraits<V>::kKahan;
-  const V* __restrict__ mu = reinterpret_cast<const V*>(a.mu) + a.row0;
-  constexpr int NS = TS::NS;
-  constexpr int K = 2 * R + 1;
-  extern __shared__ __align__(16) unsigned char smem[];
-  float4* sb = reinterpret_cast<float4*>(smem);
-  Tap* taps = reinterpret_cast<Tap*>(smem + TS::kSbBytes);
-  float* s_psf = reinterpret_cast<float*>(smem + TS::kSbBytes + TS::kTapBytes);
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ntile = (a.nx + kTXC - 1) / kTXC;
-  const int nsl = a.bslabs, slots = nsl + 1;
-  const int slab = blockIdx.x % nsl;
-  const int item = blockIdx.x / nsl;
-  const int g = item / ntile;
-  const int cam = c0 + g;
-  const int x0 = (item % ntile) * kTXC;
-  const int yb = lane * 4;
-  const bool yok = lane_rows_ok(a, yb);
-  const int zper = (a.nz + nsl - 1) / nsl;
-  const int zbeg = slab * zper, zend = min(a.nz, zbeg + zper);
-  if (zbeg >= zend) return;  // uniform over the CTA
-  if (PSF && !PTAB) {  // this slab's planes only
-    for (int i = zbeg * 2 * K + threadIdx.x; i < zend * 2 * K; i += blockDim.x) {
-      const int j = i % (2 * K), base = i - j;
-      // transpose of a convolution = correlation: reverse each kernel
-      const int src = !ADJ ? i : (j < K ? base + (K - 1 - j) : base + K + (2 * K - 1 - j));
-      s_psf[i] = __ldg(a.psf + src);
-    }
-  }
-  const CamRows cr = cam_rows(a.geom[cam].fwd);
-  const size_t vol = static_cast<size_t>(a.nz) * a.nx * a.cs;  // one scratch volume
-  const bool scatter = ADJ && !a.det;  // uniform over the launch
-  float* __restrict__ tmp = scatter ? a.out + a.row0 : a.temp + vol * g;
-  const float* __restrict__ srow = a.sino + static_cast<size_t>(cam) * a.nx * a.cy + a.row0;
-
-  float4 Tc[TS::kOwn], cTc[TS::kOwn];  // transmission per sampled column (+ Kahan compensation)
-#pragma unroll
-  for (int k = 0; k < TS::kOwn; ++k) {
-    Tc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    cTc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    const int xp = x0 - R + warp + kW * k;
-    if (ATT && warp + kW * k < NS && xp >= 0 && xp < a.nx && yok)
-      Tc[k] = ldg4(a.slab_T + ((static_cast<size_t>(cam) * slots + slab) * a.nx + xp) * a.cy + a.row0 + yb);
-  }
-  ybuf_zero_pads();
-  __syncthreads();
-
-  for (int z = zbeg; z < zend; ++z) {
-    const int b = z & 1;
-    float4* sbuf = sb + b * NS * 32;
-    Tap* tb = taps + b * TS::kTapSlots;
-    if ((ATT || ADJ) && lane < TS::kOwn) {
-      const int c = warp + kW * lane;
-      if (c < NS) {
-        const int xp = x0 - R + c;
-        tb[tap_slot<R>(c)] = make_tap(xp, z, cr.m00, cr.m02, cr.m03, cr.m20, cr.m22, cr.m23, a.nx, a.nz, a.cy,
-                         xp >= 0 && xp < a.nx);
-      }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < TS::kOwn; ++k) {
-      const int c = warp + kW * k;
-      if (c < NS) {
-        const int xp = x0 - R + c;
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (xp >= 0 && xp < a.nx && yok) s = ldg4(srow + static_cast<size_t>(xp) * a.cy + yb);
-        if (ATT) {
-          depth_add4<KAHAN>(Tc[k], cTc[k], sample4(mu, tb[tap_slot<R>(c)], yb, yok));
-          s = mul4(s, exp_neg4(depth_value4<KAHAN>(Tc[k], cTc[k])));
-        }
-        sbuf[c * 32 + lane] = s;
-      }
-    }
-    __syncthreads();
-    auto emit = [&](int i, const float4& v) {
-      const int x = x0 + warp * kTXW + i;
-      if (x >= a.nx || !yok) return;
-      if (scatter) {
-        // halo rows lack part of their PSF support: their owner window adds them
-        if (lane_writes(a, yb)) scatter4(tmp, tb[tap_slot<R>(warp * kTXW + i + R)], yb, v);
-      } else {
-        *reinterpret_cast<float4*>(tmp + (static_cast<size_t>(z) * a.nx + x) * a.cs + yb) = v;
-      }
-    };
-    if (PSF) {
-      if constexpr (PTAB && ADJ) {  // transpose of a convolution = correlation: both kernels reversed
-        const float* kr = ptab + z * 2 * K;
-        rowpass_from_tile<R>(sbuf, warp * kTXW, emit, Reversed<R>{kr}, Reversed<R>{kr + K}, lane, a.ny);
-      } else {
-        const float* kr = (PTAB ? ptab : s_psf) + z * 2 * K;
-        rowpass_from_tile<R>(sbuf, warp * kTXW, emit, kr, kr + K, lane, a.ny);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < kTXW; ++i) emit(i, sbuf[(warp * kTXW + i) * 32 + lane]);
-    }
-  }
-}
-
-template <int R, bool PSF, bool ATT, bool ADJ, class V, int CTAS = 2>
-__global__ void __launch_bounds__(32 * kW, CTAS) k_spread_yg(const YgArgs a, int c0) {
-  spread_body<R, PSF, ATT, ADJ, V, false>(a, c0, nullptr);
-}
-
-template <int R, bool ATT, bool ADJ, class V, int CTAS = 2>
-__global__ void __launch_bounds__(32 * kW, CTAS)
-    k_spread_ptab_yg(const YgArgs a, int c0, const __grid_constant__ PsfTable t) {
-  spread_body<R, true, ATT, ADJ, V, true>(a, c0, t.c);
-}
-
-// Reference-mode spread of a mirror unit -- camera c and its mate m at the
-// opposite angle about the grid centre -- into ONE scratch volume in c's
-// rotated frame:
-//   U(x', y, z') = PSF_z'[s_c e^{-T}](x') + PSF'_{nz-1-z'}[s_m(nx-1-x') e^{-T'}](x')
-// with T the inclusive mu sum along c's column from its detector side, T'
-// the inclusive sum from the other end (the mate's detector side), and PSF'
-// the mate's plane nz-1-z' with the row kernel reversed.  The mate's inverse
-// matrix is c's mirrored in x and z, so gathering U with c's inverse matrix
-// adds both cameras' terms: one mu scan, one scratch volume and one gather
-// per pair.  A unit without a mate spreads its camera alone.  CTA = (unit,
-// x-tile, depth slab); the PSF planes of the slab only sit in shared memory.
-//
-// ADJ: the exact transpose of the mirror-unit projector instead: both terms in
-// c's frame go through the transposed PSF (camera: both kernels reversed;
-// mate: row kernel forward, column kernel reversed) and, summed, are
-// scattered with c's bilinear weights into the accumulator a.out (the mate's
-// footprint of its mirrored column is c's), or with a.det written to the
-// group scratch for k_tgather_yg.
-//
-// V = bfloat16 (mu stored in bfloat16): the forward transmission is summed
-// with Kahan compensation (the compensation of each sampled column in shared
-// memory), the mate's transmission is the column total minus the compensated
-// forward sum (no second running sum), and the tiles are single-buffered (a
-// second barrier per plane) so that two CTAs per SM still fit.
-template <int R, class V>
-__host__ __device__ constexpr size_t spread_pair_fixed_smem() {
-  using TS = TileShape<R>;
-  constexpr bool KAHAN = StorageTraits<V>::kKahan;
-  return (KAHAN ? 1 : 2) * TS::kSbBytes + TS::kTapBytes + (KAHAN ? sizeof(float4) * TS::kOwn * 32 * kW : 0);
-}
-
-template <int R, bool PSF, bool ATT, bool ADJ, bool PTAB, class V = float>
-__device__ __forceinline__ void spread_pair_body(const YgArgs& a, int u0, const float* ptab) {
-  using TS = TileShape<R>;
-  constexpr bool KAHAN = StorageTraits<V>::kKahan;
-  constexpr int NB = KAHAN ? 1 : 2;  // tile buffers
-  constexpr int NS = TS::NS;
-  constexpr int K = 2 * R + 1;
-  const V* __restrict__ mu = reinterpret_cast<const V*>(a.mu) + a.row0;
-  extern __shared__ __align__(16) unsigned char smem[];
-  float4* sb = reinterpret_cast<float4*>(smem);                              // [NB stages][2][NS][32]
-  Tap* taps = reinterpret_cast<Tap*>(smem + NB * TS::kSbBytes);               // [2][kTapSlots]
-  float4* scomp = reinterpret_cast<float4*>(smem + NB * TS::kSbBytes + TS::kTapBytes);  // [kOwn][256] (KAHAN)
-  float* s_psf = reinterpret_cast<float*>(smem + spread_pair_fixed_smem<R, V>());  // [zper][2K], mate's next
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ntile = (a.nx + kTXC - 1) / kTXC;
-  const int nsl = a.bslabs, slots = nsl + 1;
-  const int slab = blockIdx.x % nsl;
-  const int item = blockIdx.x / nsl;
-  const int g = item / ntile;
-  const int unit = u0 + g;
-  const int2 uc = a.units[unit];
-  const int cam = uc.x, mate = uc.y;
-  const bool paired = mate >= 0;  // uniform over the CTA
-  const int x0 = (item % ntile) * kTXC;
-  const int yb = lane * 4;
-  const bool yok = lane_rows_ok(a, yb);
-  const int zper = (a.nz + nsl - 1) / nsl;
-  const int zbeg = slab * zper, zend = min(a.nz, zbeg + zper);
-  if (zbeg >= zend) return;  // uniform over the CTA
-  float* s_psf_m = s_psf + zper * 2 * K;
-  if (PSF && !PTAB) {
-    // reversed index of a row (j < K) or column (j >= K) kernel entry
-    auto rev = [&](int j) { return j < K ? K - 1 - j : 3 * K - 1 - j; };
-    for (int i = threadIdx.x; i < (zend - zbeg) * 2 * K; i += blockDim.x) {
-      const int z = zbeg + i / (2 * K), j = i % (2 * K);
-      s_psf[i] = __ldg(a.psf + z * 2 * K + (ADJ ? rev(j) : j));
-      if (paired) {  // mate: reference row reversed; transpose column reversed
-        const int jm = (j < K) != ADJ ? rev(j) : j;
-        s_psf_m[i] = __ldg(a.psf + (a.nz - 1 - z) * 2 * K + jm);
-      }
-    }
-  }
-  const CamRows cr = cam_rows(a.geom[cam].fwd);
-  const size_t vol = static_cast<size_t>(a.nz) * a.nx * a.cs;  // one scratch volume
-  const bool scatter = ADJ && !a.det;  // uniform over the launch
-  float* __restrict__ tmp = scatter ? a.out + a.row0 : a.temp + vol * g;
-  const float* __restrict__ srow = a.sino + static_cast<size_t>(cam) * a.nx * a.cy + a.row0;
-  const float* __restrict__ mrow = a.sino + static_cast<size_t>(paired ? mate : cam) * a.nx * a.cy + a.row0;
-
-  // transmissions per sampled column: forward (from the slab carry) and, for
-  // the mate, from the far end (column total minus the carry; with KAHAN Tr
-  // holds the column total)
-  float4 Tc[TS::kOwn], Tr[TS::kOwn];
-#pragma unroll
-  for (int k = 0; k < TS::kOwn; ++k) {
-    Tc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    Tr[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (KAHAN) scomp[k * 32 * kW + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
-    const int xp = x0 - R + warp + kW * k;
-    if (ATT && warp + kW * k < NS && xp >= 0 && xp < a.nx && yok) {
-      const float* cp = a.slab_T + ((static_cast<size_t>(cam) * slots + slab) * a.nx + xp) * a.cy + a.row0 + yb;
-      Tc[k] = ldg4(cp);
-      if (paired) {
-        const float4 tot = ldg4(cp + static_cast<size_t>(nsl - slab) * a.nx * a.cy);
-        Tr[k] = KAHAN ? tot : make_float4(tot.x - Tc[k].x, tot.y - Tc[k].y, tot.z - Tc[k].z, tot.w - Tc[k].w);
-      }
-    }
-  }
-  ybuf_zero_pads();
-  __syncthreads();
-
-  for (int z = zbeg; z < zend; ++z) {
-    const int b = z & 1;
-    float4* sc = sb + (NB == 2 ? b : 0) * 2 * NS * 32;
-    float4* sm = sc + NS * 32;
-    Tap* tb = taps + b * TS::kTapSlots;
-    if ((ATT || ADJ) && lane < TS::kOwn) {
-      const int c = warp + kW * lane;
-      if (c < NS) {
-        const int xp = x0 - R + c;
-        tb[tap_slot<R>(c)] = make_tap(xp, z, cr.m00, cr.m02, cr.m03, cr.m20, cr.m22, cr.m23, a.nx, a.nz, a.cy,
-                                      xp >= 0 && xp < a.nx);
-      }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < TS::kOwn; ++k) {
-      const int c = warp + kW * k;
-      if (c < NS) {
-        const int xp = x0 - R + c;
-        const bool ok = xp >= 0 && xp < a.nx && yok;
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f), q = s;
-        if (ok) s = ldg4(srow + static_cast<size_t>(xp) * a.cy + yb);
-        if (paired && ok) q = ldg4(mrow + static_cast<size_t>(a.nx - 1 - xp) * a.cy + yb);
-        if (ATT) {
-          // the branch: the predicated form leaves too few registers beside the
-          // two transmissions (128^3 x 120: 0.298 ms a launch, predicated 0.349)
-          const float4 m = sample4_branch(mu, tb[tap_slot<R>(c)], yb, yok);
-          if constexpr (KAHAN) {
-            float4 cc = scomp[k * 32 * kW + threadIdx.x];
-            kahan_add4p(Tc[k], cc, m);
-            scomp[k * 32 * kW + threadIdx.x] = cc;
-            const float4 tv = kahan_value4p(Tc[k], cc);
-            s = mul4p(s, exp_neg4(tv));
-            if (paired) {  // sum from the far end, inclusive: total - forward sum + this plane
-              const Pair4 tot = pair4(Tr[k]), v = pair4(tv), mm = pair4(m);
-              q = mul4p(q, exp_neg4(unpair4({add2(sub2(tot.lo, v.lo), mm.lo), add2(sub2(tot.hi, v.hi), mm.hi)})));
-            }
-          } else {
-            add4p(Tc[k], m);
-            s = mul4p(s, exp_neg4(Tc[k]));
-            if (paired) {
-              q = mul4p(q, exp_neg4(Tr[k]));
-              const Pair4 tr = pair4(Tr[k]), mm = pair4(m);
-              Tr[k] = unpair4({sub2(tr.lo, mm.lo), sub2(tr.hi, mm.hi)});
-            }
-          }
-        }
-        sc[c * 32 + lane] = s;
-        if (paired) sm[c * 32 + lane] = q;
-      }
-    }
-    __syncthreads();
-    auto write = [&](int i, const float4& v) {
-      const int x = x0 + warp * kTXW + i;
-      if (x >= a.nx || !yok) return;
-      if (scatter) {
-        // halo rows lack part of their PSF support: their owner window adds them
-        if (lane_writes(a, yb)) scatter4(tmp, tb[tap_slot<R>(warp * kTXW + i + R)], yb, v);
-      } else {
-        *reinterpret_cast<float4*>(tmp + (static_cast<size_t>(z) * a.nx + x) * a.cs + yb) = v;
-      }
-    };
-    float4 pend;  // the mate's term of the output being written
-    auto keep = [&](int i, const float4& v) { pend = v; };
-    auto write_sum = [&](int i, float4 v) {
-      add4p(v, pend);
-      write(i, v);
-    };
-    if (PSF) {
-      const float* kr = PTAB ? ptab + z * 2 * K : s_psf + (z - zbeg) * 2 * K;
-      if (paired) {  // both row passes in one sweep over the two tiles
-        if constexpr (PTAB && ADJ) {
-          const float* km = ptab + (a.nz - 1 - z) * 2 * K;
-          rowpass2_from_tiles<R>(sc, sm, warp * kTXW, write_sum, Reversed<R>{kr}, Reversed<R>{kr + K}, keep, km,
-                                 Reversed<R>{km + K}, lane, a.ny);
-        } else if constexpr (PTAB) {
-          const float* km = ptab + (a.nz - 1 - z) * 2 * K;
-          rowpass2_from_tiles<R>(sc, sm, warp * kTXW, write_sum, kr, kr + K, keep, Reversed<R>{km}, km + K, lane,
-                                 a.ny);
-        } else {
-          const float* km = s_psf_m + (z - zbeg) * 2 * K;
-          rowpass2_from_tiles<R>(sc, sm, warp * kTXW, write_sum, kr, kr + K, keep, km, km + K, lane, a.ny);
-        }
-      } else if constexpr (PTAB && ADJ) {
-        rowpass_from_tile<R>(sc, warp * kTXW, write, Reversed<R>{kr}, Reversed<R>{kr + K}, lane, a.ny);
-      } else {
-        rowpass_from_tile<R>(sc, warp * kTXW, write, kr, kr + K, lane, a.ny);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < kTXW; ++i) {
-        float4 v = sc[(warp * kTXW + i) * 32 + lane];
-        if (paired) add4(v, sm[(warp * kTXW + i) * 32 + lane]);
-        write(i, v);
-      }
-    }
-    if (NB == 1) __syncthreads();  // the single tile buffer is rewritten next plane
-  }
-}
-
-template <int R, bool PSF, bool ATT, bool ADJ, class V = float>
-__global__ void __launch_bounds__(32 * kW, 2) k_spread_pair_yg(const YgArgs a, int u0) {
-  spread_pair_body<R, PSF, ATT, ADJ, false, V>(a, u0, nullptr);
-}
-
-template <int R, bool ATT, bool ADJ, class V = float>
-__global__ void __launch_bounds__(32 * kW, 2)
-    k_spread_pair_ptab_yg(const YgArgs a, int u0, const __grid_constant__ PsfTable t) {
-  spread_pair_body<R, true, ATT, ADJ, true, V>(a, u0, t.c);
 }
 
 // ------------------------------------ backprojector: inverse-rotation gather
@@ -415,27 +79,21 @@ __global__ void __launch_bounds__(32 * kW, 2)
 // With a.units, g runs over units and B_g is the unit's first camera's.
 // first: assign instead of adding to a.out; clamp: the last group of the
 // window with a.truncate -- negative sums become zero as they are stored.
-template <int U>
+// L lanes hold one column, 32 / L lane groups per warp; footprints of
+// kGatherTaps units at a time sit in shared memory.
+template <int U, int L>
 __global__ void __launch_bounds__(32 * kGatherWarps) k_gather_yg(const YgArgs a, int c0, int gcount, int first,
                                                                 int clamp) {
-  constexpr int C = kGatherCols;
-  extern __shared__ Tap s_gtap[];  // [kGatherWarps][C * group]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int C = kGatherCols, GROUPS = 32 * kGatherWarps / L;
+  __shared__ Tap s_gtap[GROUPS][kGatherTaps * C];
+  const int grp = threadIdx.x / L, lane = threadIdx.x % L;
   const int nchunk = (a.nx + C - 1) / C;
-  const int item = blockIdx.x * kGatherWarps + warp;
-  if (item >= nchunk * a.nz) return;
+  const int item = blockIdx.x * GROUPS + grp;
   const int Z = item / nchunk;
   const int X0 = (item % nchunk) * C;
   const int yb = lane * 4;
-  Tap* tap = s_gtap + warp * C * a.group;
-  for (int e = lane; e < C * gcount; e += 32) {
-    const int g = e / C, X = X0 + e % C;
-    const CamRows cr = cam_rows(a.geom[a.units ? a.units[c0 + g].x : c0 + g].bwd);
-    // footprints in the scratch (column stride cs)
-    tap[e] = make_tap(X, Z, cr.m00, cr.m02, cr.m03, cr.m20, cr.m22, cr.m23, a.nx, a.nz, a.cs, X < a.nx);
-  }
-  __syncwarp();
-  if (!lane_rows_ok(a, yb) || !lane_writes(a, yb)) return;
+  const bool rows = Z < a.nz && lane_rows_ok(a, yb) && lane_writes(a, yb);
+  Tap* tap = s_gtap[grp];
   const size_t vol = static_cast<size_t>(a.nz) * a.nx * a.cs;
   // camera outer, columns inner: neighbouring accumulator columns of one
   // camera share footprint columns, which then hit in L1; the loads of U
@@ -444,23 +102,37 @@ __global__ void __launch_bounds__(32 * kGatherWarps) k_gather_yg(const YgArgs a,
   float4 acc[C];
 #pragma unroll
   for (int i = 0; i < C; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  int g = 0;
-  for (; g + U <= gcount; g += U) {
-    float4 v[U][C];
+  for (int g0 = 0; g0 < gcount; g0 += kGatherTaps) {
+    const int n = min(kGatherTaps, gcount - g0);
+    if (Z < a.nz)
+      for (int e = lane; e < C * n; e += L) {
+        const int g = c0 + g0 + e / C, X = X0 + e % C;
+        const CamRows cr = cam_rows(a.geom[a.units ? a.units[g].x : g].bwd);
+        // footprints in the scratch (column stride cs)
+        tap[e] = make_tap(X, Z, cr.m00, cr.m02, cr.m03, cr.m20, cr.m22, cr.m23, a.nx, a.nz, a.cs, X < a.nx);
+      }
+    __syncwarp();
+    if (rows) {
+      const float* src = a.temp + vol * g0;
+      int g = 0;
+      for (; g + U <= n; g += U) {
+        float4 v[U][C];
 #pragma unroll
-    for (int u = 0; u < U; ++u)
+        for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int i = 0; i < C; ++i) v[u][i] = sample4_loaded(a.temp + vol * (g + u), tap[(g + u) * C + i], yb);
+          for (int i = 0; i < C; ++i) v[u][i] = sample4_loaded(src + vol * (g + u), tap[(g + u) * C + i], yb);
 #pragma unroll
-    for (int u = 0; u < U; ++u)
+        for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int i = 0; i < C; ++i) add4(acc[i], v[u][i]);
+          for (int i = 0; i < C; ++i) add4(acc[i], v[u][i]);
+      }
+      for (; g < n; ++g)
+#pragma unroll
+        for (int i = 0; i < C; ++i) add4(acc[i], sample4(src + vol * g, tap[g * C + i], yb, true));
+    }
+    __syncwarp();
   }
-  for (; g < gcount; ++g) {
-    const float* src = a.temp + vol * g;
-#pragma unroll
-    for (int i = 0; i < C; ++i) add4(acc[i], sample4(src, tap[g * C + i], yb, true));
-  }
+  if (!rows) return;
 #pragma unroll
   for (int i = 0; i < C; ++i) {
     const int X = X0 + i;
@@ -574,120 +246,20 @@ void launch_tgather(const YgArgs& b, int c0, int gcount, int clamp, cudaStream_t
   k_tgather_yg<<<blocks, 32 * kGatherWarps, 0, st>>>(b, c0, gcount, c0 == 0 ? 1 : 0, clamp);
 }
 
-void launch_gather(const YgArgs& b, int c0, int gcount, int clamp, int blocks, size_t smem, cudaStream_t st) {
+template <int L>
+void launch_gather_lanes(const YgArgs& b, int c0, int gcount, int clamp, cudaStream_t st) {
+  constexpr int GROUPS = 32 * kGatherWarps / L;
+  const int items = (b.nx + kGatherCols - 1) / kGatherCols * b.nz;
   NRGB_LAUNCH_SCOPE("k_gather_yg", st);
-  k_gather_yg<kGatherUnits><<<blocks, 32 * kGatherWarps, smem, st>>>(b, c0, gcount, c0 == 0 ? 1 : 0, clamp);
+  k_gather_yg<kGatherUnits, L>
+      <<<(items + GROUPS - 1) / GROUPS, 32 * kGatherWarps, 0, st>>>(b, c0, gcount, c0 == 0 ? 1 : 0, clamp);
 }
 
-// The separated PSF of a.nz planes as a kernel-parameter table, or null when
-// it is not available on the host or does not fit.
-template <int R>
-const PsfTable* psf_table(const YgArgs& a) {
-  if (!a.psf || !a.psf_host || static_cast<size_t>(a.nz) * 2 * (2 * R + 1) > kPsfTableFloats) return nullptr;
-  static thread_local PsfTable table;
-  std::memcpy(table.c, a.psf_host, sizeof(float) * a.nz * 2 * (2 * R + 1));
-  return &table;
-}
-
-template <int R, bool ADJ>
-int launch_spread_R(const YgArgs& a, int c0, int gcount, cudaStream_t st) {
-  const int ntile = (a.nx + kTXC - 1) / kTXC;
-  const dim3 grid(gcount * ntile * a.bslabs), block(32 * kW);
-  const bool psf = a.psf != nullptr;
-  const PsfTable* tab = psf_table<R>(a);
-  const size_t smem = tile_smem_bytes<R>(psf && !tab ? a.nz : 0);
-  auto go = [&](auto k) {
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    NRGB_LAUNCH_SCOPE(ADJ ? "k_adjoint_yg" : "k_spread_yg", st);
-    k<<<grid, block, smem, st>>>(a, c0);
-  };
-  auto go_tab = [&](auto k) {
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    NRGB_LAUNCH_SCOPE(ADJ ? "k_adjoint_yg" : "k_spread_yg", st);
-    k<<<grid, block, smem, st>>>(a, c0, *tab);
-  };
-  // only mu is sampled from storage here (the sinogram is float32)
-  const bool bf16 = a.storage == kStorageBF16;
-  const bool three = 3 * (smem + kYBufBytes + 1024) <= 228 * 1024;
-  if (psf && tab) {
-    if (a.mu && bf16) {
-      go_tab(k_spread_ptab_yg<R, true, ADJ, __nv_bfloat16>);
-    } else if (a.mu) {
-      if constexpr (!ADJ) {
-        if (three)
-          go_tab(k_spread_ptab_yg<R, true, false, float, 3>);
-        else
-          go_tab(k_spread_ptab_yg<R, true, false, float>);
-      } else {
-        go_tab(k_spread_ptab_yg<R, true, true, float>);
-      }
-    } else {
-      go_tab(k_spread_ptab_yg<R, false, ADJ, float>);
-    }
-  } else if (psf) {
-    if (a.mu && bf16) {
-      go(k_spread_yg<R, true, true, ADJ, __nv_bfloat16>);
-    } else if (a.mu) {
-      if constexpr (!ADJ) {
-        if (three)
-          go(k_spread_yg<R, true, true, false, float, 3>);
-        else
-          go(k_spread_yg<R, true, true, false, float>);
-      } else {
-        go(k_spread_yg<R, true, true, true, float>);
-      }
-    } else {
-      go(k_spread_yg<R, true, false, ADJ, float>);
-    }
-  } else {
-    if (a.mu && bf16) go(k_spread_yg<0, false, true, ADJ, __nv_bfloat16>);
-    else if (a.mu) go(k_spread_yg<0, false, true, ADJ, float>);
-    else go(k_spread_yg<0, false, false, ADJ, float>);
-  }
-  return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
-}
-
-template <int R, bool ADJ>
-int launch_spread_pair_R(const YgArgs& a, int u0, int gcount, cudaStream_t st) {
-  using TS = TileShape<R>;
-  const int ntile = (a.nx + kTXC - 1) / kTXC;
-  const dim3 grid(gcount * ntile * a.bslabs), block(32 * kW);
-  const bool psf = a.psf != nullptr;
-  const int zper = (a.nz + a.bslabs - 1) / a.bslabs;
-  const PsfTable* tab = psf_table<R>(a);
-  // bfloat16 mu: the Kahan form (reference mode only)
-  const bool bf16 = a.storage == kStorageBF16 && a.mu && !ADJ;
-  const size_t smem = (bf16 ? spread_pair_fixed_smem<R, __nv_bfloat16>() : spread_pair_fixed_smem<R, float>()) +
-                      (psf && !tab ? sizeof(float) * 2 * zper * 2 * (2 * R + 1) : 0);
-  auto go = [&](auto k) {
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    NRGB_LAUNCH_SCOPE(ADJ ? "k_adjoint_pair_yg" : "k_spread_pair_yg", st);
-    k<<<grid, block, smem, st>>>(a, u0);
-  };
-  auto go_tab = [&](auto k) {
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    NRGB_LAUNCH_SCOPE(ADJ ? "k_adjoint_pair_yg" : "k_spread_pair_yg", st);
-    k<<<grid, block, smem, st>>>(a, u0, *tab);
-  };
-  if constexpr (!ADJ) {
-    if (bf16) {
-      if (psf && tab) go_tab(k_spread_pair_ptab_yg<R, true, false, __nv_bfloat16>);
-      else if (psf) go(k_spread_pair_yg<R, true, true, false, __nv_bfloat16>);
-      else go(k_spread_pair_yg<0, false, true, false, __nv_bfloat16>);
-      return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
-    }
-  }
-  if (psf && tab) {
-    if (a.mu) go_tab(k_spread_pair_ptab_yg<R, true, ADJ>);
-    else go_tab(k_spread_pair_ptab_yg<R, false, ADJ>);
-  } else if (psf) {
-    if (a.mu) go(k_spread_pair_yg<R, true, true, ADJ>);
-    else go(k_spread_pair_yg<R, true, false, ADJ>);
-  } else {
-    if (a.mu) go(k_spread_pair_yg<0, false, true, ADJ>);
-    else go(k_spread_pair_yg<0, false, false, ADJ>);
-  }
-  return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
+void launch_gather(const YgArgs& b, int c0, int gcount, int clamp, cudaStream_t st) {
+  const int lanes = column_lanes(b.ny);
+  if (lanes == 8) launch_gather_lanes<8>(b, c0, gcount, clamp, st);
+  else if (lanes == 16) launch_gather_lanes<16>(b, c0, gcount, clamp, st);
+  else launch_gather_lanes<32>(b, c0, gcount, clamp, st);
 }
 
 template <bool ADJ>
@@ -751,15 +323,23 @@ namespace {
 
 // Carries of units (or cameras) [u0, u0 + n).
 int mu_carry_range(const YgArgs& a_in, float* out, int u0, int n, cudaStream_t st) {
-  const int nchunk = (a_in.nx + kCarryCols - 1) / kCarryCols;
   for (const Window& w : row_windows(a_in.ny, 0)) {  // carries need no halo
     YgArgs a = windowed(a_in, w);
     a.slab_T = out;
-    NRGB_LAUNCH_SCOPE("k_mu_carry_yg", st);
-    if (a.storage == kStorageBF16)
-      k_mu_carry_yg<__nv_bfloat16><<<n * nchunk, 32 * a.bslabs, 0, st>>>(a, u0);
-    else
-      k_mu_carry_yg<float><<<n * nchunk, 32 * a.bslabs, 0, st>>>(a, u0);
+    auto go = [&](auto v, auto lanes) {
+      using V = decltype(v);
+      constexpr int L = decltype(lanes)::value, C = kCarryCols * (32 / L);
+      NRGB_LAUNCH_SCOPE("k_mu_carry_yg", st);
+      k_mu_carry_yg<V, L><<<n * ((a.nx + C - 1) / C), 32 * a.bslabs, 0, st>>>(a, u0);
+    };
+    auto pick = [&](auto v) {
+      const int lanes = column_lanes(a.ny);
+      if (lanes == 8) go(v, std::integral_constant<int, 8>());
+      else if (lanes == 16) go(v, std::integral_constant<int, 16>());
+      else go(v, std::integral_constant<int, 32>());
+    };
+    if (a.storage == kStorageBF16) pick(__nv_bfloat16());
+    else pick(0.0f);
   }
   return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
 }
@@ -853,12 +433,12 @@ int yg_backproject(const YgArgs& a_in, cudaStream_t st) {
     return pair ? spread_pair_by_radius<false>(R, b, c0, gcount, ss) : spread_by_radius(R, b, c0, gcount, ss);
   };
   // with a.truncate the window's last group clamps the result as it stores it
-  auto gather_on = [&](const YgArgs& b, int c0, int gcount, int blocks, size_t smem, cudaStream_t gs) {
+  auto gather_on = [&](const YgArgs& b, int c0, int gcount, cudaStream_t gs) {
     const int clamp = a.truncate && c0 + gcount == nunits ? 1 : 0;
     if (tgather)
       launch_tgather(b, c0, gcount, clamp, gs);
     else
-      launch_gather(b, c0, gcount, clamp, blocks, smem, gs);
+      launch_gather(b, c0, gcount, clamp, gs);
   };
   auto spread = [&](const YgArgs& b, int c0, int gcount) { return spread_on(b, c0, gcount, st); };
   if (a.back_mode == kBackAdjoint && !a.gradient && !a.det) {
@@ -873,11 +453,6 @@ int yg_backproject(const YgArgs& a_in, cudaStream_t st) {
     }
     return kOk;
   }
-  const int nchunk = (a.nx + kGatherCols - 1) / kGatherCols;
-  const int gblocks = (nchunk * a.nz + kGatherWarps - 1) / kGatherWarps;
-  const size_t gsmem = sizeof(Tap) * kGatherWarps * kGatherCols * group;
-  cudaFuncSetAttribute(k_gather_yg<kGatherUnits>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       static_cast<int>(gsmem));
   if (!a.pipelined) {
     for (const Window& w : wins) {
       YgArgs b = windowed(a, w);
@@ -886,7 +461,7 @@ int yg_backproject(const YgArgs& a_in, cudaStream_t st) {
         const int gcount = std::min(group, nunits - c0);
         int st_ = spread(b, c0, gcount);
         if (st_ != kOk) return st_;
-        gather_on(b, c0, gcount, gblocks, gsmem, st);
+        gather_on(b, c0, gcount, st);
       }
     }
     return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
@@ -910,7 +485,7 @@ int yg_backproject(const YgArgs& a_in, cudaStream_t st) {
       if (st_ != kOk) return st_;
       cudaEventRecord(pp->spread_done[slot], ss);
       cudaStreamWaitEvent(pp->aux, pp->spread_done[slot], 0);
-      gather_on(b, c0, gcount, gblocks, gsmem, pp->aux);
+      gather_on(b, c0, gcount, pp->aux);
       cudaEventRecord(pp->gather_done[slot], pp->aux);
     }
   }

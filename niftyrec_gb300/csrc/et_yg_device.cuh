@@ -45,8 +45,14 @@ namespace {
 namespace cg = cooperative_groups;
 
 constexpr int kW = 8;             // warps per CTA of the tile engine
-constexpr int kTXW = 4;           // output columns per warp
-constexpr int kTXC = kW * kTXW;   // output columns per CTA
+constexpr int kTXW = 4;           // output columns per lane group
+// Lane groups: L lanes (32, 16 or 8) hold one column of up to 4 L rows, so a
+// warp works on 32 / L columns at once and a CTA has kGroups<L> groups and
+// kTX<L> output columns (see window_lanes for which L a row window takes).
+template <int L>
+constexpr int kGroups = 32 * kW / L;
+template <int L>
+constexpr int kTX = kGroups<L> * kTXW;
 constexpr int kSlabsP = 4;        // depth slabs (= cluster size) of the batched projector
 constexpr int kSlabsB = 16;       // backprojector depth slabs
 constexpr int kCarrySlots = kSlabsB + 1;  // carries per camera: slab prefixes, column total
@@ -54,6 +60,7 @@ constexpr int kCarryCols = 64 / kSlabsB;  // columns per CTA of the carry pass (
 constexpr int kGatherWarps = 4;   // warps per CTA of the inverse-rotation gather
 constexpr int kGatherCols = 2;    // accumulator columns per warp in the gather
 constexpr int kGatherUnits = 2;   // scratch volumes whose loads a gather warp has in flight at once
+constexpr int kGatherTaps = 16;   // scratch volumes whose footprints a gather group holds at once
 constexpr unsigned kFull = 0xffffffffu;
 
 __host__ __device__ constexpr size_t round_up16(size_t b) { return (b + 15) / 16 * 16; }
@@ -343,32 +350,41 @@ __device__ __forceinline__ float4 yconv4(const float4& u, KC kc, int lane) {
 }
 
 // Column pass through shared memory: each lane stores its 4 rows in its
-// warp's row buffer and reads the neighbour rows back with 16-byte loads (one
+// group's row buffer and reads the neighbour rows back with 16-byte loads (one
 // store and 2 ceil(R/4) loads in place of 2R shuffles and 2R selects).  Two
-// buffers per warp alternate, so one warp barrier per call orders a store
+// buffers per group alternate, so one warp barrier per call orders a store
 // after the loads of the call before the previous one.  Rows outside the
-// warp's 128 read zero pads, written by ybuf_zero_pads before a kernel's
+// group's 4 L read zero pads, written by ybuf_zero_pads before a kernel's
 // first row pass.
 constexpr int kYPad = 2;  // pad chunks (4 rows each) on either side: R <= 8
-__shared__ __align__(16) float4 s_ybuf[kW][2][32 + 2 * kYPad];
-constexpr size_t kYBufBytes = sizeof(float4) * kW * 2 * (32 + 2 * kYPad);  // static, per CTA
+template <int L>
+constexpr int kYRow = L + 2 * kYPad;  // chunks of one group's row buffer
+template <int L>
+constexpr size_t kYBufBytes = sizeof(float4) * kGroups<L> * 2 * kYRow<L>;  // static, per CTA
 
+template <int L>
+__device__ __forceinline__ float4* ybuf(int grp, int b) {
+  __shared__ __align__(16) float4 buf[kGroups<L>][2][kYRow<L>];
+  return buf[grp][b];
+}
+
+template <int L>
 __device__ __forceinline__ void ybuf_zero_pads() {
-  for (int i = threadIdx.x; i < kW * 2 * 2 * kYPad; i += blockDim.x) {
-    const int w = i / (4 * kYPad), r = i % (4 * kYPad);
+  for (int i = threadIdx.x; i < kGroups<L> * 2 * 2 * kYPad; i += blockDim.x) {
+    const int g = i / (4 * kYPad), r = i % (4 * kYPad);
     const int b = r / (2 * kYPad), q = r % (2 * kYPad);
-    s_ybuf[w][b][q < kYPad ? q : 32 + q] = make_float4(0.f, 0.f, 0.f, 0.f);
+    ybuf<L>(g, b)[q < kYPad ? q : L + q] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
 }
 
-template <int R, class KC>
+template <int R, int L, class KC>
 __device__ __forceinline__ float4 yconv4s(const float4& u, KC kc, int lane, int b) {
   if constexpr (R == 0) {
     return yconv4<0>(u, kc, lane);
   } else {
     constexpr int C = (R + 3) / 4;
     static_assert(C <= kYPad, "row-buffer pads");
-    float4* row = &s_ybuf[threadIdx.x >> 5][b][kYPad];
+    float4* row = ybuf<L>(threadIdx.x / L, b) + kYPad;
     row[lane] = u;
     __syncwarp();
     float w[2 * R + 4];
@@ -487,6 +503,13 @@ struct PsfTable {
   float c[kPsfTableFloats];
 };
 
+// Whether the separated PSF travels in the kernel parameters: the host copy is
+// given and fits.
+template <int R>
+bool psf_in_parameters(const YgArgs& a) {
+  return a.psf && a.psf_host && static_cast<size_t>(a.nz) * 2 * (2 * R + 1) <= kPsfTableFloats;
+}
+
 // A row kernel read backwards (k -> p[2R - k]): a mirror camera's row pass.
 template <int R>
 struct Reversed {
@@ -495,60 +518,65 @@ struct Reversed {
 };
 
 // ------------------------------------------------------------ tile engine
-// A CTA of kW warps owns kTXC = kW * kTXW consecutive output columns of one
-// camera and walks one depth slab.  At every depth step the NS = kTXC + 2R
+// A CTA of kGroups<L> lane groups owns kTX<L> consecutive output columns of one
+// camera and walks one depth slab.  At every depth step the NS = kTX<L> + 2R
 // sampled columns (outputs plus the PSF row halo) are produced once per CTA
-// -- column c by warp c % kW -- into a double-buffered shared tile; after one
-// barrier each warp runs the row pass (register sliding window over its
-// kTXW + 2R tile columns), the column pass and its consumer for its kTXW
+// -- column c by group c % kGroups<L> -- into a double-buffered shared tile;
+// after one barrier each group runs the row pass (register sliding window over
+// its kTXW + 2R tile columns), the column pass and its consumer for its kTXW
 // outputs.  Writes of step z+1 go to the other buffer, so one barrier per
 // step suffices.
-template <int R>
+template <int R, int L>
 struct TileShape {
-  static constexpr int NS = kTXC + 2 * R;            // sampled columns per CTA
-  static constexpr int kOwn = (NS + kW - 1) / kW;    // sampled columns per warp (max)
-  static constexpr int kTapSlots = kW * kOwn;         // footprint slots per stage (see tap_slot)
-  static constexpr size_t kSbBytes = sizeof(float4) * 2 * NS * 32;
+  static constexpr int G = kGroups<L>;
+  static constexpr int NS = kTX<L> + 2 * R;          // sampled columns per CTA
+  static constexpr int kOwn = (NS + G - 1) / G;      // sampled columns per group (max)
+  static_assert(kOwn <= L, "one lane per footprint");
+  static constexpr int kTapSlots = G * kOwn;          // footprint slots per stage (see tap_slot)
+  static constexpr size_t kSbBytes = sizeof(float4) * 2 * NS * L;
   static constexpr size_t kTapBytes = sizeof(Tap) * 2 * kTapSlots;
   // Projector: 2 x steps tile buffers (steps depth planes sampled per
   // barrier); the region also holds the slab-merge buffers after the walk (T
   // and P per output column, and with a mirror camera its P).
   __host__ __device__ static constexpr size_t sb_bytes(bool pair, int steps = 1) {
-    return sizeof(float4) * 32 * (2 * steps * NS > (pair ? 3 : 2) * kTXC ? 2 * steps * NS : (pair ? 3 : 2) * kTXC);
+    return sizeof(float4) * L *
+           (2 * steps * NS > (pair ? 3 : 2) * kTX<L> ? 2 * steps * NS : (pair ? 3 : 2) * kTX<L>);
   }
   __host__ __device__ static constexpr size_t tap_bytes(int steps = 1) { return sizeof(Tap) * 2 * steps * kTapSlots; }
   // Projector serving mirror cameras from bfloat16 storage: the Kahan
   // compensations of T, P and the mate's Q, one float4 per thread and output
-  // column each, in shared memory ([3][kTXC][32]) -- registers hold the sums.
-  __host__ __device__ static constexpr size_t comp_bytes(bool on) { return on ? sizeof(float4) * 3 * kTXC * 32 : 0; }
+  // column each, in shared memory ([3][kTX][L]) -- registers hold the sums.
+  __host__ __device__ static constexpr size_t comp_bytes(bool on) {
+    return on ? sizeof(float4) * 3 * kTX<L> * L : 0;
+  }
 };
 
-// Footprint slot of sampled column c in the tap buffer: the columns one warp
-// computes (c = warp + kW * k) sit next to each other, so the footprint
+// Footprint slot of sampled column c in the tap buffer: the columns one group
+// computes (c = group + G * k) sit next to each other, so the footprint
 // stores of a warp do not collide in shared-memory banks.
-template <int R>
+template <int R, int L>
 __device__ __forceinline__ int tap_slot(int c) {
-  return (c % kW) * TileShape<R>::kOwn + c / kW;
+  return (c % kGroups<L>) * TileShape<R, L>::kOwn + c / kGroups<L>;
 }
 
 // Tile, footprints and the separated PSF of nz planes (twice with a mirror
 // camera: its kernels are the mirrored planes, row kernels reversed).
-template <int R>
+template <int R, int L>
 __host__ __device__ constexpr size_t tile_smem_bytes(int nz, bool pair = false, int steps = 1) {
-  return TileShape<R>::sb_bytes(pair, steps) + TileShape<R>::tap_bytes(steps) +
+  return TileShape<R, L>::sb_bytes(pair, steps) + TileShape<R, L>::tap_bytes(steps) +
          sizeof(float) * static_cast<size_t>(nz) * 2 * (2 * R + 1) * (pair ? 2 : 1);
 }
 
 // The projector's: the tile above plus, for mirror cameras from bfloat16
 // storage, the shared-memory Kahan compensations.
-template <int R>
+template <int R, int L>
 __host__ __device__ constexpr size_t project_smem_bytes(int nz, bool pair, bool kahan, int steps = 1) {
-  return tile_smem_bytes<R>(nz, pair, steps) + TileShape<R>::comp_bytes(pair && kahan);
+  return tile_smem_bytes<R, L>(nz, pair, steps) + TileShape<R, L>::comp_bytes(pair && kahan);
 }
 
-// Row pass from the shared tile: outputs i = 0..kTXW-1 of this warp use tile
-// columns base + i .. base + i + 2R (base = warp * kTXW).
-template <int R, class EmitFn, class KR, class KC>
+// Row pass from the shared tile: outputs i = 0..kTXW-1 of this group use tile
+// columns base + i .. base + i + 2R (base = group * kTXW).
+template <int R, int L, class EmitFn, class KR, class KC>
 __device__ __forceinline__ void rowpass_from_tile(const float4* __restrict__ sbuf, int base, EmitFn emit, KR kr, KC kc,
                                                   int lane, int ny) {
   constexpr int K = 2 * R + 1;
@@ -558,7 +586,7 @@ __device__ __forceinline__ void rowpass_from_tile(const float4* __restrict__ sbu
   for (int q = 0; q < K; ++q) u[q] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
   for (int j = 0; j < NJ; ++j) {
-    const float4 r = sbuf[(base + j) * 32 + lane];
+    const float4 r = sbuf[(base + j) * L + lane];
 #pragma unroll
     for (int d = 0; d < K; ++d) {
       const int i = j - d;
@@ -566,7 +594,7 @@ __device__ __forceinline__ void rowpass_from_tile(const float4* __restrict__ sbu
     }
     const int i = j - 2 * R;
     if (i >= 0 && i < kTXW) {
-      emit(i, mask_rows(yconv4s<R>(u[i % K], kc, lane, i & 1), 4 * lane, ny));
+      emit(i, mask_rows(yconv4s<R, L>(u[i % K], kc, lane, i & 1), 4 * lane, ny));
       u[i % K] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
@@ -576,7 +604,7 @@ __device__ __forceinline__ void rowpass_from_tile(const float4* __restrict__ sbu
 // one fma.rn.f32x2 per two rows; the same roundings in the same order), used
 // by the projector.  The spread keeps the scalar forms: its two transmission
 // arrays leave no registers for the broadcast coefficient pairs.
-template <int R, class EmitFn, class KR, class KC>
+template <int R, int L, class EmitFn, class KR, class KC>
 __device__ __forceinline__ void rowpass_from_tile_p(const float4* __restrict__ sbuf, int base, EmitFn emit, KR kr, KC kc,
                                                   int lane, int ny) {
   constexpr int K = 2 * R + 1;
@@ -587,7 +615,7 @@ __device__ __forceinline__ void rowpass_from_tile_p(const float4* __restrict__ s
   for (int q = 0; q < kTXW; ++q) u[q] = {zero, zero};
 #pragma unroll
   for (int j = 0; j < NJ; ++j) {
-    const Pair4 r = pair4(sbuf[(base + j) * 32 + lane]);
+    const Pair4 r = pair4(sbuf[(base + j) * L + lane]);
 #pragma unroll
     for (int d = 0; d < K; ++d) {
       const int i = j - d;
@@ -597,7 +625,7 @@ __device__ __forceinline__ void rowpass_from_tile_p(const float4* __restrict__ s
       }
     }
     const int i = j - 2 * R;
-    if (i >= 0 && i < kTXW) emit(i, mask_rows(yconv4s<R>(unpair4(u[i]), kc, lane, i & 1), 4 * lane, ny));
+    if (i >= 0 && i < kTXW) emit(i, mask_rows(yconv4s<R, L>(unpair4(u[i]), kc, lane, i & 1), 4 * lane, ny));
   }
 }
 
@@ -605,7 +633,7 @@ __device__ __forceinline__ void rowpass_from_tile_p(const float4* __restrict__ s
 // its mirror camera in the projector: each tile column is read once and feeds
 // both sliding windows) or over two tiles (the mirror-unit spread); output i
 // of camera b is emitted before output i of camera a.
-template <int R, class EmitA, class EmitB, class KRA, class KCA, class KRB, class KCB>
+template <int R, int L, class EmitA, class EmitB, class KRA, class KCA, class KRB, class KCB>
 __device__ __forceinline__ void rowpass2_from_tiles(const float4* __restrict__ sa, const float4* __restrict__ sbt,
                                                     int base, EmitA emit_a, KRA kra, KCA kca, EmitB emit_b, KRB krb,
                                                     KCB kcb, int lane, int ny) {
@@ -618,8 +646,8 @@ __device__ __forceinline__ void rowpass2_from_tiles(const float4* __restrict__ s
   }
 #pragma unroll
   for (int j = 0; j < NJ; ++j) {
-    const float4 r = sa[(base + j) * 32 + lane];
-    const float4 rb = sbt == sa ? r : sbt[(base + j) * 32 + lane];
+    const float4 r = sa[(base + j) * L + lane];
+    const float4 rb = sbt == sa ? r : sbt[(base + j) * L + lane];
 #pragma unroll
     for (int d = 0; d <= 2 * R; ++d) {
       const int i = j - d;
@@ -630,13 +658,13 @@ __device__ __forceinline__ void rowpass2_from_tiles(const float4* __restrict__ s
     }
     const int i = j - 2 * R;
     if (i >= 0 && i < kTXW) {
-      emit_b(i, mask_rows(yconv4s<R>(ub[i], kcb, lane, 0), 4 * lane, ny));
-      emit_a(i, mask_rows(yconv4s<R>(ua[i], kca, lane, 1), 4 * lane, ny));
+      emit_b(i, mask_rows(yconv4s<R, L>(ub[i], kcb, lane, 0), 4 * lane, ny));
+      emit_a(i, mask_rows(yconv4s<R, L>(ua[i], kca, lane, 1), 4 * lane, ny));
     }
   }
 }
 
-template <int R, class EmitA, class EmitB, class KRA, class KCA, class KRB, class KCB>
+template <int R, int L, class EmitA, class EmitB, class KRA, class KCA, class KRB, class KCB>
 __device__ __forceinline__ void rowpass2_from_tiles_p(const float4* __restrict__ sa, const float4* __restrict__ sbt,
                                                     int base, EmitA emit_a, KRA kra, KCA kca, EmitB emit_b, KRB krb,
                                                     KCB kcb, int lane, int ny) {
@@ -650,9 +678,9 @@ __device__ __forceinline__ void rowpass2_from_tiles_p(const float4* __restrict__
   }
 #pragma unroll
   for (int j = 0; j < NJ; ++j) {
-    const float4 rf = sa[(base + j) * 32 + lane];
+    const float4 rf = sa[(base + j) * L + lane];
     const Pair4 r = pair4(rf);
-    const Pair4 rb = sbt == sa ? r : pair4(sbt[(base + j) * 32 + lane]);
+    const Pair4 rb = sbt == sa ? r : pair4(sbt[(base + j) * L + lane]);
 #pragma unroll
     for (int d = 0; d <= 2 * R; ++d) {
       const int i = j - d;
@@ -664,22 +692,22 @@ __device__ __forceinline__ void rowpass2_from_tiles_p(const float4* __restrict__
     }
     const int i = j - 2 * R;
     if (i >= 0 && i < kTXW) {
-      emit_b(i, mask_rows(yconv4s<R>(unpair4(ub[i]), kcb, lane, 0), 4 * lane, ny));
-      emit_a(i, mask_rows(yconv4s<R>(unpair4(ua[i]), kca, lane, 1), 4 * lane, ny));
+      emit_b(i, mask_rows(yconv4s<R, L>(unpair4(ub[i]), kcb, lane, 0), 4 * lane, ny));
+      emit_a(i, mask_rows(yconv4s<R, L>(unpair4(ua[i]), kca, lane, 1), 4 * lane, ny));
     }
   }
 }
 
-template <int R, class EmitA, class EmitB, class KRA, class KCA, class KRB, class KCB>
+template <int R, int L, class EmitA, class EmitB, class KRA, class KCA, class KRB, class KCB>
 __device__ __forceinline__ void rowpass2_from_tile(const float4* __restrict__ sbuf, int base, EmitA emit_a, KRA kra,
                                                    KCA kca, EmitB emit_b, KRB krb, KCB kcb, int lane, int ny) {
-  rowpass2_from_tiles<R>(sbuf, sbuf, base, emit_a, kra, kca, emit_b, krb, kcb, lane, ny);
+  rowpass2_from_tiles<R, L>(sbuf, sbuf, base, emit_a, kra, kca, emit_b, krb, kcb, lane, ny);
 }
 
-template <int R, class EmitA, class EmitB, class KRA, class KCA, class KRB, class KCB>
+template <int R, int L, class EmitA, class EmitB, class KRA, class KCA, class KRB, class KCB>
 __device__ __forceinline__ void rowpass2_from_tile_p(const float4* __restrict__ sbuf, int base, EmitA emit_a, KRA kra,
                                                      KCA kca, EmitB emit_b, KRB krb, KCB kcb, int lane, int ny) {
-  rowpass2_from_tiles_p<R>(sbuf, sbuf, base, emit_a, kra, kca, emit_b, krb, kcb, lane, ny);
+  rowpass2_from_tiles_p<R, L>(sbuf, sbuf, base, emit_a, kra, kca, emit_b, krb, kcb, lane, ny);
 }
 
 // Vector reduction of 4 floats into global memory (sm_90+).
@@ -714,7 +742,7 @@ __device__ __forceinline__ void scatter4(float* __restrict__ base, const Tap& t,
 __device__ __forceinline__ bool lane_rows_ok(const YgArgs& a, int yb) { return yb < ((a.ny + 3) & ~3); }
 __device__ __forceinline__ bool lane_writes(const YgArgs& a, int yb) { return yb >= a.out_lo && yb < a.out_hi; }
 
-// One projector work item: camera `cam`, output columns x0 .. x0 + kTXC - 1;
+// One projector work item: camera `cam`, output columns x0 .. x0 + kTX<L> - 1;
 // the CTAs of the cluster walk the depth slabs and merge (T, p) through
 // distributed shared memory: p = p0 + exp(-T0) p1 + exp(-T0-T1) p2 + ...
 // V: storage type of activity and mu (float or bfloat16; bfloat16 sums with
@@ -738,10 +766,10 @@ constexpr float kMateMaxT = 40.0f;
 // STEPS: depth planes sampled per barrier (2 x STEPS tile buffers).  Two
 // planes per barrier measured no faster on GB300 (128^3 x 120: 0.676 against
 // 0.674 ms; 256^3 x 180: 11.9 against 11.2 ms), so the kernels use one.
-template <int R, bool PSF, bool ATT, class V, bool PAIR = false, bool PTAB = false, int STEPS = 1>
+template <int R, bool PSF, bool ATT, class V, bool PAIR = false, bool PTAB = false, int L = 32, int STEPS = 1>
 __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate, int x0, unsigned char* smem,
                                              const float* ptab = nullptr) {
-  using TS = TileShape<R>;
+  using TS = TileShape<R, L>;
   constexpr bool KAHAN = StorageTraits<V>::kKahan;
   // mirror cameras from bfloat16 storage: compensations in shared memory
   constexpr bool SCOMP = PAIR && KAHAN;
@@ -750,14 +778,14 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
   constexpr int NS = TS::NS;
   constexpr int K = 2 * R + 1;
   constexpr size_t kSb = TS::sb_bytes(PAIR, STEPS);
-  float4* sb = reinterpret_cast<float4*>(smem);                    // [2 * STEPS][NS][32]
+  float4* sb = reinterpret_cast<float4*>(smem);                    // [2 * STEPS][NS][L]
   Tap* taps = reinterpret_cast<Tap*>(smem + kSb);                   // [2 * STEPS][kTapSlots]
-  float4* scomp = reinterpret_cast<float4*>(smem + kSb + TS::tap_bytes(STEPS));  // [3][kTXC][32] (SCOMP)
+  float4* scomp = reinterpret_cast<float4*>(smem + kSb + TS::tap_bytes(STEPS));  // [3][kTX][L] (SCOMP)
   float* s_psf = reinterpret_cast<float*>(smem + kSb + TS::tap_bytes(STEPS) + TS::comp_bytes(SCOMP));  // [nz][2K]
   float* s_psf_m = s_psf + static_cast<size_t>(a.nz) * 2 * K;       // [nz][2K] (mate)
   cg::cluster_group cluster = cg::this_cluster();
   const int slab = static_cast<int>(cluster.block_rank());
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int grp = threadIdx.x / L, lane = threadIdx.x % L;
   const int yb = lane * 4;
   const bool yok = lane_rows_ok(a, yb);
   const bool paired = PAIR && mate >= 0;  // uniform over the cluster
@@ -779,20 +807,20 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
   auto mate_pass = [&](const float4* sbuf, int z, auto emit_m) {
     if constexpr (PTAB) {
       const float* m = ptab + (a.nz - 1 - z) * 2 * K;
-      rowpass_from_tile_p<R>(sbuf, warp * kTXW, emit_m, Reversed<R>{m}, m + K, lane, a.ny);
+      rowpass_from_tile_p<R, L>(sbuf, grp * kTXW, emit_m, Reversed<R>{m}, m + K, lane, a.ny);
     } else {
       const float* m = s_psf_m + z * 2 * K;
-      rowpass_from_tile_p<R>(sbuf, warp * kTXW, emit_m, m, m + K, lane, a.ny);
+      rowpass_from_tile_p<R, L>(sbuf, grp * kTXW, emit_m, m, m + K, lane, a.ny);
     }
   };
   auto both_pass = [&](const float4* sbuf, int z, auto emit, auto emit_m) {
     const float* kr = (PTAB ? ptab : s_psf) + z * 2 * K;
     if constexpr (PTAB) {
       const float* m = ptab + (a.nz - 1 - z) * 2 * K;
-      rowpass2_from_tile_p<R>(sbuf, warp * kTXW, emit, kr, kr + K, emit_m, Reversed<R>{m}, m + K, lane, a.ny);
+      rowpass2_from_tile_p<R, L>(sbuf, grp * kTXW, emit, kr, kr + K, emit_m, Reversed<R>{m}, m + K, lane, a.ny);
     } else {
       const float* m = s_psf_m + z * 2 * K;
-      rowpass2_from_tile_p<R>(sbuf, warp * kTXW, emit, kr, kr + K, emit_m, m, m + K, lane, a.ny);
+      rowpass2_from_tile_p<R, L>(sbuf, grp * kTXW, emit, kr, kr + K, emit_m, m, m + K, lane, a.ny);
     }
   };
   const CamRows cr = cam_rows(a.geom[cam].fwd);
@@ -801,7 +829,7 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
   float4 T[kTXW], P[kTXW], cT[NC], cP[NC];  // c*: Kahan compensations (KAHAN without SCOMP)
   float4 Q[PAIR ? kTXW : 1];                // mate's slab partial
   // compensation slot of quantity q (0 T, 1 P, 2 Q) of output i (SCOMP)
-  auto cslot = [&](int q, int i) { return scomp + (q * kTXC + warp * kTXW + i) * 32 + lane; };
+  auto cslot = [&](int q, int i) { return scomp + (q * kTX<L> + grp * kTXW + i) * L + lane; };
   // s += v, Kahan-compensated (KAHAN) or plain; value of a compensated sum
   auto kadd = [&](float4& s, float4* creg, int q, int i, const float4& v) {
     if constexpr (SCOMP) {
@@ -833,7 +861,7 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
     if (PAIR) Q[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int q = 0; q < 3; ++q) kclear(q, i);
   }
-  ybuf_zero_pads();
+  ybuf_zero_pads<L>();
   __syncthreads();
 
   // A depth step at plane z through tile buffer b: produce (footprints and
@@ -842,27 +870,27 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
   // form); MODE 1: the mate alone, direct weights (walked from the slab's
   // far end).
   auto produce = [&](int z, int b) {
-    float4* sbuf = sb + b * NS * 32;
+    float4* sbuf = sb + b * NS * L;
     Tap* tb = taps + b * TS::kTapSlots;
-    // footprints of the columns this warp samples (c = warp + kW * k)
+    // footprints of the columns this group samples (c = grp + G * k)
     if (lane < TS::kOwn) {
-      const int c = warp + kW * lane;
+      const int c = grp + TS::G * lane;
       if (c < NS) {
         const int xp = x0 - R + c;
-        tb[tap_slot<R>(c)] = make_tap(xp, z, cr.m00, cr.m02, cr.m03, cr.m20, cr.m22, cr.m23, a.nx, a.nz, a.cy,
+        tb[tap_slot<R, L>(c)] = make_tap(xp, z, cr.m00, cr.m02, cr.m03, cr.m20, cr.m22, cr.m23, a.nx, a.nz, a.cy,
                                       xp >= 0 && xp < a.nx);
       }
     }
     __syncwarp();
 #pragma unroll
     for (int k = 0; k < TS::kOwn; ++k) {
-      const int c = warp + kW * k;
-      if (c < NS) sbuf[c * 32 + lane] = sample4(act, tb[tap_slot<R>(c)], yb, yok);
+      const int c = grp + TS::G * k;
+      if (c < NS) sbuf[c * L + lane] = sample4(act, tb[tap_slot<R, L>(c)], yb, yok);
     }
   };
   auto consume = [&](int z, int b, auto mode) {
     constexpr int MODE = decltype(mode)::value;
-    const float4* sbuf = sb + b * NS * 32;
+    const float4* sbuf = sb + b * NS * L;
     const Tap* tb = taps + b * TS::kTapSlots;
     auto emit_m = [&](int i, const float4& v) {
       if (!ATT) {
@@ -876,7 +904,7 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
           fma4p(Q[i], v, exp_neg4(make_float4(-T[i].x, -T[i].y, -T[i].z, -T[i].w)));
         }
       } else {  // T runs from the slab's far end, inclusive
-        const float4 m = sample4(mu, tb[tap_slot<R>(warp * kTXW + i + R)], yb, yok);
+        const float4 m = sample4(mu, tb[tap_slot<R, L>(grp * kTXW + i + R)], yb, yok);
         if (KAHAN) {
           kadd(T[i], &cT[SCOMP ? 0 : i], 0, i, m);
           kadd(Q[i], nullptr, 2, i, mul4p(v, exp_neg4(kval(T[i], &cT[SCOMP ? 0 : i], 0, i))));
@@ -891,11 +919,11 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
         mate_pass(sbuf, z, emit_m);
       } else {
 #pragma unroll
-        for (int i = 0; i < kTXW; ++i) emit_m(i, sbuf[(warp * kTXW + i) * 32 + lane]);
+        for (int i = 0; i < kTXW; ++i) emit_m(i, sbuf[(grp * kTXW + i) * L + lane]);
       }
       return;
     }
-    // float32, PSF radius <= 5: mu of the warp's output columns sampled
+    // float32, PSF radius <= 5: mu of the group's output columns sampled
     // before the row pass, so that the gathers' latency overlaps the PSF
     // arithmetic (128^3 x 120, PSF 11: projector 0.608 -> 0.586 ms); wider
     // PSFs would spill registers (radius 7: slower)
@@ -903,11 +931,11 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
     float4 mv[kTXW];
     if constexpr (kEarlyMu) {
 #pragma unroll
-      for (int i = 0; i < kTXW; ++i) mv[i] = sample4(mu, tb[tap_slot<R>(warp * kTXW + i + R)], yb, yok);
+      for (int i = 0; i < kTXW; ++i) mv[i] = sample4(mu, tb[tap_slot<R, L>(grp * kTXW + i + R)], yb, yok);
     }
     auto emit = [&](int i, const float4& v) {
       if (ATT) {
-        const float4 m = kEarlyMu ? mv[i] : sample4(mu, tb[tap_slot<R>(warp * kTXW + i + R)], yb, yok);
+        const float4 m = kEarlyMu ? mv[i] : sample4(mu, tb[tap_slot<R, L>(grp * kTXW + i + R)], yb, yok);
         if (KAHAN) {
           kadd(T[i], &cT[SCOMP ? 0 : i], 0, i, m);
           kadd(P[i], &cP[SCOMP ? 0 : i], 1, i, mul4p(v, exp_neg4(kval(T[i], &cT[SCOMP ? 0 : i], 0, i))));
@@ -924,12 +952,12 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
         both_pass(sbuf, z, emit, emit_m);
       } else {
         const float* kr = (PTAB ? ptab : s_psf) + z * 2 * K;
-        rowpass_from_tile_p<R>(sbuf, warp * kTXW, emit, kr, kr + K, lane, a.ny);
+        rowpass_from_tile_p<R, L>(sbuf, grp * kTXW, emit, kr, kr + K, lane, a.ny);
       }
     } else {
 #pragma unroll
       for (int i = 0; i < kTXW; ++i) {
-        const float4 v = sbuf[(warp * kTXW + i) * 32 + lane];
+        const float4 v = sbuf[(grp * kTXW + i) * L + lane];
         if (PAIR && paired) emit_m(i, v);
         emit(i, v);
       }
@@ -954,7 +982,7 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
   auto stash_mid = [&]() {
 #pragma unroll
     for (int i = 0; i < kTXW; ++i) {
-      const int o = warp * kTXW + i;
+      const int o = grp * kTXW + i;
       if (x0 + o < a.nx && yok && lane_writes(a, yb))
         *reinterpret_cast<float4*>(carry_at(o, 2 * slab + 1)) = kval(T[i], &cT[SCOMP ? 0 : i], 0, i);
     }
@@ -1006,17 +1034,17 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
 
   // cluster merge of the depth slabs (the shared tile is free after this barrier)
   __syncthreads();
-  float4* sT = sb;                // [kTXC][32]
-  float4* sP = sb + kTXC * 32;    // [kTXC][32]
-  float4* sQ = sb + 2 * kTXC * 32;  // [kTXC][32] (PAIR)
+  float4* sT = sb;                    // [kTX][L]
+  float4* sP = sb + kTX<L> * L;       // [kTX][L]
+  float4* sQ = sb + 2 * kTX<L> * L;   // [kTX][L] (PAIR)
 #pragma unroll
   for (int i = 0; i < kTXW; ++i) {
-    sT[(warp * kTXW + i) * 32 + lane] = kval(T[i], &cT[SCOMP ? 0 : i], 0, i);
-    sP[(warp * kTXW + i) * 32 + lane] = kval(P[i], &cP[SCOMP ? 0 : i], 1, i);
-    if (PAIR && paired) sQ[(warp * kTXW + i) * 32 + lane] = kval(Q[i], nullptr, 2, i);
+    sT[(grp * kTXW + i) * L + lane] = kval(T[i], &cT[SCOMP ? 0 : i], 0, i);
+    sP[(grp * kTXW + i) * L + lane] = kval(P[i], &cP[SCOMP ? 0 : i], 1, i);
+    if (PAIR && paired) sQ[(grp * kTXW + i) * L + lane] = kval(Q[i], nullptr, 2, i);
   }
   cluster.sync();
-  const int per_rank = kTXC / nslabs;  // outputs merged by each CTA of the cluster
+  const int per_rank = kTX<L> / nslabs;  // outputs merged by each CTA of the cluster
   auto store = [&](int c, int x, float4 Pt) {
     if (a.truncate) {
       Pt.x = fmaxf(Pt.x, 0.f);
@@ -1031,14 +1059,14 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
   const bool carry = ATT && a.carry_out;
 #pragma unroll
   for (int i = 0; i < kTXW; ++i) {
-    const int o = warp * kTXW + i;
+    const int o = grp * kTXW + i;
     const int x = x0 + o;
     if (o / per_rank != slab || x >= a.nx || !yok || !lane_writes(a, yb)) continue;
     float4 Pt = make_float4(0.f, 0.f, 0.f, 0.f), Tt = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int s = 0; s < nslabs; ++s) {
       const float4* rT = cluster.map_shared_rank(sT, s);
       const float4* rP = cluster.map_shared_rank(sP, s);
-      const float4 ps = rP[o * 32 + lane];
+      const float4 ps = rP[o * L + lane];
       if (ATT) {
         if (carry) {
           *reinterpret_cast<float4*>(carry_at(o, split ? 2 * s : s)) = Tt;
@@ -1050,7 +1078,7 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
           }
         }
         fma4(Pt, exp_neg4(Tt), ps);
-        add4(Tt, rT[o * 32 + lane]);
+        add4(Tt, rT[o * L + lane]);
       } else {
         add4(Pt, ps);
       }
@@ -1061,10 +1089,10 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
       Pt = make_float4(0.f, 0.f, 0.f, 0.f);
       Tt = make_float4(0.f, 0.f, 0.f, 0.f);
       for (int s = nslabs - 1; s >= 0; --s) {
-        const float4 qs = cluster.map_shared_rank(sQ, s)[o * 32 + lane];
+        const float4 qs = cluster.map_shared_rank(sQ, s)[o * L + lane];
         if (ATT) {
           fma4(Pt, exp_neg4(Tt), qs);
-          add4(Tt, cluster.map_shared_rank(sT, s)[o * 32 + lane]);
+          add4(Tt, cluster.map_shared_rank(sT, s)[o * L + lane]);
         } else {
           add4(Pt, qs);
         }
@@ -1075,7 +1103,7 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
   cluster.sync();  // keep this CTA's shared memory alive until the others have read it
 }
 
-constexpr int kWindowRows = 128;  // rows one warp covers (32 lanes x 4)
+constexpr int kWindowRows = 128;  // rows 32 lanes cover (4 each)
 
 // Row windows of a volume for a PSF halo: window starts and valid ranges are
 // multiples of 4 (the halo is rounded up), every row is valid in exactly one
@@ -1085,6 +1113,31 @@ constexpr int kWindowRows = 128;  // rows one warp covers (32 lanes x 4)
 struct Window {
   int row0, rows, lo, hi;  // rows [row0, row0 + rows); valid [row0 + lo, row0 + hi)
 };
+
+// Lanes per column of the tile engine for a window of `rows` rows of nx
+// columns: the fewest x-tiles among the lane counts that hold the rows, the
+// larger count on a tie.  A CTA costs about the same for every L (the same
+// outputs per thread), so a window of up to 64 or 32 rows costs a half or a
+// quarter where the volume is wide enough; with 32 lanes it costs as much as
+// 128 rows (256^3 x 180, PSF 15, windows of 128, 128 and 32 rows: pair 22.9 ms
+// with 32 lanes throughout, 17.6 ms; 8 uneven volumes of 64, 96, 128 and 160
+// rows: OSEM 21.3 -> 18.7 ms).
+int window_lanes(int rows, int nx) {
+  int lanes = 32, tiles = (nx + kTX<32> - 1) / kTX<32>;
+  for (int l : {16, 8}) {
+    const int t = (nx + 1024 / l - 1) / (1024 / l);
+    if (rows <= 4 * l && t < tiles) {
+      lanes = l;
+      tiles = t;
+    }
+  }
+  return lanes;
+}
+static_assert(kTX<32> == 32 && kTX<16> == 64 && kTX<8> == 128, "1024 / L output columns per CTA");
+
+// The same for the gather and the carries, whose lane groups take any column:
+// the fewest lanes that hold the rows.
+int column_lanes(int rows) { return rows <= 32 ? 8 : rows <= 64 ? 16 : 32; }
 
 std::vector<Window> row_windows(int ny, int halo) {
   const int h = (halo + 3) & ~3;
@@ -1114,6 +1167,7 @@ YgArgs windowed(const YgArgs& a, const Window& w) {
   b.out_lo = w.lo;
   b.out_hi = w.hi;
   b.cs = round_up(w.rows, 4);
+  b.lanes = window_lanes(w.rows, a.nx);
   return b;
 }
 

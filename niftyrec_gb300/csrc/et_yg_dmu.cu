@@ -21,7 +21,7 @@ namespace {
 
 template <int R, bool PSF, bool PTAB>
 __device__ __forceinline__ void dmu_item(const YgArgs& a, int cam, int x0, unsigned char* smem, const float* ptab) {
-  using TS = TileShape<R>;
+  using TS = TileShape<R, 32>;
   const float* __restrict__ act = a.act + a.row0;
   const float* __restrict__ mu = a.mu + a.row0;
   float* __restrict__ out = a.out + a.row0;
@@ -51,7 +51,7 @@ __device__ __forceinline__ void dmu_item(const YgArgs& a, int cam, int x0, unsig
     T[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     P[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  ybuf_zero_pads();
+  ybuf_zero_pads<32>();
   __syncthreads();
 
   auto produce = [&](int z, int b) {
@@ -61,7 +61,7 @@ __device__ __forceinline__ void dmu_item(const YgArgs& a, int cam, int x0, unsig
       const int c = warp + kW * lane;
       if (c < NS) {
         const int xp = x0 - R + c;
-        tb[tap_slot<R>(c)] = make_tap(xp, z, cr.m00, cr.m02, cr.m03, cr.m20, cr.m22, cr.m23, a.nx, a.nz, a.cy,
+        tb[tap_slot<R, 32>(c)] = make_tap(xp, z, cr.m00, cr.m02, cr.m03, cr.m20, cr.m22, cr.m23, a.nx, a.nz, a.cy,
                                       xp >= 0 && xp < a.nx);
       }
     }
@@ -69,7 +69,7 @@ __device__ __forceinline__ void dmu_item(const YgArgs& a, int cam, int x0, unsig
 #pragma unroll
     for (int k = 0; k < TS::kOwn; ++k) {
       const int c = warp + kW * k;
-      if (c < NS) sbuf[c * 32 + lane] = sample4(act, tb[tap_slot<R>(c)], yb, yok);
+      if (c < NS) sbuf[c * 32 + lane] = sample4(act, tb[tap_slot<R, 32>(c)], yb, yok);
     }
   };
   // the PSF-convolved activity of this warp's output columns at plane z
@@ -77,7 +77,7 @@ __device__ __forceinline__ void dmu_item(const YgArgs& a, int cam, int x0, unsig
     const float4* sbuf = sb + b * NS * 32;
     if (PSF) {
       const float* kr = (PTAB ? ptab : s_psf) + z * 2 * K;
-      rowpass_from_tile<R>(sbuf, warp * kTXW, emit, kr, kr + K, lane, a.ny);
+      rowpass_from_tile<R, 32>(sbuf, warp * kTXW, emit, kr, kr + K, lane, a.ny);
     } else {
 #pragma unroll
       for (int i = 0; i < kTXW; ++i) emit(i, sbuf[(warp * kTXW + i) * 32 + lane]);
@@ -95,7 +95,7 @@ __device__ __forceinline__ void dmu_item(const YgArgs& a, int cam, int x0, unsig
   walk([&](int z, int b) {
     const Tap* tb = taps + b * TS::kTapSlots;
     pass(z, b, [&](int i, const float4& v) {
-      add4(T[i], sample4(mu, tb[tap_slot<R>(warp * kTXW + i + R)], yb, yok));
+      add4(T[i], sample4(mu, tb[tap_slot<R, 32>(warp * kTXW + i + R)], yb, yok));
       fma4(P[i], v, exp_neg4(T[i]));
     });
   });
@@ -103,7 +103,7 @@ __device__ __forceinline__ void dmu_item(const YgArgs& a, int cam, int x0, unsig
   // exchange through distributed shared memory (the tile region is free)
   __syncthreads();
   float4* sT = sb;
-  float4* sP = sb + kTXC * 32;
+  float4* sP = sb + kTX<32> * 32;
 #pragma unroll
   for (int i = 0; i < kTXW; ++i) {
     sT[(warp * kTXW + i) * 32 + lane] = T[i];
@@ -139,7 +139,7 @@ __device__ __forceinline__ void dmu_item(const YgArgs& a, int cam, int x0, unsig
   walk([&](int z, int b) {
     const Tap* tb = taps + b * TS::kTapSlots;
     pass(z, b, [&](int i, const float4& v) {
-      const Tap& t = tb[tap_slot<R>(warp * kTXW + i + R)];
+      const Tap& t = tb[tap_slot<R, 32>(warp * kTXW + i + R)];
       add4(T[i], sample4(mu, t, yb, yok));
       const float4 d = make_float4(fmaf(Bq[i].x, P[i].x, A[i].x), fmaf(Bq[i].y, P[i].y, A[i].y),
                                    fmaf(Bq[i].z, P[i].z, A[i].z), fmaf(Bq[i].w, P[i].w, A[i].w));
@@ -157,26 +157,26 @@ __device__ __forceinline__ void dmu_item(const YgArgs& a, int cam, int x0, unsig
 template <int R, bool PSF>
 __global__ void __launch_bounds__(32 * kW, 2) k_dmu_yg(const YgArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int ntile = (a.nx + kTXC - 1) / kTXC;
+  const int ntile = (a.nx + kTX<32> - 1) / kTX<32>;
   const int item = blockIdx.x / a.pslabs;
-  dmu_item<R, PSF, false>(a, a.cam0 + item / ntile, (item % ntile) * kTXC, smem, nullptr);
+  dmu_item<R, PSF, false>(a, a.cam0 + item / ntile, (item % ntile) * kTX<32>, smem, nullptr);
 }
 
 template <int R>
 __global__ void __launch_bounds__(32 * kW, 2) k_dmu_ptab_yg(const YgArgs a, const __grid_constant__ PsfTable t) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int ntile = (a.nx + kTXC - 1) / kTXC;
+  const int ntile = (a.nx + kTX<32> - 1) / kTX<32>;
   const int item = blockIdx.x / a.pslabs;
-  dmu_item<R, true, true>(a, a.cam0 + item / ntile, (item % ntile) * kTXC, smem, t.c);
+  dmu_item<R, true, true>(a, a.cam0 + item / ntile, (item % ntile) * kTX<32>, smem, t.c);
 }
 
 template <int R>
 int launch_dmu_R(const YgArgs& a_in, cudaStream_t st) {
   YgArgs a = a_in;
-  const int ntile = (a.nx + kTXC - 1) / kTXC;
+  const int ntile = (a.nx + kTX<32> - 1) / kTX<32>;
   const bool psf = a.psf != nullptr;
   const bool ptab = psf && a.psf_host && static_cast<size_t>(a.nz) * 2 * (2 * R + 1) <= kPsfTableFloats;
-  const size_t smem = tile_smem_bytes<R>(psf && !ptab ? a.nz : 0);
+  const size_t smem = tile_smem_bytes<R, 32>(psf && !ptab ? a.nz : 0);
   // depth slabs: the fewest of 2, 4, 8 giving four waves of two CTAs per SM
   if (a.pslabs != 2 && a.pslabs != 4 && a.pslabs != 8) {
     a.pslabs = 8;

@@ -28,7 +28,7 @@ namespace {
 template <int R, bool PSF, bool PTAB>
 __device__ __forceinline__ void grad_item(const YgArgs& a, int cam, int g, int x0, unsigned char* smem,
                                           const float* ptab) {
-  using TS = TileShape<R>;
+  using TS = TileShape<R, 32>;
   constexpr int NS = TS::NS;
   constexpr int OWN = TS::kOwn;
   constexpr int K = 2 * R + 1;
@@ -62,7 +62,7 @@ __device__ __forceinline__ void grad_item(const YgArgs& a, int cam, int g, int x
       const int c = warp + kW * lane;
       if (c < NS) {
         const int xp = x0 - R + c;
-        tb[tap_slot<R>(c)] = make_tap(xp, z, cr.m00, cr.m02, cr.m03, cr.m20, cr.m22, cr.m23, a.nx, a.nz, a.cy,
+        tb[tap_slot<R, 32>(c)] = make_tap(xp, z, cr.m00, cr.m02, cr.m03, cr.m20, cr.m22, cr.m23, a.nx, a.nz, a.cy,
                                       xp >= 0 && xp < a.nx);
       }
     }
@@ -70,7 +70,7 @@ __device__ __forceinline__ void grad_item(const YgArgs& a, int cam, int g, int x
     return tb;
   };
 
-  ybuf_zero_pads();  // ordered before walk 2 by the cluster barriers
+  ybuf_zero_pads<32>();  // ordered before walk 2 by the cluster barriers
 
   // walk 1: the slab's transmission and partial per sampled column
   float4 T[OWN], P[OWN];
@@ -85,7 +85,7 @@ __device__ __forceinline__ void grad_item(const YgArgs& a, int cam, int g, int x
     for (int k = 0; k < OWN; ++k) {
       const int c = warp + kW * k;
       if (c < NS) {
-        const Tap& t = tb[tap_slot<R>(c)];
+        const Tap& t = tb[tap_slot<R, 32>(c)];
         add4(T[k], sample4(mu, t, yb, yok));
         fma4(P[k], sample4(act, t, yb, yok), exp_neg4(T[k]));
       }
@@ -133,7 +133,7 @@ __device__ __forceinline__ void grad_item(const YgArgs& a, int cam, int g, int x
     for (int k = 0; k < OWN; ++k) {
       const int c = warp + kW * k;
       if (c < NS) {
-        const Tap& t = tb[tap_slot<R>(c)];
+        const Tap& t = tb[tap_slot<R, 32>(c)];
         const float4 m = sample4(mu, t, yb, yok);
         fma4(P[k], sample4(act, t, yb, yok), exp_neg4(T[k]));
         T[k] = make_float4(T[k].x - m.x, T[k].y - m.y, T[k].z - m.z, T[k].w - m.w);
@@ -150,7 +150,7 @@ __device__ __forceinline__ void grad_item(const YgArgs& a, int cam, int g, int x
     };
     if (PSF) {
       const float* kr = (PTAB ? ptab : s_psf) + z * 2 * K;
-      rowpass_from_tile<R>(sbuf, warp * kTXW, emit, kr, kr + K, lane, a.ny);
+      rowpass_from_tile<R, 32>(sbuf, warp * kTXW, emit, kr, kr + K, lane, a.ny);
     } else {
 #pragma unroll
       for (int i = 0; i < kTXW; ++i) emit(i, sbuf[(warp * kTXW + i) * 32 + lane]);
@@ -162,29 +162,29 @@ __device__ __forceinline__ void grad_item(const YgArgs& a, int cam, int g, int x
 template <int R, bool PSF>
 __global__ void __launch_bounds__(32 * kW, 2) k_grad_spread_yg(const YgArgs a, int c0) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int ntile = (a.nx + kTXC - 1) / kTXC;
+  const int ntile = (a.nx + kTX<32> - 1) / kTX<32>;
   const int item = blockIdx.x / a.pslabs;
   const int g = item / ntile;
-  grad_item<R, PSF, false>(a, c0 + g, g, (item % ntile) * kTXC, smem, nullptr);
+  grad_item<R, PSF, false>(a, c0 + g, g, (item % ntile) * kTX<32>, smem, nullptr);
 }
 
 template <int R>
 __global__ void __launch_bounds__(32 * kW, 2)
     k_grad_spread_ptab_yg(const YgArgs a, int c0, const __grid_constant__ PsfTable t) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int ntile = (a.nx + kTXC - 1) / kTXC;
+  const int ntile = (a.nx + kTX<32> - 1) / kTX<32>;
   const int item = blockIdx.x / a.pslabs;
   const int g = item / ntile;
-  grad_item<R, true, true>(a, c0 + g, g, (item % ntile) * kTXC, smem, t.c);
+  grad_item<R, true, true>(a, c0 + g, g, (item % ntile) * kTX<32>, smem, t.c);
 }
 
 template <int R>
 int launch_grad_R(const YgArgs& a_in, int c0, int gcount, cudaStream_t st) {
   YgArgs a = a_in;
-  const int ntile = (a.nx + kTXC - 1) / kTXC;
+  const int ntile = (a.nx + kTX<32> - 1) / kTX<32>;
   const bool psf = a.psf != nullptr;
   const bool ptab = psf && a.psf_host && static_cast<size_t>(a.nz) * 2 * (2 * R + 1) <= kPsfTableFloats;
-  const size_t smem = tile_smem_bytes<R>(psf && !ptab ? a.nz : 0);
+  const size_t smem = tile_smem_bytes<R, 32>(psf && !ptab ? a.nz : 0);
   // depth slabs: the fewest of 2, 4, 8 giving four waves of two CTAs per SM
   if (a.pslabs != 2 && a.pslabs != 4 && a.pslabs != 8) {
     a.pslabs = 8;

@@ -28,7 +28,7 @@ int project_slabs(int items, int ctas_per_sm, int nz) {
 }
 
 int yg_pair_project_slabs(int nunits, int nx, int nz) {
-  return project_slabs(nunits * ((nx + kTXC - 1) / kTXC), 2, nz);
+  return project_slabs(nunits * ((nx + kTX<32> - 1) / kTX<32>), 2, nz);
 }
 
 namespace {
@@ -60,16 +60,20 @@ __global__ void __cluster_dims__(kSlabsP, 1, 1) __launch_bounds__(32 * kW, CTAS)
     int v = 0;
     while (v + 1 < sel.n && item >= sel.begin[v + 1]) ++v;
     const BatchStepDesc& d = descs[sel.desc[v]];
-    const int ntile = (d.proj.nx + kTXC - 1) / kTXC;
-    const int per_win = d.proj.ncam * ntile;
-    const int local = item - sel.begin[v];
-    const int w = local / per_win, r = local % per_win;
+    int r = item - sel.begin[v], w = 0;
+    while (w + 1 < d.nwin && r >= d.tiles[w] * d.proj.ncam) r -= d.tiles[w++] * d.proj.ncam;
+    const int ntile = d.tiles[w];
     YgArgs a = d.proj;
     a.row0 = d.win[w][0];
     a.ny = d.win[w][1];
     a.out_lo = d.win[w][2];
     a.out_hi = d.win[w][3];
-    project_item<R, PSF, ATT, float>(a, r / ntile, -1, (r % ntile) * kTXC, smem);
+    const int cam = r / ntile, t = r % ntile;
+    switch (d.lanes[w]) {  // uniform over the cluster
+      case 8: project_item<R, PSF, ATT, float, false, false, 8>(a, cam, -1, t * kTX<8>, smem); break;
+      case 16: project_item<R, PSF, ATT, float, false, false, 16>(a, cam, -1, t * kTX<16>, smem); break;
+      default: project_item<R, PSF, ATT, float, false, false, 32>(a, cam, -1, t * kTX<32>, smem);
+    }
   }
 }
 
@@ -93,8 +97,12 @@ int batch_clusters(int ctas) { return sm_count() * ctas / kSlabsP; }
 template <int R, bool PSF>
 int launch_project_batch_R(const BatchStepDesc* d, const BatchSel& sel, bool att, int max_nz, int* counter,
                            cudaStream_t st) {
-  const size_t smem = tile_smem_bytes<R>(PSF ? max_nz : 0);
-  const bool three = 3 * (smem + kYBufBytes + 1024) <= 228 * 1024;
+  // one launch runs windows of any lane count: the largest tile of the three
+  const int planes = PSF ? max_nz : 0;
+  const size_t smem =
+      std::max({tile_smem_bytes<R, 32>(planes), tile_smem_bytes<R, 16>(planes), tile_smem_bytes<R, 8>(planes)});
+  const size_t fixed = kYBufBytes<32> + kYBufBytes<16> + kYBufBytes<8>;
+  const bool three = 3 * (smem + fixed + 1024) <= 228 * 1024;
   auto go = [&](auto k, int ctas) {
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     NRGB_LAUNCH_SCOPE("k_project_batch_yg", st);
@@ -136,12 +144,21 @@ int yg_project_batch(const BatchStepDesc* d_desc, const BatchSel& sel, int psf_k
 
 int yg_project(const YgArgs& a, cudaStream_t st, int* slabs_used) {
   const int R = a.psf ? (a.psf_k - 1) / 2 : 0;
-  int used = 0;
-  for (const Window& w : row_windows(a.ny, R)) {
-    const int s = project_by_radius(R, windowed(a, w), st, &used);
+  const std::vector<Window> wins = row_windows(a.ny, R);
+  int pslabs = a.pslabs;
+  for (size_t i = 0; i < wins.size(); ++i) {
+    int used[2] = {0, 0};
+    YgArgs b = windowed(a, wins[i]);
+    b.pslabs = pslabs;
+    const int s = project_by_radius(R, b, st, used);
     if (s != kOk) return s;
-    // every window launches with the same slab count (same sizes, same kernel)
-    if (slabs_used) *slabs_used = used;
+    if (a.carry_out) {
+      // the carries of every window have the slabs of the first; a window
+      // whose kernel fell back from 16 takes the others with it
+      if (i > 0 && used[1] != pslabs) i = static_cast<size_t>(-1);
+      pslabs = used[1];
+    }
+    if (slabs_used) *slabs_used = used[0];
   }
   return kOk;
 }

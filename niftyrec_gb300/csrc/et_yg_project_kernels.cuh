@@ -19,52 +19,47 @@ namespace {
 // for -- 3 (80 registers, more warps to hide the gathers' latency) where
 // three tiles fit in shared memory and the storage is float32, else 2 (128
 // registers; bfloat16 needs them for its Kahan compensations).
-template <int R, bool PSF, bool ATT, class V, int CTAS, bool PAIR>
+template <int R, bool PSF, bool ATT, class V, int CTAS, bool PAIR, int L>
 __global__ void __launch_bounds__(32 * kW, CTAS) k_project_yg(const YgArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int ntile = (a.nx + kTXC - 1) / kTXC;
+  const int ntile = (a.nx + kTX<L> - 1) / kTX<L>;
   const int item = blockIdx.x / a.pslabs;
   const int u = item / ntile;
   const int2 uc = PAIR ? a.units[u] : make_int2(u, -1);
-  project_item<R, PSF, ATT, V, PAIR>(a, uc.x, uc.y, (item % ntile) * kTXC, smem);
+  project_item<R, PSF, ATT, V, PAIR, false, L>(a, uc.x, uc.y, (item % ntile) * kTX<L>, smem);
 }
 
 // The same with the separated PSF in the kernel parameters (PsfTable).
-template <int R, bool ATT, class V, int CTAS, bool PAIR>
+template <int R, bool ATT, class V, int CTAS, bool PAIR, int L>
 __global__ void __launch_bounds__(32 * kW, CTAS) k_project_ptab_yg(const YgArgs a, const __grid_constant__ PsfTable t) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int ntile = (a.nx + kTXC - 1) / kTXC;
+  const int ntile = (a.nx + kTX<L> - 1) / kTX<L>;
   const int item = blockIdx.x / a.pslabs;
   const int u = item / ntile;
   const int2 uc = PAIR ? a.units[u] : make_int2(u, -1);
-  project_item<R, true, ATT, V, PAIR, true>(a, uc.x, uc.y, (item % ntile) * kTXC, smem, t.c);
+  project_item<R, true, ATT, V, PAIR, true, L>(a, uc.x, uc.y, (item % ntile) * kTX<L>, smem, t.c);
 }
 
-}  // namespace
-
-// Launch the per-call projector of PSF radius R (R = 0: no PSF) for one row
-// window; explicitly instantiated in et_yg_proj_r*.cu.  slabs_used (if
-// non-null) receives the depth-slab count of the launch (the slabs of the
-// carries written to a.carry_out).
-template <int R>
-int launch_project_R(const YgArgs& a_in, cudaStream_t st, int* slabs_used) {
+// L lanes per column (L < 32: narrow row windows; no PSF, or the PSF in the
+// kernel parameters).
+template <int R, int L>
+int launch_project_lanes(const YgArgs& a_in, cudaStream_t st, int* slabs_used) {
   YgArgs a = a_in;
-  const int ntile = (a.nx + kTXC - 1) / kTXC;
+  const int ntile = (a.nx + kTX<L> - 1) / kTX<L>;
   const bool psf = a.psf != nullptr;
   const bool bf16 = a.storage == kStorageBF16;
-  // the PSF in the kernel parameters when the host copy is given and fits
-  const bool ptab = psf && a.psf_host && static_cast<size_t>(a.nz) * 2 * (2 * R + 1) <= kPsfTableFloats;
+  const bool ptab = psf_in_parameters<R>(a);
   // mirror cameras: float32 always; bfloat16 (Kahan compensations in shared
   // memory) where two CTAs per SM still fit
   bool pair = a.units != nullptr && a.nunits > 0;
-  size_t smem = project_smem_bytes<R>(psf && !ptab ? a.nz : 0, pair, bf16);
-  if (pair && bf16 && 2 * (smem + kYBufBytes + 1024) > 228 * 1024) {
+  size_t smem = project_smem_bytes<R, L>(psf && !ptab ? a.nz : 0, pair, bf16);
+  if (pair && bf16 && 2 * (smem + kYBufBytes<L> + 1024) > 228 * 1024) {
     pair = false;
-    smem = project_smem_bytes<R>(psf && !ptab ? a.nz : 0, false, true);
+    smem = project_smem_bytes<R, L>(psf && !ptab ? a.nz : 0, false, true);
   }
   const int nunits = pair ? a.nunits : a.ncam;
   // three CTAs per SM need three tiles (plus 1 KB reserved each) in the 228 KB
-  const bool three = 3 * (smem + kYBufBytes + 1024) <= 228 * 1024;
+  const bool three = 3 * (smem + kYBufBytes<L> + 1024) <= 228 * 1024;
   if (a.pslabs != 2 && a.pslabs != 4 && a.pslabs != 8 && a.pslabs != 16)
     a.pslabs = project_slabs(nunits * ntile, three && !bf16 && !pair ? 3 : 2, a.nz);
   // carry split: the slab's halves must be the backprojector's slabs of twice
@@ -102,7 +97,10 @@ int launch_project_R(const YgArgs& a_in, cudaStream_t st, int* slabs_used) {
     }
     cfg.gridDim = dim3(nunits * ntile * a.pslabs);
     attr[0].val.clusterDim.x = a.pslabs;
-    if (slabs_used) *slabs_used = a.carry_split ? 2 * a.pslabs : a.pslabs;
+    if (slabs_used) {
+      slabs_used[0] = a.carry_split ? 2 * a.pslabs : a.pslabs;
+      slabs_used[1] = a.pslabs;
+    }
     NRGB_LAUNCH_SCOPE("k_project_yg", st);
     if (cudaLaunchKernelEx(&cfg, k, a, extra...) != cudaSuccess) launch_err = true;
   };
@@ -117,14 +115,16 @@ int launch_project_R(const YgArgs& a_in, cudaStream_t st, int* slabs_used) {
     constexpr int C = decltype(ctas)::value;
     constexpr bool P = decltype(paired)::value;
     if (psf && ptab) {
-      if (a.mu) go_tab(k_project_ptab_yg<R, true, V, C, P>);
-      else go_tab(k_project_ptab_yg<R, false, V, C, P>);
+      if (a.mu) go_tab(k_project_ptab_yg<R, true, V, C, P, L>);
+      else go_tab(k_project_ptab_yg<R, false, V, C, P, L>);
     } else if (psf) {
-      if (a.mu) go(k_project_yg<R, true, true, V, C, P>);
-      else go(k_project_yg<R, true, false, V, C, P>);
-    } else {
-      if (a.mu) go(k_project_yg<0, false, true, V, C, P>);
-      else go(k_project_yg<0, false, false, V, C, P>);
+      if constexpr (L == 32) {
+        if (a.mu) go(k_project_yg<R, true, true, V, C, P, L>);
+        else go(k_project_yg<R, true, false, V, C, P, L>);
+      }
+    } else if constexpr (R == 0) {
+      if (a.mu) go(k_project_yg<0, false, true, V, C, P, L>);
+      else go(k_project_yg<0, false, false, V, C, P, L>);
     }
   };
   using Off = std::false_type;
@@ -141,6 +141,21 @@ int launch_project_R(const YgArgs& a_in, cudaStream_t st, int* slabs_used) {
   else
     pick(0.0f, std::integral_constant<int, 2>(), Off());
   return cudaGetLastError() == cudaSuccess && !launch_err ? kOk : kErrKernel;
+}
+
+}  // namespace
+
+// Launch the per-call projector of PSF radius R (R = 0: no PSF) for one row
+// window; explicitly instantiated in et_yg_proj_r*.cu.  slabs_used (if
+// non-null) receives the slab count of the carries written to a.carry_out and
+// the depth-slab count of the launch.
+template <int R>
+int launch_project_R(const YgArgs& a, cudaStream_t st, int* slabs_used) {
+  if (!a.psf || psf_in_parameters<R>(a)) {
+    if (a.lanes == 8) return launch_project_lanes<R, 8>(a, st, slabs_used);
+    if (a.lanes == 16) return launch_project_lanes<R, 16>(a, st, slabs_used);
+  }
+  return launch_project_lanes<R, 32>(a, st, slabs_used);
 }
 
 }  // namespace nrgb

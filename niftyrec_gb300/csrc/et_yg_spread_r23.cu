@@ -1,0 +1,11 @@
+// Reference spread kernels for PSF radii 2 and 3.
+#include "et_yg_spread_kernels.cuh"
+
+namespace nrgb {
+
+template int launch_spread_R<2, false>(const YgArgs& a, int c0, int gcount, cudaStream_t st);
+template int launch_spread_pair_R<2, false>(const YgArgs& a, int u0, int gcount, cudaStream_t st);
+template int launch_spread_R<3, false>(const YgArgs& a, int c0, int gcount, cudaStream_t st);
+template int launch_spread_pair_R<3, false>(const YgArgs& a, int u0, int gcount, cudaStream_t st);
+
+}  // namespace nrgb

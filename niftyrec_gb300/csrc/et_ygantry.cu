@@ -177,12 +177,18 @@ int yg_row_windows(int ny, int psf_k, int* out, int max_windows) {
   return static_cast<int>(w.size());
 }
 
+void yg_window_lanes(int rows, int nx, int* lanes, int* tiles) {
+  *lanes = window_lanes(rows, nx);
+  const int columns = 1024 / *lanes;
+  *tiles = (nx + columns - 1) / columns;
+}
+
 bool yg_supported(int nx, int ny, int nz, int psf_k) {
   const int cy = round_up(ny, 4);
   if (nx < 1 || ny < 1 || nz < 1) return false;
   if (psf_k != 0 && (psf_k % 2 != 1 || psf_k > 15)) return false;
   // the PSF table of one CTA lives in shared memory next to the tile
-  if (psf_k != 0 && tile_smem_bytes<7>(nz) > 110 * 1024) return false;
+  if (psf_k != 0 && tile_smem_bytes<7, 32>(nz) > 110 * 1024) return false;
   // 32-bit element offsets inside one volume
   if (static_cast<size_t>(nz) * nx * cy >= (1u << 31)) return false;
   return true;
