@@ -151,6 +151,9 @@ bool use_fused_x(const Problem& pb) {
 namespace {
 
 size_t vol_n(const Problem& pb) { return static_cast<size_t>(pb.nx) * pb.ny * pb.nz; }
+// Cameras per launch of the general path and its three sets of work volumes.
+int gen_group(const Problem& pb) { return general_group(vol_n(pb), sizeof(float), pb.cams.n); }
+size_t gen_n(const Problem& pb) { return vol_n(pb) * gen_group(pb); }
 size_t col_n(const Problem& pb) { return static_cast<size_t>(pb.nx) * round_up(pb.ny, 4) * pb.nz; }
 size_t sino_col_n(const Problem& pb) { return static_cast<size_t>(pb.nx) * round_up(pb.ny, 4) * pb.cams.n; }
 constexpr size_t kSlack = 8 * 256;
@@ -273,11 +276,11 @@ int widen_inputs(const Problem& pb, Carver& cv, const float** act, const float**
 
 size_t project_workspace(const Problem& pb, bool has_act, bool has_att) {
   size_t b = common_bytes(pb);
-  if (use_fused_x(pb) && has_act) return b + vol_n(pb) * 3 * sizeof(float) + widen_bytes(pb);  // or general
+  if (use_fused_x(pb) && has_act) return b + gen_n(pb) * 3 * sizeof(float) + widen_bytes(pb);  // or general
   if (use_fused(pb) && has_act)
     b += sizeof(float) * (col_n(pb) * (has_att ? 2 : 1) + sino_col_n(pb));
   else
-    b += sizeof(float) * vol_n(pb) * 3 + widen_bytes(pb);
+    b += sizeof(float) * gen_n(pb) * 3 + widen_bytes(pb);
   return b;
 }
 
@@ -285,18 +288,18 @@ size_t backproject_workspace(const Problem& pb, bool has_att) {
   size_t b = common_bytes(pb);
   if (use_fused_x(pb))  // the fused form's scratch, or the general path's volumes
     return b + std::max(yg_backproject_workspace(pb.ny, pb.nx, pb.nz, pb.cams.n, pb.group) + kSlack,
-                        sizeof(float) * vol_n(pb) * 3 + widen_bytes(pb));
+                        sizeof(float) * gen_n(pb) * 3 + widen_bytes(pb));
   if (use_fused(pb))
     b += sizeof(float) * (col_n(pb) * (has_att ? 2 : 1) + sino_col_n(pb)) +
          yg_backproject_workspace(pb.nx, pb.ny, pb.nz, pb.cams.n, pb.group) + kSlack;
   else
-    b += sizeof(float) * vol_n(pb) * 3 + widen_bytes(pb);
+    b += sizeof(float) * gen_n(pb) * 3 + widen_bytes(pb);
   return b;
 }
 
 namespace {
-// The general-orientation path's three work volumes.
-size_t general3_workspace(const Problem& pb) { return common_bytes(pb) + sizeof(float) * vol_n(pb) * 3; }
+// The general-orientation path's work volumes.
+size_t general3_workspace(const Problem& pb) { return common_bytes(pb) + sizeof(float) * gen_n(pb) * 3; }
 int grad_group(const Problem& pb) { return std::max(1, std::min(pb.group, pb.cams.n)); }
 }  // namespace
 
@@ -393,9 +396,10 @@ int project_device(const Problem& pb, const float* d_act, const float* d_att, fl
   g.bg = pb.bg;
   g.bg_att = pb.bg_att;
   g.truncate = pb.truncate;
-  g.ws_act = cv.take<float>(vol_n(pb));
-  g.ws_att = cv.take<float>(vol_n(pb));
-  g.ws_tmp = cv.take<float>(vol_n(pb));
+  g.group = gen_group(pb);
+  g.ws_act = cv.take<float>(gen_n(pb));
+  g.ws_att = cv.take<float>(gen_n(pb));
+  g.ws_tmp = cv.take<float>(gen_n(pb));
   if (!g.ws_act || !g.ws_att || !g.ws_tmp) return kErrAllocGpu;
   return check(general_project(g, st));
 }
@@ -524,9 +528,10 @@ int backproject_device(const Problem& pb, const float* d_sino, const float* d_at
   g.bg = pb.bg;
   g.bg_att = pb.bg_att;
   g.truncate = pb.truncate;
-  g.ws_act = cv.take<float>(vol_n(pb));
-  g.ws_att = cv.take<float>(vol_n(pb));
-  g.ws_tmp = cv.take<float>(vol_n(pb));
+  g.group = gen_group(pb);
+  g.ws_act = cv.take<float>(gen_n(pb));
+  g.ws_att = cv.take<float>(gen_n(pb));
+  g.ws_tmp = cv.take<float>(gen_n(pb));
   if (!g.ws_act || !g.ws_att || !g.ws_tmp) return kErrAllocGpu;
   return check(pb.back_mode == kBackAdjoint ? general_adjoint(g, st) : general_backproject(g, st));
 }
@@ -636,7 +641,7 @@ int pair_device(const Problem& pb, const Problem& pb_back, const float* d_act, c
   return check(from_column(out_c, d_bk, pb.nx, pb.ny, cy, pb.nz, pb.truncate, st));
 }
 
-size_t partial_workspace(const Problem& pb) { return common_bytes(pb) + sizeof(float) * vol_n(pb) * 3 + 3 * 256; }
+size_t partial_workspace(const Problem& pb) { return common_bytes(pb) + sizeof(float) * gen_n(pb) * 3 + 3 * 256; }
 
 int project_partial_device(const Problem& pb, const float* d_act, const float* d_att, const float* d_bg_image,
                            float* d_sino, float* d_partial, int do_rotate, char* ws, size_t ws_bytes, Staging* stg,
@@ -660,9 +665,10 @@ int project_partial_device(const Problem& pb, const float* d_act, const float* d
   g.bg = pb.bg;
   g.bg_att = pb.bg_att;
   g.truncate = pb.truncate;
-  g.ws_act = cv.take<float>(vol_n(pb));
-  g.ws_att = cv.take<float>(vol_n(pb));
-  g.ws_tmp = cv.take<float>(vol_n(pb));
+  g.group = gen_group(pb);
+  g.ws_act = cv.take<float>(gen_n(pb));
+  g.ws_att = cv.take<float>(gen_n(pb));
+  g.ws_tmp = cv.take<float>(gen_n(pb));
   if (!g.ws_act || !g.ws_att || !g.ws_tmp) return kErrAllocGpu;
   return check(general_project_partial(g, d_bg_image, d_partial, do_rotate, st));
 }
@@ -753,9 +759,10 @@ int dmu_device(const Problem& pb, const float* d_g, const float* d_act, const fl
   g.psf_k = pb.psf_k;
   g.bg = pb.bg;
   g.bg_att = pb.bg_att;
-  g.ws_act = cv.take<float>(vol_n(pb));
-  g.ws_att = cv.take<float>(vol_n(pb));
-  g.ws_tmp = cv.take<float>(vol_n(pb));
+  g.group = gen_group(pb);
+  g.ws_act = cv.take<float>(gen_n(pb));
+  g.ws_att = cv.take<float>(gen_n(pb));
+  g.ws_tmp = cv.take<float>(gen_n(pb));
   if (!g.ws_act || !g.ws_att || !g.ws_tmp) return kErrAllocGpu;
   return check(general_dmu(g, st));
 }
@@ -834,16 +841,18 @@ int gradient_device(const Problem& pb, const float* d_sino, const float* d_act, 
   g.bg = pb.bg;
   g.bg_att = pb.bg_att;
   g.truncate = pb.truncate;
-  g.ws_act = cv.take<float>(vol_n(pb));
-  g.ws_att = cv.take<float>(vol_n(pb));
-  g.ws_tmp = cv.take<float>(vol_n(pb));
+  g.group = gen_group(pb);
+  g.ws_act = cv.take<float>(gen_n(pb));
+  g.ws_att = cv.take<float>(gen_n(pb));
+  g.ws_tmp = cv.take<float>(gen_n(pb));
   if (!g.ws_act || !g.ws_att || !g.ws_tmp) return kErrAllocGpu;
   return check(general_gradient(g, st));
 }
 
 // ------------------------------------------------------------ float64 run
 size_t workspace64(const Problem& pb) {
-  return sizeof(double) * (3 * vol_n(pb) + static_cast<size_t>(2 * pb.psf_k) * pb.nz) + kSlack;
+  const size_t group = general_group(vol_n(pb), sizeof(double), pb.cams.n);
+  return sizeof(double) * (3 * vol_n(pb) * group + static_cast<size_t>(2 * pb.psf_k) * pb.nz) + kSlack;
 }
 
 namespace {
@@ -871,9 +880,10 @@ int setup64(const Problem& pb, const float* psf_host, Carver& cv, std::vector<Ca
       return kErrTransferGpu;
     g->psf_sep = d;
   }
-  g->ws_act = cv.take<double>(vol_n(pb));
-  g->ws_att = cv.take<double>(vol_n(pb));
-  g->ws_tmp = cv.take<double>(vol_n(pb));
+  g->group = general_group(vol_n(pb), sizeof(double), pb.cams.n);
+  g->ws_act = cv.take<double>(vol_n(pb) * g->group);
+  g->ws_att = cv.take<double>(vol_n(pb) * g->group);
+  g->ws_tmp = cv.take<double>(vol_n(pb) * g->group);
   return (g->ws_act && g->ws_att && g->ws_tmp) ? kOk : kErrAllocGpu;
 }
 

@@ -2,10 +2,16 @@
 // any background values, any grid.  Volumes in nifti layout.  Each stage is a
 // separate kernel following the reference's float operation order (products
 // and sums rounded separately), so this path reproduces the reference CPU
-// path up to the last bit of expf.  The fused kernels of et_yg_*.cu cover
-// the common gantry case; this path covers everything else.
+// path up to the last bit of expf.  A launch covers a group of cameras (their
+// matrices are launch parameters, the work volumes sit one after another), so
+// the per-ray scans of one camera -- a few thousand threads -- do not leave the
+// GPU idle.  The fused kernels of et_yg_*.cu cover the common gantry case;
+// this path covers everything else.
 #include "et_kernels.h"
 #include "et_profile.h"
+
+#include <algorithm>
+#include <type_traits>
 
 namespace nrgb {
 
@@ -30,48 +36,70 @@ __device__ __forceinline__ double flo(double v) { return floor(v); }
 __device__ __forceinline__ float ex(float v) { return expf(v); }
 __device__ __forceinline__ double ex(double v) { return exp(v); }
 
-// Trilinear resampling of one voxel, reg-lib/_reg_resampling.cpp:334-450
-// (positions from reg-lib/_reg_affineTransformation.cpp:116-132 with an
-// identity voxel-to-world matrix).  With bg != 0 every neighbour outside the
-// grid adds bg * xBasis[.] to a separate background weight, as the reference
-// does (:366-396).
+// Matrices of a group of cameras, a kernel parameter.
 template <class T>
-__device__ __forceinline__ T trilinear_ref(const T* __restrict__ src, int nx, int ny, int nz, const Affine34T<T>& A,
-                                           int x, int y, int z, T bg) {
-  const T fx = static_cast<T>(x), fy = static_cast<T>(y), fz = static_cast<T>(z);
-  T pos[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-    pos[i] = fa(fa(fa(fm(A.m[4 * i + 0], fx), fm(A.m[4 * i + 1], fy)), fm(A.m[4 * i + 2], fz)), A.m[4 * i + 3]);
+struct AffineSetT {
+  T m[kGeneralGroup][12];
+};
+
+// Footprint of one voxel: floor positions and the two weights per axis
+// (reg-lib/_reg_affineTransformation.cpp:116-132 with an identity
+// voxel-to-world matrix, reg-lib/_reg_resampling.cpp:334-364).
+template <class T>
+struct Foot {
   int prev[3];
   T b0[3], b1[3];
+};
+
+template <class T>
+__device__ __forceinline__ Foot<T> footprint(const T* m, int x, int y, int z) {
+  const T fx = static_cast<T>(x), fy = static_cast<T>(y), fz = static_cast<T>(z);
+  Foot<T> f;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    prev[i] = static_cast<int>(flo(pos[i]));
-    T rel = fs(pos[i], static_cast<T>(prev[i]));
+    const T pos = fa(fa(fa(fm(m[4 * i + 0], fx), fm(m[4 * i + 1], fy)), fm(m[4 * i + 2], fz)), m[4 * i + 3]);
+    f.prev[i] = static_cast<int>(flo(pos));
+    T rel = fs(pos, static_cast<T>(f.prev[i]));
     if (rel < T(0)) rel = T(0);
-    b0[i] = fs(T(1), rel);
-    b1[i] = rel;
+    f.b0[i] = fs(T(1), rel);
+    f.b1[i] = rel;
   }
-  const T bx[2] = {b0[0], b1[0]};
-  const T by[2] = {b0[1], b1[1]};
-  const T bz[2] = {b0[2], b1[2]};
+  return f;
+}
+
+// Trilinear value of a footprint, reg-lib/_reg_resampling.cpp:365-450.  With
+// bg != 0 every neighbour outside the grid adds bg * xBasis[.] to a separate
+// background weight, as the reference does (:366-396).  A footprint inside
+// the grid -- nearly all -- takes the same sums without the tests.
+template <class T>
+__device__ __forceinline__ T trilinear_ref(const T* __restrict__ src, int nx, int ny, int nz, const Foot<T>& f, T bg) {
+  const int px = f.prev[0], py = f.prev[1], pz = f.prev[2];
+  if (px >= 0 && px + 1 < nx && py >= 0 && py + 1 < ny && pz >= 0 && pz + 1 < nz) {
+    const T* p = src + (static_cast<size_t>(pz) * ny + py) * nx + px;
+    const T* q = p + static_cast<size_t>(ny) * nx;
+    auto line = [&](const T* r) { return fa(fm(__ldg(r), f.b0[0]), fm(__ldg(r + 1), f.b1[0])); };
+    auto plane = [&](const T* r) { return fa(fm(line(r), f.b0[1]), fm(line(r + nx), f.b1[1])); };
+    return fa(fm(plane(p), f.b0[2]), fm(plane(q), f.b1[2]));
+  }
+  const T bx[2] = {f.b0[0], f.b1[0]};
+  const T by[2] = {f.b0[1], f.b1[1]};
+  const T bz[2] = {f.b0[2], f.b1[2]};
   T val = T(0), bgw = T(0);
   const bool use_bg = (bg != T(0));
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
-    const int Z = prev[2] + c;
+    const int Z = pz + c;
     if (Z >= 0 && Z < nz) {
       T ysum = T(0);
 #pragma unroll
       for (int b = 0; b < 2; ++b) {
-        const int Y = prev[1] + b;
+        const int Y = py + b;
         if (Y >= 0 && Y < ny) {
           const T* row = src + (static_cast<size_t>(Z) * ny + Y) * nx;
           T xsum = T(0);
 #pragma unroll
           for (int a = 0; a < 2; ++a) {
-            const int X = prev[0] + a;
+            const int X = px + a;
             if (X >= 0 && X < nx)
               xsum = fa(xsum, fm(__ldg(row + X), bx[a]));
             else if (use_bg)
@@ -91,70 +119,85 @@ __device__ __forceinline__ T trilinear_ref(const T* __restrict__ src, int nx, in
   return val;
 }
 
-template <bool ACCUM, class T = float>
-__global__ void k_resample(const T* __restrict__ src, T* __restrict__ dst, int nx, int ny, int nz, Affine34T<T> A,
-                           T bg) {
+// Voxel of this thread in a launch of 32 x 8-voxel blocks over (x-tile,
+// y-tile, z, camera of the group); one set of 32-bit divisions per block.
+struct Voxel {
+  int x, y, z, g;
+};
+
+__device__ __forceinline__ Voxel block_voxel(int nx, int ny, int nz) {
+  const int tx = (nx + 31) / 32, ty = (ny + 7) / 8;
+  int b = blockIdx.x;
+  Voxel v;
+  v.x = b % tx * 32 + threadIdx.x;
+  b /= tx;
+  v.y = b % ty * 8 + threadIdx.y;
+  b /= ty;
+  v.z = b % nz;
+  v.g = b / nz;
+  return v;
+}
+
+// dst[g] = src resampled at the positions of camera g; with src2 the same for
+// a second volume (activity and mu share their footprints).
+template <class T>
+__global__ void __launch_bounds__(256)
+    k_resample(const T* __restrict__ src, T* __restrict__ dst, T bg, const T* __restrict__ src2, T* __restrict__ dst2,
+               T bg2, int nx, int ny, int nz, const __grid_constant__ AffineSetT<T> A) {
+  const Voxel v = block_voxel(nx, ny, nz);
+  if (v.x >= nx || v.y >= ny) return;
+  const Foot<T> f = footprint(A.m[v.g], v.x, v.y, v.z);
+  const size_t o = ((static_cast<size_t>(v.g) * nz + v.z) * ny + v.y) * nx + v.x;
+  if (src) dst[o] = trilinear_ref(src, nx, ny, nz, f, bg);
+  if (src2) dst2[o] = trilinear_ref(src2, nx, ny, nz, f, bg2);
+}
+
+// dst (+)= sum over the group's cameras, in camera order, of src[g] resampled
+// at camera g's positions; first: assign; clamp: store negative sums as zero.
+template <class T>
+__global__ void __launch_bounds__(256)
+    k_resample_sum(const T* __restrict__ src, T* __restrict__ dst, int n, int first, int clamp, T bg, int nx, int ny,
+                   int nz, const __grid_constant__ AffineSetT<T> A) {
+  const Voxel v = block_voxel(nx, ny, nz);
+  if (v.x >= nx || v.y >= ny) return;
   const size_t nvox = static_cast<size_t>(nx) * ny * nz;
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < nvox;
-       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const int x = static_cast<int>(i % nx);
-    const int y = static_cast<int>((i / nx) % ny);
-    const int z = static_cast<int>(i / (static_cast<size_t>(nx) * ny));
-    const T v = trilinear_ref<T>(src, nx, ny, nz, A, x, y, z, bg);
-    if (ACCUM)
-      dst[i] = fa(dst[i], v);
-    else
-      dst[i] = v;
-  }
+  const size_t o = (static_cast<size_t>(v.z) * ny + v.y) * nx + v.x;
+  T acc = first ? T(0) : dst[o];
+  for (int g = 0; g < n; ++g)
+    acc = fa(acc, trilinear_ref(src + nvox * g, nx, ny, nz, footprint(A.m[g], v.x, v.y, v.z), bg));
+  dst[o] = clamp && acc < T(0) ? T(0) : acc;
 }
 
 // Transpose of trilinear_ref with bg = 0: add v * weight to each in-grid
-// corner of the footprint of (x, y, z) (atomics: footprints overlap).
-__device__ __forceinline__ void trilinear_scatter(float* __restrict__ dst, int nx, int ny, int nz, const Affine34& A,
-                                                  int x, int y, int z, float v) {
-  const float fx = static_cast<float>(x), fy = static_cast<float>(y), fz = static_cast<float>(z);
-  int prev[3];
-  float b0[3], b1[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const float pos =
-        fa(fa(fa(fm(A.m[4 * i + 0], fx), fm(A.m[4 * i + 1], fy)), fm(A.m[4 * i + 2], fz)), A.m[4 * i + 3]);
-    prev[i] = static_cast<int>(floorf(pos));
-    float rel = __fsub_rn(pos, static_cast<float>(prev[i]));
-    if (rel < 0.0f) rel = 0.0f;
-    b0[i] = __fsub_rn(1.0f, rel);
-    b1[i] = rel;
-  }
+// corner of the footprint (atomics: footprints overlap).
+__device__ __forceinline__ void trilinear_scatter(float* __restrict__ dst, int nx, int ny, int nz,
+                                                  const Foot<float>& f, float v) {
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
-    const int Z = prev[2] + c;
+    const int Z = f.prev[2] + c;
     if (Z < 0 || Z >= nz) continue;
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
-      const int Y = prev[1] + b;
+      const int Y = f.prev[1] + b;
       if (Y < 0 || Y >= ny) continue;
 #pragma unroll
       for (int a = 0; a < 2; ++a) {
-        const int X = prev[0] + a;
+        const int X = f.prev[0] + a;
         if (X < 0 || X >= nx) continue;
-        const float w = (a ? b1[0] : b0[0]) * (b ? b1[1] : b0[1]) * (c ? b1[2] : b0[2]);
+        const float w = (a ? f.b1[0] : f.b0[0]) * (b ? f.b1[1] : f.b0[1]) * (c ? f.b1[2] : f.b0[2]);
         if (w != 0.0f) atomicAdd(dst + (static_cast<size_t>(Z) * ny + Y) * nx + X, v * w);
       }
     }
   }
 }
 
-__global__ void k_scatter(const float* __restrict__ src, float* __restrict__ dst, int nx, int ny, int nz, Affine34 A) {
-  const size_t nvox = static_cast<size_t>(nx) * ny * nz;
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < nvox;
-       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const float v = src[i];
-    if (v == 0.0f) continue;
-    const int x = static_cast<int>(i % nx);
-    const int y = static_cast<int>((i / nx) % ny);
-    const int z = static_cast<int>(i / (static_cast<size_t>(nx) * ny));
-    trilinear_scatter(dst, nx, ny, nz, A, x, y, z, v);
-  }
+__global__ void __launch_bounds__(256) k_scatter(const float* __restrict__ src, float* __restrict__ dst, int nx, int ny,
+                                                 int nz, const __grid_constant__ AffineSetT<float> A) {
+  const Voxel v = block_voxel(nx, ny, nz);
+  if (v.x >= nx || v.y >= ny) return;
+  const float s = src[((static_cast<size_t>(v.g) * nz + v.z) * ny + v.y) * nx + v.x];
+  if (s == 0.0f) return;
+  trilinear_scatter(dst, nx, ny, nz, footprint(A.m[v.g], v.x, v.y, v.z), s);
 }
 
 // Row (x) then column (y) pass of emission-lib/_et_convolveSeparable2D.cpp:13-40:
@@ -187,47 +230,141 @@ __global__ void k_conv(const T* __restrict__ in, T* __restrict__ out, int nx, in
   }
 }
 
-// Attenuated line integral along z, emission-lib/_et_line_integral_attenuated.cpp:14-68.
+// Both passes of one 32 x 32 tile of a plane through shared memory, PSF radius
+// R <= 7: the tile and its halo are read once (zeros outside the plane), a
+// thread then sums four consecutive outputs of a row, and of a column, from
+// 4 + 2R values.  Same products and order as k_conv<ROWS> then k_conv<columns>
+// (a zero outside the plane adds nothing), which read every tap from L1/L2 and
+// took two passes over the volume.  With FLIP both are correlations.
+// The row kernel index advances with the plane of the volume: plane z of
+// camera g of the group.
+template <int R, bool FLIP, class T>
+__global__ void __launch_bounds__(256)
+    k_conv2(const T* __restrict__ in, T* __restrict__ out, int nx, int ny, int nz, const T* __restrict__ sep) {
+  constexpr int K = 2 * R + 1, W = 32 + 2 * R, N = 4;
+  __shared__ T s_in[W][W + 1];
+  __shared__ T s_row[W][33];
+  const int tx = (nx + 31) / 32, ty = (ny + 31) / 32;
+  int b = blockIdx.x;
+  const int x0 = b % tx * 32;
+  b /= tx;
+  const int y0 = b % ty * 32;
+  b /= ty;  // plane of the group: camera * nz + z
+  const T* src = in + static_cast<size_t>(b) * ny * nx;
+  const T* k = sep + static_cast<size_t>(2 * K) * (b % nz);
+  for (int e = threadIdx.x; e < W * W; e += 256) {
+    const int r = e / W, c = e % W;
+    const int x = x0 - R + c, y = y0 - R + r;
+    s_in[r][c] = x >= 0 && x < nx && y >= 0 && y < ny ? __ldg(src + static_cast<size_t>(y) * nx + x) : T(0);
+  }
+  T kr[K], kc[K];
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    kr[j] = __ldg(k + (FLIP ? j : 2 * R - j));
+    kc[j] = __ldg(k + K + (FLIP ? j : 2 * R - j));
+  }
+  __syncthreads();
+  // a coefficient that is not finite must not meet the zeros outside the plane
+  bool finite = true;
+#pragma unroll
+  for (int j = 0; j < K; ++j) finite = finite && isfinite(kr[j]) && isfinite(kc[j]);
+  const int c = threadIdx.x % 32, r = threadIdx.x / 32 * N;
+  T s[N];
+  auto both = [&](auto check) {
+    constexpr bool CHECK = decltype(check)::value;
+    for (int e = threadIdx.x; e < W * (32 / N); e += 256) {
+      const int er = e % W, ec = e / W * N;
+#pragma unroll
+      for (int i = 0; i < N; ++i) s[i] = T(0);
+#pragma unroll
+      for (int j = 0; j < N + 2 * R; ++j) {
+        const T v = s_in[er][ec + j];
+        const int x = x0 - R + ec + j;
+        if (CHECK && (x < 0 || x >= nx)) continue;
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+          if (j - i >= 0 && j - i < K) s[i] = fa(s[i], fm(v, kr[j - i]));
+      }
+#pragma unroll
+      for (int i = 0; i < N; ++i) s_row[er][ec + i] = s[i];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < N; ++i) s[i] = T(0);
+#pragma unroll
+    for (int j = 0; j < N + 2 * R; ++j) {
+      const T v = s_row[r + j][c];
+      const int y = y0 - R + r + j;
+      if (CHECK && (y < 0 || y >= ny)) continue;
+#pragma unroll
+      for (int i = 0; i < N; ++i)
+        if (j - i >= 0 && j - i < K) s[i] = fa(s[i], fm(v, kc[j - i]));
+    }
+  };
+  if (finite) both(std::false_type());
+  else both(std::true_type());  // uniform over the block: one plane's coefficients
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (x0 + c < nx && y0 + r + i < ny)
+      out[(static_cast<size_t>(b) * ny + y0 + r + i) * nx + x0 + c] = s[i];
+}
+
+constexpr int kScanDepth = 8;  // depth planes whose loads a ray scan has in flight
+
+// Attenuated line integral along z, emission-lib/_et_line_integral_attenuated.cpp:14-68;
+// blockIdx.y: camera of the group.
 template <class R = float>
 __global__ void k_line_integral(const R* __restrict__ act, const R* __restrict__ att, R* __restrict__ out, int nx,
-                                int ny, int nz, R bg) {
-  const int nxy = nx * ny;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+                                int ny, int nz, R bg, int truncate) {
+  const size_t nxy = static_cast<size_t>(nx) * ny;
+  const size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   if (i >= nxy) return;
+  const size_t vol = nxy * nz * blockIdx.y;
+  if (act) act += vol + i;
+  if (att) att += vol + i;
   R p = R(0), T = R(0);
-  if (act && att) {
-    for (int z = 0; z < nz; ++z) {
-      T = fa(T, __ldg(att + static_cast<size_t>(z) * nxy + i));
-      p = fa(p, fm(__ldg(act + static_cast<size_t>(z) * nxy + i), ex(-T)));
+  for (int z0 = 0; z0 < nz; z0 += kScanDepth) {
+    R a[kScanDepth], m[kScanDepth];
+#pragma unroll
+    for (int d = 0; d < kScanDepth; ++d) {
+      const bool in = z0 + d < nz;
+      a[d] = act && in ? __ldg(act + nxy * (z0 + d)) : R(0);
+      m[d] = att && in ? __ldg(att + nxy * (z0 + d)) : R(0);
     }
-    p = fa(p, fm(bg, ex(-T)));
-  } else if (act) {
-    for (int z = 0; z < nz; ++z) p = fa(p, __ldg(act + static_cast<size_t>(z) * nxy + i));
-    p = fa(p, bg);
-  } else {
-    for (int z = 0; z < nz; ++z) T = fa(T, __ldg(att + static_cast<size_t>(z) * nxy + i));
-    p = fm(bg, ex(-T));
+#pragma unroll
+    for (int d = 0; d < kScanDepth; ++d) {
+      if (z0 + d >= nz) break;
+      if (att) T = fa(T, m[d]);
+      if (act) p = fa(p, att ? fm(a[d], ex(-T)) : a[d]);
+    }
   }
-  out[i] = p;
+  if (act && att) p = fa(p, fm(bg, ex(-T)));
+  else if (act) p = fa(p, bg);
+  else p = fm(bg, ex(-T));
+  if (truncate && p < R(0)) p = R(0);
+  out[nxy * blockIdx.y + i] = p;
 }
 
 // Spread along z, emission-lib/_et_line_backproject_attenuated.cpp:17-36 and
-// emission-lib/_et_line_backproject.cpp:17-30.
+// emission-lib/_et_line_backproject.cpp:17-30; blockIdx.y: camera of the group.
 template <class R = float>
 __global__ void k_spread(const R* __restrict__ plane, const R* __restrict__ att, R* __restrict__ vol, int nx, int ny,
                          int nz) {
-  const int nxy = nx * ny;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t nxy = static_cast<size_t>(nx) * ny;
+  const size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   if (i >= nxy) return;
-  const R s = __ldg(plane + i);
+  const size_t off = nxy * nz * blockIdx.y + i;
+  const R s = __ldg(plane + nxy * blockIdx.y + i);
   R T = R(0);
-  for (int z = 0; z < nz; ++z) {
-    const size_t j = static_cast<size_t>(z) * nxy + i;
-    if (att) {
-      T = fa(T, __ldg(att + j));
-      vol[j] = fm(s, ex(-T));
-    } else {
-      vol[j] = s;
+  for (int z0 = 0; z0 < nz; z0 += kScanDepth) {
+    R m[kScanDepth];
+#pragma unroll
+    for (int d = 0; d < kScanDepth; ++d) m[d] = att && z0 + d < nz ? __ldg(att + off + nxy * (z0 + d)) : R(0);
+#pragma unroll
+    for (int d = 0; d < kScanDepth; ++d) {
+      if (z0 + d >= nz) break;
+      T = fa(T, m[d]);
+      vol[off + nxy * (z0 + d)] = att ? fm(s, ex(-T)) : s;
     }
   }
 }
@@ -243,6 +380,11 @@ __global__ void k_line_partial(const float* __restrict__ act, const float* __res
   const int nxy = nx * ny;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nxy) return;
+  const size_t off = static_cast<size_t>(nxy) * nz * blockIdx.y, off2 = static_cast<size_t>(nxy) * blockIdx.y;
+  if (act) act += off;
+  if (att) att += off;
+  partial += off;
+  out += off2;
   float s = bg;
   if (bg_image) s = fm(s, __ldg(bg_image + i));
   for (int z = nz - 1; z >= 0; --z) {
@@ -258,13 +400,6 @@ __global__ void k_line_partial(const float* __restrict__ act, const float* __res
   out[i] = s;
 }
 
-template <class R>
-__global__ void k_truncate_t(R* __restrict__ buf, size_t n) {
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<size_t>(gridDim.x) * blockDim.x)
-    if (buf[i] < R(0)) buf[i] = R(0);
-}
-
 // Attenuation-gradient scan, emission-lib_gpu/_et_attenuation_gradient_gpu_kernels.cu:24-39:
 // pass 1 stores the inclusive prefix T_z, pass 2 (far to near) accumulates
 // a_z * exp(-T_z) and stores s * acc.
@@ -273,6 +408,11 @@ __global__ void k_grad_scan(const float* __restrict__ act, const float* __restri
   const int nxy = nx * ny;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nxy) return;
+  const size_t off = static_cast<size_t>(nxy) * nz * blockIdx.y, off2 = static_cast<size_t>(nxy) * blockIdx.y;
+  if (act) act += off;
+  if (att) att += off;
+  vol += off;
+  plane += off2;
   float T = 0.0f;
   for (int z = 0; z < nz; ++z) {
     const size_t j = static_cast<size_t>(z) * nxy + i;
@@ -300,6 +440,11 @@ __global__ void k_dmu_scan(const float* __restrict__ v, const float* __restrict_
   const int nxy = nx * ny;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nxy) return;
+  const size_t off = static_cast<size_t>(nxy) * nz * blockIdx.y, off2 = static_cast<size_t>(nxy) * blockIdx.y;
+  v += off;
+  m += off;
+  out += off;
+  g_plane += off2;
   float T = 0.0f, Pv = 0.0f;
   for (int z = 0; z < nz; ++z) {
     const size_t j = static_cast<size_t>(z) * nxy + i;
@@ -325,67 +470,129 @@ int grid_for(size_t n, int block) {
   return static_cast<int>(g < cap ? g : cap);
 }
 
+// Launches of one call's stages over groups of cameras.
 template <class T>
-Affine34T<T> affine_of(const T* m12) {
-  Affine34T<T> a;
-  for (int i = 0; i < 12; ++i) a.m[i] = m12[i];
-  return a;
-}
+struct General {
+  const GeneralArgsT<T>& a;
+  cudaStream_t st;
+  size_t nvox, nxy;
+  int cam0 = 0, n = 0;  // the current group
 
-template <class T>
-void launch_truncate_t(T* buf, size_t n, cudaStream_t st) {
-  NRGB_LAUNCH_SCOPE("k_truncate", st);
-  k_truncate_t<T><<<grid_for(n, 256), 256, 0, st>>>(buf, n);
-}
+  General(const GeneralArgsT<T>& args, cudaStream_t stream) : a(args), st(stream) {
+    nxy = static_cast<size_t>(a.nx) * a.ny;
+    nvox = nxy * a.nz;
+  }
+
+  template <class Body>
+  int groups(Body body) {
+    const int group = std::max(1, std::min(a.group, kGeneralGroup));
+    for (cam0 = 0; cam0 < a.ncam; cam0 += group) {
+      n = std::min(group, a.ncam - cam0);
+      body();
+    }
+    return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
+  }
+
+  bool last() const { return cam0 + n == a.ncam; }
+
+  AffineSetT<T> matrices(bool back) const {
+    AffineSetT<T> s = {};
+    for (int g = 0; g < n; ++g) {
+      const T* m = back ? a.geom_host[cam0 + g].bwd : a.geom_host[cam0 + g].fwd;
+      std::copy(m, m + 12, s.m[g]);
+    }
+    return s;
+  }
+
+  // blocks of 32 x rows voxels over `volumes` volumes
+  unsigned blocks(int rows, int volumes) const {
+    return static_cast<unsigned>((a.nx + 31) / 32) * ((a.ny + rows - 1) / rows) * a.nz * volumes;
+  }
+  dim3 rays() const { return dim3(static_cast<unsigned>((nxy + 127) / 128), n); }
+
+  // rotate one or two volumes (either may be null) into work volumes
+  void rotate(const T* src, T* dst, T bg, const T* src2, T* dst2, T bg2) {
+    if (!src && !src2) return;
+    NRGB_LAUNCH_SCOPE("k_resample", st);
+    k_resample<T><<<blocks(8, n), dim3(32, 8), 0, st>>>(src, dst, bg, src2, dst2, bg2, a.nx, a.ny, a.nz,
+                                                        matrices(false));
+  }
+
+  // PSF of the group's volumes; returns where the result is (tmp, or vol for
+  // radii beyond the fused kernel, whose two passes go through tmp)
+  template <bool FLIP = false>
+  T* convolve(T* vol, T* tmp) {
+    if (!a.psf_sep) return vol;
+    auto go = [&](auto k) {
+      NRGB_LAUNCH_SCOPE("k_conv2", st);
+      k<<<blocks(32, n), 256, 0, st>>>(vol, tmp, a.nx, a.ny, a.nz, a.psf_sep);
+    };
+    switch ((a.psf_k - 1) / 2) {
+      case 0: go(k_conv2<0, FLIP, T>); return tmp;
+      case 1: go(k_conv2<1, FLIP, T>); return tmp;
+      case 2: go(k_conv2<2, FLIP, T>); return tmp;
+      case 3: go(k_conv2<3, FLIP, T>); return tmp;
+      case 4: go(k_conv2<4, FLIP, T>); return tmp;
+      case 5: go(k_conv2<5, FLIP, T>); return tmp;
+      case 6: go(k_conv2<6, FLIP, T>); return tmp;
+      case 7: go(k_conv2<7, FLIP, T>); return tmp;
+      default: break;
+    }
+    for (int g = 0; g < n; ++g) {
+      T *v = vol + nvox * g, *t = tmp + nvox * g;
+      NRGB_LAUNCH_SCOPE("k_conv", st);
+      k_conv<true, FLIP, T><<<grid_for(nvox, 256), 256, 0, st>>>(v, t, a.nx, a.ny, a.nz, a.psf_sep, a.psf_k);
+      k_conv<false, FLIP, T><<<grid_for(nvox, 256), 256, 0, st>>>(t, v, a.nx, a.ny, a.nz, a.psf_sep, a.psf_k);
+    }
+    return vol;
+  }
+
+  void spread(const T* att, T* vol) {
+    NRGB_LAUNCH_SCOPE("k_spread", st);
+    k_spread<T><<<rays(), 128, 0, st>>>(a.sino + nxy * cam0, att, vol, a.nx, a.ny, a.nz);
+  }
+
+  // rotate the group's volumes back and add them to the output
+  void gather(const T* src, T bg) {
+    NRGB_LAUNCH_SCOPE("k_resample_sum", st);
+    k_resample_sum<T><<<blocks(8, 1), dim3(32, 8), 0, st>>>(src, a.out, n, cam0 == 0, a.truncate && last(), bg, a.nx,
+                                                            a.ny, a.nz, matrices(true));
+  }
+};
 
 // et_project (emission-lib/_et.cpp:218-281): per camera rotate activity and
-// mu, PSF, attenuated line integral; truncation at the end (:283-292).
+// mu, PSF, attenuated line integral, truncation (:283-292).
 template <class T>
 int general_project_t(const GeneralArgsT<T>& a, cudaStream_t st) {
-  const int nx = a.nx, ny = a.ny, nz = a.nz;
-  const size_t nvox = static_cast<size_t>(nx) * ny * nz, nxy = static_cast<size_t>(nx) * ny;
-  const int B = 256;
-  for (int cam = 0; cam < a.ncam; ++cam) {
-    const Affine34T<T> F = affine_of<T>(a.geom_host[cam].fwd);
-    if (a.act) { NRGB_LAUNCH_SCOPE("k_resample", st); k_resample<false, T><<<grid_for(nvox, B), B, 0, st>>>(a.act, a.ws_act, nx, ny, nz, F, a.bg); }
-    if (a.att) { NRGB_LAUNCH_SCOPE("k_resample", st); k_resample<false, T><<<grid_for(nvox, B), B, 0, st>>>(a.att, a.ws_att, nx, ny, nz, F, a.bg_att); }
-    if (a.psf_sep && a.act) {
-      { NRGB_LAUNCH_SCOPE("k_conv", st); k_conv<true, false, T><<<grid_for(nvox, B), B, 0, st>>>(a.ws_act, a.ws_tmp, nx, ny, nz, a.psf_sep, a.psf_k); }
-      { NRGB_LAUNCH_SCOPE("k_conv", st); k_conv<false, false, T><<<grid_for(nvox, B), B, 0, st>>>(a.ws_tmp, a.ws_act, nx, ny, nz, a.psf_sep, a.psf_k); }
-    }
-    { NRGB_LAUNCH_SCOPE("k_line_integral", st); k_line_integral<T><<<static_cast<int>((nxy + B - 1) / B), B, 0, st>>>(a.act ? a.ws_act : nullptr,
-                                                                      a.att ? a.ws_att : nullptr,
-                                                                      a.out + nxy * cam, nx, ny, nz, a.bg); }
-  }
-  if (a.truncate) launch_truncate_t<T>(a.out, nxy * a.ncam, st);
-  return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
+  General<T> p(a, st);
+  return p.groups([&] {
+    p.rotate(a.act, a.ws_act, a.bg, a.att, a.ws_att, a.bg_att);
+    const T* v = a.act ? p.convolve(a.ws_act, a.ws_tmp) : nullptr;
+    NRGB_LAUNCH_SCOPE("k_line_integral", st);
+    k_line_integral<T><<<p.rays(), 128, 0, st>>>(v, a.att ? a.ws_att : nullptr, a.out + p.nxy * p.cam0, a.nx, a.ny,
+                                                 a.nz, a.bg, a.truncate);
+  });
 }
 
 // et_backproject (emission-lib/_et.cpp:415-499): per camera rotate mu, spread
 // the attenuated plane, PSF, rotate back with the inverse matrix, accumulate.
 template <class T>
 int general_backproject_t(const GeneralArgsT<T>& a, cudaStream_t st) {
-  const int nx = a.nx, ny = a.ny, nz = a.nz;
-  const size_t nvox = static_cast<size_t>(nx) * ny * nz, nxy = static_cast<size_t>(nx) * ny;
-  const int B = 256;
-  cudaMemsetAsync(a.out, 0, nvox * sizeof(T), st);
-  for (int cam = 0; cam < a.ncam; ++cam) {
-    const Affine34T<T> F = affine_of<T>(a.geom_host[cam].fwd);
-    const Affine34T<T> Bk = affine_of<T>(a.geom_host[cam].bwd);
-    if (a.att) { NRGB_LAUNCH_SCOPE("k_resample", st); k_resample<false, T><<<grid_for(nvox, B), B, 0, st>>>(a.att, a.ws_att, nx, ny, nz, F, a.bg_att); }
-    { NRGB_LAUNCH_SCOPE("k_spread", st); k_spread<T><<<static_cast<int>((nxy + B - 1) / B), B, 0, st>>>(a.sino + nxy * cam, a.att ? a.ws_att : nullptr,
-                                                               a.ws_act, nx, ny, nz); }
-    if (a.psf_sep) {
-      { NRGB_LAUNCH_SCOPE("k_conv", st); k_conv<true, false, T><<<grid_for(nvox, B), B, 0, st>>>(a.ws_act, a.ws_tmp, nx, ny, nz, a.psf_sep, a.psf_k); }
-      { NRGB_LAUNCH_SCOPE("k_conv", st); k_conv<false, false, T><<<grid_for(nvox, B), B, 0, st>>>(a.ws_tmp, a.ws_act, nx, ny, nz, a.psf_sep, a.psf_k); }
-    }
-    { NRGB_LAUNCH_SCOPE("k_resample", st); k_resample<true, T><<<grid_for(nvox, B), B, 0, st>>>(a.ws_act, a.out, nx, ny, nz, Bk, a.bg); }
-  }
-  if (a.truncate) launch_truncate_t<T>(a.out, nvox, st);
-  return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
+  General<T> p(a, st);
+  return p.groups([&] {
+    p.rotate(nullptr, nullptr, T(0), a.att, a.ws_att, a.bg_att);
+    p.spread(a.att ? a.ws_att : nullptr, a.ws_act);
+    p.gather(p.convolve(a.ws_act, a.ws_tmp), a.bg);
+  });
 }
 
 }  // namespace
+
+int general_group(size_t nvox, size_t element, int ncam) {
+  const size_t most = kGeneralScratch / (3 * element * std::max<size_t>(nvox, 1));
+  return static_cast<int>(std::max<size_t>(1, std::min<size_t>({most, static_cast<size_t>(kGeneralGroup),
+                                                                static_cast<size_t>(std::max(1, ncam))})));
+}
 
 // et_project_partial_gpu (emission-lib/_et.cpp:2106-2436): per camera rotate
 // activity (bg) and mu (bg_att), PSF, partial-sum line integral; with
@@ -393,32 +600,28 @@ int general_backproject_t(const GeneralArgsT<T>& a, cudaStream_t st) {
 // (-theta, ZYX, background bg, :2373-2404).  partial: [ncam][nz][ny][nx].
 int general_project_partial(const GeneralArgs& a, const float* bg_image, float* partial, int do_rotate,
                             cudaStream_t st) {
-  const int nx = a.nx, ny = a.ny, nz = a.nz;
-  const size_t nvox = static_cast<size_t>(nx) * ny * nz, nxy = static_cast<size_t>(nx) * ny;
-  const int B = 256;
-  for (int cam = 0; cam < a.ncam; ++cam) {
-    const Affine34 F = affine_of(a.geom_host[cam].fwd);
-    if (a.act) { NRGB_LAUNCH_SCOPE("k_resample", st); k_resample<false><<<grid_for(nvox, B), B, 0, st>>>(a.act, a.ws_act, nx, ny, nz, F, a.bg); }
-    if (a.att) { NRGB_LAUNCH_SCOPE("k_resample", st); k_resample<false><<<grid_for(nvox, B), B, 0, st>>>(a.att, a.ws_att, nx, ny, nz, F, a.bg_att); }
-    if (a.psf_sep && a.act) {
-      { NRGB_LAUNCH_SCOPE("k_conv", st); k_conv<true><<<grid_for(nvox, B), B, 0, st>>>(a.ws_act, a.ws_tmp, nx, ny, nz, a.psf_sep, a.psf_k); }
-      { NRGB_LAUNCH_SCOPE("k_conv", st); k_conv<false><<<grid_for(nvox, B), B, 0, st>>>(a.ws_tmp, a.ws_act, nx, ny, nz, a.psf_sep, a.psf_k); }
-    }
-    float* dst = partial + nvox * cam;
+  General<float> p(a, st);
+  const int s = p.groups([&] {
+    p.rotate(a.act, a.ws_act, a.bg, a.att, a.ws_att, a.bg_att);
+    const float* v = a.act ? p.convolve(a.ws_act, a.ws_tmp) : nullptr;
+    float* dst = partial + p.nvox * p.cam0;
+    // the sums to rotate back go where the scan no longer reads
+    float* sums = v == a.ws_tmp ? a.ws_act : a.ws_tmp;
     {
       NRGB_LAUNCH_SCOPE("k_line_partial", st);
-      k_line_partial<<<static_cast<int>((nxy + B - 1) / B), B, 0, st>>>(
-          a.act ? a.ws_act : nullptr, a.att ? a.ws_att : nullptr, bg_image, a.out + nxy * cam,
-          do_rotate ? a.ws_tmp : dst, nx, ny, nz, a.bg);
+      k_line_partial<<<p.rays(), 128, 0, st>>>(v, a.att ? a.ws_att : nullptr, bg_image, a.out + p.nxy * p.cam0,
+                                               do_rotate ? sums : dst, a.nx, a.ny, a.nz, a.bg);
     }
-    if (do_rotate) {
+    for (int g = 0; do_rotate && g < p.n; ++g) {
+      AffineSetT<float> m = {};
+      std::copy(a.geom_host[p.cam0 + g].bwd, a.geom_host[p.cam0 + g].bwd + 12, m.m[0]);
       NRGB_LAUNCH_SCOPE("k_resample", st);
-      k_resample<false><<<grid_for(nvox, B), B, 0, st>>>(a.ws_tmp, dst, nx, ny, nz, affine_of(a.geom_host[cam].bwd),
-                                                          a.bg);
+      k_resample<float><<<p.blocks(8, 1), dim3(32, 8), 0, st>>>(sums + p.nvox * g, dst + p.nvox * g, a.bg, nullptr,
+                                                                nullptr, 0.0f, a.nx, a.ny, a.nz, m);
     }
-  }
-  if (a.truncate) launch_truncate_t<float>(a.out, nxy * a.ncam, st);
-  return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
+  });
+  if (s == kOk && a.truncate) launch_truncate(a.out, p.nxy * a.ncam, st);
+  return cudaGetLastError() == cudaSuccess ? s : kErrKernel;
 }
 
 int general_project(const GeneralArgs& a, cudaStream_t st) { return general_project_t<float>(a, st); }
@@ -426,70 +629,56 @@ int general_backproject(const GeneralArgs& a, cudaStream_t st) { return general_
 int general_project64(const GeneralArgs64& a, cudaStream_t st) { return general_project_t<double>(a, st); }
 int general_backproject64(const GeneralArgs64& a, cudaStream_t st) { return general_backproject_t<double>(a, st); }
 
+namespace {
+
+void scatter(const General<float>& p, const float* src) {
+  NRGB_LAUNCH_SCOPE("k_scatter", p.st);
+  k_scatter<<<p.blocks(8, p.n), dim3(32, 8), 0, p.st>>>(src, p.a.out, p.a.nx, p.a.ny, p.a.nz, p.matrices(false));
+}
+
+}  // namespace
+
 // Exact transpose of general_project for fixed mu (bg terms dropped: the
 // transpose of the projector's linear part): spread, transposed PSF
-// (correlation, column pass first), transposed trilinear scatter.
+// (correlation), transposed trilinear scatter.
 int general_adjoint(const GeneralArgs& a, cudaStream_t st) {
-  const int nx = a.nx, ny = a.ny, nz = a.nz;
-  const size_t nvox = static_cast<size_t>(nx) * ny * nz, nxy = static_cast<size_t>(nx) * ny;
-  const int B = 256;
-  cudaMemsetAsync(a.out, 0, nvox * sizeof(float), st);
-  for (int cam = 0; cam < a.ncam; ++cam) {
-    const Affine34 F = affine_of(a.geom_host[cam].fwd);
-    if (a.att) { NRGB_LAUNCH_SCOPE("k_resample", st); k_resample<false><<<grid_for(nvox, B), B, 0, st>>>(a.att, a.ws_att, nx, ny, nz, F, a.bg_att); }
-    { NRGB_LAUNCH_SCOPE("k_spread", st); k_spread<<<static_cast<int>((nxy + B - 1) / B), B, 0, st>>>(a.sino + nxy * cam, a.att ? a.ws_att : nullptr,
-                                                               a.ws_act, nx, ny, nz); }
-    if (a.psf_sep) {
-      { NRGB_LAUNCH_SCOPE("k_conv", st); k_conv<false, true><<<grid_for(nvox, B), B, 0, st>>>(a.ws_act, a.ws_tmp, nx, ny, nz, a.psf_sep, a.psf_k); }
-      { NRGB_LAUNCH_SCOPE("k_conv", st); k_conv<true, true><<<grid_for(nvox, B), B, 0, st>>>(a.ws_tmp, a.ws_act, nx, ny, nz, a.psf_sep, a.psf_k); }
-    }
-    { NRGB_LAUNCH_SCOPE("k_scatter", st); k_scatter<<<grid_for(nvox, B), B, 0, st>>>(a.ws_act, a.out, nx, ny, nz, F); }
-  }
-  return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
+  General<float> p(a, st);
+  cudaMemsetAsync(a.out, 0, p.nvox * sizeof(float), st);
+  return p.groups([&] {
+    p.rotate(nullptr, nullptr, 0.0f, a.att, a.ws_att, a.bg_att);
+    p.spread(a.att ? a.ws_att : nullptr, a.ws_act);
+    scatter(p, p.convolve<true>(a.ws_act, a.ws_tmp));
+  });
 }
 
 // Gradient of sum(g * project(act, mu)) with respect to mu (a.sino = g),
 // into a.out.  Per camera: rotate activity and mu, PSF on the activity,
 // k_dmu_scan, transposed trilinear scatter of the rotated-frame gradient.
 int general_dmu(const GeneralArgs& a, cudaStream_t st) {
-  const int nx = a.nx, ny = a.ny, nz = a.nz;
-  const size_t nvox = static_cast<size_t>(nx) * ny * nz, nxy = static_cast<size_t>(nx) * ny;
-  const int B = 256;
-  cudaMemsetAsync(a.out, 0, nvox * sizeof(float), st);
-  for (int cam = 0; cam < a.ncam; ++cam) {
-    const Affine34 F = affine_of(a.geom_host[cam].fwd);
-    { NRGB_LAUNCH_SCOPE("k_resample", st); k_resample<false><<<grid_for(nvox, B), B, 0, st>>>(a.act, a.ws_act, nx, ny, nz, F, a.bg); }
-    { NRGB_LAUNCH_SCOPE("k_resample", st); k_resample<false><<<grid_for(nvox, B), B, 0, st>>>(a.att, a.ws_att, nx, ny, nz, F, a.bg_att); }
-    if (a.psf_sep) {
-      { NRGB_LAUNCH_SCOPE("k_conv", st); k_conv<true><<<grid_for(nvox, B), B, 0, st>>>(a.ws_act, a.ws_tmp, nx, ny, nz, a.psf_sep, a.psf_k); }
-      { NRGB_LAUNCH_SCOPE("k_conv", st); k_conv<false><<<grid_for(nvox, B), B, 0, st>>>(a.ws_tmp, a.ws_act, nx, ny, nz, a.psf_sep, a.psf_k); }
+  General<float> p(a, st);
+  cudaMemsetAsync(a.out, 0, p.nvox * sizeof(float), st);
+  return p.groups([&] {
+    p.rotate(a.act, a.ws_act, a.bg, a.att, a.ws_att, a.bg_att);
+    const float* v = p.convolve(a.ws_act, a.ws_tmp);
+    float* d = v == a.ws_tmp ? a.ws_act : a.ws_tmp;
+    {
+      NRGB_LAUNCH_SCOPE("k_dmu_scan", st);
+      k_dmu_scan<<<p.rays(), 128, 0, st>>>(v, a.ws_att, a.sino + p.nxy * p.cam0, d, a.nx, a.ny, a.nz, a.bg);
     }
-    { NRGB_LAUNCH_SCOPE("k_dmu_scan", st); k_dmu_scan<<<static_cast<int>((nxy + B - 1) / B), B, 0, st>>>(a.ws_act, a.ws_att, a.sino + nxy * cam, a.ws_tmp, nx, ny, nz, a.bg); }
-    { NRGB_LAUNCH_SCOPE("k_scatter", st); k_scatter<<<grid_for(nvox, B), B, 0, st>>>(a.ws_tmp, a.out, nx, ny, nz, F); }
-  }
-  return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
+    scatter(p, d);
+  });
 }
 
 int general_gradient(const GeneralArgs& a, cudaStream_t st) {
-  const int nx = a.nx, ny = a.ny, nz = a.nz;
-  const size_t nvox = static_cast<size_t>(nx) * ny * nz, nxy = static_cast<size_t>(nx) * ny;
-  const int B = 256;
-  cudaMemsetAsync(a.out, 0, nvox * sizeof(float), st);
-  for (int cam = 0; cam < a.ncam; ++cam) {
-    const Affine34 F = affine_of(a.geom_host[cam].fwd);
-    const Affine34 Bk = affine_of(a.geom_host[cam].bwd);
-    { NRGB_LAUNCH_SCOPE("k_resample", st); k_resample<false><<<grid_for(nvox, B), B, 0, st>>>(a.att, a.ws_att, nx, ny, nz, F, a.bg_att); }
-    { NRGB_LAUNCH_SCOPE("k_resample", st); k_resample<false><<<grid_for(nvox, B), B, 0, st>>>(a.act, a.ws_act, nx, ny, nz, F, a.bg); }
-    { NRGB_LAUNCH_SCOPE("k_grad_scan", st); k_grad_scan<<<static_cast<int>((nxy + B - 1) / B), B, 0, st>>>(a.ws_act, a.ws_att, a.sino + nxy * cam,
-                                                                  a.ws_tmp, nx, ny, nz); }
-    if (a.psf_sep) {
-      { NRGB_LAUNCH_SCOPE("k_conv", st); k_conv<true><<<grid_for(nvox, B), B, 0, st>>>(a.ws_tmp, a.ws_act, nx, ny, nz, a.psf_sep, a.psf_k); }
-      { NRGB_LAUNCH_SCOPE("k_conv", st); k_conv<false><<<grid_for(nvox, B), B, 0, st>>>(a.ws_act, a.ws_tmp, nx, ny, nz, a.psf_sep, a.psf_k); }
+  General<float> p(a, st);
+  return p.groups([&] {
+    p.rotate(a.act, a.ws_act, a.bg, a.att, a.ws_att, a.bg_att);
+    {
+      NRGB_LAUNCH_SCOPE("k_grad_scan", st);
+      k_grad_scan<<<p.rays(), 128, 0, st>>>(a.ws_act, a.ws_att, a.sino + p.nxy * p.cam0, a.ws_tmp, a.nx, a.ny, a.nz);
     }
-    { NRGB_LAUNCH_SCOPE("k_resample", st); k_resample<true><<<grid_for(nvox, B), B, 0, st>>>(a.ws_tmp, a.out, nx, ny, nz, Bk, a.bg); }
-  }
-  if (a.truncate) launch_truncate(a.out, nvox, st);
-  return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
+    p.gather(p.convolve(a.ws_tmp, a.ws_act), a.bg);
+  });
 }
 
 namespace {
@@ -528,8 +717,15 @@ int general_convolve2d(const float* src, float* dst, int nx, int ny, int nz, con
 }
 
 int general_rotate(const float* src, float* dst, int nx, int ny, int nz, const float* m12, float bg, cudaStream_t st) {
-  const size_t nvox = static_cast<size_t>(nx) * ny * nz;
-  { NRGB_LAUNCH_SCOPE("k_resample", st); k_resample<false><<<grid_for(nvox, 256), 256, 0, st>>>(src, dst, nx, ny, nz, affine_of(m12), bg); }
+  GeneralArgs a;
+  a.nx = nx;
+  a.ny = ny;
+  a.nz = nz;
+  AffineSetT<float> m = {};
+  std::copy(m12, m12 + 12, m.m[0]);
+  NRGB_LAUNCH_SCOPE("k_resample", st);
+  k_resample<float><<<General<float>(a, st).blocks(8, 1), dim3(32, 8), 0, st>>>(src, dst, bg, nullptr, nullptr, 0.0f,
+                                                                                nx, ny, nz, m);
   return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
 }
 

@@ -21,10 +21,17 @@ struct GeneralArgsT {
   int psf_k = 0;
   T bg = 0, bg_att = 0;
   int truncate = 0;
-  T* ws_act = nullptr;  // three nvox work volumes
+  int group = 1;        // cameras per launch (at most kGeneralGroup)
+  T* ws_act = nullptr;  // three sets of `group` nvox work volumes
   T* ws_att = nullptr;
   T* ws_tmp = nullptr;
 };
+// Cameras per launch of the general path: as many as kGeneralGroup (their
+// matrices are launch parameters) while the three sets of work volumes stay
+// within kGeneralScratch bytes; at least one.
+constexpr int kGeneralGroup = 8;
+constexpr size_t kGeneralScratch = static_cast<size_t>(256) << 20;
+int general_group(size_t nvox, size_t element, int ncam);
 using GeneralArgs = GeneralArgsT<float>;
 // The same projector / backprojector evaluated in float64 (every product,
 // sum, position and exp in double): the float64 reference run that the

@@ -130,7 +130,9 @@ int plan_project(Plan& p, int subset, const float* d_act, float* d_sino, int lay
   g.bg = pb.bg;
   g.bg_att = pb.bg_att;
   g.truncate = truncate;
-  const size_t nv = static_cast<size_t>(pb.nx) * pb.ny * pb.nz;
+  size_t nv = static_cast<size_t>(pb.nx) * pb.ny * pb.nz;
+  g.group = general_group(nv, sizeof(float), pb.cams.n);
+  nv *= g.group;
   g.ws_act = p.work;
   g.ws_att = p.work + nv;
   g.ws_tmp = p.work + 2 * nv;
@@ -193,7 +195,9 @@ int plan_backproject(Plan& p, int subset, const float* d_sino, float* d_out, int
   g.bg = pb.bg;
   g.bg_att = pb.bg_att;
   g.truncate = truncate;
-  const size_t nv = static_cast<size_t>(pb.nx) * pb.ny * pb.nz;
+  size_t nv = static_cast<size_t>(pb.nx) * pb.ny * pb.nz;
+  g.group = general_group(nv, sizeof(float), pb.cams.n);
+  nv *= g.group;
   g.ws_act = p.work;
   g.ws_att = p.work + nv;
   g.ws_tmp = p.work + 2 * nv;
@@ -308,7 +312,7 @@ int nrgb_plan_create(void** out_plan, const int* size, const float* cameras, con
                     sizeof(float) * static_cast<size_t>(ncam) * yg_carry_slabs() * nx * p->cy;
   } else {
     bytes += al(sizeof(float) * nv) * (p->has_att ? 1 : 0);
-    p->work_bytes = sizeof(float) * nv * 3;
+    p->work_bytes = sizeof(float) * nv * 3 * general_group(nv, sizeof(float), ncam);
   }
   bytes += al(p->work_bytes);
   if (cudaMalloc(&p->mem, bytes) != cudaSuccess) {
