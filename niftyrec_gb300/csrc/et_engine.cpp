@@ -202,20 +202,17 @@ int upload_common(const Problem& pb, Carver& cv, CamGeom** d_geom, float** d_psf
   const std::vector<CamGeom>& geom = engine_x ? pb.geom_x : pb.geom;
   const std::vector<float>& psf_sep = engine_x ? pb.psf_sep_x : pb.psf_sep;
   const std::vector<int>& units = engine_x ? pb.units_x : pb.units;
-  *d_geom = cv.take<CamGeom>(pb.cams.n);
-  *d_psf = nullptr;
-  if (!*d_geom) return kErrAllocGpu;
-  if (pb.psf_k) {
-    *d_psf = cv.take<float>(psf_sep.size());
-    if (!*d_psf) return kErrAllocGpu;
-  }
-  const size_t ubytes = d_units ? sizeof(int) * units.size() : 0;
-  if (d_units) {
-    *d_units = nullptr;
-    if (ubytes && !(*d_units = cv.take<int2>(units.size() / 2))) return kErrAllocGpu;
-  }
+  // one region and one copy for all of them, each on a 256-byte boundary
+  auto al = [](size_t n) { return (n + 255) / 256 * 256; };
   const size_t gbytes = sizeof(CamGeom) * pb.cams.n;
   const size_t pbytes = sizeof(float) * psf_sep.size();
+  const size_t ubytes = d_units ? sizeof(int) * units.size() : 0;
+  const size_t poff = al(gbytes), uoff = poff + al(pbytes), total = uoff + al(ubytes);
+  char* d = cv.take<char>(total);
+  if (!d) return kErrAllocGpu;
+  *d_geom = reinterpret_cast<CamGeom*>(d);
+  *d_psf = pb.psf_k ? reinterpret_cast<float*>(d + poff) : nullptr;
+  if (d_units) *d_units = ubytes ? reinterpret_cast<int2*>(d + uoff) : nullptr;
   const int slot = stg->slot;
   stg->slot ^= 1;
   if (stg->done[slot]) {
@@ -223,11 +220,11 @@ int upload_common(const Problem& pb, Carver& cv, CamGeom** d_geom, float** d_psf
   } else if (cudaEventCreateWithFlags(&stg->done[slot], cudaEventDisableTiming) != cudaSuccess) {
     return kErrUnspecified;
   }
-  if (stg->bytes[slot] < gbytes + pbytes + ubytes) {
+  if (stg->bytes[slot] < total) {
     if (stg->pinned[slot]) cudaFreeHost(stg->pinned[slot]);
     stg->pinned[slot] = nullptr;
     stg->bytes[slot] = 0;
-    const size_t want = std::max(gbytes + pbytes + ubytes, static_cast<size_t>(1) << 20);
+    const size_t want = std::max(total, static_cast<size_t>(1) << 20);
     if (cudaMallocHost(&stg->pinned[slot], want) != cudaSuccess) {
       cudaGetLastError();
       return kErrAllocCpu;
@@ -236,15 +233,9 @@ int upload_common(const Problem& pb, Carver& cv, CamGeom** d_geom, float** d_psf
   }
   char* h = stg->pinned[slot];
   std::memcpy(h, geom.data(), gbytes);
-  if (pbytes) std::memcpy(h + gbytes, psf_sep.data(), pbytes);
-  if (cudaMemcpyAsync(*d_geom, h, gbytes, cudaMemcpyHostToDevice, st) != cudaSuccess) return kErrTransferGpu;
-  if (pbytes && cudaMemcpyAsync(*d_psf, h + gbytes, pbytes, cudaMemcpyHostToDevice, st) != cudaSuccess)
-    return kErrTransferGpu;
-  if (ubytes) {
-    std::memcpy(h + gbytes + pbytes, units.data(), ubytes);
-    if (cudaMemcpyAsync(*d_units, h + gbytes + pbytes, ubytes, cudaMemcpyHostToDevice, st) != cudaSuccess)
-      return kErrTransferGpu;
-  }
+  if (pbytes) std::memcpy(h + poff, psf_sep.data(), pbytes);
+  if (ubytes) std::memcpy(h + uoff, units.data(), ubytes);
+  if (cudaMemcpyAsync(d, h, uoff + ubytes, cudaMemcpyHostToDevice, st) != cudaSuccess) return kErrTransferGpu;
   cudaEventRecord(stg->done[slot], st);
   return kOk;
 }
