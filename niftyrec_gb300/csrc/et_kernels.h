@@ -28,9 +28,9 @@ struct GeneralArgsT {
 };
 // Cameras per launch of the general path: as many as kGeneralGroup (their
 // matrices are launch parameters) while the three sets of work volumes stay
-// within kGeneralScratch bytes; at least one.
+// within kGeneralScratch bytes, which stay in L2; at least one.
 constexpr int kGeneralGroup = 8;
-constexpr size_t kGeneralScratch = static_cast<size_t>(256) << 20;
+constexpr size_t kGeneralScratch = static_cast<size_t>(96) << 20;
 int general_group(size_t nvox, size_t element, int ncam);
 using GeneralArgs = GeneralArgsT<float>;
 // The same projector / backprojector evaluated in float64 (every product,
@@ -92,9 +92,10 @@ struct YgArgs {
   float* slab_T = nullptr;
   float* temp = nullptr;
   int group = 16;
-  // Backprojector depth slabs (1..16): carries hold bslabs + 1 slots per
-  // camera (every slab's exclusive prefix, then the column total).
-  int bslabs = 16;
+  // Backprojector depth slabs (1..16; 0: chosen by yg_backproject): carries
+  // hold bslabs + 1 slots per camera (every slab's exclusive prefix, then the
+  // column total).
+  int bslabs = 0;
   // Projector: non-null -> also write the transmission carries of its own
   // depth slabs ([ncam][pslabs + 1][nx][cy], the layout above with bslabs =
   // the projector's slab count; with units, at each unit's first camera).
@@ -143,9 +144,16 @@ size_t yg_backproject_workspace(int nx, int ny, int nz, int ncam, int group, int
 // Camera-group size the backprojector uses for n units and a requested group
 // (groups as even as possible, at most `group` units each).
 int yg_even_group(int n, int group);
-// Depth slabs the per-call projector chooses for nunits mirror units (or
-// cameras) of an nx-wide volume with nz planes, two CTAs per SM.
-int yg_pair_project_slabs(int nunits, int nx, int nz);
+// Depth slabs (13..16) of the spread for `items` (unit, x-tile) items of nz
+// planes: the projector's rule without clusters, the larger on a tie.
+// 128^3 x 15 cameras backprojected in 154 us with 16 slabs, 141 us with the 15
+// that fill two rounds of three CTAs per SM; 30 mirrored cameras 196 -> 189 us;
+// 120 cameras the same within 1 %.
+int yg_spread_slabs(int items, int nz, int ctas_per_sm);
+// The same for a launch over n units (or cameras) of an nx x ny x nz volume.
+int yg_backproject_slabs(int nx, int ny, int nz, int n, int ctas_per_sm);
+// Cost of `rounds` rounds of CTAs in plane steps of one CTA alone on an SM.
+double slab_rounds(double rounds, double ctas, int ctas_per_sm);
 // slabs_used (if non-null): the slab count of the carries written to
 // a.carry_out (the projector's depth slabs, twice that with a carry split).
 int yg_project(const YgArgs& a, cudaStream_t st, int* slabs_used = nullptr);

@@ -37,7 +37,8 @@ struct Plan {
   CamGeom* geom_b = nullptr;
   float* psf = nullptr;
   float* mu = nullptr;     // column layout (fused) or nifti copy (general)
-  float* carry = nullptr;  // [ncam][slots][nx][cy] (fused with attenuation)
+  float* carry = nullptr;  // [ncam][bslabs + 1][nx][cy] (fused with attenuation)
+  int bslabs = 0;          // depth slabs of the spread and the carries
   float* act_c = nullptr;  // column staging for nifti-layout calls (fused)
   float* sino_c = nullptr;
   float* out_c = nullptr;
@@ -172,7 +173,8 @@ int plan_backproject(Plan& p, int subset, const float* d_sino, float* d_out, int
     a.truncate = truncate;
     a.group = std::min(pb.group, tuned_group(pb.nx, pb.ny, pb.nz, n));  // by the subset's camera count
     a.work = p.work;
-    a.carry = p.carry ? p.carry + static_cast<size_t>(b) * yg_carry_slabs() * pb.nx * p.cy : nullptr;
+    a.carry = p.carry ? p.carry + static_cast<size_t>(b) * (p.bslabs + 1) * pb.nx * p.cy : nullptr;
+    a.bslabs = p.bslabs;
     a.pipelined = pipelined;
     int s = yg_backproject(a, st);
     if (s != kOk) return s;
@@ -342,6 +344,12 @@ int nrgb_plan_create(void** out_plan, const int* size, const float* cameras, con
     cudaMemcpyAsync(p->units_b, hu_b.data(), sizeof(int) * hu_b.size(), cudaMemcpyHostToDevice, st);
   }
   if (p->fused) {
+    // slabs for the largest subset's launches
+    int units = 0;
+    for (int i = 0; i < n_subsets; ++i) units = std::max(units, p->ucnt_b.empty() ? 0 : p->ucnt_b[i]);
+    const bool pair = units > 0;
+    const int n = yg_even_group(pair ? units : std::max(max_sub, 1), p->back.group);
+    p->bslabs = yg_backproject_slabs(nx, ny, nz, n, pair || !p->has_att ? 2 : 3);
     if (p->has_att) p->mu = cv.take<float>(ncv);
     p->act_c = cv.take<float>(ncv);
     p->out_c = cv.take<float>(ncv);
@@ -357,6 +365,7 @@ int nrgb_plan_create(void** out_plan, const int* size, const float* cameras, con
       a.ncam = ncam;
       a.geom = p->geom_b;
       a.mu = p->mu;
+      a.bslabs = p->bslabs;
       if (s == kOk) s = yg_mu_carry(a, p->carry, st);
     }
   } else if (p->has_att) {

@@ -81,10 +81,10 @@ __global__ void __launch_bounds__(32 * kSlabsB) k_mu_carry_yg(const YgArgs a, in
 // window with a.truncate -- negative sums become zero as they are stored.
 // L lanes hold one column, 32 / L lane groups per warp; footprints of
 // kGatherTaps units at a time sit in shared memory.
-template <int U, int L>
+template <int U, int L, int C>
 __global__ void __launch_bounds__(32 * kGatherWarps) k_gather_yg(const YgArgs a, int c0, int gcount, int first,
                                                                 int clamp) {
-  constexpr int C = kGatherCols, GROUPS = 32 * kGatherWarps / L;
+  constexpr int GROUPS = 32 * kGatherWarps / L;
   __shared__ Tap s_gtap[GROUPS][kGatherTaps * C];
   const int grp = threadIdx.x / L, lane = threadIdx.x % L;
   const int nchunk = (a.nx + C - 1) / C;
@@ -246,13 +246,25 @@ void launch_tgather(const YgArgs& b, int c0, int gcount, int clamp, cudaStream_t
   k_tgather_yg<<<blocks, 32 * kGatherWarps, 0, st>>>(b, c0, gcount, c0 == 0 ? 1 : 0, clamp);
 }
 
+template <int U, int L, int C>
+void launch_gather_as(const YgArgs& b, int c0, int gcount, int clamp, cudaStream_t st) {
+  constexpr int GROUPS = 32 * kGatherWarps / L;
+  const int items = (b.nx + C - 1) / C * b.nz;
+  NRGB_LAUNCH_SCOPE("k_gather_yg", st);
+  k_gather_yg<U, L, C>
+      <<<(items + GROUPS - 1) / GROUPS, 32 * kGatherWarps, 0, st>>>(b, c0, gcount, c0 == 0 ? 1 : 0, clamp);
+}
+
+// Two columns and two units in flight per lane group; where that leaves fewer
+// than four CTAs per SM (64^3 and below) one column and four units, so that
+// the grid has twice the warps and each as many loads in flight.
 template <int L>
 void launch_gather_lanes(const YgArgs& b, int c0, int gcount, int clamp, cudaStream_t st) {
-  constexpr int GROUPS = 32 * kGatherWarps / L;
-  const int items = (b.nx + kGatherCols - 1) / kGatherCols * b.nz;
-  NRGB_LAUNCH_SCOPE("k_gather_yg", st);
-  k_gather_yg<kGatherUnits, L>
-      <<<(items + GROUPS - 1) / GROUPS, 32 * kGatherWarps, 0, st>>>(b, c0, gcount, c0 == 0 ? 1 : 0, clamp);
+  const int ctas = (b.nx + 1) / 2 * b.nz / (32 * kGatherWarps / L);
+  if (ctas < 4 * sm_count())
+    launch_gather_as<2 * kGatherUnits, L, 1>(b, c0, gcount, clamp, st);
+  else
+    launch_gather_as<kGatherUnits, L, kGatherCols>(b, c0, gcount, clamp, st);
 }
 
 void launch_gather(const YgArgs& b, int c0, int gcount, int clamp, cudaStream_t st) {
@@ -318,6 +330,11 @@ size_t yg_gradient_workspace(int nx, int ny, int nz, int ncam, int group, int sl
 }
 
 int yg_carry_slabs() { return kCarrySlots; }
+
+int yg_backproject_slabs(int nx, int ny, int nz, int n, int ctas_per_sm) {
+  const int columns = 1024 / window_lanes(std::min(ny, kWindowRows), nx);
+  return yg_spread_slabs(n * ((nx + columns - 1) / columns), nz, ctas_per_sm);
+}
 
 namespace {
 
@@ -395,7 +412,7 @@ void yg_tgather(const YgArgs& a, int c0, int gcount, int clamp, cudaStream_t st)
 // gather of step g; a slot is spread again only after its gather.
 int yg_backproject(const YgArgs& a_in, cudaStream_t st) {
   YgArgs a = a_in;
-  if (a.bslabs < 1 || a.bslabs > kSlabsB) return kErrParameters;
+  if (a.bslabs < 0 || a.bslabs > kSlabsB) return kErrParameters;
   const int R = a.psf ? (a.psf_k - 1) / 2 : 0;
   // mirror units: float32 mu, or bfloat16 mu in reference mode
   const bool pair = !a.gradient && a.units && a.nunits > 0 &&
@@ -407,6 +424,11 @@ int yg_backproject(const YgArgs& a_in, cudaStream_t st) {
   const int nunits = pair ? a.nunits : a.ncam;  // scratch volumes to spread and gather
   // even groups of at most a.group units
   int group = yg_even_group(nunits, a.group);
+  if (a.bslabs == 0) {
+    const bool scatter = a.back_mode == kBackAdjoint && !a.gradient && !a.det;  // every unit in one launch
+    const bool three = !pair && a.mu && a.storage != kStorageBF16 && a.back_mode != kBackAdjoint;
+    a.bslabs = yg_backproject_slabs(a.nx, a.ny, a.nz, scatter ? nunits : group, three ? 3 : 2);
+  }
   const std::vector<Window> wins = row_windows(a.ny, R);
   // work space: slab carries first (unless given), then the scratch slot(s)
   const size_t vol = static_cast<size_t>(a.nz) * a.nx * scratch_rows(a.ny);

@@ -790,7 +790,7 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
   const bool yok = lane_rows_ok(a, yb);
   const bool paired = PAIR && mate >= 0;  // uniform over the cluster
 
-  const int nslabs = static_cast<int>(cluster.num_blocks());  // depth slabs = cluster size (2, 4 or 8)
+  const int nslabs = static_cast<int>(cluster.num_blocks());  // depth slabs = cluster size
   const int zper = (a.nz + nslabs - 1) / nslabs;
   const int zbeg = slab * zper, zend = min(a.nz, zbeg + zper);
   if (PSF && !PTAB) {  // this slab's planes only
@@ -1044,7 +1044,6 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
     if (PAIR && paired) sQ[(grp * kTXW + i) * L + lane] = kval(Q[i], nullptr, 2, i);
   }
   cluster.sync();
-  const int per_rank = kTX<L> / nslabs;  // outputs merged by each CTA of the cluster
   auto store = [&](int c, int x, float4 Pt) {
     if (a.truncate) {
       Pt.x = fmaxf(Pt.x, 0.f);
@@ -1061,7 +1060,8 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
   for (int i = 0; i < kTXW; ++i) {
     const int o = grp * kTXW + i;
     const int x = x0 + o;
-    if (o / per_rank != slab || x >= a.nx || !yok || !lane_writes(a, yb)) continue;
+    // output o is merged by CTA o % nslabs of the cluster
+    if (o % nslabs != slab || x >= a.nx || !yok || !lane_writes(a, yb)) continue;
     float4 Pt = make_float4(0.f, 0.f, 0.f, 0.f), Tt = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int s = 0; s < nslabs; ++s) {
       const float4* rT = cluster.map_shared_rank(sT, s);

@@ -2,24 +2,35 @@
 // the persistent batched projector, and the public entry points.
 #include "et_yg_device.cuh"
 
+#include <cmath>
+#include <functional>
+#include <tuple>
+
 namespace nrgb {
 
 template <int R>
 int launch_project_R(const YgArgs& a, cudaStream_t st, int* slabs_used);  // et_yg_project_kernels.cuh
 
 // ------------------------------------------------------------- dispatch
-// Depth slabs (cluster size) of the projector: the fewest of 2, 4, 8 (16
-// with at least 8 planes per slab) that give at least three waves of CTAs
-// (fewer slabs merge less; more slabs fill the GPU for small problems, e.g.
-// the 15-camera subsets of an OSEM step).  Measured on GB300 without mirror
-// units: 128^3 x 120 cameras 4 (0.84 ms; 2: 0.87, 8: 0.87), 256^3 x 180: 2
-// (15.9 ms; 4: 16.7), 64^3 x 60: 8 (0.149 ms; 4: 0.158); with mirror units
-// (60 units at 128^3 x 120): 4 (0.612 ms; 8: 0.640, 16: 0.858).
-int project_slabs(int items, int ctas_per_sm, int nz) {
+double slab_rounds(double rounds, double ctas, int ctas_per_sm) {
+  static const double step[2][3] = {{1.0, 1.5, 1.5}, {1.0, 1.28, 1.7}};
+  const double* t = step[ctas_per_sm > 2 ? 1 : 0];
+  const int most = ctas_per_sm > 2 ? 3 : 2;
+  const double full = std::floor(rounds), rest = rounds - full;
+  double cost = full * t[most - 1];
+  if (rest > 0) {
+    const int per_sm = static_cast<int>(std::ceil(ctas * rest / rounds / sm_count()));
+    cost += t[std::min(std::max(per_sm, 1), most) - 1];
+  }
+  return cost;
+}
+
+namespace {
+
+// The fewest of 2, 4, 8 (16 with 128 planes) slabs that give three waves of
+// CTAs; four where one round of them holds every item.
+int three_wave_slabs(int items, int nz, int ctas_per_sm) {
   const int slots = sm_count() * ctas_per_sm;
-  // few items (an OSEM subset: 15 cameras x 4 tiles at 128^3): one round of
-  // 4-slab clusters beats several rounds of shorter slabs (8 subsets at
-  // 128^3 x 120: 2.42 against 2.49 ms per iteration with 16 slabs)
   if (items * 4 <= slots) return 4;
   const int most = nz >= 128 ? 16 : 8;
   for (int s = 2; s < most; s *= 2)
@@ -27,8 +38,69 @@ int project_slabs(int items, int ctas_per_sm, int nz) {
   return most;
 }
 
-int yg_pair_project_slabs(int nunits, int nx, int nz) {
-  return project_slabs(nunits * ((nx + kTX<32> - 1) / kTX<32>), 2, nz);
+}  // namespace
+
+int project_slabs(int items, int nz, int ctas_per_sm, bool pair, const std::function<int(int)>& clusters) {
+  const int waves = three_wave_slabs(items, nz, ctas_per_sm);
+  const int least = std::min(waves, pair ? 8 : 6);
+  int best = least;
+  double cost = 0.0;
+  for (int s : {2, 4, 6, 8, 16}) {
+    if (s < least || (pair && s == 6)) continue;
+    const int resident = clusters(s);
+    if (resident < 1) continue;
+    const double c = ((nz + s - 1) / s + 2) *
+                     slab_rounds(static_cast<double>(items) / resident, static_cast<double>(items) * s, ctas_per_sm);
+    if (cost == 0.0 || c < cost) {
+      best = s;
+      cost = c;
+    }
+  }
+  return best;
+}
+
+int yg_spread_slabs(int items, int nz, int ctas_per_sm) {
+  int best = kSlabsB;
+  double cost = 0.0;
+  for (int s = kSlabsB; s > 12; --s) {
+    const double ctas = static_cast<double>(items) * s;
+    const double c =
+        ((nz + s - 1) / s + 1) * slab_rounds(ctas / (sm_count() * ctas_per_sm), ctas, ctas_per_sm);
+    if (cost == 0.0 || c < cost) {
+      best = s;
+      cost = c;
+    }
+  }
+  return best;
+}
+
+int max_active_clusters(const void* kernel, int cluster, int threads, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, const void*, int, int, size_t>, int> known;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const auto key = std::make_tuple(dev, kernel, cluster, threads, smem);
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = known.find(key);
+  if (it != known.end()) return it->second;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cluster);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if ((cluster > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+      cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  return known[key] = n;
 }
 
 namespace {

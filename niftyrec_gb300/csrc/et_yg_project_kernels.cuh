@@ -5,11 +5,28 @@
 
 #include "et_yg_device.cuh"
 
+#include <functional>
+
 namespace nrgb {
 
-// Depth slabs (cluster size) of the projector for `items` cluster work items
-// at `ctas_per_sm` CTAs per SM and nz depth planes (et_yg_project.cu).
-int project_slabs(int items, int ctas_per_sm, int nz);
+// Depth slabs (cluster size 2, 4, 6, 8 or 16) of the projector for `items`
+// cluster work items of nz depth planes: the least planes per slab times the
+// rounds of resident clusters (clusters(s): how many of size s fit at once,
+// cudaOccupancyMaxActiveClusters).  A round is weighted by the CTAs that share
+// an SM -- a plane step of 2 (3) of them takes 1.28 (1.7) times as long as of
+// one alone, 1.5 times with mirror units; measured at 128^3 -- and two planes
+// stand for a slab's start and merge.  Against the count for three waves of
+// CTAs: 128^3 x 30 cameras of a half-turn 258 -> 196 us (6 slabs), x 15 125 ->
+// 114, 256^3 x 18 PSF 15 1.66 -> 1.25 ms, 64^3 x 60 plain 25 -> 19 us (8),
+// 32^3 x 8 27 -> 15 us (16); 128^3 x 120 keeps 4 (0.504 ms; 8: 0.519).
+// Left out: 5 and 7 (128^3 x 15: 131 and 136 us although they fit one round),
+// with mirror units 6 (96 x 96 x 80 x 90: 206 us, 8: 200), and fewer than the
+// three-wave count (6 or 8 at least): longer float sums for nothing more than
+// 7 % (96 x 96 x 80 x 90 with 2 slabs, error 2.4e-7 -> 3.2e-7).
+int project_slabs(int items, int nz, int ctas_per_sm, bool pair, const std::function<int(int)>& clusters);
+// Clusters of `cluster` CTAs of a kernel that are resident at once (0: none);
+// asked of the driver once per device, kernel and shape.
+int max_active_clusters(const void* kernel, int cluster, int threads, size_t smem);
 
 namespace {
 
@@ -60,15 +77,12 @@ int launch_project_lanes(const YgArgs& a_in, cudaStream_t st, int* slabs_used) {
   const int nunits = pair ? a.nunits : a.ncam;
   // three CTAs per SM need three tiles (plus 1 KB reserved each) in the 228 KB
   const bool three = 3 * (smem + kYBufBytes<L> + 1024) <= 228 * 1024;
-  if (a.pslabs != 2 && a.pslabs != 4 && a.pslabs != 8 && a.pslabs != 16)
-    a.pslabs = project_slabs(nunits * ntile, three && !bf16 && !pair ? 3 : 2, a.nz);
   // carry split: the slab's halves must be the backprojector's slabs of twice
   // the count, with at most 8 of them
   auto split_ok = [&](int p) {
     return a.carry_out && a.mu && a.carry_split && 2 * p <= 8 &&
            (a.nz + p - 1) / p == 2 * ((a.nz + 2 * p - 1) / (2 * p));
   };
-  a.carry_split = split_ok(a.pslabs) ? 1 : 0;
   // one cluster of a.pslabs CTAs per (unit, x-tile); 16 is a non-portable
   // cluster size: it falls back to 8 where the kernel cannot be resident so
   bool launch_err = false;
@@ -84,17 +98,14 @@ int launch_project_lanes(const YgArgs& a_in, cudaStream_t st, int* slabs_used) {
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (a.pslabs == 16) {
-      int clusters = 0;
-      cfg.gridDim = dim3(nunits * ntile * 16);
-      attr[0].val.clusterDim.x = 16;
-      if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-          cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess || clusters < 1) {
-        cudaGetLastError();
-        a.pslabs = 8;
-        a.carry_split = split_ok(8) ? 1 : 0;
-      }
-    }
+    auto clusters = [&](int s) {
+      return max_active_clusters(reinterpret_cast<const void*>(k), s, 32 * kW, smem);
+    };
+    if (a.pslabs < 2 || (a.pslabs > 8 && a.pslabs != 16))
+      a.pslabs = project_slabs(nunits * ntile, a.nz, three && !bf16 && !pair ? 3 : 2, pair || a.carry_out, clusters);
+    else if (a.pslabs == 16 && clusters(16) < 1)
+      a.pslabs = 8;
+    a.carry_split = split_ok(a.pslabs) ? 1 : 0;
     cfg.gridDim = dim3(nunits * ntile * a.pslabs);
     attr[0].val.clusterDim.x = a.pslabs;
     if (slabs_used) {
