@@ -337,6 +337,9 @@ int nrgb_plan_create(void **out_plan, const int *size, const float *cameras, con
 int nrgb_plan_destroy(void *plan);
 int nrgb_plan_shape(void *plan, int *out);
 int nrgb_plan_subset_cameras(void *plan, int subset, int *idx_out);
+/* Counts of all cameras (device, nifti planes in creation order) into column
+ * layout [n_cameras][nx][cy], planes in subset order (fused plans only). */
+int nrgb_plan_split_counts(void *plan, const float *d_counts, float *d_out, void *stream);
 int nrgb_plan_project(void *plan, int subset, const float *d_activity, float *d_sinogram, int layout,
                       int truncate, void *stream);
 int nrgb_plan_backproject(void *plan, int subset, const float *d_sinogram, float *d_out, int layout,

@@ -79,6 +79,7 @@ PROTOTYPES = {
     "nrgb_plan_destroy": (_I, [_P]),
     "nrgb_plan_shape": (_I, [_P, _PI]),
     "nrgb_plan_subset_cameras": (_I, [_P, _I, _PI]),
+    "nrgb_plan_split_counts": (_I, [_P, _P, _P, _P]),
     "nrgb_plan_project": (_I, [_P, _I, _P, _P, _I, _I, _P]),
     "nrgb_plan_backproject": (_I, [_P, _I, _P, _P, _I, _I, _P]),
     "nrgb_plan_osem_prepare": (_I, [_P, _I, _P]),

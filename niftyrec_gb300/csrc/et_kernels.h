@@ -237,6 +237,9 @@ int fisher_pairs(const float* proj, int npx, int npy, const int* coords, const i
 // ---- layout conversion and elementwise helpers ----
 // planes x [ny][nx] (nifti) <-> planes x [nx][cy] (column), zero pads.
 int to_column(const float* src, float* dst, int nx, int ny, int cy, int planes, cudaStream_t st);
+// The same with destination plane p = source plane order[p] (device array).
+int to_column_planes(const float* src, float* dst, const int* order, int nx, int ny, int cy, int planes,
+                     cudaStream_t st);
 // Two volumes of the same shape laid out in one launch (two launches where
 // the 16-byte form does not apply).
 int to_column2(const float* src_a, float* dst_a, const float* src_b, float* dst_b, int nx, int ny, int cy, int planes,

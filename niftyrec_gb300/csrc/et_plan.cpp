@@ -35,6 +35,7 @@ struct Plan {
   size_t bytes = 0;
   CamGeom* geom_p = nullptr;
   CamGeom* geom_b = nullptr;
+  int* d_order = nullptr;  // `order` on the device
   float* psf = nullptr;
   float* mu = nullptr;     // column layout (fused) or nifti copy (general)
   float* carry = nullptr;  // [ncam][bslabs + 1][nx][cy] (fused with attenuation)
@@ -306,7 +307,7 @@ int nrgb_plan_create(void** out_plan, const int* size, const float* cameras, con
   const size_t ncv = static_cast<size_t>(nx) * p->cy * nz;
   const size_t nsc = static_cast<size_t>(nx) * p->cy * ncam;
   size_t bytes = al(sizeof(CamGeom) * ncam) * 2 + al(sizeof(float) * p->proj.psf_sep.size()) +
-                 al(sizeof(int) * hu_p.size()) + al(sizeof(int) * hu_b.size());
+                 al(sizeof(int) * hu_p.size()) + al(sizeof(int) * hu_b.size()) + al(sizeof(int) * ncam);
   if (p->fused) {
     bytes += al(sizeof(float) * ncv) * (p->has_att ? 4 : 3) + al(sizeof(float) * nsc);
     if (p->has_att) bytes += al(sizeof(float) * static_cast<size_t>(ncam) * yg_carry_slabs() * nx * p->cy);
@@ -326,10 +327,12 @@ int nrgb_plan_create(void** out_plan, const int* size, const float* cameras, con
   Carver cv(p->mem, bytes);
   p->geom_p = cv.take<CamGeom>(ncam);
   p->geom_b = cv.take<CamGeom>(ncam);
+  p->d_order = cv.take<int>(ncam);
   if (!p->proj.psf_sep.empty()) p->psf = cv.take<float>(p->proj.psf_sep.size());
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaMemcpyAsync(p->geom_p, p->proj.geom.data(), sizeof(CamGeom) * ncam, cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(p->geom_b, p->back.geom.data(), sizeof(CamGeom) * ncam, cudaMemcpyHostToDevice, st);
+  cudaMemcpyAsync(p->d_order, p->order.data(), sizeof(int) * ncam, cudaMemcpyHostToDevice, st);
   if (p->psf)
     cudaMemcpyAsync(p->psf, p->proj.psf_sep.data(), sizeof(float) * p->proj.psf_sep.size(), cudaMemcpyHostToDevice,
                     st);
@@ -420,6 +423,18 @@ int nrgb_plan_subset_cameras(void* plan, int subset, int* idx_out) {
   if (idx_out)
     for (int i = b; i < e; ++i) idx_out[i - b] = p->order[i];
   return e - b;
+}
+
+// Counts of all cameras, device [n_cameras][ny][nx] in the order given to
+// nrgb_plan_create, into column layout [n_cameras][nx][cy] in subset order:
+// the planes of subset 0 first, then subset 1, ... (nrgb_plan_subset_cameras).
+int nrgb_plan_split_counts(void* plan, const float* d_counts, float* d_out, void* stream) {
+  NRGB_API("nrgb_plan_split_counts");
+  Plan* p = static_cast<Plan*>(plan);
+  if (!p || !p->fused || !d_counts || !d_out) return kErrParameters;
+  const Problem& pb = p->proj;
+  return to_column_planes(d_counts, d_out, p->d_order, pb.nx, pb.ny, p->cy, pb.cams.n,
+                          static_cast<cudaStream_t>(stream));
 }
 
 // Project the cameras of `subset` (-1: all) of d_activity into d_sinogram
@@ -730,12 +745,7 @@ int nrgb_batch_set_counts(void* batch, int v, const float* d_counts, void* strea
   const Plan& p = *b->plans[v];
   const Problem& pb = p.proj;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const size_t in_plane = static_cast<size_t>(pb.nx) * pb.ny, out_plane = static_cast<size_t>(pb.nx) * p.cy;
-  for (int i = 0; i < pb.cams.n; ++i) {
-    const int s = to_column(d_counts + in_plane * p.order[i], b->counts[v] + out_plane * i, pb.nx, pb.ny, p.cy, 1, st);
-    if (s != kOk) return s;
-  }
-  return kOk;
+  return to_column_planes(d_counts, b->counts[v], p.d_order, pb.nx, pb.ny, p.cy, pb.cams.n, st);
 }
 
 // Activity of volume v in and out, device (nz, ny, nx) nifti.

@@ -362,29 +362,32 @@ constexpr int kYRow = L + 2 * kYPad;  // chunks of one group's row buffer
 template <int L>
 constexpr size_t kYBufBytes = sizeof(float4) * kGroups<L> * 2 * kYRow<L>;  // static, per CTA
 
-template <int L>
+// YB: the lane count whose row buffers the kernel holds -- L, or in a kernel
+// that runs windows of several lane counts the one with the largest (8).
+template <int L, int YB>
 __device__ __forceinline__ float4* ybuf(int grp, int b) {
-  __shared__ __align__(16) float4 buf[kGroups<L>][2][kYRow<L>];
-  return buf[grp][b];
+  static_assert(kYBufBytes<L> <= kYBufBytes<YB>, "row buffers of L lanes fit");
+  __shared__ __align__(16) float4 buf[kYBufBytes<YB> / sizeof(float4)];
+  return buf + (grp * 2 + b) * kYRow<L>;
 }
 
-template <int L>
+template <int L, int YB = L>
 __device__ __forceinline__ void ybuf_zero_pads() {
   for (int i = threadIdx.x; i < kGroups<L> * 2 * 2 * kYPad; i += blockDim.x) {
     const int g = i / (4 * kYPad), r = i % (4 * kYPad);
     const int b = r / (2 * kYPad), q = r % (2 * kYPad);
-    ybuf<L>(g, b)[q < kYPad ? q : L + q] = make_float4(0.f, 0.f, 0.f, 0.f);
+    ybuf<L, YB>(g, b)[q < kYPad ? q : L + q] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
 }
 
-template <int R, int L, class KC>
+template <int R, int L, int YB, class KC>
 __device__ __forceinline__ float4 yconv4s(const float4& u, KC kc, int lane, int b) {
   if constexpr (R == 0) {
     return yconv4<0>(u, kc, lane);
   } else {
     constexpr int C = (R + 3) / 4;
     static_assert(C <= kYPad, "row-buffer pads");
-    float4* row = ybuf<L>(threadIdx.x / L, b) + kYPad;
+    float4* row = ybuf<L, YB>(threadIdx.x / L, b) + kYPad;
     row[lane] = u;
     __syncwarp();
     float w[2 * R + 4];
@@ -576,7 +579,7 @@ __host__ __device__ constexpr size_t project_smem_bytes(int nz, bool pair, bool 
 
 // Row pass from the shared tile: outputs i = 0..kTXW-1 of this group use tile
 // columns base + i .. base + i + 2R (base = group * kTXW).
-template <int R, int L, class EmitFn, class KR, class KC>
+template <int R, int L, int YB, class EmitFn, class KR, class KC>
 __device__ __forceinline__ void rowpass_from_tile(const float4* __restrict__ sbuf, int base, EmitFn emit, KR kr, KC kc,
                                                   int lane, int ny) {
   constexpr int K = 2 * R + 1;
@@ -594,7 +597,7 @@ __device__ __forceinline__ void rowpass_from_tile(const float4* __restrict__ sbu
     }
     const int i = j - 2 * R;
     if (i >= 0 && i < kTXW) {
-      emit(i, mask_rows(yconv4s<R, L>(u[i % K], kc, lane, i & 1), 4 * lane, ny));
+      emit(i, mask_rows(yconv4s<R, L, YB>(u[i % K], kc, lane, i & 1), 4 * lane, ny));
       u[i % K] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
@@ -604,7 +607,7 @@ __device__ __forceinline__ void rowpass_from_tile(const float4* __restrict__ sbu
 // one fma.rn.f32x2 per two rows; the same roundings in the same order), used
 // by the projector.  The spread keeps the scalar forms: its two transmission
 // arrays leave no registers for the broadcast coefficient pairs.
-template <int R, int L, class EmitFn, class KR, class KC>
+template <int R, int L, int YB, class EmitFn, class KR, class KC>
 __device__ __forceinline__ void rowpass_from_tile_p(const float4* __restrict__ sbuf, int base, EmitFn emit, KR kr, KC kc,
                                                   int lane, int ny) {
   constexpr int K = 2 * R + 1;
@@ -625,7 +628,7 @@ __device__ __forceinline__ void rowpass_from_tile_p(const float4* __restrict__ s
       }
     }
     const int i = j - 2 * R;
-    if (i >= 0 && i < kTXW) emit(i, mask_rows(yconv4s<R, L>(unpair4(u[i]), kc, lane, i & 1), 4 * lane, ny));
+    if (i >= 0 && i < kTXW) emit(i, mask_rows(yconv4s<R, L, YB>(unpair4(u[i]), kc, lane, i & 1), 4 * lane, ny));
   }
 }
 
@@ -633,7 +636,7 @@ __device__ __forceinline__ void rowpass_from_tile_p(const float4* __restrict__ s
 // its mirror camera in the projector: each tile column is read once and feeds
 // both sliding windows) or over two tiles (the mirror-unit spread); output i
 // of camera b is emitted before output i of camera a.
-template <int R, int L, class EmitA, class EmitB, class KRA, class KCA, class KRB, class KCB>
+template <int R, int L, int YB, class EmitA, class EmitB, class KRA, class KCA, class KRB, class KCB>
 __device__ __forceinline__ void rowpass2_from_tiles(const float4* __restrict__ sa, const float4* __restrict__ sbt,
                                                     int base, EmitA emit_a, KRA kra, KCA kca, EmitB emit_b, KRB krb,
                                                     KCB kcb, int lane, int ny) {
@@ -658,13 +661,13 @@ __device__ __forceinline__ void rowpass2_from_tiles(const float4* __restrict__ s
     }
     const int i = j - 2 * R;
     if (i >= 0 && i < kTXW) {
-      emit_b(i, mask_rows(yconv4s<R, L>(ub[i], kcb, lane, 0), 4 * lane, ny));
-      emit_a(i, mask_rows(yconv4s<R, L>(ua[i], kca, lane, 1), 4 * lane, ny));
+      emit_b(i, mask_rows(yconv4s<R, L, YB>(ub[i], kcb, lane, 0), 4 * lane, ny));
+      emit_a(i, mask_rows(yconv4s<R, L, YB>(ua[i], kca, lane, 1), 4 * lane, ny));
     }
   }
 }
 
-template <int R, int L, class EmitA, class EmitB, class KRA, class KCA, class KRB, class KCB>
+template <int R, int L, int YB, class EmitA, class EmitB, class KRA, class KCA, class KRB, class KCB>
 __device__ __forceinline__ void rowpass2_from_tiles_p(const float4* __restrict__ sa, const float4* __restrict__ sbt,
                                                     int base, EmitA emit_a, KRA kra, KCA kca, EmitB emit_b, KRB krb,
                                                     KCB kcb, int lane, int ny) {
@@ -692,22 +695,22 @@ __device__ __forceinline__ void rowpass2_from_tiles_p(const float4* __restrict__
     }
     const int i = j - 2 * R;
     if (i >= 0 && i < kTXW) {
-      emit_b(i, mask_rows(yconv4s<R, L>(unpair4(ub[i]), kcb, lane, 0), 4 * lane, ny));
-      emit_a(i, mask_rows(yconv4s<R, L>(unpair4(ua[i]), kca, lane, 1), 4 * lane, ny));
+      emit_b(i, mask_rows(yconv4s<R, L, YB>(unpair4(ub[i]), kcb, lane, 0), 4 * lane, ny));
+      emit_a(i, mask_rows(yconv4s<R, L, YB>(unpair4(ua[i]), kca, lane, 1), 4 * lane, ny));
     }
   }
 }
 
-template <int R, int L, class EmitA, class EmitB, class KRA, class KCA, class KRB, class KCB>
+template <int R, int L, int YB, class EmitA, class EmitB, class KRA, class KCA, class KRB, class KCB>
 __device__ __forceinline__ void rowpass2_from_tile(const float4* __restrict__ sbuf, int base, EmitA emit_a, KRA kra,
                                                    KCA kca, EmitB emit_b, KRB krb, KCB kcb, int lane, int ny) {
-  rowpass2_from_tiles<R, L>(sbuf, sbuf, base, emit_a, kra, kca, emit_b, krb, kcb, lane, ny);
+  rowpass2_from_tiles<R, L, YB>(sbuf, sbuf, base, emit_a, kra, kca, emit_b, krb, kcb, lane, ny);
 }
 
-template <int R, int L, class EmitA, class EmitB, class KRA, class KCA, class KRB, class KCB>
+template <int R, int L, int YB, class EmitA, class EmitB, class KRA, class KCA, class KRB, class KCB>
 __device__ __forceinline__ void rowpass2_from_tile_p(const float4* __restrict__ sbuf, int base, EmitA emit_a, KRA kra,
                                                      KCA kca, EmitB emit_b, KRB krb, KCB kcb, int lane, int ny) {
-  rowpass2_from_tiles_p<R, L>(sbuf, sbuf, base, emit_a, kra, kca, emit_b, krb, kcb, lane, ny);
+  rowpass2_from_tiles_p<R, L, YB>(sbuf, sbuf, base, emit_a, kra, kca, emit_b, krb, kcb, lane, ny);
 }
 
 // Vector reduction of 4 floats into global memory (sm_90+).
@@ -766,7 +769,7 @@ constexpr float kMateMaxT = 40.0f;
 // STEPS: depth planes sampled per barrier (2 x STEPS tile buffers).  Two
 // planes per barrier measured no faster on GB300 (128^3 x 120: 0.676 against
 // 0.674 ms; 256^3 x 180: 11.9 against 11.2 ms), so the kernels use one.
-template <int R, bool PSF, bool ATT, class V, bool PAIR = false, bool PTAB = false, int L = 32, int STEPS = 1>
+template <int R, bool PSF, bool ATT, class V, bool PAIR = false, bool PTAB = false, int L = 32, int YB = L, int STEPS = 1>
 __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate, int x0, unsigned char* smem,
                                              const float* ptab = nullptr) {
   using TS = TileShape<R, L>;
@@ -807,20 +810,20 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
   auto mate_pass = [&](const float4* sbuf, int z, auto emit_m) {
     if constexpr (PTAB) {
       const float* m = ptab + (a.nz - 1 - z) * 2 * K;
-      rowpass_from_tile_p<R, L>(sbuf, grp * kTXW, emit_m, Reversed<R>{m}, m + K, lane, a.ny);
+      rowpass_from_tile_p<R, L, YB>(sbuf, grp * kTXW, emit_m, Reversed<R>{m}, m + K, lane, a.ny);
     } else {
       const float* m = s_psf_m + z * 2 * K;
-      rowpass_from_tile_p<R, L>(sbuf, grp * kTXW, emit_m, m, m + K, lane, a.ny);
+      rowpass_from_tile_p<R, L, YB>(sbuf, grp * kTXW, emit_m, m, m + K, lane, a.ny);
     }
   };
   auto both_pass = [&](const float4* sbuf, int z, auto emit, auto emit_m) {
     const float* kr = (PTAB ? ptab : s_psf) + z * 2 * K;
     if constexpr (PTAB) {
       const float* m = ptab + (a.nz - 1 - z) * 2 * K;
-      rowpass2_from_tile_p<R, L>(sbuf, grp * kTXW, emit, kr, kr + K, emit_m, Reversed<R>{m}, m + K, lane, a.ny);
+      rowpass2_from_tile_p<R, L, YB>(sbuf, grp * kTXW, emit, kr, kr + K, emit_m, Reversed<R>{m}, m + K, lane, a.ny);
     } else {
       const float* m = s_psf_m + z * 2 * K;
-      rowpass2_from_tile_p<R, L>(sbuf, grp * kTXW, emit, kr, kr + K, emit_m, m, m + K, lane, a.ny);
+      rowpass2_from_tile_p<R, L, YB>(sbuf, grp * kTXW, emit, kr, kr + K, emit_m, m, m + K, lane, a.ny);
     }
   };
   const CamRows cr = cam_rows(a.geom[cam].fwd);
@@ -861,7 +864,7 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
     if (PAIR) Q[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int q = 0; q < 3; ++q) kclear(q, i);
   }
-  ybuf_zero_pads<L>();
+  ybuf_zero_pads<L, YB>();
   __syncthreads();
 
   // A depth step at plane z through tile buffer b: produce (footprints and
@@ -952,7 +955,7 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
         both_pass(sbuf, z, emit, emit_m);
       } else {
         const float* kr = (PTAB ? ptab : s_psf) + z * 2 * K;
-        rowpass_from_tile_p<R, L>(sbuf, grp * kTXW, emit, kr, kr + K, lane, a.ny);
+        rowpass_from_tile_p<R, L, YB>(sbuf, grp * kTXW, emit, kr, kr + K, lane, a.ny);
       }
     } else {
 #pragma unroll

@@ -150,7 +150,7 @@ __device__ __forceinline__ void grad_item(const YgArgs& a, int cam, int g, int x
     };
     if (PSF) {
       const float* kr = (PTAB ? ptab : s_psf) + z * 2 * K;
-      rowpass_from_tile<R, 32>(sbuf, warp * kTXW, emit, kr, kr + K, lane, a.ny);
+      rowpass_from_tile<R, 32, 32>(sbuf, warp * kTXW, emit, kr, kr + K, lane, a.ny);
     } else {
 #pragma unroll
       for (int i = 0; i < kTXW; ++i) emit(i, sbuf[(warp * kTXW + i) * 32 + lane]);

@@ -142,9 +142,9 @@ __global__ void __cluster_dims__(kSlabsP, 1, 1) __launch_bounds__(32 * kW, CTAS)
     a.out_hi = d.win[w][3];
     const int cam = r / ntile, t = r % ntile;
     switch (d.lanes[w]) {  // uniform over the cluster
-      case 8: project_item<R, PSF, ATT, float, false, false, 8>(a, cam, -1, t * kTX<8>, smem); break;
-      case 16: project_item<R, PSF, ATT, float, false, false, 16>(a, cam, -1, t * kTX<16>, smem); break;
-      default: project_item<R, PSF, ATT, float, false, false, 32>(a, cam, -1, t * kTX<32>, smem);
+      case 8: project_item<R, PSF, ATT, float, false, false, 8, 8>(a, cam, -1, t * kTX<8>, smem); break;
+      case 16: project_item<R, PSF, ATT, float, false, false, 16, 8>(a, cam, -1, t * kTX<16>, smem); break;
+      default: project_item<R, PSF, ATT, float, false, false, 32, 8>(a, cam, -1, t * kTX<32>, smem);
     }
   }
 }
@@ -173,8 +173,7 @@ int launch_project_batch_R(const BatchStepDesc* d, const BatchSel& sel, bool att
   const int planes = PSF ? max_nz : 0;
   const size_t smem =
       std::max({tile_smem_bytes<R, 32>(planes), tile_smem_bytes<R, 16>(planes), tile_smem_bytes<R, 8>(planes)});
-  const size_t fixed = kYBufBytes<32> + kYBufBytes<16> + kYBufBytes<8>;
-  const bool three = 3 * (smem + fixed + 1024) <= 228 * 1024;
+  const bool three = 3 * (smem + kYBufBytes<8> + 1024) <= 228 * 1024;
   auto go = [&](auto k, int ctas) {
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     NRGB_LAUNCH_SCOPE("k_project_batch_yg", st);

@@ -115,10 +115,10 @@ __device__ __forceinline__ void spread_body(const YgArgs& a, int c0, const float
     if (PSF) {
       if constexpr (PTAB && ADJ) {  // transpose of a convolution = correlation: both kernels reversed
         const float* kr = ptab + z * 2 * K;
-        rowpass_from_tile<R, L>(sbuf, grp * kTXW, emit, Reversed<R>{kr}, Reversed<R>{kr + K}, lane, a.ny);
+        rowpass_from_tile<R, L, L>(sbuf, grp * kTXW, emit, Reversed<R>{kr}, Reversed<R>{kr + K}, lane, a.ny);
       } else {
         const float* kr = (PTAB ? ptab : s_psf) + z * 2 * K;
-        rowpass_from_tile<R, L>(sbuf, grp * kTXW, emit, kr, kr + K, lane, a.ny);
+        rowpass_from_tile<R, L, L>(sbuf, grp * kTXW, emit, kr, kr + K, lane, a.ny);
       }
     } else {
 #pragma unroll
@@ -314,20 +314,20 @@ __device__ __forceinline__ void spread_pair_body(const YgArgs& a, int u0, const 
       if (paired) {  // both row passes in one sweep over the two tiles
         if constexpr (PTAB && ADJ) {
           const float* km = ptab + (a.nz - 1 - z) * 2 * K;
-          rowpass2_from_tiles<R, L>(sc, sm, grp * kTXW, write_sum, Reversed<R>{kr}, Reversed<R>{kr + K}, keep, km,
+          rowpass2_from_tiles<R, L, L>(sc, sm, grp * kTXW, write_sum, Reversed<R>{kr}, Reversed<R>{kr + K}, keep, km,
                                  Reversed<R>{km + K}, lane, a.ny);
         } else if constexpr (PTAB) {
           const float* km = ptab + (a.nz - 1 - z) * 2 * K;
-          rowpass2_from_tiles<R, L>(sc, sm, grp * kTXW, write_sum, kr, kr + K, keep, Reversed<R>{km}, km + K, lane,
+          rowpass2_from_tiles<R, L, L>(sc, sm, grp * kTXW, write_sum, kr, kr + K, keep, Reversed<R>{km}, km + K, lane,
                                  a.ny);
         } else {
           const float* km = s_psf_m + (z - zbeg) * 2 * K;
-          rowpass2_from_tiles<R, L>(sc, sm, grp * kTXW, write_sum, kr, kr + K, keep, km, km + K, lane, a.ny);
+          rowpass2_from_tiles<R, L, L>(sc, sm, grp * kTXW, write_sum, kr, kr + K, keep, km, km + K, lane, a.ny);
         }
       } else if constexpr (PTAB && ADJ) {
-        rowpass_from_tile<R, L>(sc, grp * kTXW, write, Reversed<R>{kr}, Reversed<R>{kr + K}, lane, a.ny);
+        rowpass_from_tile<R, L, L>(sc, grp * kTXW, write, Reversed<R>{kr}, Reversed<R>{kr + K}, lane, a.ny);
       } else {
-        rowpass_from_tile<R, L>(sc, grp * kTXW, write, kr, kr + K, lane, a.ny);
+        rowpass_from_tile<R, L, L>(sc, grp * kTXW, write, kr, kr + K, lane, a.ny);
       }
     } else {
 #pragma unroll

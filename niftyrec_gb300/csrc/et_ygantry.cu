@@ -8,15 +8,16 @@ namespace {
 // --------------------------------------------------------------- layouts
 // dst[p][x][r] = src[p][row0 + r][x] for r < rows, zero pads up to cy.
 // src planes have ny_src rows.
+// With order, destination plane p is source plane order[p].
 __global__ void k_to_col(const float* __restrict__ src, float* __restrict__ dst, int nx, int ny_src, int row0,
-                         int rows, int cy) {
+                         int rows, int cy, const int* __restrict__ order) {
   __shared__ float tile[32][33];
-  const int p = blockIdx.z;
+  const int p = blockIdx.z, q = order ? order[p] : p;
   const int xb = blockIdx.x * 32, yb = blockIdx.y * 32;
   const int tx = threadIdx.x;
   for (int dy = threadIdx.y; dy < 32; dy += blockDim.y) {
     const int r = yb + dy, x = xb + tx;
-    tile[dy][tx] = (r < rows && x < nx) ? src[(static_cast<size_t>(p) * ny_src + row0 + r) * nx + x] : 0.0f;
+    tile[dy][tx] = (r < rows && x < nx) ? src[(static_cast<size_t>(q) * ny_src + row0 + r) * nx + x] : 0.0f;
   }
   __syncthreads();
   for (int dx = threadIdx.y; dx < 32; dx += blockDim.y) {
@@ -34,7 +35,8 @@ __global__ void k_to_col(const float* __restrict__ src, float* __restrict__ dst,
 // lay out src2 into dst2: two volumes in one launch.
 __global__ void __launch_bounds__(256) k_to_col4(const float* __restrict__ src, float* __restrict__ dst, int nx,
                                                  int ny_src, int row0, int rows, int cy, const float* __restrict__ src2,
-                                                 float* __restrict__ dst2, int planes) {
+                                                 float* __restrict__ dst2, int planes,
+                                                 const int* __restrict__ order) {
   __shared__ float tile[32][129];
   int p = blockIdx.z;
   if (p >= planes) {  // uniform over the CTA
@@ -42,6 +44,7 @@ __global__ void __launch_bounds__(256) k_to_col4(const float* __restrict__ src, 
     src = src2;
     dst = dst2;
   }
+  const int q = order ? order[p] : p;
   const int xb = blockIdx.x * 128, yb = blockIdx.y * 32;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   float4 v[4];
@@ -49,7 +52,7 @@ __global__ void __launch_bounds__(256) k_to_col4(const float* __restrict__ src, 
   for (int i = 0; i < 4; ++i) {
     const int r = yb + w + 8 * i, x = xb + 4 * lane;
     v[i] = (r < rows && x < nx)
-               ? *reinterpret_cast<const float4*>(src + (static_cast<size_t>(p) * ny_src + row0 + r) * nx + x)
+               ? *reinterpret_cast<const float4*>(src + (static_cast<size_t>(q) * ny_src + row0 + r) * nx + x)
                : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
 #pragma unroll
@@ -194,18 +197,38 @@ bool yg_supported(int nx, int ny, int nz, int psf_k) {
   return true;
 }
 
-int to_column_rows(const float* src, float* dst, int nx, int ny_src, int row0, int rows, int cy, int planes,
-                   cudaStream_t st) {
+namespace {
+
+int to_column_ordered(const float* src, float* dst, int nx, int ny_src, int row0, int rows, int cy, int planes,
+                      const int* order, cudaStream_t st) {
   if (wide_rows(src, nx)) {
     const dim3 grid((nx + 127) / 128, (cy + 31) / 32, planes);
     NRGB_LAUNCH_SCOPE("k_to_col4", st);
-    k_to_col4<<<grid, 256, 0, st>>>(src, dst, nx, ny_src, row0, rows, cy, nullptr, nullptr, planes);
+    k_to_col4<<<grid, 256, 0, st>>>(src, dst, nx, ny_src, row0, rows, cy, nullptr, nullptr, planes, order);
   } else {
     const dim3 grid((nx + 31) / 32, (cy + 31) / 32, planes), block(32, 8);
     NRGB_LAUNCH_SCOPE("k_to_col", st);
-    k_to_col<<<grid, block, 0, st>>>(src, dst, nx, ny_src, row0, rows, cy);
+    k_to_col<<<grid, block, 0, st>>>(src, dst, nx, ny_src, row0, rows, cy, order);
   }
   return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
+}
+
+}  // namespace
+
+int to_column_rows(const float* src, float* dst, int nx, int ny_src, int row0, int rows, int cy, int planes,
+                   cudaStream_t st) {
+  return to_column_ordered(src, dst, nx, ny_src, row0, rows, cy, planes, nullptr, st);
+}
+
+int to_column_planes(const float* src, float* dst, const int* order, int nx, int ny, int cy, int planes,
+                     cudaStream_t st) {
+  // at most 65535 planes a launch
+  for (int p = 0; p < planes; p += 65535) {
+    const int s = to_column_ordered(src, dst + static_cast<size_t>(p) * nx * cy, nx, ny, 0, ny, cy,
+                                    std::min(planes - p, 65535), order + p, st);
+    if (s != kOk) return s;
+  }
+  return kOk;
 }
 
 int from_column_rows(const float* src, float* dst, int nx, int cy, int r_begin, int r_end, int row0, int ny_dst,
@@ -264,7 +287,7 @@ int to_column2(const float* src_a, float* dst_a, const float* src_b, float* dst_
   }
   const dim3 grid((nx + 127) / 128, (cy + 31) / 32, 2 * planes);
   NRGB_LAUNCH_SCOPE("k_to_col4", st);
-  k_to_col4<<<grid, 256, 0, st>>>(src_a, dst_a, nx, ny, 0, ny, cy, src_b, dst_b, planes);
+  k_to_col4<<<grid, 256, 0, st>>>(src_a, dst_a, nx, ny, 0, ny, cy, src_b, dst_b, planes, nullptr);
   return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
 }
 

@@ -170,6 +170,17 @@ class Plan:
     def split_counts(self, counts, layout="column"):
         """Per-subset count sinograms in subset camera order from a full (n, ny, nx) tensor."""
         out = []
+        nz, ny, nx = self.shape
+        if (_layout(layout) == COLUMN and self.fused and counts.is_cuda and counts.dtype == self.torch.float32
+                and counts.ndim == 3 and counts.shape[0] >= self.n_cameras and tuple(counts.shape[1:]) == (ny, nx)):
+            # every subset in one launch, as slices of one tensor
+            c = counts.contiguous()
+            cols = self.torch.empty((self.n_cameras, nx, self.cy), dtype=self.torch.float32, device=counts.device)
+            st = self.L.nrgb_plan_split_counts(self.handle, _vp(c.data_ptr()), _vp(cols.data_ptr()), self._stream())
+            if st:
+                raise NiftyRecError("nrgb_plan_split_counts", st)
+            sizes = [self.subset_size(s) for s in range(self.n_subsets)]
+            return list(cols.split(sizes))
         for s in range(self.n_subsets):
             idx = self.torch.as_tensor(self.subset_cameras(s), device=counts.device)
             y = counts.index_select(0, idx).contiguous()

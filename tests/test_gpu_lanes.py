@@ -58,3 +58,21 @@ def test_narrow_windows(o32, shape, k, cams):
     want = float(np.sum(so.astype(np.float64) * d)) / 2
     # the central difference is exact to second order in h; 1e-4 of the terms' size
     assert abs(float(np.sum(g * h)) - want) < 1e-4 * float(np.linalg.norm(g) * np.linalg.norm(h))
+
+
+@pytest.mark.parametrize("shape,subsets", [((9, 12, 16), 4), ((8, 13, 15), 3), ((6, 130, 10), 5)])
+def test_counts_split_in_one_launch(shape, subsets):
+    """The one-launch split equals plane-by-plane selection and layout, exactly
+    (16-byte and 4-byte layout kernels; a row stride that is padded)."""
+    from niftyrec_gb300.plan import Plan
+
+    nz, ny, nx = shape
+    ids = np.random.default_rng(2).integers(0, subsets, 11).astype(np.int32)
+    ids[:subsets] = np.arange(subsets)
+    plan = Plan(shape, S.cameras_about_y(11), subsets=ids)
+    y = torch.rand((11, ny, nx), device="cuda")
+    parts = plan.split_counts(y)
+    assert len(parts) == subsets
+    for s, p in enumerate(parts):
+        sel = y[torch.as_tensor(np.flatnonzero(ids == s), device="cuda")].contiguous()
+        assert torch.equal(p, plan.to_column(sel))
