@@ -24,6 +24,7 @@ SOURCES = ["et_geometry.cpp", "et_engine.cpp", "et_api.cpp", "et_profile.cpp", "
            "et_yg_project.cu", "et_yg_proj_r01.cu", "et_yg_proj_r23.cu", "et_yg_proj_r45.cu", "et_yg_proj_r67.cu",
            "et_yg_spread_r01.cu", "et_yg_spread_r23.cu", "et_yg_spread_r45.cu", "et_yg_spread_r67.cu",
            "et_yg_adjoint_r01.cu", "et_yg_adjoint_r23.cu", "et_yg_adjoint_r45.cu", "et_yg_adjoint_r67.cu",
+           "et_yg_dmu_r01.cu", "et_yg_dmu_r23.cu", "et_yg_dmu_r45.cu", "et_yg_dmu_r67.cu",
            "et_yg_back.cu", "et_yg_dmu.cu", "et_yg_grad.cu", "et_update.cu", "et_noalloc.cu", "et_plan.cpp", "et_fisher.cu", "et_nifti.cpp"]
 TOOL = os.path.join(HERE, "rec_spect")  # command-line reconstruction (csrc/rec_spect.cpp)
 

@@ -667,11 +667,10 @@ int project_partial_device(const Problem& pb, const float* d_act, const float* d
 size_t dmu_workspace(const Problem& pb) {
   if (use_fused_x(pb) && pb.storage == kStorageF32)  // the fused form's scratch, or the general path's volumes
     return std::max(general3_workspace(pb),
-                    common_bytes(pb) + (pb.det ? yg_dmu_det_workspace(pb.ny, pb.nx, pb.nz, pb.cams.n, pb.group) : 0) +
-                        kSlack);
+                    common_bytes(pb) + yg_dmu_workspace(pb.ny, pb.nx, pb.nz, pb.cams.n, pb.group) + kSlack);
   if (use_fused(pb) && pb.storage == kStorageF32)
     return common_bytes(pb) + sizeof(float) * (3 * col_n(pb) + sino_col_n(pb)) + 4 * 256 +
-           (pb.det ? yg_dmu_det_workspace(pb.nx, pb.ny, pb.nz, pb.cams.n, pb.group) + kSlack : 0);
+           yg_dmu_workspace(pb.nx, pb.ny, pb.nz, pb.cams.n, pb.group) + kSlack;
   return general3_workspace(pb);
 }
 
@@ -681,27 +680,25 @@ int dmu_device(const Problem& pb, const float* d_g, const float* d_act, const fl
     Carver cx(ws, ws_bytes);
     CamGeom* d_geom;
     float* d_psf;
-    int s = upload_common(pb, cx, &d_geom, &d_psf, stg, st, nullptr, true);
+    int2* d_units;
+    int s = upload_common(pb, cx, &d_geom, &d_psf, stg, st, &d_units, true);
     if (s != kOk) return s;
-    YgArgs a = x_args(pb, d_geom, d_psf, nullptr);
-    a.units = nullptr;
-    a.nunits = 0;
+    YgArgs a = x_args(pb, d_geom, d_psf, d_units);
     a.act = d_act;
     a.mu = d_att;
     a.sino = d_g;
     a.out = d_out;
-    if (pb.det) {
-      a.det = 1;
-      a.group = pb.group;
-      a.work = cx.take<float>(yg_dmu_det_workspace(a.nx, a.ny, a.nz, a.ncam, a.group) / sizeof(float));
-      if (!a.work) return kErrAllocGpu;
-    }
+    a.det = pb.det;
+    a.group = pb.group;
+    a.work = cx.take<float>(yg_dmu_workspace(a.nx, a.ny, a.nz, a.ncam, a.group) / sizeof(float));
+    if (!a.work) return kErrAllocGpu;
     return check(yg_dmu(a, st));
   }
   Carver cv(ws, ws_bytes);
   CamGeom* d_geom;
   float* d_psf;
-  int s = upload_common(pb, cv, &d_geom, &d_psf, stg, st);
+  int2* d_units;
+  int s = upload_common(pb, cv, &d_geom, &d_psf, stg, st, &d_units);
   if (s != kOk) return s;
   if (use_fused(pb) && pb.storage == kStorageF32) {
     const int cy = round_up(pb.ny, 4);
@@ -727,12 +724,12 @@ int dmu_device(const Problem& pb, const float* d_g, const float* d_act, const fl
     a.psf = d_psf;
     a.psf_host = pb.psf_k ? pb.psf_sep.data() : nullptr;
     a.psf_k = pb.psf_k;
-    if (pb.det) {
-      a.det = 1;
-      a.group = pb.group;
-      a.work = cv.take<float>(yg_dmu_det_workspace(a.nx, a.ny, a.nz, a.ncam, a.group) / sizeof(float));
-      if (!a.work) return kErrAllocGpu;
-    }
+    a.units = d_units;
+    a.nunits = static_cast<int>(pb.units.size() / 2);
+    a.det = pb.det;
+    a.group = pb.group;
+    a.work = cv.take<float>(yg_dmu_workspace(a.nx, a.ny, a.nz, a.ncam, a.group) / sizeof(float));
+    if (!a.work) return kErrAllocGpu;
     if ((s = yg_dmu(a, st)) != kOk) return s;
     return check(from_column(out_c, d_out, pb.nx, pb.ny, cy, pb.nz, 0, st));
   }

@@ -127,7 +127,10 @@ struct YgArgs {
   // the rotated-frame values go into the group scratch instead of vector
   // reductions into a.out, and a transposed gather (fixed order) sums them.
   int det = 0;
-  // d/dmu: first camera of the launch (scratch volume g = camera - cam0).
+  // d/dmu: first unit (or camera) of the launch, the scratch volume of an
+  // item's terms (its mirror camera's: group + vol0), the rays' coefficients.
+  int vol0 = 0;
+  float* coef = nullptr;
   int cam0 = 0;
 };
 // Carry slots per camera of the backprojector's transmission carries (the
@@ -161,8 +164,9 @@ int yg_project(const YgArgs& a, cudaStream_t st, int* slabs_used = nullptr);
 // (column layouts: a.act, a.mu; a.sino = g [ncam][nx][cy]; a.out = the
 // gradient [nz][nx][cy], zeroed here); no backgrounds.
 int yg_dmu(const YgArgs& a, cudaStream_t st);
-// Work space of yg_dmu with a.det (one scratch slot of a camera group).
-size_t yg_dmu_det_workspace(int nx, int ny, int nz, int ncam, int group);
+// Work space of yg_dmu: a group's scratch volumes and ray coefficients.
+constexpr int kDmuSlabs = 8;  // depth slabs at most
+size_t yg_dmu_workspace(int nx, int ny, int nz, int ncam, int group);
 // Deterministic transposed gather of scratch volumes a.temp[0 .. gcount) of
 // units (or cameras) c0 .. c0 + gcount - 1 into a.out (assigned when c0 == 0,
 // else added; clamp: negative results stored as zero), rows of the window a

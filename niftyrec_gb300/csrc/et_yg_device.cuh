@@ -766,10 +766,19 @@ __device__ __forceinline__ bool lane_writes(const YgArgs& a, int yb) { return yb
 constexpr float kMateMaxT = 40.0f;
 
 //
+// TERMS (d/dmu; float32 with mu): instead of the projection, the terms
+// v exp(-T) (T local to the slab) of every output column and plane go to the
+// scratch volume a.vol0 of a.temp, and per slab the coefficients A, B of
+//   -g S(z) = A + B * (the slab's terms before z),  S(z) = sum of the ray's terms from z on,
+// to a.coef ([volume][slab][nx][A, B][cs]); g = a.sino.  The mirror camera's go
+// to volume a.group + a.vol0, in this camera's frame: its depth sum runs
+// towards this camera, so its S(z) is A + B * (the slab's terms up to and with z).
+//
 // STEPS: depth planes sampled per barrier (2 x STEPS tile buffers).  Two
 // planes per barrier measured no faster on GB300 (128^3 x 120: 0.676 against
 // 0.674 ms; 256^3 x 180: 11.9 against 11.2 ms), so the kernels use one.
-template <int R, bool PSF, bool ATT, class V, bool PAIR = false, bool PTAB = false, int L = 32, int YB = L, int STEPS = 1>
+template <int R, bool PSF, bool ATT, class V, bool PAIR = false, bool PTAB = false, int L = 32, int YB = L,
+          bool TERMS = false, int STEPS = 1>
 __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate, int x0, unsigned char* smem,
                                              const float* ptab = nullptr) {
   using TS = TileShape<R, L>;
@@ -827,6 +836,13 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
     }
   };
   const CamRows cr = cam_rows(a.geom[cam].fwd);
+  const size_t tvol = static_cast<size_t>(a.nz) * a.nx * a.cs;
+  auto put_term = [&](int volume, int i, int z, const float4& w) {  // TERMS
+    const int x = x0 + grp * kTXW + i;
+    if (x < a.nx && yok && lane_writes(a, yb))
+      *reinterpret_cast<float4*>(a.temp + tvol * volume + (static_cast<size_t>(z) * a.nx + x) * a.cs + yb) = w;
+  };
+  __shared__ int s_direct;  // TERMS: the mate's terms carry the direct weights
 
   constexpr int NC = SCOMP ? 1 : kTXW;
   float4 T[kTXW], P[kTXW], cT[NC], cP[NC];  // c*: Kahan compensations (KAHAN without SCOMP)
@@ -904,7 +920,14 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
           const float4 e = kval(T[i], &cT[SCOMP ? 0 : i], 0, i);
           kadd(Q[i], nullptr, 2, i, mul4p(v, exp_neg4(make_float4(-e.x, -e.y, -e.z, -e.w))));
         } else {
-          fma4p(Q[i], v, exp_neg4(make_float4(-T[i].x, -T[i].y, -T[i].z, -T[i].w)));
+          const float4 e = exp_neg4(make_float4(-T[i].x, -T[i].y, -T[i].z, -T[i].w));
+          if constexpr (TERMS) {
+            const float4 w = mul4p(v, e);
+            add4p(Q[i], w);
+            put_term(a.group + a.vol0, i, z, w);
+          } else {
+            fma4p(Q[i], v, e);
+          }
         }
       } else {  // T runs from the slab's far end, inclusive
         const float4 m = sample4(mu, tb[tap_slot<R, L>(grp * kTXW + i + R)], yb, yok);
@@ -913,7 +936,13 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
           kadd(Q[i], nullptr, 2, i, mul4p(v, exp_neg4(kval(T[i], &cT[SCOMP ? 0 : i], 0, i))));
         } else {
           add4p(T[i], m);
-          fma4p(Q[i], v, exp_neg4(T[i]));
+          if constexpr (TERMS) {
+            const float4 w = mul4p(v, exp_neg4(T[i]));
+            add4p(Q[i], w);
+            put_term(a.group + a.vol0, i, z, w);
+          } else {
+            fma4p(Q[i], v, exp_neg4(T[i]));
+          }
         }
       }
     };
@@ -944,7 +973,13 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
           kadd(P[i], &cP[SCOMP ? 0 : i], 1, i, mul4p(v, exp_neg4(kval(T[i], &cT[SCOMP ? 0 : i], 0, i))));
         } else {
           add4p(T[i], m);
-          fma4p(P[i], v, exp_neg4(T[i]));
+          if constexpr (TERMS) {
+            const float4 w = mul4p(v, exp_neg4(T[i]));
+            add4p(P[i], w);
+            put_term(a.vol0, i, z, w);
+          } else {
+            fma4p(P[i], v, exp_neg4(T[i]));
+          }
         }
       } else {
         kadd(P[i], &cP[SCOMP ? 0 : i], 1, i, v);
@@ -1016,7 +1051,9 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
       redo |= !(T[i].x <= kMateMaxT && T[i].y <= kMateMaxT && T[i].z <= kMateMaxT && T[i].w <= kMateMaxT);
       redo |= !(isfinite(Q[i].x) && isfinite(Q[i].y) && isfinite(Q[i].z) && isfinite(Q[i].w));
     }
-    if (__syncthreads_or(redo)) {  // uniform over the CTA
+    const bool again = __syncthreads_or(redo);  // uniform over the CTA
+    if (TERMS && threadIdx.x == 0) s_direct = again;
+    if (again) {
 #pragma unroll
       for (int i = 0; i < kTXW; ++i) {
         Q[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1066,6 +1103,50 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
     // output o is merged by CTA o % nslabs of the cluster
     if (o % nslabs != slab || x >= a.nx || !yok || !lane_writes(a, yb)) continue;
     float4 Pt = make_float4(0.f, 0.f, 0.f, 0.f), Tt = make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (TERMS) {
+      const size_t step = static_cast<size_t>(a.nx) * 2 * a.cs;
+      auto coefs = [&](int volume) {
+        return a.coef + (static_cast<size_t>(volume) * nslabs * a.nx + x) * 2 * a.cs + yb;
+      };
+      auto plane = [&](int c, int column) {
+        return ldg4(a.sino + (static_cast<size_t>(c) * a.nx + column) * a.cy + a.row0 + yb);
+      };
+      auto put = [&](float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; };
+      auto neg_mul = [](const float4& g, const float4& v) {
+        return make_float4(-g.x * v.x, -g.y * v.y, -g.z * v.z, -g.w * v.w);
+      };
+      float* cf = coefs(a.vol0);
+      float4 g = plane(cam, x);
+      for (int s = 0; s < nslabs; ++s) {  // the slab's weighted partial, for now, and B = g exp(-T before it)
+        const float4 w = exp_neg4(Tt);
+        put(cf + s * step, mul4(w, cluster.map_shared_rank(sP, s)[o * L + lane]));
+        put(cf + s * step + a.cs, mul4(g, w));
+        add4(Tt, cluster.map_shared_rank(sT, s)[o * L + lane]);
+      }
+      for (int s = nslabs - 1; s >= 0; --s) {  // A = -g * (partials from this slab on)
+        add4(Pt, *reinterpret_cast<const float4*>(cf + s * step));
+        put(cf + s * step, neg_mul(g, Pt));
+      }
+      if (PAIR && paired) {
+        cf = coefs(a.group + a.vol0);
+        g = plane(mate, a.nx - 1 - x);
+        Tt = Pt = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int s = nslabs - 1; s >= 0; --s) {  // from the mate's side: Tt the mu between it and the slab
+          const float4 ts = cluster.map_shared_rank(sT, s)[o * L + lane];
+          put(cf + s * step, mul4(exp_neg4(Tt), cluster.map_shared_rank(sQ, s)[o * L + lane]));
+          float4 far = Tt;  // forward-form terms still lack exp(-slab)
+          add4(far, ts);
+          put(cf + s * step + a.cs, neg_mul(g, exp_neg4(*cluster.map_shared_rank(&s_direct, s) ? Tt : far)));
+          Tt = far;
+        }
+        for (int s = 0; s < nslabs; ++s) {  // A = -g * (partials before this slab)
+          const float4 own = *reinterpret_cast<const float4*>(cf + s * step);
+          put(cf + s * step, neg_mul(g, Pt));
+          add4(Pt, own);
+        }
+      }
+      continue;
+    }
     for (int s = 0; s < nslabs; ++s) {
       const float4* rT = cluster.map_shared_rank(sT, s);
       const float4* rP = cluster.map_shared_rank(sP, s);
