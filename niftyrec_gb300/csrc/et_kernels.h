@@ -214,8 +214,9 @@ struct BatchElems {
 };
 // Row windows the fused launchers use for ny rows and PSF width psf_k (0: no
 // PSF); writes 4 ints per window (row0, rows, lo, hi), returns the count or
-// -1 if more than max_windows.
-int yg_row_windows(int ny, int psf_k, int* out, int max_windows);
+// -1 if more than max_windows.  nx: columns, for the split of the last window
+// (0, or where the split does not fit max_windows: unsplit).
+int yg_row_windows(int ny, int psf_k, int* out, int max_windows, int nx = 0);
 // Lanes per column the tile kernels take for a window of `rows` rows of nx
 // columns, and the x-tiles that gives.
 void yg_window_lanes(int rows, int nx, int* lanes, int* tiles);

@@ -688,7 +688,7 @@ int nrgb_batch_create(void** out_batch, void* const* plans, int n_plans, void* s
       a.psf = p->psf;
       a.psf_k = pb.psf_k;
       a.truncate = 1;
-      d.nwin = yg_row_windows(pb.ny, pb.psf_k, &d.win[0][0], kMaxWindows);
+      d.nwin = yg_row_windows(pb.ny, pb.psf_k, &d.win[0][0], kMaxWindows, pb.nx);
       if (d.nwin < 0) {
         cudaFree(b->mem);
         destroy_batch_streams(b);

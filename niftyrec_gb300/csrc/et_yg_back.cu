@@ -80,68 +80,53 @@ __global__ void __launch_bounds__(32 * kSlabsB) k_mu_carry_yg(const YgArgs a, in
 // first: assign instead of adding to a.out; clamp: the last group of the
 // window with a.truncate -- negative sums become zero as they are stored.
 // L lanes hold one column, 32 / L lane groups per warp; footprints of
-// kGatherTaps units at a time sit in shared memory.
-template <int U, int L, int C>
+// kGatherTaps units at a time sit in shared memory.  One column and four units
+// in flight per group: 60 us a 30-unit group at 128^3 (two columns and two
+// units, the same loads in flight from half the warps, 66 us; three units 72).
+template <int U, int L>
 __global__ void __launch_bounds__(32 * kGatherWarps) k_gather_yg(const YgArgs a, int c0, int gcount, int first,
                                                                 int clamp) {
   constexpr int GROUPS = 32 * kGatherWarps / L;
-  __shared__ Tap s_gtap[GROUPS][kGatherTaps * C];
+  __shared__ Tap s_gtap[GROUPS][kGatherTaps];
   const int grp = threadIdx.x / L, lane = threadIdx.x % L;
-  const int nchunk = (a.nx + C - 1) / C;
   const int item = blockIdx.x * GROUPS + grp;
-  const int Z = item / nchunk;
-  const int X0 = (item % nchunk) * C;
+  const int Z = item / a.nx, X = item % a.nx;
   const int yb = lane * 4;
   const bool rows = Z < a.nz && lane_rows_ok(a, yb) && lane_writes(a, yb);
   Tap* tap = s_gtap[grp];
   const size_t vol = static_cast<size_t>(a.nz) * a.nx * a.cs;
-  // camera outer, columns inner: neighbouring accumulator columns of one
-  // camera share footprint columns, which then hit in L1; the loads of U
-  // units' volumes in flight at once (every footprint offset is inside its
-  // volume, see make_tap), added in unit order
-  float4 acc[C];
-#pragma unroll
-  for (int i = 0; i < C; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  // the loads of U units' volumes in flight at once (every footprint offset is
+  // inside its volume, see make_tap), added in unit order
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int g0 = 0; g0 < gcount; g0 += kGatherTaps) {
     const int n = min(kGatherTaps, gcount - g0);
     if (Z < a.nz)
-      for (int e = lane; e < C * n; e += L) {
-        const int g = c0 + g0 + e / C, X = X0 + e % C;
+      for (int e = lane; e < n; e += L) {
+        const int g = c0 + g0 + e;
         const CamRows cr = cam_rows(a.geom[a.units ? a.units[g].x : g].bwd);
         // footprints in the scratch (column stride cs)
-        tap[e] = make_tap(X, Z, cr.m00, cr.m02, cr.m03, cr.m20, cr.m22, cr.m23, a.nx, a.nz, a.cs, X < a.nx);
+        tap[e] = make_tap(X, Z, cr.m00, cr.m02, cr.m03, cr.m20, cr.m22, cr.m23, a.nx, a.nz, a.cs, true);
       }
     __syncwarp();
     if (rows) {
       const float* src = a.temp + vol * g0;
       int g = 0;
       for (; g + U <= n; g += U) {
-        float4 v[U][C];
+        float4 v[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u)
+        for (int u = 0; u < U; ++u) v[u] = sample4_loaded(src + vol * (g + u), tap[g + u], yb);
 #pragma unroll
-          for (int i = 0; i < C; ++i) v[u][i] = sample4_loaded(src + vol * (g + u), tap[(g + u) * C + i], yb);
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-          for (int i = 0; i < C; ++i) add4(acc[i], v[u][i]);
+        for (int u = 0; u < U; ++u) add4(acc, v[u]);
       }
-      for (; g < n; ++g)
-#pragma unroll
-        for (int i = 0; i < C; ++i) add4(acc[i], sample4(src + vol * g, tap[g * C + i], yb, true));
+      for (; g < n; ++g) add4(acc, sample4(src + vol * g, tap[g], yb, true));
     }
     __syncwarp();
   }
   if (!rows) return;
-#pragma unroll
-  for (int i = 0; i < C; ++i) {
-    const int X = X0 + i;
-    if (X >= a.nx) continue;
-    float4* dst = reinterpret_cast<float4*>(a.out + (static_cast<size_t>(Z) * a.nx + X) * a.cy + a.row0 + yb);
-    if (!first) add4(acc[i], *dst);
-    if (clamp) acc[i] = clamp0(acc[i]);
-    *dst = acc[i];
-  }
+  float4* dst = reinterpret_cast<float4*>(a.out + (static_cast<size_t>(Z) * a.nx + X) * a.cy + a.row0 + yb);
+  if (!first) add4(acc, *dst);
+  if (clamp) acc = clamp0(acc);
+  *dst = acc;
 }
 
 // Forward bilinear weight of corner (X, Z) in the footprint of rotated column
@@ -246,32 +231,20 @@ void launch_tgather(const YgArgs& b, int c0, int gcount, int clamp, cudaStream_t
   k_tgather_yg<<<blocks, 32 * kGatherWarps, 0, st>>>(b, c0, gcount, c0 == 0 ? 1 : 0, clamp);
 }
 
-template <int U, int L, int C>
+template <int L>
 void launch_gather_as(const YgArgs& b, int c0, int gcount, int clamp, cudaStream_t st) {
   constexpr int GROUPS = 32 * kGatherWarps / L;
-  const int items = (b.nx + C - 1) / C * b.nz;
+  const int items = b.nx * b.nz;
   NRGB_LAUNCH_SCOPE("k_gather_yg", st);
-  k_gather_yg<U, L, C>
+  k_gather_yg<kGatherUnits, L>
       <<<(items + GROUPS - 1) / GROUPS, 32 * kGatherWarps, 0, st>>>(b, c0, gcount, c0 == 0 ? 1 : 0, clamp);
-}
-
-// Two columns and two units in flight per lane group; where that leaves fewer
-// than four CTAs per SM (64^3 and below) one column and four units, so that
-// the grid has twice the warps and each as many loads in flight.
-template <int L>
-void launch_gather_lanes(const YgArgs& b, int c0, int gcount, int clamp, cudaStream_t st) {
-  const int ctas = (b.nx + 1) / 2 * b.nz / (32 * kGatherWarps / L);
-  if (ctas < 4 * sm_count())
-    launch_gather_as<2 * kGatherUnits, L, 1>(b, c0, gcount, clamp, st);
-  else
-    launch_gather_as<kGatherUnits, L, kGatherCols>(b, c0, gcount, clamp, st);
 }
 
 void launch_gather(const YgArgs& b, int c0, int gcount, int clamp, cudaStream_t st) {
   const int lanes = column_lanes(b.ny);
-  if (lanes == 8) launch_gather_lanes<8>(b, c0, gcount, clamp, st);
-  else if (lanes == 16) launch_gather_lanes<16>(b, c0, gcount, clamp, st);
-  else launch_gather_lanes<32>(b, c0, gcount, clamp, st);
+  if (lanes == 8) launch_gather_as<8>(b, c0, gcount, clamp, st);
+  else if (lanes == 16) launch_gather_as<16>(b, c0, gcount, clamp, st);
+  else launch_gather_as<32>(b, c0, gcount, clamp, st);
 }
 
 template <bool ADJ>
@@ -340,7 +313,7 @@ namespace {
 
 // Carries of units (or cameras) [u0, u0 + n).
 int mu_carry_range(const YgArgs& a_in, float* out, int u0, int n, cudaStream_t st) {
-  for (const Window& w : row_windows(a_in.ny, 0)) {  // carries need no halo
+  for (const Window& w : row_windows(a_in.ny, 0, a_in.nx)) {  // carries need no halo
     YgArgs a = windowed(a_in, w);
     a.slab_T = out;
     auto go = [&](auto v, auto lanes) {
@@ -429,7 +402,7 @@ int yg_backproject(const YgArgs& a_in, cudaStream_t st) {
     const bool three = !pair && a.mu && a.storage != kStorageBF16 && a.back_mode != kBackAdjoint;
     a.bslabs = yg_backproject_slabs(a.nx, a.ny, a.nz, scatter ? nunits : group, three ? 3 : 2);
   }
-  const std::vector<Window> wins = row_windows(a.ny, R);
+  const std::vector<Window> wins = call_windows(a, R);
   // work space: slab carries first (unless given), then the scratch slot(s)
   const size_t vol = static_cast<size_t>(a.nz) * a.nx * scratch_rows(a.ny);
   float* slot0;

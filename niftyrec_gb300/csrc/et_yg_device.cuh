@@ -58,8 +58,7 @@ constexpr int kSlabsB = 16;       // backprojector depth slabs
 constexpr int kCarrySlots = kSlabsB + 1;  // carries per camera: slab prefixes, column total
 constexpr int kCarryCols = 64 / kSlabsB;  // columns per CTA of the carry pass (32 KB of slab sums)
 constexpr int kGatherWarps = 4;   // warps per CTA of the inverse-rotation gather
-constexpr int kGatherCols = 2;    // accumulator columns per warp in the gather
-constexpr int kGatherUnits = 2;   // scratch volumes whose loads a gather warp has in flight at once
+constexpr int kGatherUnits = 4;   // scratch volumes whose loads a gather group has in flight at once
 constexpr int kGatherTaps = 16;   // scratch volumes whose footprints a gather group holds at once
 constexpr unsigned kFull = 0xffffffffu;
 
@@ -1223,18 +1222,32 @@ static_assert(kTX<32> == 32 && kTX<16> == 64 && kTX<8> == 128, "1024 / L output 
 // the fewest lanes that hold the rows.
 int column_lanes(int rows) { return rows <= 32 ? 8 : rows <= 64 ? 16 : 32; }
 
-std::vector<Window> row_windows(int ny, int halo) {
+//
+// nx > 0: a last window of 65 rows or more that a 64-row and a 32-row window
+// cover for fewer x-tiles is split so (192 rows with a halo of 8: 128 + 64 + 32
+// rows; 192^3 x 120 in bfloat16, PSF 15: pair 6.33 -> 6.06 ms).
+std::vector<Window> row_windows(int ny, int halo, int nx = 0) {
   const int h = (halo + 3) & ~3;
   std::vector<Window> w;
+  auto tiles = [&](int lanes) { return (nx + 1024 / lanes - 1) / (1024 / lanes); };
+  auto last = [&](int in0, int lo) {
+    const int rows = ny - in0, rest = rows - 64 + 2 * h;
+    if (nx > 0 && rows > 64 && rest <= 32 && lo < 64 - h && tiles(16) + tiles(8) < tiles(32)) {
+      w.push_back({in0, 64, lo, 64 - h});
+      w.push_back({in0 + 64 - 2 * h, rest, h, rest});
+    } else {
+      w.push_back({in0, rows, lo, rows});
+    }
+  };
   if (ny <= kWindowRows) {
-    w.push_back({0, ny, 0, ny});
+    last(0, 0);
     return w;
   }
   int out0 = 0;
   while (out0 < ny) {
     const int in0 = std::max(0, out0 - h);
     if (in0 + kWindowRows >= ny) {
-      w.push_back({in0, ny - in0, out0 - in0, ny - in0});
+      last(in0, out0 - in0);
       break;
     }
     const int out1 = in0 + kWindowRows - h;
@@ -1244,6 +1257,19 @@ std::vector<Window> row_windows(int ny, int halo) {
   return w;
 }
 
+// Whether the window kernels of this call take narrow windows with fewer lanes:
+// not with the separated PSF in shared memory, nor the attenuation gradient.
+bool narrow_windows(const YgArgs& a) {
+  if (a.gradient) return false;
+  return !a.psf || (a.psf_host && static_cast<size_t>(a.nz) * 2 * a.psf_k <= kPsfTableFloats);
+}
+
+// The row windows of a call for a PSF halo (the transposed gather of the
+// deterministic form works on whole warps: no split).
+std::vector<Window> call_windows(const YgArgs& a, int halo) {
+  return row_windows(a.ny, halo, narrow_windows(a) && !a.det ? a.nx : 0);
+}
+
 YgArgs windowed(const YgArgs& a, const Window& w) {
   YgArgs b = a;
   b.row0 = w.row0;
@@ -1251,7 +1277,7 @@ YgArgs windowed(const YgArgs& a, const Window& w) {
   b.out_lo = w.lo;
   b.out_hi = w.hi;
   b.cs = round_up(w.rows, 4);
-  b.lanes = window_lanes(w.rows, a.nx);
+  b.lanes = narrow_windows(a) ? window_lanes(w.rows, a.nx) : 32;
   return b;
 }
 

@@ -200,7 +200,7 @@ int yg_dmu(const YgArgs& a_in, cudaStream_t st) {
     const size_t full = static_cast<size_t>(a.nz) * a.nx * a.cy;
     if (cudaMemsetAsync(a.out, 0, sizeof(float) * full, st) != cudaSuccess) return kErrKernel;
   }
-  for (const Window& w : row_windows(a.ny, R)) {
+  for (const Window& w : call_windows(a, R)) {
     YgArgs b = windowed(a, w);
     b.temp = a.work;
     for (int c0 = 0; c0 < units; c0 += group) {

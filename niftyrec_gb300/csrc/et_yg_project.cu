@@ -215,7 +215,7 @@ int yg_project_batch(const BatchStepDesc* d_desc, const BatchSel& sel, int psf_k
 
 int yg_project(const YgArgs& a, cudaStream_t st, int* slabs_used) {
   const int R = a.psf ? (a.psf_k - 1) / 2 : 0;
-  const std::vector<Window> wins = row_windows(a.ny, R);
+  const std::vector<Window> wins = call_windows(a, R);
   int pslabs = a.pslabs;
   for (size_t i = 0; i < wins.size(); ++i) {
     int used[2] = {0, 0};

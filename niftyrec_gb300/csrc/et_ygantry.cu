@@ -168,8 +168,10 @@ bool wide_rows(const void* p, int nx) { return nx % 4 == 0 && (reinterpret_cast<
 
 }  // namespace
 
-int yg_row_windows(int ny, int psf_k, int* out, int max_windows) {
-  const std::vector<Window> w = row_windows(ny, psf_k > 0 ? (psf_k - 1) / 2 : 0);
+int yg_row_windows(int ny, int psf_k, int* out, int max_windows, int nx) {
+  const int halo = psf_k > 0 ? (psf_k - 1) / 2 : 0;
+  std::vector<Window> w = row_windows(ny, halo, nx);
+  if (static_cast<int>(w.size()) > max_windows) w = row_windows(ny, halo);
   if (static_cast<int>(w.size()) > max_windows) return -1;
   for (size_t i = 0; i < w.size(); ++i) {
     out[4 * i + 0] = w[i].row0;

@@ -22,7 +22,8 @@ def o32():
 
 
 @pytest.mark.parametrize("shape,k", [((20, 32, 68), 7), ((12, 30, 132), 11), ((14, 28, 130), 15), ((16, 64, 66), 0),
-                                     ((15, 61, 66), 15), ((13, 33, 65), 9), ((12, 65, 70), 5), ((10, 140, 132), 11),
+                                     ((15, 61, 66), 15), ((13, 33, 65), 9), ((12, 65, 70), 5), ((10, 140, 132), 11), ((9, 80, 100), 13),
+                                     ((8, 192, 98), 15), ((10, 81, 100), 11), ((9, 88, 129), 9),
                                      ((9, 160, 66), 13), ((12, 31, 32), 3), ((11, 4, 129), 5)])
 @pytest.mark.parametrize("cams", ["opposite", "half-turn"])
 def test_narrow_windows(o32, shape, k, cams):
