@@ -761,12 +761,10 @@ int gradient_device(const Problem& pb, const float* d_sino, const float* d_act, 
     Carver cx(ws, ws_bytes);
     CamGeom* d_geom;
     float* d_psf;
-    int s = upload_common(pb, cx, &d_geom, &d_psf, stg, st, nullptr, true);
+    int2* d_units;
+    int s = upload_common(pb, cx, &d_geom, &d_psf, stg, st, &d_units, true);
     if (s != kOk) return s;
-    YgArgs a = x_args(pb, d_geom, d_psf, nullptr);
-    a.units = nullptr;
-    a.nunits = 0;
-    a.gradient = 1;
+    YgArgs a = x_args(pb, d_geom, d_psf, d_units);
     a.act = d_act;
     a.mu = d_att;
     a.sino = d_sino;
@@ -774,12 +772,13 @@ int gradient_device(const Problem& pb, const float* d_sino, const float* d_act, 
     a.group = grad_group(pb);
     a.work = cx.take<float>(yg_gradient_workspace(pb.ny, pb.nx, pb.nz, pb.cams.n, a.group) / sizeof(float));
     if (!a.work) return kErrAllocGpu;
-    return check(yg_backproject(a, st));  // the last gathers clamp when truncating
+    return check(yg_gradient(a, st));
   }
   Carver cv(ws, ws_bytes);
   CamGeom* d_geom;
   float* d_psf;
-  int s = upload_common(pb, cv, &d_geom, &d_psf, stg, st);
+  int2* d_units;
+  int s = upload_common(pb, cv, &d_geom, &d_psf, stg, st, &d_units);
   if (s != kOk) return s;
   if (use_fused(pb) && pb.storage == kStorageF32) {
     const int cy = round_up(pb.ny, 4);
@@ -807,11 +806,11 @@ int gradient_device(const Problem& pb, const float* d_sino, const float* d_act, 
     a.psf = d_psf;
     a.psf_host = pb.psf_k ? pb.psf_sep.data() : nullptr;
     a.psf_k = pb.psf_k;
-    a.pslabs = pb.pslabs;
-    a.gradient = 1;
+    a.units = d_units;
+    a.nunits = static_cast<int>(pb.units.size() / 2);
     a.group = group;
     a.work = work;
-    if ((s = yg_backproject(a, st)) != kOk) return s;
+    if ((s = yg_gradient(a, st)) != kOk) return s;
     return check(from_column(out_c, d_out, pb.nx, pb.ny, cy, pb.nz, pb.truncate, st));
   }
   GeneralArgs g;

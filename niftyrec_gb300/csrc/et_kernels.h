@@ -119,10 +119,8 @@ struct YgArgs {
   const float* carry = nullptr;
   // yg_backproject (reference form, deterministic transpose): the window's
   // last gather stores max(result, 0) when a.truncate is set.
-  // Non-zero: yg_backproject spreads the reference's attenuation gradient
-  // instead (a.act and a.mu sampled, a.sino the camera planes; no carries,
-  // no mirror units), then gathers it like the reference-mode backprojection.
-  int gradient = 0;
+  // Gather: 1 takes the units' mirror cameras (skipping units without one).
+  int mates = 0;
   // Non-zero (exact-transpose backprojector, d/dmu): deterministic form --
   // the rotated-frame values go into the group scratch instead of vector
   // reductions into a.out, and a transposed gather (fixed order) sums them.
@@ -173,12 +171,15 @@ size_t yg_dmu_workspace(int nx, int ny, int nz, int ncam, int group);
 // describes.
 void yg_tgather(const YgArgs& a, int c0, int gcount, int clamp, cudaStream_t st);
 int yg_backproject(const YgArgs& a, cudaStream_t st);
-// Spread of the reference attenuation gradient for cameras [c0, c0 + gcount)
-// into the scratch volumes a.temp (one row window: a.row0, a.ny, a.cs).
-int yg_grad_spread(const YgArgs& a, int c0, int gcount, cudaStream_t st);
-// Bytes of work space of the fused attenuation gradient (`slots` scratch
-// volumes of `group` cameras each; no carries).
-size_t yg_gradient_workspace(int nx, int ny, int nz, int ncam, int group, int slots = 2);
+// Inverse-rotation gather of scratch volumes a.temp[0 .. gcount) of units (or
+// cameras) c0 .. into a.out (first: assign, else add; clamp: negative results
+// stored as zero), rows of the window a describes.
+void yg_gather(const YgArgs& a, int c0, int gcount, int first, int clamp, cudaStream_t st);
+// The reference's attenuation gradient (a.act, a.mu sampled, a.sino the camera
+// planes, a.out the gradient; with a.truncate negative results are stored as
+// zero); a.work holds yg_gradient_workspace bytes.
+int yg_gradient(const YgArgs& a, cudaStream_t st);
+size_t yg_gradient_workspace(int nx, int ny, int nz, int ncam, int group);
 
 // ---- batches of volumes (one OSEM subset step of many plans at once) ----
 constexpr int kMaxBatch = 64;    // volumes per batched launch

@@ -103,9 +103,10 @@ __global__ void __launch_bounds__(32 * kGatherWarps) k_gather_yg(const YgArgs a,
     if (Z < a.nz)
       for (int e = lane; e < n; e += L) {
         const int g = c0 + g0 + e;
-        const CamRows cr = cam_rows(a.geom[a.units ? a.units[g].x : g].bwd);
-        // footprints in the scratch (column stride cs)
-        tap[e] = make_tap(X, Z, cr.m00, cr.m02, cr.m03, cr.m20, cr.m22, cr.m23, a.nx, a.nz, a.cs, true);
+        const int cam = !a.units ? g : a.mates ? a.units[g].y : a.units[g].x;
+        // footprints in the scratch (column stride cs); none without a camera
+        const CamRows cr = cam_rows(a.geom[max(cam, 0)].bwd);
+        tap[e] = make_tap(X, Z, cr.m00, cr.m02, cr.m03, cr.m20, cr.m22, cr.m23, a.nx, a.nz, a.cs, cam >= 0);
       }
     __syncwarp();
     if (rows) {
@@ -232,20 +233,24 @@ void launch_tgather(const YgArgs& b, int c0, int gcount, int clamp, cudaStream_t
 }
 
 template <int L>
-void launch_gather_as(const YgArgs& b, int c0, int gcount, int clamp, cudaStream_t st) {
+void launch_gather_as(const YgArgs& b, int c0, int gcount, int first, int clamp, cudaStream_t st) {
   constexpr int GROUPS = 32 * kGatherWarps / L;
   const int items = b.nx * b.nz;
   NRGB_LAUNCH_SCOPE("k_gather_yg", st);
   k_gather_yg<kGatherUnits, L>
-      <<<(items + GROUPS - 1) / GROUPS, 32 * kGatherWarps, 0, st>>>(b, c0, gcount, c0 == 0 ? 1 : 0, clamp);
+      <<<(items + GROUPS - 1) / GROUPS, 32 * kGatherWarps, 0, st>>>(b, c0, gcount, first, clamp);
 }
 
-void launch_gather(const YgArgs& b, int c0, int gcount, int clamp, cudaStream_t st) {
+}  // namespace
+
+void yg_gather(const YgArgs& b, int c0, int gcount, int first, int clamp, cudaStream_t st) {
   const int lanes = column_lanes(b.ny);
-  if (lanes == 8) launch_gather_as<8>(b, c0, gcount, clamp, st);
-  else if (lanes == 16) launch_gather_as<16>(b, c0, gcount, clamp, st);
-  else launch_gather_as<32>(b, c0, gcount, clamp, st);
+  if (lanes == 8) launch_gather_as<8>(b, c0, gcount, first, clamp, st);
+  else if (lanes == 16) launch_gather_as<16>(b, c0, gcount, first, clamp, st);
+  else launch_gather_as<32>(b, c0, gcount, first, clamp, st);
 }
+
+namespace {
 
 template <bool ADJ>
 int spread_pair_by_radius(int R, const YgArgs& a, int u0, int gcount, cudaStream_t st) {
@@ -295,11 +300,6 @@ size_t yg_backproject_workspace(int nx, int ny, int nz, int ncam, int group, int
   const size_t slabs = static_cast<size_t>(ncam) * kCarrySlots * nx * cy;  // at most kSlabsB slabs
   // with two slots the spread of group g+1 overlaps the gather of group g
   return sizeof(float) * (slabs + static_cast<size_t>(slots) * vol * std::max(1, std::min(group, ncam)));
-}
-
-size_t yg_gradient_workspace(int nx, int ny, int nz, int ncam, int group, int slots) {
-  const size_t vol = static_cast<size_t>(nz) * nx * scratch_rows(ny);
-  return sizeof(float) * static_cast<size_t>(slots) * vol * std::max(1, std::min(group, ncam));
 }
 
 int yg_carry_slabs() { return kCarrySlots; }
@@ -388,7 +388,7 @@ int yg_backproject(const YgArgs& a_in, cudaStream_t st) {
   if (a.bslabs < 0 || a.bslabs > kSlabsB) return kErrParameters;
   const int R = a.psf ? (a.psf_k - 1) / 2 : 0;
   // mirror units: float32 mu, or bfloat16 mu in reference mode
-  const bool pair = !a.gradient && a.units && a.nunits > 0 &&
+  const bool pair = a.units && a.nunits > 0 &&
                     (a.storage != kStorageBF16 || a.back_mode != kBackAdjoint);
   if (!pair) {
     a.units = nullptr;
@@ -398,7 +398,7 @@ int yg_backproject(const YgArgs& a_in, cudaStream_t st) {
   // even groups of at most a.group units
   int group = yg_even_group(nunits, a.group);
   if (a.bslabs == 0) {
-    const bool scatter = a.back_mode == kBackAdjoint && !a.gradient && !a.det;  // every unit in one launch
+    const bool scatter = a.back_mode == kBackAdjoint && !a.det;  // every unit in one launch
     const bool three = !pair && a.mu && a.storage != kStorageBF16 && a.back_mode != kBackAdjoint;
     a.bslabs = yg_backproject_slabs(a.nx, a.ny, a.nz, scatter ? nunits : group, three ? 3 : 2);
   }
@@ -408,7 +408,7 @@ int yg_backproject(const YgArgs& a_in, cudaStream_t st) {
   float* slot0;
   // carries of every unit first (computing group g+1's carries on the gather
   // stream while group g spreads measured no faster on GB300)
-  if (a.gradient || a.carry || !a.mu) {  // carries given, or not needed
+  if (a.carry || !a.mu) {  // carries given, or not needed
     a.slab_T = const_cast<float*>(a.carry);
     slot0 = a.work;
   } else {
@@ -420,9 +420,8 @@ int yg_backproject(const YgArgs& a_in, cudaStream_t st) {
   if (a.sino_ready) cudaStreamWaitEvent(st, static_cast<cudaEvent_t>(a.sino_ready), 0);
   a.group = group;
   // the exact transpose in its deterministic form: group scratch + transposed gather
-  const bool tgather = a.back_mode == kBackAdjoint && !a.gradient && a.det;
+  const bool tgather = a.back_mode == kBackAdjoint && a.det;
   auto spread_on = [&](const YgArgs& b, int c0, int gcount, cudaStream_t ss) {
-    if (a.gradient) return yg_grad_spread(b, c0, gcount, ss);
     if (tgather)
       return pair ? spread_pair_by_radius<true>(R, b, c0, gcount, ss) : spread_by_radius_t<true>(R, b, c0, gcount, ss);
     return pair ? spread_pair_by_radius<false>(R, b, c0, gcount, ss) : spread_by_radius(R, b, c0, gcount, ss);
@@ -433,10 +432,10 @@ int yg_backproject(const YgArgs& a_in, cudaStream_t st) {
     if (tgather)
       launch_tgather(b, c0, gcount, clamp, gs);
     else
-      launch_gather(b, c0, gcount, clamp, gs);
+      yg_gather(b, c0, gcount, c0 == 0 ? 1 : 0, clamp, gs);
   };
   auto spread = [&](const YgArgs& b, int c0, int gcount) { return spread_on(b, c0, gcount, st); };
-  if (a.back_mode == kBackAdjoint && !a.gradient && !a.det) {
+  if (a.back_mode == kBackAdjoint && !a.det) {
     // transpose of the projector: one launch per window over all cameras,
     // scattered straight into the zeroed accumulator
     const size_t full = static_cast<size_t>(a.nz) * a.nx * a.cy;

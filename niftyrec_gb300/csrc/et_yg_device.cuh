@@ -1258,9 +1258,8 @@ std::vector<Window> row_windows(int ny, int halo, int nx = 0) {
 }
 
 // Whether the window kernels of this call take narrow windows with fewer lanes:
-// not with the separated PSF in shared memory, nor the attenuation gradient.
+// not with the separated PSF in shared memory.
 bool narrow_windows(const YgArgs& a) {
-  if (a.gradient) return false;
   return !a.psf || (a.psf_host && static_cast<size_t>(a.nz) * 2 * a.psf_k <= kPsfTableFloats);
 }
 

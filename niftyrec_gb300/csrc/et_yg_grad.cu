@@ -5,241 +5,366 @@
 // inclusive depth sum of m, s the sinogram plane):
 //   w(x, y, z) = s(x, y) * sum_{z' >= z} a_z' exp(-T_z'),
 // then the per-plane PSF (as in the projector) and the inverse-rotation
-// gather into the accumulator.  The gather and the camera-group pipeline are
-// the reference-mode backprojector's; this file holds the spread that writes
-// PSF(w) of a camera group into the scratch volumes.
-//
-// Work item as the projector's: a cluster of depth-slab CTAs per (camera,
-// 32-column tile), every CTA owning the NS = 32 + 2R sampled columns its PSF
-// needs.  Walk 1 sums the slab's local transmission T_s and partial
-// P_s = sum a exp(-T_local) per sampled column; the cluster exchanges them
-// through distributed shared memory, so slab s knows the transmission before
-// it (Tb) and the weighted partials of the slabs after it
-// (later = sum_{r > s} exp(-Tb_r) P_r).  Walk 2 runs from the slab's far end
-// with the global transmission V = Tb + T_s (decremented by each plane's mu)
-// and the suffix W = later + sum a exp(-V), so every term is added, none
-// cancelled; s * W goes into the shared tile and the row / column passes of
-// the plane write PSF(w) to the scratch.
+// gather into the accumulator.  Three kernels per group of cameras:
+//   k_grad_weights_yg: w of a camera and its mirror camera from one set of
+//     samples (no PSF halo: every column once), each in its own frame;
+//   k_grad_conv_yg: the PSF of the w volumes into the scratch volumes;
+//   the backprojector's gather, each volume at its own camera's positions.
+// Every sum over depth adds its terms (none is taken as a difference): the
+// camera's suffix and the mirror camera's, which is a prefix in this frame,
+// run over terms that the first walk left in the volume itself.
+// 128^3 x 120, PSF 11: 1.26 ms, against 2.10 ms of one spread kernel per camera
+// that sampled activity and mu twice, halo columns included.
 #include "et_yg_device.cuh"
 
 namespace nrgb {
 namespace {
 
-template <int R, bool PSF, bool PTAB>
-__device__ __forceinline__ void grad_item(const YgArgs& a, int cam, int g, int x0, unsigned char* smem,
-                                          const float* ptab) {
-  using TS = TileShape<R, 32>;
-  constexpr int NS = TS::NS;
-  constexpr int OWN = TS::kOwn;
-  constexpr int K = 2 * R + 1;
-  constexpr size_t kSb = TS::sb_bytes(false);
-  static_assert(kSb >= sizeof(float4) * 2 * NS * 32, "the exchange needs two NS x 32 arrays");
+constexpr int kGradCols = 2;    // columns per lane group of k_grad_weights_yg
+constexpr int kGradPlanes = 8;  // planes whose terms its second walk has in flight
+
+// One warp per depth slab (kSlabsB of them), 32 / L lane groups of kGradCols
+// columns each; a block holds its columns' whole depth, so the slabs exchange
+// through shared memory.  Volume g of a.temp: w of the unit's camera (walk 1
+// leaves the terms a exp(-T) there, T local to the slab); volume a.group + g,
+// in the mirror camera's frame: the mate's (walk 1: the running sum of
+// a exp(E), E the slab's mu before the plane; a slab whose mu exceeds kMateMaxT
+// is summed again with the direct weights exp(E - slab)).
+// Bound by gather latency and by the volumes' traffic.  One block per SM with
+// the registers it wants: 1.24 ms a call at 128^3 x 120, 1.37 ms with two blocks
+// of 64 registers, which spill.
+template <int L>
+__global__ void __launch_bounds__(32 * kSlabsB) k_grad_weights_yg(const YgArgs a, int u0) {
+  constexpr int C = kGradCols, GW = 32 / L;
   const float* __restrict__ act = a.act + a.row0;
   const float* __restrict__ mu = a.mu + a.row0;
-  float4* sb = reinterpret_cast<float4*>(smem);                         // [2][NS][32]
-  Tap* taps = reinterpret_cast<Tap*>(smem + kSb);                        // [2][kTapSlots]
-  float* s_psf = reinterpret_cast<float*>(smem + kSb + TS::kTapBytes);   // [nz][2K]
-
-  cg::cluster_group cluster = cg::this_cluster();
-  const int slab = static_cast<int>(cluster.block_rank());
-  const int nslabs = static_cast<int>(cluster.num_blocks());
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  extern __shared__ __align__(16) unsigned char smem[];
+  float4(*sT)[C][32] = reinterpret_cast<float4(*)[C][32]>(smem);  // [kSlabsB][C][32], then P, Q
+  float4(*sP)[C][32] = sT + kSlabsB;
+  float4(*sQ)[C][32] = sP + kSlabsB;
+  __shared__ Tap s_tap[kSlabsB][GW][C];
+  const int slab = threadIdx.x >> 5, wlane = threadIdx.x & 31, sub = wlane / L, lane = wlane % L;
+  const int nchunk = (a.nx + C * GW - 1) / (C * GW);
+  const int g = blockIdx.x / nchunk;
+  const int2 uc = a.units ? a.units[u0 + g] : make_int2(u0 + g, -1);
+  const bool paired = uc.y >= 0;  // uniform over the block
+  const int x0 = ((blockIdx.x % nchunk) * GW + sub) * C;
   const int yb = lane * 4;
   const bool yok = lane_rows_ok(a, yb);
-  const int zper = (a.nz + nslabs - 1) / nslabs;
+  const CamRows cr = cam_rows(a.geom[uc.x].fwd);
+  const int zper = (a.nz + kSlabsB - 1) / kSlabsB;
   const int zbeg = slab * zper, zend = min(a.nz, zbeg + zper);
-  if (PSF && !PTAB)
-    for (int i = zbeg * 2 * K + threadIdx.x; i < zend * 2 * K; i += blockDim.x) s_psf[i] = __ldg(a.psf + i);
-  const CamRows cr = cam_rows(a.geom[cam].fwd);
-  const float* __restrict__ srow = a.sino + static_cast<size_t>(cam) * a.nx * a.cy + a.row0;
-  float* __restrict__ tmp = a.temp + static_cast<size_t>(a.nz) * a.nx * a.cs * g;
+  const size_t vol = static_cast<size_t>(a.nz) * a.nx * a.cs;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto mine = [&](int z, int x) {  // the camera's w at (z, x)
+    return reinterpret_cast<float4*>(a.temp + vol * g + (static_cast<size_t>(z) * a.nx + x) * a.cs + yb);
+  };
+  auto mates = [&](int z, int x) {  // the mate's, in its own frame
+    return reinterpret_cast<float4*>(a.temp + vol * (a.group + g) +
+                                     (static_cast<size_t>(a.nz - 1 - z) * a.nx + a.nx - 1 - x) * a.cs + yb);
+  };
+  auto footprints = [&](int z) {
+    if (lane < C)
+      s_tap[slab][sub][lane] = make_tap(x0 + lane, z, cr.m00, cr.m02, cr.m03, cr.m20, cr.m22, cr.m23, a.nx, a.nz,
+                                        a.cy, x0 + lane < a.nx);
+    __syncwarp();
+  };
 
-  // footprints of the columns this warp samples (c = warp + kW * k), shared
-  // within the warp through buffer b of the tap slots
-  auto footprints = [&](int z, int b) {
-    Tap* tb = taps + b * TS::kTapSlots;
-    if (lane < OWN) {
-      const int c = warp + kW * lane;
-      if (c < NS) {
-        const int xp = x0 - R + c;
-        tb[tap_slot<R, 32>(c)] = make_tap(xp, z, cr.m00, cr.m02, cr.m03, cr.m20, cr.m22, cr.m23, a.nx, a.nz, a.cy,
-                                      xp >= 0 && xp < a.nx);
+  // walk 1: terms, and the slab's transmission and partials
+  float4 T[C], P[C], Q[C];
+#pragma unroll
+  for (int i = 0; i < C; ++i) T[i] = P[i] = Q[i] = zero;
+  for (int z = zbeg; z < zend; ++z) {
+    footprints(z);
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+      const Tap& t = s_tap[slab][sub][i];
+      const float4 m = sample4(mu, t, yb, yok), x = sample4(act, t, yb, yok);
+      const bool ok = x0 + i < a.nx && yok;
+      if (paired) {
+        add4p(Q[i], mul4p(x, exp_neg4(make_float4(-T[i].x, -T[i].y, -T[i].z, -T[i].w))));
+        if (ok) *mates(z, x0 + i) = Q[i];
       }
+      add4p(T[i], m);
+      const float4 e = mul4p(x, exp_neg4(T[i]));
+      add4p(P[i], e);
+      if (ok) *mine(z, x0 + i) = e;
     }
     __syncwarp();
-    return tb;
+  }
+  bool direct = false;  // uniform over the warp: the mate's sums carry the direct weights
+  if (paired) {
+    bool redo = false;
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+      redo |= !(T[i].x <= kMateMaxT && T[i].y <= kMateMaxT && T[i].z <= kMateMaxT && T[i].w <= kMateMaxT);
+      redo |= !(isfinite(Q[i].x) && isfinite(Q[i].y) && isfinite(Q[i].z) && isfinite(Q[i].w));
+    }
+    direct = __any_sync(kFull, redo);
+    if (direct) {
+      float4 E[C];
+#pragma unroll
+      for (int i = 0; i < C; ++i) E[i] = Q[i] = zero;
+      for (int z = zbeg; z < zend; ++z) {
+        footprints(z);
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+          const Tap& t = s_tap[slab][sub][i];
+          const float4 after = make_float4(T[i].x - E[i].x, T[i].y - E[i].y, T[i].z - E[i].z, T[i].w - E[i].w);
+          fma4(Q[i], sample4(act, t, yb, yok), exp_neg4(after));
+          if (x0 + i < a.nx && yok) *mates(z, x0 + i) = Q[i];
+          add4(E[i], sample4(mu, t, yb, yok));
+        }
+        __syncwarp();
+      }
+    }
+  }
+
+  // slabs: w = exp(-mu before), later = the weighted partials after this slab;
+  // the mate's from the other end
+#pragma unroll
+  for (int i = 0; i < C; ++i) sT[slab][i][wlane] = T[i];
+  __syncthreads();
+  float4 w[C], wm[C];
+#pragma unroll
+  for (int i = 0; i < C; ++i) {
+    float4 before = zero, after = direct ? zero : T[i];
+    for (int s = 0; s < slab; ++s) add4(before, sT[s][i][wlane]);
+    for (int s = kSlabsB - 1; s > slab; --s) add4(after, sT[s][i][wlane]);
+    w[i] = exp_neg4(before);
+    wm[i] = exp_neg4(after);
+    sP[slab][i][wlane] = mul4(w[i], P[i]);
+    sQ[slab][i][wlane] = mul4(wm[i], Q[i]);
+  }
+  __syncthreads();
+  // walk 2: w = s * (later + weight * running sum), in place
+#pragma unroll
+  for (int i = 0; i < C; ++i) {
+    const int x = x0 + i;
+    if (x >= a.nx || !yok) continue;
+    float4 later = zero, run = zero;
+    for (int s = kSlabsB - 1; s > slab; --s) add4(later, sP[s][i][wlane]);
+    const float4 sc = ldg4(a.sino + (static_cast<size_t>(uc.x) * a.nx + x) * a.cy + a.row0 + yb);
+    for (int z = zend - 1; z >= zbeg; z -= kGradPlanes) {
+      float4 e[kGradPlanes];  // loaded before the stores below, which the compiler cannot move them over
+#pragma unroll
+      for (int q = 0; q < kGradPlanes; ++q) e[q] = z - q >= zbeg ? *mine(z - q, x) : zero;
+#pragma unroll
+      for (int q = 0; q < kGradPlanes; ++q) {
+        if (z - q < zbeg) break;
+        float4 v = later;
+        add4p(run, e[q]);
+        fma4p(v, w[i], run);
+        *mine(z - q, x) = mul4p(sc, v);
+      }
+    }
+    if (paired) {
+      float4 earlier = zero;
+      for (int s = 0; s < slab; ++s) add4(earlier, sQ[s][i][wlane]);
+      const float4 sm = ldg4(a.sino + (static_cast<size_t>(uc.y) * a.nx + a.nx - 1 - x) * a.cy + a.row0 + yb);
+      for (int z = zbeg; z < zend; z += kGradPlanes) {
+        float4 e[kGradPlanes];
+#pragma unroll
+        for (int q = 0; q < kGradPlanes; ++q) e[q] = z + q < zend ? *mates(z + q, x) : zero;
+#pragma unroll
+        for (int q = 0; q < kGradPlanes; ++q) {
+          if (z + q >= zend) break;
+          float4 v = earlier;
+          fma4p(v, wm[i], e[q]);
+          *mates(z + q, x) = mul4p(sm, v);
+        }
+      }
+    }
+  }
+}
+
+// PSF of the w volumes: volume v of the launch from a.temp to a.out (both
+// [v][nz][nx][cs]); with a.units the volumes from a.nunits on are the mirror
+// cameras' (skipped where a unit has none).  CTA = (volume, x-tile, depth slab).
+template <int R, bool PTAB, int L>
+__device__ __forceinline__ void grad_conv_body(const YgArgs& a, int u0, int n, const float* ptab) {
+  using TS = TileShape<R, L>;
+  constexpr int NS = TS::NS, K = 2 * R + 1;
+  extern __shared__ __align__(16) unsigned char smem[];
+  float4* sb = reinterpret_cast<float4*>(smem);                       // [2][NS][L]
+  float* s_psf = reinterpret_cast<float*>(smem + TS::kSbBytes);        // [nz][2K]
+  const int grp = threadIdx.x / L, lane = threadIdx.x % L;
+  const int ntile = (a.nx + kTX<L> - 1) / kTX<L>;
+  const int slab = blockIdx.x % a.bslabs, item = blockIdx.x / a.bslabs;
+  const int x0 = (item % ntile) * kTX<L>;
+  int v = item / ntile;
+  if (v >= n) {
+    if (a.units[u0 + v - n].y < 0) return;  // uniform over the CTA
+    v += a.group - n;
+  }
+  const int yb = lane * 4;
+  const bool yok = lane_rows_ok(a, yb);
+  const int zper = (a.nz + a.bslabs - 1) / a.bslabs;
+  const int zbeg = slab * zper, zend = min(a.nz, zbeg + zper);
+  if (!PTAB)
+    for (int i = zbeg * 2 * K + threadIdx.x; i < zend * 2 * K; i += blockDim.x) s_psf[i] = __ldg(a.psf + i);
+  const size_t vol = static_cast<size_t>(a.nz) * a.nx * a.cs;
+  const float* __restrict__ src = a.temp + vol * v + yb;
+  float* __restrict__ dst = a.out + vol * v + yb;
+  ybuf_zero_pads<L>();
+  __syncthreads();
+  auto load = [&](int z, float4 (&r)[TS::kOwn]) {
+#pragma unroll
+    for (int k = 0; k < TS::kOwn; ++k) {
+      const int c = grp + TS::G * k, xp = x0 - R + c;
+      r[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c < NS && xp >= 0 && xp < a.nx && yok) r[k] = ldg4(src + (static_cast<size_t>(z) * a.nx + xp) * a.cs);
+    }
   };
-
-  ybuf_zero_pads<32>();  // ordered before walk 2 by the cluster barriers
-
-  // walk 1: the slab's transmission and partial per sampled column
-  float4 T[OWN], P[OWN];
-#pragma unroll
-  for (int k = 0; k < OWN; ++k) {
-    T[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    P[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
+  float4 next[TS::kOwn];  // the next plane's columns, in flight during this plane's passes
+  if (zbeg < zend) load(zbeg, next);
   for (int z = zbeg; z < zend; ++z) {
-    const Tap* tb = footprints(z, z & 1);
+    float4* sbuf = sb + (z & 1) * NS * L;
 #pragma unroll
-    for (int k = 0; k < OWN; ++k) {
-      const int c = warp + kW * k;
-      if (c < NS) {
-        const Tap& t = tb[tap_slot<R, 32>(c)];
-        add4(T[k], sample4(mu, t, yb, yok));
-        fma4(P[k], sample4(act, t, yb, yok), exp_neg4(T[k]));
-      }
-    }
-  }
-
-  // exchange through distributed shared memory (the tile region is unused so far)
-  float4* sT = sb;
-  float4* sP = sb + NS * 32;
-#pragma unroll
-  for (int k = 0; k < OWN; ++k) {
-    const int c = warp + kW * k;
-    if (c < NS) {
-      sT[c * 32 + lane] = T[k];
-      sP[c * 32 + lane] = P[k];
-    }
-  }
-  cluster.sync();
-  // V: global transmission at the slab's last plane; W: the suffix from the
-  // slabs after this one
-#pragma unroll
-  for (int k = 0; k < OWN; ++k) {
-    const int c = warp + kW * k;
-    if (c >= NS) continue;
-    float4 tacc = make_float4(0.f, 0.f, 0.f, 0.f), later = tacc, before = tacc;
-    for (int s = 0; s < nslabs; ++s) {
-      if (s == slab) before = tacc;
-      if (s > slab) fma4(later, exp_neg4(tacc), cluster.map_shared_rank(sP, s)[c * 32 + lane]);
-      add4(tacc, cluster.map_shared_rank(sT, s)[c * 32 + lane]);
-    }
-    add4(before, T[k]);
-    T[k] = before;  // V
-    P[k] = later;   // W
-  }
-  cluster.sync();  // every CTA's exchange reads are done before the tiles are rewritten
-
-  // walk 2, from the slab's far end
-  const int n = zend - zbeg;
-  for (int j = 0; j < n; ++j) {
-    const int z = zend - 1 - j;
-    const int b = j & 1;
-    float4* sbuf = sb + b * NS * 32;
-    const Tap* tb = footprints(z, b);
-#pragma unroll
-    for (int k = 0; k < OWN; ++k) {
-      const int c = warp + kW * k;
-      if (c < NS) {
-        const Tap& t = tb[tap_slot<R, 32>(c)];
-        const float4 m = sample4(mu, t, yb, yok);
-        fma4(P[k], sample4(act, t, yb, yok), exp_neg4(T[k]));
-        T[k] = make_float4(T[k].x - m.x, T[k].y - m.y, T[k].z - m.z, T[k].w - m.w);
-        const int xp = x0 - R + c;
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (xp >= 0 && xp < a.nx && yok) s = ldg4(srow + static_cast<size_t>(xp) * a.cy + yb);
-        sbuf[c * 32 + lane] = mul4(s, P[k]);
-      }
+    for (int k = 0; k < TS::kOwn; ++k) {
+      const int c = grp + TS::G * k;
+      if (c < NS) sbuf[c * L + lane] = next[k];
     }
     __syncthreads();
-    auto emit = [&](int i, const float4& v) {
-      const int x = x0 + warp * kTXW + i;
-      if (x < a.nx && yok) *reinterpret_cast<float4*>(tmp + (static_cast<size_t>(z) * a.nx + x) * a.cs + yb) = v;
-    };
-    if (PSF) {
-      const float* kr = (PTAB ? ptab : s_psf) + z * 2 * K;
-      rowpass_from_tile<R, 32, 32>(sbuf, warp * kTXW, emit, kr, kr + K, lane, a.ny);
-    } else {
-#pragma unroll
-      for (int i = 0; i < kTXW; ++i) emit(i, sbuf[(warp * kTXW + i) * 32 + lane]);
-    }
+    if (z + 1 < zend) load(z + 1, next);
+    const float* kr = (PTAB ? ptab : s_psf) + z * 2 * K;
+    rowpass_from_tile_p<R, L, L>(
+        sbuf, grp * kTXW,
+        [&](int i, const float4& o) {
+          const int x = x0 + grp * kTXW + i;
+          if (x < a.nx && yok) *reinterpret_cast<float4*>(dst + (static_cast<size_t>(z) * a.nx + x) * a.cs) = o;
+        },
+        kr, kr + K, lane, a.ny);
   }
 }
 
-// Grid: (camera g of the group, x-tile) items x depth slabs (the cluster).
-template <int R, bool PSF>
-__global__ void __launch_bounds__(32 * kW, 2) k_grad_spread_yg(const YgArgs a, int c0) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int ntile = (a.nx + kTX<32> - 1) / kTX<32>;
-  const int item = blockIdx.x / a.pslabs;
-  const int g = item / ntile;
-  grad_item<R, PSF, false>(a, c0 + g, g, (item % ntile) * kTX<32>, smem, nullptr);
+template <int R, int L>
+__global__ void __launch_bounds__(32 * kW, 3) k_grad_conv_yg(const YgArgs a, int u0, int n) {
+  grad_conv_body<R, false, L>(a, u0, n, nullptr);
 }
 
-template <int R>
-__global__ void __launch_bounds__(32 * kW, 2)
-    k_grad_spread_ptab_yg(const YgArgs a, int c0, const __grid_constant__ PsfTable t) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int ntile = (a.nx + kTX<32> - 1) / kTX<32>;
-  const int item = blockIdx.x / a.pslabs;
-  const int g = item / ntile;
-  grad_item<R, true, true>(a, c0 + g, g, (item % ntile) * kTX<32>, smem, t.c);
+template <int R, int L>
+__global__ void __launch_bounds__(32 * kW, 3)
+    k_grad_conv_ptab_yg(const YgArgs a, int u0, int n, const __grid_constant__ PsfTable t) {
+  grad_conv_body<R, true, L>(a, u0, n, t.c);
 }
 
-template <int R>
-int launch_grad_R(const YgArgs& a_in, int c0, int gcount, cudaStream_t st) {
+template <int R, int L>
+int launch_grad_conv(const YgArgs& a_in, int u0, int n, cudaStream_t st) {
   YgArgs a = a_in;
-  const int ntile = (a.nx + kTX<32> - 1) / kTX<32>;
-  const bool psf = a.psf != nullptr;
-  const bool ptab = psf && a.psf_host && static_cast<size_t>(a.nz) * 2 * (2 * R + 1) <= kPsfTableFloats;
-  const size_t smem = tile_smem_bytes<R, 32>(psf && !ptab ? a.nz : 0);
-  // depth slabs: the fewest of 2, 4, 8 giving four waves of two CTAs per SM
-  if (a.pslabs != 2 && a.pslabs != 4 && a.pslabs != 8) {
-    a.pslabs = 8;
-    for (int s = 2; s < 8; s *= 2)
-      if (gcount * ntile * s >= 4 * 2 * sm_count()) {
-        a.pslabs = s;
-        break;
-      }
-  }
-  bool launch_err = false;
-  auto launch = [&](auto k, auto&&... extra) {
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(gcount * ntile * a.pslabs);
-    cfg.blockDim = dim3(32 * kW);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = a.pslabs;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    NRGB_LAUNCH_SCOPE("k_grad_spread_yg", st);
-    if (cudaLaunchKernelEx(&cfg, k, a, c0, extra...) != cudaSuccess) launch_err = true;
-  };
+  const int ntile = (a.nx + kTX<L> - 1) / kTX<L>;
+  const int volumes = a.units ? 2 * n : n;
+  a.bslabs = yg_spread_slabs(volumes * ntile, a.nz, 3);
+  const bool ptab = psf_in_parameters<R>(a);
+  const size_t smem = TileShape<R, L>::kSbBytes + (ptab ? 0 : sizeof(float) * a.nz * 2 * (2 * R + 1));
+  const dim3 grid(volumes * ntile * a.bslabs), block(32 * kW);
   if (ptab) {
     static thread_local PsfTable table;
     std::memcpy(table.c, a.psf_host, sizeof(float) * a.nz * 2 * (2 * R + 1));
-    launch(k_grad_spread_ptab_yg<R>, table);
-  } else if (psf) {
-    launch(k_grad_spread_yg<R, true>);
-  } else {
-    launch(k_grad_spread_yg<0, false>);
+    auto k = k_grad_conv_ptab_yg<R, L>;
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    NRGB_LAUNCH_SCOPE("k_grad_conv_yg", st);
+    k<<<grid, block, smem, st>>>(a, u0, n, table);
+  } else if constexpr (L == 32) {
+    auto k = k_grad_conv_yg<R, L>;
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    NRGB_LAUNCH_SCOPE("k_grad_conv_yg", st);
+    k<<<grid, block, smem, st>>>(a, u0, n);
   }
-  return cudaGetLastError() == cudaSuccess && !launch_err ? kOk : kErrKernel;
+  return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
+}
+
+template <int R>
+int grad_conv_R(const YgArgs& a, int u0, int n, cudaStream_t st) {
+  if (psf_in_parameters<R>(a)) {
+    if (a.lanes == 8) return launch_grad_conv<R, 8>(a, u0, n, st);
+    if (a.lanes == 16) return launch_grad_conv<R, 16>(a, u0, n, st);
+  }
+  return launch_grad_conv<R, 32>(a, u0, n, st);
+}
+
+int grad_conv_by_radius(int R, const YgArgs& a, int u0, int n, cudaStream_t st) {
+  switch (R) {
+    case 0: return grad_conv_R<0>(a, u0, n, st);
+    case 1: return grad_conv_R<1>(a, u0, n, st);
+    case 2: return grad_conv_R<2>(a, u0, n, st);
+    case 3: return grad_conv_R<3>(a, u0, n, st);
+    case 4: return grad_conv_R<4>(a, u0, n, st);
+    case 5: return grad_conv_R<5>(a, u0, n, st);
+    case 6: return grad_conv_R<6>(a, u0, n, st);
+    case 7: return grad_conv_R<7>(a, u0, n, st);
+    default: return kErrParameters;
+  }
+}
+
+int launch_weights(const YgArgs& a, int u0, int n, cudaStream_t st) {
+  constexpr size_t smem = sizeof(float4) * 3 * kSlabsB * kGradCols * 32;
+  auto go = [&](auto lanes) {
+    constexpr int L = decltype(lanes)::value, C = kGradCols * (32 / L);
+    auto k = k_grad_weights_yg<L>;
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    NRGB_LAUNCH_SCOPE("k_grad_weights_yg", st);
+    k<<<n * ((a.nx + C - 1) / C), 32 * kSlabsB, smem, st>>>(a, u0);
+  };
+  const int lanes = column_lanes(a.ny);
+  if (lanes == 8) go(std::integral_constant<int, 8>());
+  else if (lanes == 16) go(std::integral_constant<int, 16>());
+  else go(std::integral_constant<int, 32>());
+  return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
+}
+
+// Units (or cameras) per group: their w and PSF volumes, two of each per mirror
+// unit, in three scratch slots of the backprojector.
+int grad_units(int n, int ncam, int group, bool pair) {
+  const int volumes = 3 * std::max(1, std::min(group, ncam));
+  return yg_even_group(n, std::max(1, volumes / (pair ? 4 : 2)));
 }
 
 }  // namespace
 
-int yg_grad_spread(const YgArgs& a, int c0, int gcount, cudaStream_t st) {
-  if (!a.mu || !a.act || !a.sino || !a.temp) return kErrParameters;
+int yg_gradient(const YgArgs& a_in, cudaStream_t st) {
+  YgArgs a = a_in;
+  if (!a.mu || !a.act || !a.sino || !a.out || !a.work) return kErrParameters;
   const int R = a.psf ? (a.psf_k - 1) / 2 : 0;
-  switch (R) {
-    case 0: return launch_grad_R<0>(a, c0, gcount, st);
-    case 1: return launch_grad_R<1>(a, c0, gcount, st);
-    case 2: return launch_grad_R<2>(a, c0, gcount, st);
-    case 3: return launch_grad_R<3>(a, c0, gcount, st);
-    case 4: return launch_grad_R<4>(a, c0, gcount, st);
-    case 5: return launch_grad_R<5>(a, c0, gcount, st);
-    case 6: return launch_grad_R<6>(a, c0, gcount, st);
-    case 7: return launch_grad_R<7>(a, c0, gcount, st);
-    default: return kErrParameters;
+  const bool pair = a.units && a.nunits > 0;
+  if (!pair) a.units = nullptr;
+  const int units = pair ? a.nunits : a.ncam;
+  const int group = grad_units(units, a.ncam, a.group, pair);
+  const int slots = pair ? 2 * group : group;  // volumes of a group
+  a.group = group;
+  for (const Window& w : call_windows(a, R)) {
+    YgArgs b = windowed(a, w);
+    const size_t vol = static_cast<size_t>(b.nz) * b.nx * b.cs;
+    float* weights = a.work;
+    float* blurred = a.psf ? a.work + vol * slots : weights;
+    for (int u0 = 0; u0 < units; u0 += group) {
+      const int n = std::min(group, units - u0);
+      b.temp = weights;
+      int s = launch_weights(b, u0, n, st);
+      if (s == kOk && a.psf) {
+        YgArgs c = b;
+        c.out = blurred;
+        s = grad_conv_by_radius(R, c, u0, n, st);
+      }
+      if (s != kOk) return s;
+      const bool last = u0 + n == units;
+      b.temp = blurred;
+      yg_gather(b, u0, n, u0 == 0, a.truncate && last && !pair, st);
+      if (pair) {
+        b.temp = blurred + vol * group;
+        b.mates = 1;
+        yg_gather(b, u0, n, 0, a.truncate && last, st);
+        b.mates = 0;
+      }
+    }
   }
+  return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
+}
+
+size_t yg_gradient_workspace(int nx, int ny, int nz, int ncam, int group) {
+  const size_t vol = static_cast<size_t>(nz) * nx * scratch_rows(ny);
+  // at least one unit: two volumes, and two blurred
+  return sizeof(float) * vol * std::max(4, 3 * std::max(1, std::min(group, ncam)));
 }
 
 }  // namespace nrgb
