@@ -379,19 +379,37 @@ __device__ __forceinline__ void ybuf_zero_pads() {
   }
 }
 
-template <int R, int L, int YB, class KC>
+// SHUF: the outermost chunk on either side, of which N rows are needed, by
+// shuffle -- one L1 wavefront a row where a 16-byte load takes four.  R = 1 and 2
+// need nothing else (no row buffer): projector at 128^3 x 120, PSF 3, 0.425 ->
+// 0.403 ms.  R = 5 (N = 1): the projector's single-camera pass 0.755 -> 0.725 ms;
+// no gain in the passes of two cameras (0.537, 0.540 ms) and in the spread,
+// d/dmu slower.  R = 6 (N = 2) slower (192^3, PSF 13: 5.02 -> 5.17 ms).
+template <int R, int L, int YB, bool SHUF, class KC>
 __device__ __forceinline__ float4 yconv4s(const float4& u, KC kc, int lane, int b) {
   if constexpr (R == 0) {
     return yconv4<0>(u, kc, lane);
   } else {
-    constexpr int C = (R + 3) / 4;
-    static_assert(C <= kYPad, "row-buffer pads");
-    float4* row = ybuf<L, YB>(threadIdx.x / L, b) + kYPad;
-    row[lane] = u;
-    __syncwarp();
+    constexpr int C = (R + 3) / 4, N = R - 4 * (C - 1);
+    constexpr int CL = SHUF ? C - 1 : C;  // chunks on either side read from the row buffer
+    static_assert(CL <= kYPad, "row-buffer pads");
     float w[2 * R + 4];
+    if constexpr (CL < C) {
 #pragma unroll
-    for (int c = -C; c <= C; ++c) {
+      for (int t = 1; t <= N; ++t) {
+        const float up = __shfl_up_sync(kFull, comp(u, 4 - t), C, L);
+        const float dn = __shfl_down_sync(kFull, comp(u, t - 1), C, L);
+        w[R - 4 * (C - 1) - t] = lane >= C ? up : 0.0f;
+        w[R + 3 + 4 * (C - 1) + t] = lane + C < L ? dn : 0.0f;
+      }
+    }
+    float4* row = CL > 0 ? ybuf<L, YB>(threadIdx.x / L, b) + kYPad : nullptr;
+    if constexpr (CL > 0) {
+      row[lane] = u;
+      __syncwarp();
+    }
+#pragma unroll
+    for (int c = -CL; c <= CL; ++c) {
       const float4 v = c == 0 ? u : row[lane + c];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
@@ -596,7 +614,7 @@ __device__ __forceinline__ void rowpass_from_tile(const float4* __restrict__ sbu
     }
     const int i = j - 2 * R;
     if (i >= 0 && i < kTXW) {
-      emit(i, mask_rows(yconv4s<R, L, YB>(u[i % K], kc, lane, i & 1), 4 * lane, ny));
+      emit(i, mask_rows(yconv4s<R, L, YB, R <= 2>(u[i % K], kc, lane, i & 1), 4 * lane, ny));
       u[i % K] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
@@ -627,7 +645,7 @@ __device__ __forceinline__ void rowpass_from_tile_p(const float4* __restrict__ s
       }
     }
     const int i = j - 2 * R;
-    if (i >= 0 && i < kTXW) emit(i, mask_rows(yconv4s<R, L, YB>(unpair4(u[i]), kc, lane, i & 1), 4 * lane, ny));
+    if (i >= 0 && i < kTXW) emit(i, mask_rows(yconv4s<R, L, YB, R <= 2 || R == 5>(unpair4(u[i]), kc, lane, i & 1), 4 * lane, ny));
   }
 }
 
@@ -660,8 +678,8 @@ __device__ __forceinline__ void rowpass2_from_tiles(const float4* __restrict__ s
     }
     const int i = j - 2 * R;
     if (i >= 0 && i < kTXW) {
-      emit_b(i, mask_rows(yconv4s<R, L, YB>(ub[i], kcb, lane, 0), 4 * lane, ny));
-      emit_a(i, mask_rows(yconv4s<R, L, YB>(ua[i], kca, lane, 1), 4 * lane, ny));
+      emit_b(i, mask_rows(yconv4s<R, L, YB, R <= 2>(ub[i], kcb, lane, 0), 4 * lane, ny));
+      emit_a(i, mask_rows(yconv4s<R, L, YB, R <= 2>(ua[i], kca, lane, 1), 4 * lane, ny));
     }
   }
 }
@@ -694,8 +712,8 @@ __device__ __forceinline__ void rowpass2_from_tiles_p(const float4* __restrict__
     }
     const int i = j - 2 * R;
     if (i >= 0 && i < kTXW) {
-      emit_b(i, mask_rows(yconv4s<R, L, YB>(unpair4(ub[i]), kcb, lane, 0), 4 * lane, ny));
-      emit_a(i, mask_rows(yconv4s<R, L, YB>(unpair4(ua[i]), kca, lane, 1), 4 * lane, ny));
+      emit_b(i, mask_rows(yconv4s<R, L, YB, R <= 2>(unpair4(ub[i]), kcb, lane, 0), 4 * lane, ny));
+      emit_a(i, mask_rows(yconv4s<R, L, YB, R <= 2>(unpair4(ua[i]), kca, lane, 1), 4 * lane, ny));
     }
   }
 }

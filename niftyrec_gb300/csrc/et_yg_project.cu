@@ -46,7 +46,7 @@ int project_slabs(int items, int nz, int ctas_per_sm, bool pair, const std::func
   int best = least;
   double cost = 0.0;
   for (int s : {2, 4, 6, 8, 16}) {
-    if (s < least || (pair && s == 6)) continue;
+    if (s < least || (pair && s == 6) || (s == 16 && nz < 128)) continue;
     const int resident = clusters(s);
     if (resident < 1) continue;
     const double c = ((nz + s - 1) / s + 2) *

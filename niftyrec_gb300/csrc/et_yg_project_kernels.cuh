@@ -18,7 +18,8 @@ namespace nrgb {
 // stand for a slab's start and merge.  Against the count for three waves of
 // CTAs: 128^3 x 30 cameras of a half-turn 258 -> 196 us (6 slabs), x 15 125 ->
 // 114, 256^3 x 18 PSF 15 1.66 -> 1.25 ms, 64^3 x 60 plain 25 -> 19 us (8),
-// 32^3 x 8 27 -> 15 us (16); 128^3 x 120 keeps 4 (0.504 ms; 8: 0.519).
+// 32^3 x 8 27 -> 19 us (8; 16: 15 us, but its slabs of two planes cost accuracy,
+// 1.0e-7 -> 1.3e-7, so 16 needs 128 planes); 128^3 x 120 keeps 4 (0.504 ms; 8: 0.519).
 // Left out: 5 and 7 (128^3 x 15: 131 and 136 us although they fit one round),
 // with mirror units 6 (96 x 96 x 80 x 90: 206 us, 8: 200), and fewer than the
 // three-wave count (6 or 8 at least): longer float sums for nothing more than
