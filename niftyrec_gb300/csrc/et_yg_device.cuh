@@ -622,8 +622,10 @@ __device__ __forceinline__ void rowpass_from_tile(const float4* __restrict__ sbu
 
 // Packed forms of the two row passes below (accumulators as float32 pairs,
 // one fma.rn.f32x2 per two rows; the same roundings in the same order), used
-// by the projector.  The spread keeps the scalar forms: its two transmission
-// arrays leave no registers for the broadcast coefficient pairs.
+// by the projector and by the spread of single cameras (128^3 x 120: 1.194 ->
+// 1.183 ms with PSF 11, 1.268 -> 1.232 with PSF 15).  The mirror-unit spread
+// keeps the scalar forms: its two transmission arrays leave no registers for
+// the broadcast coefficient pairs.
 template <int R, int L, int YB, class EmitFn, class KR, class KC>
 __device__ __forceinline__ void rowpass_from_tile_p(const float4* __restrict__ sbuf, int base, EmitFn emit, KR kr, KC kc,
                                                   int lane, int ny) {
@@ -716,12 +718,6 @@ __device__ __forceinline__ void rowpass2_from_tiles_p(const float4* __restrict__
       emit_a(i, mask_rows(yconv4s<R, L, YB, R <= 2>(unpair4(ua[i]), kca, lane, 1), 4 * lane, ny));
     }
   }
-}
-
-template <int R, int L, int YB, class EmitA, class EmitB, class KRA, class KCA, class KRB, class KCB>
-__device__ __forceinline__ void rowpass2_from_tile(const float4* __restrict__ sbuf, int base, EmitA emit_a, KRA kra,
-                                                   KCA kca, EmitB emit_b, KRB krb, KCB kcb, int lane, int ny) {
-  rowpass2_from_tiles<R, L, YB>(sbuf, sbuf, base, emit_a, kra, kca, emit_b, krb, kcb, lane, ny);
 }
 
 template <int R, int L, int YB, class EmitA, class EmitB, class KRA, class KCA, class KRB, class KCB>
@@ -972,11 +968,11 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
       }
       return;
     }
-    // float32, PSF radius <= 5: mu of the group's output columns sampled
-    // before the row pass, so that the gathers' latency overlaps the PSF
-    // arithmetic (128^3 x 120, PSF 11: projector 0.608 -> 0.586 ms); wider
-    // PSFs would spill registers (radius 7: slower)
-    constexpr bool kEarlyMu = ATT && !KAHAN && R <= 5;
+    // float32: mu of the group's output columns sampled before the row pass, so
+    // that the gathers' latency overlaps the PSF arithmetic (128^3 x 120, PSF 11:
+    // projector 0.608 -> 0.586 ms; one camera at a time, PSF 15: 0.840 -> 0.815);
+    // with mirror units only for PSF radius <= 5 (radius 7: registers, no gain)
+    constexpr bool kEarlyMu = ATT && !KAHAN && (R <= 5 || !PAIR);
     float4 mv[kTXW];
     if constexpr (kEarlyMu) {
 #pragma unroll

@@ -23,6 +23,15 @@ namespace {
 // shared memory, for the float32 reference spread; else 2).
 // PTAB: the separated PSF comes from the kernel-parameter table `ptab`
 // ([nz][2K]) instead of a shared-memory copy of the slab's planes.
+// Row pass of a single camera: packed, but for radius 4 scalar (96^3 x 72, PSF 9:
+// 0.402 ms, packed 0.405).
+template <int R, int L, class EmitFn, class KR, class KC>
+__device__ __forceinline__ void rowpass_single(const float4* __restrict__ sbuf, int base, EmitFn emit, KR kr, KC kc,
+                                               int lane, int ny) {
+  if constexpr (R == 4) rowpass_from_tile<R, L, L>(sbuf, base, emit, kr, kc, lane, ny);
+  else rowpass_from_tile_p<R, L, L>(sbuf, base, emit, kr, kc, lane, ny);
+}
+
 template <int R, bool PSF, bool ATT, bool ADJ, class V, bool PTAB, int L>
 __device__ __forceinline__ void spread_body(const YgArgs& a, int c0, const float* ptab) {
   using TS = TileShape<R, L>;
@@ -115,10 +124,10 @@ __device__ __forceinline__ void spread_body(const YgArgs& a, int c0, const float
     if (PSF) {
       if constexpr (PTAB && ADJ) {  // transpose of a convolution = correlation: both kernels reversed
         const float* kr = ptab + z * 2 * K;
-        rowpass_from_tile<R, L, L>(sbuf, grp * kTXW, emit, Reversed<R>{kr}, Reversed<R>{kr + K}, lane, a.ny);
+        rowpass_single<R, L>(sbuf, grp * kTXW, emit, Reversed<R>{kr}, Reversed<R>{kr + K}, lane, a.ny);
       } else {
         const float* kr = (PTAB ? ptab : s_psf) + z * 2 * K;
-        rowpass_from_tile<R, L, L>(sbuf, grp * kTXW, emit, kr, kr + K, lane, a.ny);
+        rowpass_single<R, L>(sbuf, grp * kTXW, emit, kr, kr + K, lane, a.ny);
       }
     } else {
 #pragma unroll
@@ -162,18 +171,25 @@ __global__ void __launch_bounds__(32 * kW, CTAS)
 // memory), the mate's transmission is the column total minus the compensated
 // forward sum (no second running sum), and the tiles are single-buffered (a
 // second barrier per plane) so that two CTAs per SM still fit.
-template <int R, int L, class V>
+//
+// float32 reference mode of radius 6 and 7 is single-buffered too: the smaller
+// tiles leave more L1 for the gathers (256^3 x 60, PSF 15: pair 6.11 -> 6.06 ms;
+// 128^3 x 120, PSF 13: backprojection 0.855 -> 0.839; PSF 11 0.828 -> 0.833).
+template <int R, bool ADJ, class V>
+constexpr bool kSingleTile = StorageTraits<V>::kKahan || (R >= 6 && !ADJ);
+
+template <int R, int L, bool ADJ, class V>
 __host__ __device__ constexpr size_t spread_pair_fixed_smem() {
   using TS = TileShape<R, L>;
   constexpr bool KAHAN = StorageTraits<V>::kKahan;
-  return (KAHAN ? 1 : 2) * TS::kSbBytes + TS::kTapBytes + (KAHAN ? sizeof(float4) * TS::kOwn * 32 * kW : 0);
+  return (kSingleTile<R, ADJ, V> ? 1 : 2) * TS::kSbBytes + TS::kTapBytes + (KAHAN ? sizeof(float4) * TS::kOwn * 32 * kW : 0);
 }
 
 template <int R, bool PSF, bool ATT, bool ADJ, bool PTAB, class V, int L>
 __device__ __forceinline__ void spread_pair_body(const YgArgs& a, int u0, const float* ptab) {
   using TS = TileShape<R, L>;
   constexpr bool KAHAN = StorageTraits<V>::kKahan;
-  constexpr int NB = KAHAN ? 1 : 2;  // tile buffers
+  constexpr int NB = kSingleTile<R, ADJ, V> ? 1 : 2;  // tile buffers
   constexpr int NS = TS::NS;
   constexpr int K = 2 * R + 1;
   const V* __restrict__ mu = reinterpret_cast<const V*>(a.mu) + a.row0;
@@ -181,7 +197,7 @@ __device__ __forceinline__ void spread_pair_body(const YgArgs& a, int u0, const 
   float4* sb = reinterpret_cast<float4*>(smem);                              // [NB stages][2][NS][L]
   Tap* taps = reinterpret_cast<Tap*>(smem + NB * TS::kSbBytes);               // [2][kTapSlots]
   float4* scomp = reinterpret_cast<float4*>(smem + NB * TS::kSbBytes + TS::kTapBytes);  // [kOwn][256] (KAHAN)
-  float* s_psf = reinterpret_cast<float*>(smem + spread_pair_fixed_smem<R, L, V>());  // [zper][2K], mate's next
+  float* s_psf = reinterpret_cast<float*>(smem + spread_pair_fixed_smem<R, L, ADJ, V>());  // [zper][2K], mate's next
 
   const int grp = threadIdx.x / L, lane = threadIdx.x % L;
   const int ntile = (a.nx + kTX<L> - 1) / kTX<L>;
@@ -431,7 +447,7 @@ int launch_spread_pair_lanes(const YgArgs& a, int u0, int gcount, cudaStream_t s
   const PsfTable* tab = psf_table<R>(a);
   // bfloat16 mu: the Kahan form (reference mode only)
   const bool bf16 = a.storage == kStorageBF16 && a.mu && !ADJ;
-  const size_t smem = (bf16 ? spread_pair_fixed_smem<R, L, __nv_bfloat16>() : spread_pair_fixed_smem<R, L, float>()) +
+  const size_t smem = (bf16 ? spread_pair_fixed_smem<R, L, ADJ, __nv_bfloat16>() : spread_pair_fixed_smem<R, L, ADJ, float>()) +
                       (psf && !tab ? sizeof(float) * 2 * zper * 2 * (2 * R + 1) : 0);
   auto go = [&](auto k) {
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
