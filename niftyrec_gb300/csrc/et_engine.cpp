@@ -154,6 +154,8 @@ size_t vol_n(const Problem& pb) { return static_cast<size_t>(pb.nx) * pb.ny * pb
 // Cameras per launch of the general path and its three sets of work volumes.
 int gen_group(const Problem& pb) { return general_group(vol_n(pb), sizeof(float), pb.cams.n); }
 size_t gen_n(const Problem& pb) { return vol_n(pb) * gen_group(pb); }
+// Its projection's and backprojection's work space (the sources' two volumes too).
+size_t gen_bytes(const Problem& pb) { return sizeof(float) * (3 * gen_n(pb) + 2 * vol_n(pb)); }
 size_t col_n(const Problem& pb) { return static_cast<size_t>(pb.nx) * round_up(pb.ny, 4) * pb.nz; }
 size_t sino_col_n(const Problem& pb) { return static_cast<size_t>(pb.nx) * round_up(pb.ny, 4) * pb.cams.n; }
 constexpr size_t kSlack = 8 * 256;
@@ -267,11 +269,11 @@ int widen_inputs(const Problem& pb, Carver& cv, const float** act, const float**
 
 size_t project_workspace(const Problem& pb, bool has_act, bool has_att) {
   size_t b = common_bytes(pb);
-  if (use_fused_x(pb) && has_act) return b + gen_n(pb) * 3 * sizeof(float) + widen_bytes(pb);  // or general
+  if (use_fused_x(pb) && has_act) return b + gen_bytes(pb) + widen_bytes(pb);  // or general
   if (use_fused(pb) && has_act)
     b += sizeof(float) * (col_n(pb) * (has_att ? 2 : 1) + sino_col_n(pb));
   else
-    b += sizeof(float) * gen_n(pb) * 3 + widen_bytes(pb);
+    b += gen_bytes(pb) + widen_bytes(pb);
   return b;
 }
 
@@ -279,12 +281,12 @@ size_t backproject_workspace(const Problem& pb, bool has_att) {
   size_t b = common_bytes(pb);
   if (use_fused_x(pb))  // the fused form's scratch, or the general path's volumes
     return b + std::max(yg_backproject_workspace(pb.ny, pb.nx, pb.nz, pb.cams.n, pb.group) + kSlack,
-                        sizeof(float) * gen_n(pb) * 3 + widen_bytes(pb));
+                        gen_bytes(pb) + widen_bytes(pb));
   if (use_fused(pb))
     b += sizeof(float) * (col_n(pb) * (has_att ? 2 : 1) + sino_col_n(pb)) +
          yg_backproject_workspace(pb.nx, pb.ny, pb.nz, pb.cams.n, pb.group) + kSlack;
   else
-    b += sizeof(float) * gen_n(pb) * 3 + widen_bytes(pb);
+    b += gen_bytes(pb) + widen_bytes(pb);
   return b;
 }
 
@@ -391,7 +393,8 @@ int project_device(const Problem& pb, const float* d_act, const float* d_att, fl
   g.ws_act = cv.take<float>(gen_n(pb));
   g.ws_att = cv.take<float>(gen_n(pb));
   g.ws_tmp = cv.take<float>(gen_n(pb));
-  if (!g.ws_act || !g.ws_att || !g.ws_tmp) return kErrAllocGpu;
+  g.ws_src = cv.take<float>(2 * vol_n(pb));
+  if (!g.ws_act || !g.ws_att || !g.ws_tmp || !g.ws_src) return kErrAllocGpu;
   return check(general_project(g, st));
 }
 
@@ -523,7 +526,8 @@ int backproject_device(const Problem& pb, const float* d_sino, const float* d_at
   g.ws_act = cv.take<float>(gen_n(pb));
   g.ws_att = cv.take<float>(gen_n(pb));
   g.ws_tmp = cv.take<float>(gen_n(pb));
-  if (!g.ws_act || !g.ws_att || !g.ws_tmp) return kErrAllocGpu;
+  g.ws_src = cv.take<float>(2 * vol_n(pb));
+  if (!g.ws_act || !g.ws_att || !g.ws_tmp || !g.ws_src) return kErrAllocGpu;
   return check(pb.back_mode == kBackAdjoint ? general_adjoint(g, st) : general_backproject(g, st));
 }
 
@@ -839,7 +843,7 @@ int gradient_device(const Problem& pb, const float* d_sino, const float* d_act, 
 // ------------------------------------------------------------ float64 run
 size_t workspace64(const Problem& pb) {
   const size_t group = general_group(vol_n(pb), sizeof(double), pb.cams.n);
-  return sizeof(double) * (3 * vol_n(pb) * group + static_cast<size_t>(2 * pb.psf_k) * pb.nz) + kSlack;
+  return sizeof(double) * (vol_n(pb) * (3 * group + 2) + static_cast<size_t>(2 * pb.psf_k) * pb.nz) + kSlack;
 }
 
 namespace {
@@ -871,7 +875,8 @@ int setup64(const Problem& pb, const float* psf_host, Carver& cv, std::vector<Ca
   g->ws_act = cv.take<double>(vol_n(pb) * g->group);
   g->ws_att = cv.take<double>(vol_n(pb) * g->group);
   g->ws_tmp = cv.take<double>(vol_n(pb) * g->group);
-  return (g->ws_act && g->ws_att && g->ws_tmp) ? kOk : kErrAllocGpu;
+  g->ws_src = cv.take<double>(2 * vol_n(pb));
+  return (g->ws_act && g->ws_att && g->ws_tmp && g->ws_src) ? kOk : kErrAllocGpu;
 }
 
 }  // namespace

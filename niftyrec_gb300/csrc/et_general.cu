@@ -11,6 +11,7 @@
 #include "et_profile.h"
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 namespace nrgb {
@@ -40,6 +41,19 @@ __device__ __forceinline__ double ex(double v) { return exp(v); }
 template <class T>
 struct AffineSetT {
   T m[kGeneralGroup][12];
+};
+
+// Grid and layout of the work volumes: planes [y][x] (x fastest, the caller's
+// order) or, with col, [x][y].
+struct Grid {
+  int nx, ny, nz, col;
+  __device__ __forceinline__ int sx() const { return col ? ny : 1; }
+  __device__ __forceinline__ int sy() const { return col ? 1 : nx; }
+  __device__ __forceinline__ size_t at(int x, int y, int z) const {
+    return static_cast<size_t>(z) * ny * nx + static_cast<size_t>(y) * sy() + static_cast<size_t>(x) * sx();
+  }
+  // index of element i of a work plane in the caller's [y][x] plane
+  __device__ __forceinline__ size_t caller(size_t i) const { return col ? i % ny * nx + i / ny : i; }
 };
 
 // Footprint of one voxel: floor positions and the two weights per axis
@@ -72,13 +86,15 @@ __device__ __forceinline__ Foot<T> footprint(const T* m, int x, int y, int z) {
 // background weight, as the reference does (:366-396).  A footprint inside
 // the grid -- nearly all -- takes the same sums without the tests.
 template <class T>
-__device__ __forceinline__ T trilinear_ref(const T* __restrict__ src, int nx, int ny, int nz, const Foot<T>& f, T bg) {
+__device__ __forceinline__ T trilinear_ref(const T* __restrict__ src, const Grid& n, const Foot<T>& f, T bg) {
+  const int nx = n.nx, ny = n.ny, nz = n.nz;
   const int px = f.prev[0], py = f.prev[1], pz = f.prev[2];
   if (px >= 0 && px + 1 < nx && py >= 0 && py + 1 < ny && pz >= 0 && pz + 1 < nz) {
-    const T* p = src + (static_cast<size_t>(pz) * ny + py) * nx + px;
+    const T* p = src + n.at(px, py, pz);
     const T* q = p + static_cast<size_t>(ny) * nx;
-    auto line = [&](const T* r) { return fa(fm(__ldg(r), f.b0[0]), fm(__ldg(r + 1), f.b1[0])); };
-    auto plane = [&](const T* r) { return fa(fm(line(r), f.b0[1]), fm(line(r + nx), f.b1[1])); };
+    const int sx = n.sx(), sy = n.sy();
+    auto line = [&](const T* r) { return fa(fm(__ldg(r), f.b0[0]), fm(__ldg(r + sx), f.b1[0])); };
+    auto plane = [&](const T* r) { return fa(fm(line(r), f.b0[1]), fm(line(r + sy), f.b1[1])); };
     return fa(fm(plane(p), f.b0[2]), fm(plane(q), f.b1[2]));
   }
   const T bx[2] = {f.b0[0], f.b1[0]};
@@ -95,13 +111,12 @@ __device__ __forceinline__ T trilinear_ref(const T* __restrict__ src, int nx, in
       for (int b = 0; b < 2; ++b) {
         const int Y = py + b;
         if (Y >= 0 && Y < ny) {
-          const T* row = src + (static_cast<size_t>(Z) * ny + Y) * nx;
           T xsum = T(0);
 #pragma unroll
           for (int a = 0; a < 2; ++a) {
             const int X = px + a;
             if (X >= 0 && X < nx)
-              xsum = fa(xsum, fm(__ldg(row + X), bx[a]));
+              xsum = fa(xsum, fm(__ldg(src + n.at(X, Y, Z)), bx[a]));
             else if (use_bg)
               bgw = fa(bgw, fm(bg, bx[a]));
           }
@@ -119,22 +134,25 @@ __device__ __forceinline__ T trilinear_ref(const T* __restrict__ src, int nx, in
   return val;
 }
 
-// Voxel of this thread in a launch of 32 x 8-voxel blocks over (x-tile,
-// y-tile, z, camera of the group); one set of 32-bit divisions per block.
+// Voxel of this thread in a launch of 32 x 8-voxel blocks (32 along the fast
+// axis) over (fast tile, slow tile, z, camera of the group); one set of 32-bit
+// divisions per block.
 struct Voxel {
   int x, y, z, g;
 };
 
-__device__ __forceinline__ Voxel block_voxel(int nx, int ny, int nz) {
-  const int tx = (nx + 31) / 32, ty = (ny + 7) / 8;
+__device__ __forceinline__ Voxel block_voxel(const Grid& n) {
+  const int tf = ((n.col ? n.ny : n.nx) + 31) / 32, ts = ((n.col ? n.nx : n.ny) + 7) / 8;
   int b = blockIdx.x;
   Voxel v;
-  v.x = b % tx * 32 + threadIdx.x;
-  b /= tx;
-  v.y = b % ty * 8 + threadIdx.y;
-  b /= ty;
-  v.z = b % nz;
-  v.g = b / nz;
+  const int fast = b % tf * 32 + threadIdx.x;
+  b /= tf;
+  const int slow = b % ts * 8 + threadIdx.y;
+  b /= ts;
+  v.x = n.col ? slow : fast;
+  v.y = n.col ? fast : slow;
+  v.z = b % n.nz;
+  v.g = b / n.nz;
   return v;
 }
 
@@ -143,29 +161,50 @@ __device__ __forceinline__ Voxel block_voxel(int nx, int ny, int nz) {
 template <class T>
 __global__ void __launch_bounds__(256)
     k_resample(const T* __restrict__ src, T* __restrict__ dst, T bg, const T* __restrict__ src2, T* __restrict__ dst2,
-               T bg2, int nx, int ny, int nz, const __grid_constant__ AffineSetT<T> A) {
-  const Voxel v = block_voxel(nx, ny, nz);
-  if (v.x >= nx || v.y >= ny) return;
+               T bg2, const Grid n, const __grid_constant__ AffineSetT<T> A) {
+  const Voxel v = block_voxel(n);
+  if (v.x >= n.nx || v.y >= n.ny) return;
   const Foot<T> f = footprint(A.m[v.g], v.x, v.y, v.z);
-  const size_t o = ((static_cast<size_t>(v.g) * nz + v.z) * ny + v.y) * nx + v.x;
-  if (src) dst[o] = trilinear_ref(src, nx, ny, nz, f, bg);
-  if (src2) dst2[o] = trilinear_ref(src2, nx, ny, nz, f, bg2);
+  const size_t o = static_cast<size_t>(v.g) * n.nz * n.ny * n.nx + n.at(v.x, v.y, v.z);
+  if (src) dst[o] = trilinear_ref(src, n, f, bg);
+  if (src2) dst2[o] = trilinear_ref(src2, n, f, bg2);
 }
 
-// dst (+)= sum over the group's cameras, in camera order, of src[g] resampled
-// at camera g's positions; first: assign; clamp: store negative sums as zero.
+// dst (the caller's layout) (+)= sum over the group's cameras, in camera order,
+// of src[g] resampled at camera g's positions; first: assign; clamp: store
+// negative sums as zero.
 template <class T>
 __global__ void __launch_bounds__(256)
-    k_resample_sum(const T* __restrict__ src, T* __restrict__ dst, int n, int first, int clamp, T bg, int nx, int ny,
-                   int nz, const __grid_constant__ AffineSetT<T> A) {
-  const Voxel v = block_voxel(nx, ny, nz);
-  if (v.x >= nx || v.y >= ny) return;
-  const size_t nvox = static_cast<size_t>(nx) * ny * nz;
-  const size_t o = (static_cast<size_t>(v.z) * ny + v.y) * nx + v.x;
+    k_resample_sum(const T* __restrict__ src, T* __restrict__ dst, int count, int first, int clamp, T bg, const Grid n,
+                   const __grid_constant__ AffineSetT<T> A) {
+  const Voxel v = block_voxel(n);
+  if (v.x >= n.nx || v.y >= n.ny) return;
+  const size_t nvox = static_cast<size_t>(n.nx) * n.ny * n.nz;
+  const size_t o = (static_cast<size_t>(v.z) * n.ny + v.y) * n.nx + v.x;
   T acc = first ? T(0) : dst[o];
-  for (int g = 0; g < n; ++g)
-    acc = fa(acc, trilinear_ref(src + nvox * g, nx, ny, nz, footprint(A.m[g], v.x, v.y, v.z), bg));
+  for (int g = 0; g < count; ++g)
+    acc = fa(acc, trilinear_ref(src + nvox * g, n, footprint(A.m[g], v.x, v.y, v.z), bg));
   dst[o] = clamp && acc < T(0) ? T(0) : acc;
+}
+
+// Planes [y][x] to [x][y] through a 32 x 32 tile.
+template <class T>
+__global__ void __launch_bounds__(256) k_transpose(const T* __restrict__ src, T* __restrict__ dst, int nx, int ny) {
+  __shared__ T tile[32][33];
+  const int tx = (nx + 31) / 32, ty = (ny + 31) / 32;
+  int b = blockIdx.x;
+  const int x0 = b % tx * 32;
+  b /= tx;
+  const int y0 = b % ty * 32;
+  b /= ty;
+  const size_t plane = static_cast<size_t>(b) * ny * nx;
+  for (int r = threadIdx.y; r < 32; r += 8)
+    if (x0 + threadIdx.x < nx && y0 + r < ny)
+      tile[r][threadIdx.x] = src[plane + static_cast<size_t>(y0 + r) * nx + x0 + threadIdx.x];
+  __syncthreads();
+  for (int c = threadIdx.y; c < 32; c += 8)
+    if (x0 + c < nx && y0 + threadIdx.x < ny)
+      dst[plane + static_cast<size_t>(x0 + c) * ny + y0 + threadIdx.x] = tile[threadIdx.x][c];
 }
 
 // Transpose of trilinear_ref with bg = 0: add v * weight to each in-grid
@@ -193,7 +232,7 @@ __device__ __forceinline__ void trilinear_scatter(float* __restrict__ dst, int n
 
 __global__ void __launch_bounds__(256) k_scatter(const float* __restrict__ src, float* __restrict__ dst, int nx, int ny,
                                                  int nz, const __grid_constant__ AffineSetT<float> A) {
-  const Voxel v = block_voxel(nx, ny, nz);
+  const Voxel v = block_voxel(Grid{nx, ny, nz, 0});
   if (v.x >= nx || v.y >= ny) return;
   const float s = src[((static_cast<size_t>(v.g) * nz + v.z) * ny + v.y) * nx + v.x];
   if (s == 0.0f) return;
@@ -240,7 +279,7 @@ __global__ void k_conv(const T* __restrict__ in, T* __restrict__ out, int nx, in
 // camera g of the group.
 template <int R, bool FLIP, class T>
 __global__ void __launch_bounds__(256)
-    k_conv2(const T* __restrict__ in, T* __restrict__ out, int nx, int ny, int nz, const T* __restrict__ sep) {
+    k_conv2(const T* __restrict__ in, T* __restrict__ out, int nx, int ny, int nz, const T* __restrict__ sep, int col) {
   constexpr int K = 2 * R + 1, W = 32 + 2 * R, N = 4;
   __shared__ T s_in[W][W + 1];
   __shared__ T s_row[W][33];
@@ -253,9 +292,10 @@ __global__ void __launch_bounds__(256)
   const T* src = in + static_cast<size_t>(b) * ny * nx;
   const T* k = sep + static_cast<size_t>(2 * K) * (b % nz);
   for (int e = threadIdx.x; e < W * W; e += 256) {
-    const int r = e / W, c = e % W;
+    const int r = col ? e % W : e / W, c = col ? e / W : e % W;  // lanes along the fast axis
     const int x = x0 - R + c, y = y0 - R + r;
-    s_in[r][c] = x >= 0 && x < nx && y >= 0 && y < ny ? __ldg(src + static_cast<size_t>(y) * nx + x) : T(0);
+    const size_t o = col ? static_cast<size_t>(x) * ny + y : static_cast<size_t>(y) * nx + x;
+    s_in[r][c] = x >= 0 && x < nx && y >= 0 && y < ny ? __ldg(src + o) : T(0);
   }
   T kr[K], kc[K];
 #pragma unroll
@@ -268,7 +308,8 @@ __global__ void __launch_bounds__(256)
   bool finite = true;
 #pragma unroll
   for (int j = 0; j < K; ++j) finite = finite && isfinite(kr[j]) && isfinite(kc[j]);
-  const int c = threadIdx.x % 32, r = threadIdx.x / 32 * N;
+  // this thread's outputs of the column pass: lanes along the fast axis
+  const int c = col ? threadIdx.x / 8 : threadIdx.x % 32, r = (col ? threadIdx.x % 8 : threadIdx.x / 32) * N;
   T s[N];
   auto both = [&](auto check) {
     constexpr bool CHECK = decltype(check)::value;
@@ -306,7 +347,8 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
   for (int i = 0; i < N; ++i)
     if (x0 + c < nx && y0 + r + i < ny)
-      out[(static_cast<size_t>(b) * ny + y0 + r + i) * nx + x0 + c] = s[i];
+      out[static_cast<size_t>(b) * ny * nx + (col ? static_cast<size_t>(x0 + c) * ny + y0 + r + i
+                                                  : static_cast<size_t>(y0 + r + i) * nx + x0 + c)] = s[i];
 }
 
 constexpr int kScanDepth = 8;  // depth planes whose loads a ray scan has in flight
@@ -314,9 +356,10 @@ constexpr int kScanDepth = 8;  // depth planes whose loads a ray scan has in fli
 // Attenuated line integral along z, emission-lib/_et_line_integral_attenuated.cpp:14-68;
 // blockIdx.y: camera of the group.
 template <class R = float>
-__global__ void k_line_integral(const R* __restrict__ act, const R* __restrict__ att, R* __restrict__ out, int nx,
-                                int ny, int nz, R bg, int truncate) {
-  const size_t nxy = static_cast<size_t>(nx) * ny;
+__global__ void k_line_integral(const R* __restrict__ act, const R* __restrict__ att, R* __restrict__ out,
+                                const Grid n, R bg, int truncate) {
+  const int nz = n.nz;
+  const size_t nxy = static_cast<size_t>(n.nx) * n.ny;
   const size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   if (i >= nxy) return;
   const size_t vol = nxy * nz * blockIdx.y;
@@ -342,19 +385,19 @@ __global__ void k_line_integral(const R* __restrict__ act, const R* __restrict__
   else if (act) p = fa(p, bg);
   else p = fm(bg, ex(-T));
   if (truncate && p < R(0)) p = R(0);
-  out[nxy * blockIdx.y + i] = p;
+  out[nxy * blockIdx.y + n.caller(i)] = p;
 }
 
 // Spread along z, emission-lib/_et_line_backproject_attenuated.cpp:17-36 and
 // emission-lib/_et_line_backproject.cpp:17-30; blockIdx.y: camera of the group.
 template <class R = float>
-__global__ void k_spread(const R* __restrict__ plane, const R* __restrict__ att, R* __restrict__ vol, int nx, int ny,
-                         int nz) {
-  const size_t nxy = static_cast<size_t>(nx) * ny;
+__global__ void k_spread(const R* __restrict__ plane, const R* __restrict__ att, R* __restrict__ vol, const Grid n) {
+  const int nz = n.nz;
+  const size_t nxy = static_cast<size_t>(n.nx) * n.ny;
   const size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   if (i >= nxy) return;
   const size_t off = nxy * nz * blockIdx.y + i;
-  const R s = __ldg(plane + nxy * blockIdx.y + i);
+  const R s = __ldg(plane + nxy * blockIdx.y + n.caller(i));
   R T = R(0);
   for (int z0 = 0; z0 < nz; z0 += kScanDepth) {
     R m[kScanDepth];
@@ -477,10 +520,39 @@ struct General {
   cudaStream_t st;
   size_t nvox, nxy;
   int cam0 = 0, n = 0;  // the current group
+  Grid grid;
 
   General(const GeneralArgsT<T>& args, cudaStream_t stream) : a(args), st(stream) {
     nxy = static_cast<size_t>(a.nx) * a.ny;
     nvox = nxy * a.nz;
+    grid = {a.nx, a.ny, a.nz, 0};
+  }
+
+  // Work volumes as planes [x][y] where that is the better order: the lanes of
+  // a resampling step along the fast axis, and a load is coalesced as far as
+  // that step stays on the axis.  Cameras turned about y (tilted heads) keep y:
+  // 96^3 x 30 cameras tilted by 7 degrees, projection + backprojection 1.53 ms
+  // along x, 1.43 along y.  Needs the fused convolution, and two volumes for
+  // the sources.
+  void choose_layout() {
+    if (!a.ws_src || a.ncam < 2 || (a.psf_sep && a.psf_k > 15)) return;
+    T off_x = 0, off_y = 0;  // how far steps along x and y leave their axis
+    for (int c = 0; c < a.ncam; ++c) {
+      const T* m = a.geom_host[c].fwd;
+      off_x += std::abs(m[4]) + std::abs(m[8]);
+      off_y += std::abs(m[1]) + std::abs(m[9]);
+    }
+    grid.col = off_y < T(0.7) * off_x;
+  }
+
+  // A source volume in the work layout (slot 0 or 1 of a.ws_src).
+  const T* source(const T* src, int slot) {
+    if (!src || !grid.col) return src;
+    T* dst = a.ws_src + nvox * slot;
+    NRGB_LAUNCH_SCOPE("k_transpose", st);
+    k_transpose<T><<<static_cast<unsigned>((a.nx + 31) / 32) * ((a.ny + 31) / 32) * a.nz, dim3(32, 8), 0, st>>>(
+        src, dst, a.nx, a.ny);
+    return dst;
   }
 
   template <class Body>
@@ -504,9 +576,10 @@ struct General {
     return s;
   }
 
-  // blocks of 32 x rows voxels over `volumes` volumes
+  // blocks of 32 (fast axis) x rows voxels over `volumes` volumes
   unsigned blocks(int rows, int volumes) const {
-    return static_cast<unsigned>((a.nx + 31) / 32) * ((a.ny + rows - 1) / rows) * a.nz * volumes;
+    const int fast = grid.col ? a.ny : a.nx, slow = grid.col ? a.nx : a.ny;
+    return static_cast<unsigned>((fast + 31) / 32) * ((slow + rows - 1) / rows) * a.nz * volumes;
   }
   dim3 rays() const { return dim3(static_cast<unsigned>((nxy + 127) / 128), n); }
 
@@ -514,8 +587,7 @@ struct General {
   void rotate(const T* src, T* dst, T bg, const T* src2, T* dst2, T bg2) {
     if (!src && !src2) return;
     NRGB_LAUNCH_SCOPE("k_resample", st);
-    k_resample<T><<<blocks(8, n), dim3(32, 8), 0, st>>>(src, dst, bg, src2, dst2, bg2, a.nx, a.ny, a.nz,
-                                                        matrices(false));
+    k_resample<T><<<blocks(8, n), dim3(32, 8), 0, st>>>(src, dst, bg, src2, dst2, bg2, grid, matrices(false));
   }
 
   // PSF of the group's volumes; returns where the result is (tmp, or vol for
@@ -525,7 +597,7 @@ struct General {
     if (!a.psf_sep) return vol;
     auto go = [&](auto k) {
       NRGB_LAUNCH_SCOPE("k_conv2", st);
-      k<<<blocks(32, n), 256, 0, st>>>(vol, tmp, a.nx, a.ny, a.nz, a.psf_sep);
+      k<<<blocks(32, n), 256, 0, st>>>(vol, tmp, a.nx, a.ny, a.nz, a.psf_sep, grid.col);
     };
     switch ((a.psf_k - 1) / 2) {
       case 0: go(k_conv2<0, FLIP, T>); return tmp;
@@ -549,14 +621,14 @@ struct General {
 
   void spread(const T* att, T* vol) {
     NRGB_LAUNCH_SCOPE("k_spread", st);
-    k_spread<T><<<rays(), 128, 0, st>>>(a.sino + nxy * cam0, att, vol, a.nx, a.ny, a.nz);
+    k_spread<T><<<rays(), 128, 0, st>>>(a.sino + nxy * cam0, att, vol, grid);
   }
 
   // rotate the group's volumes back and add them to the output
   void gather(const T* src, T bg) {
     NRGB_LAUNCH_SCOPE("k_resample_sum", st);
-    k_resample_sum<T><<<blocks(8, 1), dim3(32, 8), 0, st>>>(src, a.out, n, cam0 == 0, a.truncate && last(), bg, a.nx,
-                                                            a.ny, a.nz, matrices(true));
+    k_resample_sum<T><<<blocks(8, 1), dim3(32, 8), 0, st>>>(src, a.out, n, cam0 == 0, a.truncate && last(), bg, grid,
+                                                            matrices(true));
   }
 };
 
@@ -565,12 +637,14 @@ struct General {
 template <class T>
 int general_project_t(const GeneralArgsT<T>& a, cudaStream_t st) {
   General<T> p(a, st);
+  p.choose_layout();
+  const T *act = p.source(a.act, 0), *att = p.source(a.att, 1);
   return p.groups([&] {
-    p.rotate(a.act, a.ws_act, a.bg, a.att, a.ws_att, a.bg_att);
+    p.rotate(act, a.ws_act, a.bg, att, a.ws_att, a.bg_att);
     const T* v = a.act ? p.convolve(a.ws_act, a.ws_tmp) : nullptr;
     NRGB_LAUNCH_SCOPE("k_line_integral", st);
-    k_line_integral<T><<<p.rays(), 128, 0, st>>>(v, a.att ? a.ws_att : nullptr, a.out + p.nxy * p.cam0, a.nx, a.ny,
-                                                 a.nz, a.bg, a.truncate);
+    k_line_integral<T><<<p.rays(), 128, 0, st>>>(v, a.att ? a.ws_att : nullptr, a.out + p.nxy * p.cam0, p.grid, a.bg,
+                                                 a.truncate);
   });
 }
 
@@ -579,8 +653,10 @@ int general_project_t(const GeneralArgsT<T>& a, cudaStream_t st) {
 template <class T>
 int general_backproject_t(const GeneralArgsT<T>& a, cudaStream_t st) {
   General<T> p(a, st);
+  p.choose_layout();
+  const T* att = p.source(a.att, 0);
   return p.groups([&] {
-    p.rotate(nullptr, nullptr, T(0), a.att, a.ws_att, a.bg_att);
+    p.rotate(nullptr, nullptr, T(0), att, a.ws_att, a.bg_att);
     p.spread(a.att ? a.ws_att : nullptr, a.ws_act);
     p.gather(p.convolve(a.ws_act, a.ws_tmp), a.bg);
   });
@@ -617,7 +693,7 @@ int general_project_partial(const GeneralArgs& a, const float* bg_image, float* 
       std::copy(a.geom_host[p.cam0 + g].bwd, a.geom_host[p.cam0 + g].bwd + 12, m.m[0]);
       NRGB_LAUNCH_SCOPE("k_resample", st);
       k_resample<float><<<p.blocks(8, 1), dim3(32, 8), 0, st>>>(sums + p.nvox * g, dst + p.nvox * g, a.bg, nullptr,
-                                                                nullptr, 0.0f, a.nx, a.ny, a.nz, m);
+                                                                nullptr, 0.0f, p.grid, m);
     }
   });
   if (s == kOk && a.truncate) launch_truncate(a.out, p.nxy * a.ncam, st);
@@ -725,7 +801,7 @@ int general_rotate(const float* src, float* dst, int nx, int ny, int nz, const f
   std::copy(m12, m12 + 12, m.m[0]);
   NRGB_LAUNCH_SCOPE("k_resample", st);
   k_resample<float><<<General<float>(a, st).blocks(8, 1), dim3(32, 8), 0, st>>>(src, dst, bg, nullptr, nullptr, 0.0f,
-                                                                                nx, ny, nz, m);
+                                                                                Grid{nx, ny, nz, 0}, m);
   return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
 }
 

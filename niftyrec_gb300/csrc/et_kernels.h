@@ -25,6 +25,7 @@ struct GeneralArgsT {
   T* ws_act = nullptr;  // three sets of `group` nvox work volumes
   T* ws_att = nullptr;
   T* ws_tmp = nullptr;
+  T* ws_src = nullptr;  // projection, backprojection: two volumes for sources in the work layout, or null
 };
 // Cameras per launch of the general path: as many as kGeneralGroup (their
 // matrices are launch parameters) while the three sets of work volumes stay

@@ -138,6 +138,7 @@ int plan_project(Plan& p, int subset, const float* d_act, float* d_sino, int lay
   g.ws_act = p.work;
   g.ws_att = p.work + nv;
   g.ws_tmp = p.work + 2 * nv;
+  g.ws_src = p.work + 3 * nv;
   int s = general_project(g, st);
   return s != kOk ? s : check();
 }
@@ -204,6 +205,7 @@ int plan_backproject(Plan& p, int subset, const float* d_sino, float* d_out, int
   g.ws_act = p.work;
   g.ws_att = p.work + nv;
   g.ws_tmp = p.work + 2 * nv;
+  g.ws_src = p.work + 3 * nv;
   int s = general_backproject(g, st);
   return s != kOk ? s : check();
 }
@@ -315,7 +317,7 @@ int nrgb_plan_create(void** out_plan, const int* size, const float* cameras, con
                     sizeof(float) * static_cast<size_t>(ncam) * yg_carry_slabs() * nx * p->cy;
   } else {
     bytes += al(sizeof(float) * nv) * (p->has_att ? 1 : 0);
-    p->work_bytes = sizeof(float) * nv * 3 * general_group(nv, sizeof(float), ncam);
+    p->work_bytes = sizeof(float) * nv * (3 * general_group(nv, sizeof(float), ncam) + 2);
   }
   bytes += al(p->work_bytes);
   if (cudaMalloc(&p->mem, bytes) != cudaSuccess) {

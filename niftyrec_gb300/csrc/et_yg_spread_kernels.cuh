@@ -8,6 +8,15 @@
 namespace nrgb {
 namespace {
 
+// Row pass of a single camera: packed, but for radius 4 scalar (96^3 x 72, PSF 9:
+// 0.402 ms, packed 0.405).
+template <int R, int L, class EmitFn, class KR, class KC>
+__device__ __forceinline__ void rowpass_single(const float4* __restrict__ sbuf, int base, EmitFn emit, KR kr, KC kc,
+                                               int lane, int ny) {
+  if constexpr (R == 4) rowpass_from_tile<R, L, L>(sbuf, base, emit, kr, kc, lane, ny);
+  else rowpass_from_tile_p<R, L, L>(sbuf, base, emit, kr, kc, lane, ny);
+}
+
 // ---------------------------------------- backprojector: spread + PSF
 // temp[g][z][x][y] = PSF_z( s(x', y) * exp(-T_z(x', y)) ) for camera c0+g,
 // T inclusive (emission-lib/_et_line_backproject_attenuated.cpp:24-34), PSF
@@ -23,15 +32,6 @@ namespace {
 // shared memory, for the float32 reference spread; else 2).
 // PTAB: the separated PSF comes from the kernel-parameter table `ptab`
 // ([nz][2K]) instead of a shared-memory copy of the slab's planes.
-// Row pass of a single camera: packed, but for radius 4 scalar (96^3 x 72, PSF 9:
-// 0.402 ms, packed 0.405).
-template <int R, int L, class EmitFn, class KR, class KC>
-__device__ __forceinline__ void rowpass_single(const float4* __restrict__ sbuf, int base, EmitFn emit, KR kr, KC kc,
-                                               int lane, int ny) {
-  if constexpr (R == 4) rowpass_from_tile<R, L, L>(sbuf, base, emit, kr, kc, lane, ny);
-  else rowpass_from_tile_p<R, L, L>(sbuf, base, emit, kr, kc, lane, ny);
-}
-
 template <int R, bool PSF, bool ATT, bool ADJ, class V, bool PTAB, int L>
 __device__ __forceinline__ void spread_body(const YgArgs& a, int c0, const float* ptab) {
   using TS = TileShape<R, L>;
