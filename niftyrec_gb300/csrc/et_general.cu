@@ -84,12 +84,14 @@ __device__ __forceinline__ Foot<T> footprint(const T* m, int x, int y, int z) {
 // Trilinear value of a footprint, reg-lib/_reg_resampling.cpp:365-450.  With
 // bg != 0 every neighbour outside the grid adds bg * xBasis[.] to a separate
 // background weight, as the reference does (:366-396).  A footprint inside
-// the grid -- nearly all -- takes the same sums without the tests.
+// the grid -- nearly all -- takes the same sums without the tests.  Under a
+// caller's affine matrix the floor may saturate: no neighbour's index is formed
+// before it is known to lie in the grid, so that it cannot wrap into it.
 template <class T>
 __device__ __forceinline__ T trilinear_ref(const T* __restrict__ src, const Grid& n, const Foot<T>& f, T bg) {
   const int nx = n.nx, ny = n.ny, nz = n.nz;
   const int px = f.prev[0], py = f.prev[1], pz = f.prev[2];
-  if (px >= 0 && px + 1 < nx && py >= 0 && py + 1 < ny && pz >= 0 && pz + 1 < nz) {
+  if (px >= 0 && px < nx - 1 && py >= 0 && py < ny - 1 && pz >= 0 && pz < nz - 1) {
     const T* p = src + n.at(px, py, pz);
     const T* q = p + static_cast<size_t>(ny) * nx;
     const int sx = n.sx(), sy = n.sy();
@@ -104,19 +106,16 @@ __device__ __forceinline__ T trilinear_ref(const T* __restrict__ src, const Grid
   const bool use_bg = (bg != T(0));
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
-    const int Z = pz + c;
-    if (Z >= 0 && Z < nz) {
+    if (pz >= -c && pz < nz - c) {
       T ysum = T(0);
 #pragma unroll
       for (int b = 0; b < 2; ++b) {
-        const int Y = py + b;
-        if (Y >= 0 && Y < ny) {
+        if (py >= -b && py < ny - b) {
           T xsum = T(0);
 #pragma unroll
           for (int a = 0; a < 2; ++a) {
-            const int X = px + a;
-            if (X >= 0 && X < nx)
-              xsum = fa(xsum, fm(__ldg(src + n.at(X, Y, Z)), bx[a]));
+            if (px >= -a && px < nx - a)
+              xsum = fa(xsum, fm(__ldg(src + n.at(px + a, py + b, pz + c)), bx[a]));
             else if (use_bg)
               bgw = fa(bgw, fm(bg, bx[a]));
           }
@@ -213,18 +212,16 @@ __device__ __forceinline__ void trilinear_scatter(float* __restrict__ dst, int n
                                                   const Foot<float>& f, float v) {
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
-    const int Z = f.prev[2] + c;
-    if (Z < 0 || Z >= nz) continue;
+    if (f.prev[2] < -c || f.prev[2] >= nz - c) continue;
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
-      const int Y = f.prev[1] + b;
-      if (Y < 0 || Y >= ny) continue;
+      if (f.prev[1] < -b || f.prev[1] >= ny - b) continue;
 #pragma unroll
       for (int a = 0; a < 2; ++a) {
-        const int X = f.prev[0] + a;
-        if (X < 0 || X >= nx) continue;
+        if (f.prev[0] < -a || f.prev[0] >= nx - a) continue;
         const float w = (a ? f.b1[0] : f.b0[0]) * (b ? f.b1[1] : f.b0[1]) * (c ? f.b1[2] : f.b0[2]);
-        if (w != 0.0f) atomicAdd(dst + (static_cast<size_t>(Z) * ny + Y) * nx + X, v * w);
+        if (w != 0.0f)
+          atomicAdd(dst + (static_cast<size_t>(f.prev[2] + c) * ny + f.prev[1] + b) * nx + f.prev[0] + a, v * w);
       }
     }
   }

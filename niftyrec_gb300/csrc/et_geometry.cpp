@@ -75,6 +75,16 @@ int expand_cameras(const float* cameras, int n, int ncols, const int center_size
 }
 
 template <class T>
+void bound_translations(T m[12]) {
+  const T far = static_cast<T>(1 << 30);
+  for (int i = 3; i < 12; i += 4) {
+    if (m[i] > far) m[i] = far;
+    if (m[i] < -far) m[i] = -far;
+  }
+}
+template void bound_translations<float>(float m[12]);
+
+template <class T>
 std::vector<CamGeomT<T>> camera_geometry_t(const Cameras& cams) {
   std::vector<CamGeomT<T>> g(cams.n);
   const int n = cams.n;
@@ -86,6 +96,8 @@ std::vector<CamGeomT<T>> camera_geometry_t(const Cameras& cams) {
     std::memcpy(g[c].fwd, M, sizeof(T) * 12);
     rotation_matrix_t<T>(M, -tx, -ty, -tz, cx, cy, cz, 5);
     std::memcpy(g[c].bwd, M, sizeof(T) * 12);
+    bound_translations(g[c].fwd);
+    bound_translations(g[c].bwd);
   }
   return g;
 }

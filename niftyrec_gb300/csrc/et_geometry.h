@@ -32,6 +32,13 @@ int expand_cameras(const float* cameras, int n, int ncols, const int center_size
 std::vector<CamGeom> camera_geometry(const Cameras& cams);
 std::vector<CamGeom64> camera_geometry64(const Cameras& cams);
 
+// Translations of a camera's 3x4 matrix moved to at most 2^30 voxels from the
+// origin (NaN kept).  A camera whose centre puts the grid further away samples
+// nothing either way, and the kernels' integer positions, a voxel's neighbour
+// among them, stay in range.
+template <class T>
+void bound_translations(T m[12]);
+
 // True when every camera rotates about the gantry axis only (theta_x ==
 // theta_z == 0), so that the resampling matrices are exact rotations about y.
 bool is_y_gantry(const Cameras& cams);

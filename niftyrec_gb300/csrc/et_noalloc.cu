@@ -137,6 +137,8 @@ extern "C" int nrgb_backproject_device_noalloc(const float* d_sinogram, const fl
     std::memcpy(g_geom[c].fwd, M, sizeof(float) * 12);
     rotation_matrix(M, -ang[0], -ang[1], -ang[2], cen[0], cen[1], cen[2], 5);
     std::memcpy(g_geom[c].bwd, M, sizeof(float) * 12);
+    bound_translations(g_geom[c].fwd);
+    bound_translations(g_geom[c].bwd);
   }
   if (k) {
     const int cc = (k - 1) / 2;

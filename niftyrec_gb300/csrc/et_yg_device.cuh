@@ -69,7 +69,8 @@ __device__ __forceinline__ float fa(float a, float b) { return __fadd_rn(a, b); 
 
 // Bilinear footprint of one sampled column.  Corner (a, c) sits at
 // off + a*dx + c*dz; corners outside the grid get weight 0 and a clamped
-// (valid) address, so loads never leave the volume.
+// (valid) address, so loads never leave the volume (a position's neighbour is
+// a valid int: see bound_translations).
 struct __align__(16) Tap {
   int off, dx, dz, any;
   float w00, w10, w01, w11;
