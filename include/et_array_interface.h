@@ -428,6 +428,11 @@ int nrgb_get_deterministic(void);
 int nrgb_mirror_units(const float *cameras, const int *cameras_size, const int *size, int *out_units, int max_units,
                       int *n_units);
 int nrgb_row_windows(int ny, int psf_k, int *out, int max_windows, int *n_windows);
+/* The batched projector's launch for volumes of up to max_nz planes, a PSF of
+ * width psf_k (0: none), with or without mu, on the current device: out = {CTAs
+ * per SM its kernel is built for, the kernel's static shared memory and its local
+ * memory per thread in bytes, clusters of 4 CTAs launched}. */
+int nrgb_batch_projector_info(int psf_k, int has_att, int max_nz, int *out);
 
 /* Instrumentation (no counterpart in the reference).  nrgb_launch_count: CUDA
  * kernels this library launched since it was loaded.  nrgb_profile_enable(1)

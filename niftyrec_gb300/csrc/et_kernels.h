@@ -227,6 +227,9 @@ void yg_window_lanes(int rows, int nx, int* lanes, int* tiles);
 // one launch share psf_k and whether they have mu; max_nz sizes the PSF table.
 int yg_project_batch(const BatchStepDesc* d_desc, const BatchSel& sel, int psf_k, bool att, int max_nz,
                      int* d_counter, cudaStream_t st);
+// The batched projector's launch for volumes of up to max_nz planes: {CTAs per
+// SM the kernel is built for, static shared memory, local memory per thread, clusters}.
+int yg_project_batch_info(int psf_k, bool att, int max_nz, int* info);
 // ratio (desc.proj.out <- counts / max-rule(proj.out)) and update
 // (proj.act *= num / max(sens, eps)) over all selected volumes in one launch.
 int osem_ratio_batch(const BatchStepDesc* d_desc, const BatchElems& e, float eps, cudaStream_t st);

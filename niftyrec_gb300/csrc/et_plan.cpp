@@ -839,4 +839,13 @@ int nrgb_batch_osem_step(void* batch, int step, int iterations, float epsilon, v
   return s;
 }
 
+// What the batched projector's launch would be (see the header).
+int nrgb_batch_projector_info(int psf_k, int has_att, int max_nz, int* out) {
+  NRGB_API("nrgb_batch_projector_info");
+  if (!out || psf_k < 0 || (psf_k && psf_k % 2 != 1) || psf_k > 15 || max_nz < 1 || !yg_supported(1, 1, max_nz, psf_k))
+    return kErrParameters;
+  std::fill(out, out + 4, 0);
+  return yg_project_batch_info(psf_k, has_att != 0, max_nz, out);
+}
+
 }  // extern "C"

@@ -363,12 +363,19 @@ template <int L>
 constexpr size_t kYBufBytes = sizeof(float4) * kGroups<L> * 2 * kYRow<L>;  // static, per CTA
 
 // YB: the lane count whose row buffers the kernel holds -- L, or in a kernel
-// that runs windows of several lane counts the one with the largest (8).
+// that runs windows of several lane counts the one with the largest (8).  The
+// array belongs to a function of YB alone: one object for all of the kernel's
+// lane counts.
+template <int YB>
+__device__ __forceinline__ float4* ybuf_storage() {
+  __shared__ __align__(16) float4 buf[kYBufBytes<YB> / sizeof(float4)];
+  return buf;
+}
+
 template <int L, int YB>
 __device__ __forceinline__ float4* ybuf(int grp, int b) {
   static_assert(kYBufBytes<L> <= kYBufBytes<YB>, "row buffers of L lanes fit");
-  __shared__ __align__(16) float4 buf[kYBufBytes<YB> / sizeof(float4)];
-  return buf + (grp * 2 + b) * kYRow<L>;
+  return ybuf_storage<YB>() + (grp * 2 + b) * kYRow<L>;
 }
 
 template <int L, int YB = L>

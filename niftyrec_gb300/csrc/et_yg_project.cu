@@ -111,8 +111,10 @@ namespace {
 // is drawn by the cluster's first thread and read by the other CTAs from its
 // shared memory (double-buffered: the slot of item i is rewritten at item i+2,
 // after the barriers of item i+1).
-// CTAS: CTAs per SM the kernel is built for (3: 80 registers and more warps to
-// hide the gathers' latency, where three tiles fit in shared memory; else 2).
+// CTAS: CTAs per SM the kernel is built for.  With mu 2 (128 registers): the
+// three bodies of the lane counts spill 796 bytes at the 80 registers of 3 CTAs, and
+// a step of 24 volumes takes 4.98 ms against 5.50.  Without mu nothing spills at
+// 3 CTAs, taken where more of them are resident.
 template <int R, bool PSF, bool ATT, int CTAS>
 __global__ void __cluster_dims__(kSlabsP, 1, 1) __launch_bounds__(32 * kW, CTAS)
     k_project_batch_yg(const BatchStepDesc* __restrict__ descs, const BatchSel sel, int* __restrict__ counter) {
@@ -163,44 +165,60 @@ int project_by_radius(int R, const YgArgs& a, cudaStream_t st, int* slabs_used) 
   }
 }
 
-// Persistent grid: `ctas` CTAs per SM, whole clusters.
-int batch_clusters(int ctas) { return sm_count() * ctas / kSlabsP; }
-
+// One launch of the batched projector, or with info only what that launch
+// would be: {CTAs per SM the kernel is built for, its static shared memory and
+// its local memory per thread in bytes, clusters launched}.
 template <int R, bool PSF>
 int launch_project_batch_R(const BatchStepDesc* d, const BatchSel& sel, bool att, int max_nz, int* counter,
-                           cudaStream_t st) {
+                           cudaStream_t st, int* info) {
   // one launch runs windows of any lane count: the largest tile of the three
   const int planes = PSF ? max_nz : 0;
   const size_t smem =
       std::max({tile_smem_bytes<R, 32>(planes), tile_smem_bytes<R, 16>(planes), tile_smem_bytes<R, 8>(planes)});
-  const bool three = 3 * (smem + kYBufBytes<8> + 1024) <= 228 * 1024;
-  auto go = [&](auto k, int ctas) {
+  // persistent grid: the clusters that are resident at once
+  auto clusters = [&](auto k) {
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    return max_active_clusters(reinterpret_cast<const void*>(k), kSlabsP, 32 * kW, smem);
+  };
+  auto go = [&](auto k, int ctas, int resident) {
+    const int grid = resident > 0 ? resident : sm_count() * ctas / kSlabsP;
+    if (info) {
+      cudaFuncAttributes attr = {};
+      if (cudaFuncGetAttributes(&attr, k) != cudaSuccess) return;
+      info[0] = ctas;
+      info[1] = static_cast<int>(attr.sharedSizeBytes);
+      info[2] = static_cast<int>(attr.localSizeBytes);
+      info[3] = grid;
+      return;
+    }
     NRGB_LAUNCH_SCOPE("k_project_batch_yg", st);
-    k<<<batch_clusters(ctas) * kSlabsP, 32 * kW, smem, st>>>(d, sel, counter);
+    k<<<grid * kSlabsP, 32 * kW, smem, st>>>(d, sel, counter);
   };
   if (att) {
-    if (three) go(k_project_batch_yg<R, PSF, true, 3>, 3);
-    else go(k_project_batch_yg<R, PSF, true, 2>, 2);
+    auto k = k_project_batch_yg<R, PSF, true, 2>;
+    go(k, 2, clusters(k));
   } else {
-    if (three) go(k_project_batch_yg<R, PSF, false, 3>, 3);
-    else go(k_project_batch_yg<R, PSF, false, 2>, 2);
+    auto two = k_project_batch_yg<R, PSF, false, 2>;
+    auto three = k_project_batch_yg<R, PSF, false, 3>;
+    const int n2 = clusters(two), n3 = clusters(three);
+    if (n3 > n2) go(three, 3, n3);
+    else go(two, 2, n2);
   }
   return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
 }
 
 int project_batch_by_radius(int psf_k, const BatchStepDesc* d, const BatchSel& sel, bool att, int max_nz,
-                            int* counter, cudaStream_t st) {
-  if (psf_k == 0) return launch_project_batch_R<0, false>(d, sel, att, max_nz, counter, st);
+                            int* counter, cudaStream_t st, int* info) {
+  if (psf_k == 0) return launch_project_batch_R<0, false>(d, sel, att, max_nz, counter, st, info);
   switch ((psf_k - 1) / 2) {
-    case 0: return launch_project_batch_R<0, true>(d, sel, att, max_nz, counter, st);
-    case 1: return launch_project_batch_R<1, true>(d, sel, att, max_nz, counter, st);
-    case 2: return launch_project_batch_R<2, true>(d, sel, att, max_nz, counter, st);
-    case 3: return launch_project_batch_R<3, true>(d, sel, att, max_nz, counter, st);
-    case 4: return launch_project_batch_R<4, true>(d, sel, att, max_nz, counter, st);
-    case 5: return launch_project_batch_R<5, true>(d, sel, att, max_nz, counter, st);
-    case 6: return launch_project_batch_R<6, true>(d, sel, att, max_nz, counter, st);
-    case 7: return launch_project_batch_R<7, true>(d, sel, att, max_nz, counter, st);
+    case 0: return launch_project_batch_R<0, true>(d, sel, att, max_nz, counter, st, info);
+    case 1: return launch_project_batch_R<1, true>(d, sel, att, max_nz, counter, st, info);
+    case 2: return launch_project_batch_R<2, true>(d, sel, att, max_nz, counter, st, info);
+    case 3: return launch_project_batch_R<3, true>(d, sel, att, max_nz, counter, st, info);
+    case 4: return launch_project_batch_R<4, true>(d, sel, att, max_nz, counter, st, info);
+    case 5: return launch_project_batch_R<5, true>(d, sel, att, max_nz, counter, st, info);
+    case 6: return launch_project_batch_R<6, true>(d, sel, att, max_nz, counter, st, info);
+    case 7: return launch_project_batch_R<7, true>(d, sel, att, max_nz, counter, st, info);
     default: return kErrParameters;
   }
 }
@@ -210,7 +228,11 @@ int project_batch_by_radius(int psf_k, const BatchStepDesc* d, const BatchSel& s
 int yg_project_batch(const BatchStepDesc* d_desc, const BatchSel& sel, int psf_k, bool att, int max_nz,
                      int* d_counter, cudaStream_t st) {
   if (sel.n <= 0 || sel.total <= 0) return kOk;
-  return project_batch_by_radius(psf_k, d_desc, sel, att, max_nz, d_counter, st);
+  return project_batch_by_radius(psf_k, d_desc, sel, att, max_nz, d_counter, st, nullptr);
+}
+
+int yg_project_batch_info(int psf_k, bool att, int max_nz, int* info) {
+  return project_batch_by_radius(psf_k, nullptr, BatchSel(), att, max_nz, nullptr, nullptr, info);
 }
 
 int yg_project(const YgArgs& a, cudaStream_t st, int* slabs_used) {
