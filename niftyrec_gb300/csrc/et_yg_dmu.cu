@@ -131,10 +131,13 @@ __global__ void __launch_bounds__(256, 3) k_dmu_scatter_yg(const YgArgs a, int n
           Z = zs;
         }
         const float wx0 = __fsub_rn(1.0f, rx), wz0 = __fsub_rn(1.0f, rz);
-        axpy4(n00, wx0 * wz0, d);
-        axpy4(n10, rx * wz0, d);
-        axpy4(n01, wx0 * rz, d);
-        axpy4(n11, rx * rz, d);
+        // a corner without weight takes nothing: d may be infinite (uniform tests,
+        // 128^3 x 120: 0.259 -> 0.266 ms a launch)
+        const float w00 = wx0 * wz0, w10 = rx * wz0, w01 = wx0 * rz, w11 = rx * rz;
+        if (w00 != 0.0f) axpy4(n00, w00, d);
+        if (w10 != 0.0f) axpy4(n10, w10, d);
+        if (w01 != 0.0f) axpy4(n01, w01, d);
+        if (w11 != 0.0f) axpy4(n11, w11, d);
       }
     }
   }
