@@ -89,15 +89,17 @@ bool host_memory_readable() {
 }
 
 // Project with host buffers (activity and/or attenuation may be null).
-int project_host(const Problem& pb, const float* act, const float* att, float* sino) {
+int project_host(Problem& pb, const float* act, const float* att, float* sino) {
   int s;
   DeviceState& ds = current_device_state(&s);
   if (s != kOk) return s;
   std::lock_guard<std::mutex> lk(ds.mu);
   const size_t nvox = static_cast<size_t>(pb.nx) * pb.ny * pb.nz;
   const size_t nsino = static_cast<size_t>(pb.nx) * pb.ny * pb.cams.n;
-  const size_t ws = project_workspace(pb, act != nullptr, att != nullptr);
-  if ((s = ensure_arena(ds, fbytes(2 * nvox + nsino) + 4 * 256 + ws)) != kOk) return s;
+  auto work = [&](const Problem& q) { return project_workspace(q, act != nullptr, att != nullptr); };
+  auto bytes = [&](const Problem& q) { return fbytes(2 * nvox + nsino) + 4 * 256 + work(q); };
+  if ((s = reserve_arena(ds, pb, bytes)) != kOk) return s;
+  const size_t ws = work(pb);
   Carver cv(ds.arena, ds.arena_bytes);
   float* d_act = act ? cv.take<float>(nvox) : nullptr;
   float* d_att = att ? cv.take<float>(nvox) : nullptr;
@@ -119,15 +121,17 @@ int project_host(const Problem& pb, const float* act, const float* att, float* s
   return finish(ds, s);
 }
 
-int backproject_host(const Problem& pb, const float* sino, const float* att, float* out) {
+int backproject_host(Problem& pb, const float* sino, const float* att, float* out) {
   int s;
   DeviceState& ds = current_device_state(&s);
   if (s != kOk) return s;
   std::lock_guard<std::mutex> lk(ds.mu);
   const size_t nvox = static_cast<size_t>(pb.nx) * pb.ny * pb.nz;
   const size_t nsino = static_cast<size_t>(pb.nx) * pb.ny * pb.cams.n;
-  const size_t ws = backproject_workspace(pb, att != nullptr);
-  if ((s = ensure_arena(ds, fbytes(2 * nvox + nsino) + 4 * 256 + ws)) != kOk) return s;
+  auto work = [&](const Problem& q) { return backproject_workspace(q, att != nullptr); };
+  auto bytes = [&](const Problem& q) { return fbytes(2 * nvox + nsino) + 4 * 256 + work(q); };
+  if ((s = reserve_arena(ds, pb, bytes)) != kOk) return s;
+  const size_t ws = work(pb);
   Carver cv(ds.arena, ds.arena_bytes);
   float* d_sino = cv.take<float>(nsino);
   float* d_att = att ? cv.take<float>(nvox) : nullptr;
@@ -149,15 +153,17 @@ int backproject_host(const Problem& pb, const float* sino, const float* att, flo
   return finish(ds, s);
 }
 
-int gradient_host(const Problem& pb, const float* sino, const float* act, const float* att, float* out) {
+int gradient_host(Problem& pb, const float* sino, const float* act, const float* att, float* out) {
   int s;
   DeviceState& ds = current_device_state(&s);
   if (s != kOk) return s;
   std::lock_guard<std::mutex> lk(ds.mu);
   const size_t nvox = static_cast<size_t>(pb.nx) * pb.ny * pb.nz;
   const size_t nsino = static_cast<size_t>(pb.nx) * pb.ny * pb.cams.n;
-  const size_t ws = gradient_workspace(pb);
-  if ((s = ensure_arena(ds, fbytes(3 * nvox + nsino) + 5 * 256 + ws)) != kOk) return s;
+  auto work = [&](const Problem& q) { return gradient_workspace(q); };
+  auto bytes = [&](const Problem& q) { return fbytes(3 * nvox + nsino) + 5 * 256 + work(q); };
+  if ((s = reserve_arena(ds, pb, bytes)) != kOk) return s;
+  const size_t ws = work(pb);
   Carver cv(ds.arena, ds.arena_bytes);
   float* d_sino = cv.take<float>(nsino);
   float* d_act = cv.take<float>(nvox);
@@ -184,15 +190,19 @@ int gradient_host(const Problem& pb, const float* sino, const float* act, const 
 // One OSEM step over the given camera subset on the device:
 // project (truncate) -> ratio -> backproject ratio and ones (truncate) -> update,
 // emission-lib/_et_array_interface.cpp:1017-1044.
-int osem_step_host(const Problem& pb, float* act, const float* ysub, const float* att, float eps) {
+int osem_step_host(Problem& pb, float* act, const float* ysub, const float* att, float eps) {
   int s;
   DeviceState& ds = current_device_state(&s);
   if (s != kOk) return s;
   std::lock_guard<std::mutex> lk(ds.mu);
   const size_t nvox = static_cast<size_t>(pb.nx) * pb.ny * pb.nz;
   const size_t nsino = static_cast<size_t>(pb.nx) * pb.ny * pb.cams.n;
-  const size_t ws = std::max(project_workspace(pb, true, att != nullptr), backproject_workspace(pb, att != nullptr));
-  if ((s = ensure_arena(ds, fbytes(4 * nvox + 3 * nsino) + 8 * 256 + ws)) != kOk) return s;
+  auto work = [&](const Problem& q) {
+    return std::max(project_workspace(q, true, att != nullptr), backproject_workspace(q, att != nullptr));
+  };
+  auto bytes = [&](const Problem& q) { return fbytes(4 * nvox + 3 * nsino) + 8 * 256 + work(q); };
+  if ((s = reserve_arena(ds, pb, bytes)) != kOk) return s;
+  const size_t ws = work(pb);
   Carver cv(ds.arena, ds.arena_bytes);
   float* d_act = cv.take<float>(nvox);
   float* d_att = att ? cv.take<float>(nvox) : nullptr;
@@ -285,7 +295,7 @@ int fisher_from_projection(DeviceState& ds, Carver& cv, const float* d_proj, int
   return s;
 }
 
-int project_partial_host(const Problem& pb, const float* act, const float* att, const float* bg_image, float* sino,
+int project_partial_host(Problem& pb, const float* act, const float* att, const float* bg_image, float* sino,
                          float* partial, int do_rotate) {
   int s;
   DeviceState& ds = current_device_state(&s);
@@ -295,8 +305,10 @@ int project_partial_host(const Problem& pb, const float* act, const float* att, 
   const size_t nxy = static_cast<size_t>(pb.nx) * pb.ny;
   const size_t nsino = nxy * pb.cams.n;
   const size_t npart = nvox * pb.cams.n;
-  const size_t ws = partial_workspace(pb);
-  if ((s = ensure_arena(ds, fbytes(2 * nvox + nxy + nsino + npart) + 6 * 256 + ws)) != kOk) return s;
+  auto work = [&](const Problem& q) { return partial_workspace(q); };
+  auto bytes = [&](const Problem& q) { return fbytes(2 * nvox + nxy + nsino + npart) + 6 * 256 + work(q); };
+  if ((s = reserve_arena(ds, pb, bytes)) != kOk) return s;
+  const size_t ws = work(pb);
   Carver cv(ds.arena, ds.arena_bytes);
   float* d_act = act ? cv.take<float>(nvox) : nullptr;
   float* d_att = att ? cv.take<float>(nvox) : nullptr;
@@ -855,8 +867,10 @@ int et_array_fisher_grid(float* activity_ptr, int* activity_size, float* cameras
   const size_t extra = sizeof(int) * (3 * static_cast<size_t>(n) * (ncam + 1)) +
                        sizeof(float) * (static_cast<size_t>(psf_size[0]) * psf_size[1] * psf_size[2] +
                                         2 * static_cast<size_t>(n) * n) + 8 * 256;
-  const size_t ws = project_workspace(pb, true, !no_att);
-  if ((s = ensure_arena(ds, fbytes(2 * nvox + nsino) + 4 * 256 + ws + extra)) != kOk) return s;
+  auto work = [&](const Problem& q) { return project_workspace(q, true, !no_att); };
+  auto bytes = [&](const Problem& q) { return fbytes(2 * nvox + nsino) + 4 * 256 + extra + work(q); };
+  if ((s = reserve_arena(ds, pb, bytes)) != kOk) return s;
+  const size_t ws = work(pb);
   Carver cv(ds.arena, ds.arena_bytes);
   float* d_act = cv.take<float>(nvox);
   float* d_att = no_att ? nullptr : cv.take<float>(nvox);
@@ -996,8 +1010,10 @@ int project_device_call(const float* d_activity, const float* d_attenuation, con
   DeviceState& ds = current_device_state(&s);
   if (s != kOk) return s;
   std::lock_guard<std::mutex> lk(ds.mu);
-  const size_t ws = project_workspace(pb, d_activity != nullptr, d_attenuation != nullptr);
-  if ((s = ensure_arena(ds, ws)) != kOk) return s;
+  auto work = [&](const Problem& q) {
+    return project_workspace(q, d_activity != nullptr, d_attenuation != nullptr);
+  };
+  if ((s = reserve_arena(ds, pb, work)) != kOk) return s;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaStreamWaitEvent(st, ds.last_use, 0);
   g_last_path = ((use_fused(pb) || use_fused_x(pb)) && d_activity) ? 1 : 2;
@@ -1030,8 +1046,8 @@ int backproject_device_call(const float* d_sinogram, const float* d_attenuation,
   DeviceState& ds = current_device_state(&s);
   if (s != kOk) return s;
   std::lock_guard<std::mutex> lk(ds.mu);
-  const size_t ws = backproject_workspace(pb, d_attenuation != nullptr);
-  if ((s = ensure_arena(ds, ws)) != kOk) return s;
+  auto work = [&](const Problem& q) { return backproject_workspace(q, d_attenuation != nullptr); };
+  if ((s = reserve_arena(ds, pb, work)) != kOk) return s;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaStreamWaitEvent(st, ds.last_use, 0);
   g_last_path = (use_fused(pb) || use_fused_x(pb)) ? 1 : 2;
@@ -1068,9 +1084,12 @@ int pair_device_call(const float* d_activity, const float* d_attenuation, const 
   DeviceState& ds = current_device_state(&s);
   if (s != kOk) return s;
   std::lock_guard<std::mutex> lk(ds.mu);
-  const size_t ws = std::max(pair_workspace(pb, d_attenuation != nullptr, d_backproject_input != nullptr),
-                             backproject_workspace(pbb, d_attenuation != nullptr));
-  if ((s = ensure_arena(ds, ws)) != kOk) return s;
+  auto work = [&](const Problem& q) {
+    pbb.lean = q.lean;
+    return std::max(pair_workspace(q, d_attenuation != nullptr, d_backproject_input != nullptr),
+                    backproject_workspace(pbb, d_attenuation != nullptr));
+  };
+  if ((s = reserve_arena(ds, pb, work)) != kOk) return s;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaStreamWaitEvent(st, ds.last_use, 0);
   g_last_path = (use_fused(pb) || use_fused_x(pb)) ? 1 : 2;
@@ -1165,7 +1184,7 @@ int nrgb_project_device_f64(const double* d_activity, const double* d_attenuatio
   DeviceState& ds = current_device_state(&s);
   if (s != kOk) return s;
   std::lock_guard<std::mutex> lk(ds.mu);
-  if ((s = ensure_arena(ds, workspace64(pb))) != kOk) return s;
+  if ((s = reserve_arena(ds, pb, workspace64)) != kOk) return s;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaStreamWaitEvent(st, ds.last_use, 0);
   g_last_path = 2;
@@ -1191,7 +1210,7 @@ int nrgb_backproject_device_f64(const double* d_sinogram, const double* d_attenu
   DeviceState& ds = current_device_state(&s);
   if (s != kOk) return s;
   std::lock_guard<std::mutex> lk(ds.mu);
-  if ((s = ensure_arena(ds, workspace64(pb))) != kOk) return s;
+  if ((s = reserve_arena(ds, pb, workspace64)) != kOk) return s;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaStreamWaitEvent(st, ds.last_use, 0);
   g_last_path = 2;
@@ -1235,8 +1254,7 @@ int nrgb_attenuation_grad_device(const float* d_grad_sinogram, const float* d_ac
   DeviceState& ds = current_device_state(&s);
   if (s != kOk) return s;
   std::lock_guard<std::mutex> lk(ds.mu);
-  const size_t ws = dmu_workspace(pb);
-  if ((s = ensure_arena(ds, ws)) != kOk) return s;
+  if ((s = reserve_arena(ds, pb, dmu_workspace)) != kOk) return s;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaStreamWaitEvent(st, ds.last_use, 0);
   g_last_path = (use_fused(pb) || use_fused_x(pb)) ? 1 : 2;
@@ -1263,8 +1281,7 @@ int nrgb_gradient_attenuation_device(const float* d_sinogram, const float* d_act
   DeviceState& ds = current_device_state(&s);
   if (s != kOk) return s;
   std::lock_guard<std::mutex> lk(ds.mu);
-  const size_t ws = gradient_workspace(pb);
-  if ((s = ensure_arena(ds, ws)) != kOk) return s;
+  if ((s = reserve_arena(ds, pb, gradient_workspace)) != kOk) return s;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaStreamWaitEvent(st, ds.last_use, 0);
   g_last_path = (use_fused(pb) || use_fused_x(pb)) && pb.storage == kStorageF32 ? 1 : 2;

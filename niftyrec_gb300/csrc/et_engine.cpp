@@ -151,11 +151,27 @@ bool use_fused_x(const Problem& pb) {
 namespace {
 
 size_t vol_n(const Problem& pb) { return static_cast<size_t>(pb.nx) * pb.ny * pb.nz; }
-// Cameras per launch of the general path and its three sets of work volumes.
-int gen_group(const Problem& pb) { return general_group(vol_n(pb), sizeof(float), pb.cams.n); }
-size_t gen_n(const Problem& pb) { return vol_n(pb) * gen_group(pb); }
-// Its projection's and backprojection's work space (the sources' two volumes too).
-size_t gen_bytes(const Problem& pb) { return sizeof(float) * (3 * gen_n(pb) + 2 * vol_n(pb)); }
+// Cameras per launch of the general path; its three sets of work volumes, and
+// for projection and backprojection (sources) two volumes more.
+size_t gen_group(const Problem& pb, size_t element) {
+  return pb.lean ? 1 : general_group(vol_n(pb), element, pb.cams.n);
+}
+size_t gen_src_n(const Problem& pb, bool sources) { return sources && !pb.lean ? 2 * vol_n(pb) : 0; }
+size_t gen_bytes(const Problem& pb, size_t element, bool sources) {
+  return element * (3 * vol_n(pb) * gen_group(pb, element) + gen_src_n(pb, sources));
+}
+
+template <class T>
+int gen_work(const Problem& pb, bool sources, Carver& cv, GeneralArgsT<T>* g) {
+  g->group = static_cast<int>(gen_group(pb, sizeof(T)));
+  const size_t n = vol_n(pb) * g->group, src = gen_src_n(pb, sources);
+  g->ws_act = cv.take<T>(n);
+  g->ws_att = cv.take<T>(n);
+  g->ws_tmp = cv.take<T>(n);
+  g->ws_src = src ? cv.take<T>(src) : nullptr;
+  return g->ws_act && g->ws_att && g->ws_tmp && (g->ws_src || !src) ? kOk : kErrAllocGpu;
+}
+
 size_t col_n(const Problem& pb) { return static_cast<size_t>(pb.nx) * round_up(pb.ny, 4) * pb.nz; }
 size_t sino_col_n(const Problem& pb) { return static_cast<size_t>(pb.nx) * round_up(pb.ny, 4) * pb.cams.n; }
 constexpr size_t kSlack = 8 * 256;
@@ -269,11 +285,11 @@ int widen_inputs(const Problem& pb, Carver& cv, const float** act, const float**
 
 size_t project_workspace(const Problem& pb, bool has_act, bool has_att) {
   size_t b = common_bytes(pb);
-  if (use_fused_x(pb) && has_act) return b + gen_bytes(pb) + widen_bytes(pb);  // or general
+  if (use_fused_x(pb) && has_act) return b + gen_bytes(pb, sizeof(float), true) + widen_bytes(pb);  // or general
   if (use_fused(pb) && has_act)
     b += sizeof(float) * (col_n(pb) * (has_att ? 2 : 1) + sino_col_n(pb));
   else
-    b += gen_bytes(pb) + widen_bytes(pb);
+    b += gen_bytes(pb, sizeof(float), true) + widen_bytes(pb);
   return b;
 }
 
@@ -281,29 +297,37 @@ size_t backproject_workspace(const Problem& pb, bool has_att) {
   size_t b = common_bytes(pb);
   if (use_fused_x(pb))  // the fused form's scratch, or the general path's volumes
     return b + std::max(yg_backproject_workspace(pb.ny, pb.nx, pb.nz, pb.cams.n, pb.group) + kSlack,
-                        gen_bytes(pb) + widen_bytes(pb));
+                        gen_bytes(pb, sizeof(float), true) + widen_bytes(pb));
   if (use_fused(pb))
     b += sizeof(float) * (col_n(pb) * (has_att ? 2 : 1) + sino_col_n(pb)) +
          yg_backproject_workspace(pb.nx, pb.ny, pb.nz, pb.cams.n, pb.group) + kSlack;
   else
-    b += gen_bytes(pb) + widen_bytes(pb);
+    b += gen_bytes(pb, sizeof(float), true) + widen_bytes(pb);
   return b;
 }
 
 namespace {
 // The general-orientation path's work volumes.
-size_t general3_workspace(const Problem& pb) { return common_bytes(pb) + sizeof(float) * gen_n(pb) * 3; }
-int grad_group(const Problem& pb) { return std::max(1, std::min(pb.group, pb.cams.n)); }
+size_t general3_workspace(const Problem& pb) { return common_bytes(pb) + gen_bytes(pb, sizeof(float), false); }
+// Scratch volumes of the fused attenuation gradient: three slots of the
+// backprojector's, at least one mirror unit's; two slots where memory is short.
+int grad_volumes(const Problem& pb) {
+  const int slot = std::max(1, std::min(pb.group, pb.cams.n));
+  if (pb.lean) return 2 * slot;
+  return std::max(pb.units.empty() && pb.units_x.empty() ? 2 : 4, 3 * slot);
+}
+// Cameras per group of the fused d/dmu; one unit where memory is short.
+int dmu_group(const Problem& pb) { return pb.lean ? 1 : pb.group; }
 }  // namespace
 
 size_t gradient_workspace(const Problem& pb) {
   if (pb.storage != kStorageF32) return general3_workspace(pb);
   if (use_fused_x(pb))  // the fused form's scratch, or the general path's volumes
     return std::max(general3_workspace(pb),
-                    common_bytes(pb) + yg_gradient_workspace(pb.ny, pb.nx, pb.nz, pb.cams.n, grad_group(pb)) + kSlack);
+                    common_bytes(pb) + yg_gradient_workspace(pb.ny, pb.nx, pb.nz, grad_volumes(pb)) + kSlack);
   if (use_fused(pb))
     return common_bytes(pb) + sizeof(float) * (3 * col_n(pb) + sino_col_n(pb)) +
-           yg_gradient_workspace(pb.nx, pb.ny, pb.nz, pb.cams.n, grad_group(pb)) + kSlack;
+           yg_gradient_workspace(pb.nx, pb.ny, pb.nz, grad_volumes(pb)) + kSlack;
   return general3_workspace(pb);
 }
 
@@ -389,12 +413,7 @@ int project_device(const Problem& pb, const float* d_act, const float* d_att, fl
   g.bg = pb.bg;
   g.bg_att = pb.bg_att;
   g.truncate = pb.truncate;
-  g.group = gen_group(pb);
-  g.ws_act = cv.take<float>(gen_n(pb));
-  g.ws_att = cv.take<float>(gen_n(pb));
-  g.ws_tmp = cv.take<float>(gen_n(pb));
-  g.ws_src = cv.take<float>(2 * vol_n(pb));
-  if (!g.ws_act || !g.ws_att || !g.ws_tmp || !g.ws_src) return kErrAllocGpu;
+  if ((s = gen_work(pb, true, cv, &g)) != kOk) return s;
   return check(general_project(g, st));
 }
 
@@ -522,12 +541,7 @@ int backproject_device(const Problem& pb, const float* d_sino, const float* d_at
   g.bg = pb.bg;
   g.bg_att = pb.bg_att;
   g.truncate = pb.truncate;
-  g.group = gen_group(pb);
-  g.ws_act = cv.take<float>(gen_n(pb));
-  g.ws_att = cv.take<float>(gen_n(pb));
-  g.ws_tmp = cv.take<float>(gen_n(pb));
-  g.ws_src = cv.take<float>(2 * vol_n(pb));
-  if (!g.ws_act || !g.ws_att || !g.ws_tmp || !g.ws_src) return kErrAllocGpu;
+  if ((s = gen_work(pb, true, cv, &g)) != kOk) return s;
   return check(pb.back_mode == kBackAdjoint ? general_adjoint(g, st) : general_backproject(g, st));
 }
 
@@ -636,7 +650,9 @@ int pair_device(const Problem& pb, const Problem& pb_back, const float* d_act, c
   return check(from_column(out_c, d_bk, pb.nx, pb.ny, cy, pb.nz, pb.truncate, st));
 }
 
-size_t partial_workspace(const Problem& pb) { return common_bytes(pb) + sizeof(float) * gen_n(pb) * 3 + 3 * 256; }
+size_t partial_workspace(const Problem& pb) {
+  return common_bytes(pb) + gen_bytes(pb, sizeof(float), false) + 3 * 256;
+}
 
 int project_partial_device(const Problem& pb, const float* d_act, const float* d_att, const float* d_bg_image,
                            float* d_sino, float* d_partial, int do_rotate, char* ws, size_t ws_bytes, Staging* stg,
@@ -660,21 +676,17 @@ int project_partial_device(const Problem& pb, const float* d_act, const float* d
   g.bg = pb.bg;
   g.bg_att = pb.bg_att;
   g.truncate = pb.truncate;
-  g.group = gen_group(pb);
-  g.ws_act = cv.take<float>(gen_n(pb));
-  g.ws_att = cv.take<float>(gen_n(pb));
-  g.ws_tmp = cv.take<float>(gen_n(pb));
-  if (!g.ws_act || !g.ws_att || !g.ws_tmp) return kErrAllocGpu;
+  if ((s = gen_work(pb, false, cv, &g)) != kOk) return s;
   return check(general_project_partial(g, d_bg_image, d_partial, do_rotate, st));
 }
 
 size_t dmu_workspace(const Problem& pb) {
   if (use_fused_x(pb) && pb.storage == kStorageF32)  // the fused form's scratch, or the general path's volumes
     return std::max(general3_workspace(pb),
-                    common_bytes(pb) + yg_dmu_workspace(pb.ny, pb.nx, pb.nz, pb.cams.n, pb.group) + kSlack);
+                    common_bytes(pb) + yg_dmu_workspace(pb.ny, pb.nx, pb.nz, pb.cams.n, dmu_group(pb)) + kSlack);
   if (use_fused(pb) && pb.storage == kStorageF32)
     return common_bytes(pb) + sizeof(float) * (3 * col_n(pb) + sino_col_n(pb)) + 4 * 256 +
-           yg_dmu_workspace(pb.nx, pb.ny, pb.nz, pb.cams.n, pb.group) + kSlack;
+           yg_dmu_workspace(pb.nx, pb.ny, pb.nz, pb.cams.n, dmu_group(pb)) + kSlack;
   return general3_workspace(pb);
 }
 
@@ -693,7 +705,7 @@ int dmu_device(const Problem& pb, const float* d_g, const float* d_act, const fl
     a.sino = d_g;
     a.out = d_out;
     a.det = pb.det;
-    a.group = pb.group;
+    a.group = dmu_group(pb);
     a.work = cx.take<float>(yg_dmu_workspace(a.nx, a.ny, a.nz, a.ncam, a.group) / sizeof(float));
     if (!a.work) return kErrAllocGpu;
     return check(yg_dmu(a, st));
@@ -731,7 +743,7 @@ int dmu_device(const Problem& pb, const float* d_g, const float* d_act, const fl
     a.units = d_units;
     a.nunits = static_cast<int>(pb.units.size() / 2);
     a.det = pb.det;
-    a.group = pb.group;
+    a.group = dmu_group(pb);
     a.work = cv.take<float>(yg_dmu_workspace(a.nx, a.ny, a.nz, a.ncam, a.group) / sizeof(float));
     if (!a.work) return kErrAllocGpu;
     if ((s = yg_dmu(a, st)) != kOk) return s;
@@ -751,11 +763,7 @@ int dmu_device(const Problem& pb, const float* d_g, const float* d_act, const fl
   g.psf_k = pb.psf_k;
   g.bg = pb.bg;
   g.bg_att = pb.bg_att;
-  g.group = gen_group(pb);
-  g.ws_act = cv.take<float>(gen_n(pb));
-  g.ws_att = cv.take<float>(gen_n(pb));
-  g.ws_tmp = cv.take<float>(gen_n(pb));
-  if (!g.ws_act || !g.ws_att || !g.ws_tmp) return kErrAllocGpu;
+  if ((s = gen_work(pb, false, cv, &g)) != kOk) return s;
   return check(general_dmu(g, st));
 }
 
@@ -773,8 +781,8 @@ int gradient_device(const Problem& pb, const float* d_sino, const float* d_act, 
     a.mu = d_att;
     a.sino = d_sino;
     a.out = d_out;
-    a.group = grad_group(pb);
-    a.work = cx.take<float>(yg_gradient_workspace(pb.ny, pb.nx, pb.nz, pb.cams.n, a.group) / sizeof(float));
+    a.group = grad_volumes(pb);
+    a.work = cx.take<float>(yg_gradient_workspace(pb.ny, pb.nx, pb.nz, a.group) / sizeof(float));
     if (!a.work) return kErrAllocGpu;
     return check(yg_gradient(a, st));
   }
@@ -790,8 +798,8 @@ int gradient_device(const Problem& pb, const float* d_sino, const float* d_act, 
     float* mu_c = cv.take<float>(col_n(pb));
     float* out_c = cv.take<float>(col_n(pb));
     float* sino_c = cv.take<float>(sino_col_n(pb));
-    const int group = grad_group(pb);
-    float* work = cv.take<float>(yg_gradient_workspace(pb.nx, pb.ny, pb.nz, pb.cams.n, group) / sizeof(float));
+    const int volumes = grad_volumes(pb);
+    float* work = cv.take<float>(yg_gradient_workspace(pb.nx, pb.ny, pb.nz, volumes) / sizeof(float));
     if (!act_c || !mu_c || !out_c || !sino_c || !work) return kErrAllocGpu;
     if ((s = to_column(d_act, act_c, pb.nx, pb.ny, cy, pb.nz, st)) != kOk) return s;
     if ((s = to_column(d_att, mu_c, pb.nx, pb.ny, cy, pb.nz, st)) != kOk) return s;
@@ -812,7 +820,7 @@ int gradient_device(const Problem& pb, const float* d_sino, const float* d_act, 
     a.psf_k = pb.psf_k;
     a.units = d_units;
     a.nunits = static_cast<int>(pb.units.size() / 2);
-    a.group = group;
+    a.group = volumes;
     a.work = work;
     if ((s = yg_gradient(a, st)) != kOk) return s;
     return check(from_column(out_c, d_out, pb.nx, pb.ny, cy, pb.nz, pb.truncate, st));
@@ -832,18 +840,13 @@ int gradient_device(const Problem& pb, const float* d_sino, const float* d_act, 
   g.bg = pb.bg;
   g.bg_att = pb.bg_att;
   g.truncate = pb.truncate;
-  g.group = gen_group(pb);
-  g.ws_act = cv.take<float>(gen_n(pb));
-  g.ws_att = cv.take<float>(gen_n(pb));
-  g.ws_tmp = cv.take<float>(gen_n(pb));
-  if (!g.ws_act || !g.ws_att || !g.ws_tmp) return kErrAllocGpu;
+  if ((s = gen_work(pb, false, cv, &g)) != kOk) return s;
   return check(general_gradient(g, st));
 }
 
 // ------------------------------------------------------------ float64 run
 size_t workspace64(const Problem& pb) {
-  const size_t group = general_group(vol_n(pb), sizeof(double), pb.cams.n);
-  return sizeof(double) * (vol_n(pb) * (3 * group + 2) + static_cast<size_t>(2 * pb.psf_k) * pb.nz) + kSlack;
+  return gen_bytes(pb, sizeof(double), true) + sizeof(double) * static_cast<size_t>(2 * pb.psf_k) * pb.nz + kSlack;
 }
 
 namespace {
@@ -871,12 +874,7 @@ int setup64(const Problem& pb, const float* psf_host, Carver& cv, std::vector<Ca
       return kErrTransferGpu;
     g->psf_sep = d;
   }
-  g->group = general_group(vol_n(pb), sizeof(double), pb.cams.n);
-  g->ws_act = cv.take<double>(vol_n(pb) * g->group);
-  g->ws_att = cv.take<double>(vol_n(pb) * g->group);
-  g->ws_tmp = cv.take<double>(vol_n(pb) * g->group);
-  g->ws_src = cv.take<double>(2 * vol_n(pb));
-  return (g->ws_act && g->ws_att && g->ws_tmp && g->ws_src) ? kOk : kErrAllocGpu;
+  return gen_work(pb, true, cv, g);
 }
 
 }  // namespace

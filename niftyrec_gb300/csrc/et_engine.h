@@ -44,6 +44,10 @@ struct Problem {
   // kernels (scratch + transposed gather instead of vector reductions); set
   // from the library-wide switch when the problem is made.
   int det = 0;
+  // Set where the device memory does not hold the work space the kernels like
+  // (reserve_arena): the general path's three work volumes of one camera, the
+  // attenuation gradient's two scratch slots, d/dmu unit by unit.
+  int lean = 0;
 };
 
 // Build a Problem; psf may be null.  psf_size = {kx, ky, planes}.  Returns
@@ -125,6 +129,18 @@ class Carver {
 
 // Ensure the arena holds at least `bytes`.
 int ensure_arena(DeviceState& ds, size_t bytes);
+
+// The same for bytes(pb), or where that cannot be had, with pb.lean set, for the
+// smaller work space that asks for.
+template <class Bytes>
+int reserve_arena(DeviceState& ds, Problem& pb, Bytes bytes) {
+  const size_t want = bytes(pb);
+  const int s = ensure_arena(ds, want);
+  if (s != kErrAllocGpu) return s;
+  pb.lean = 1;
+  const size_t need = bytes(pb);
+  return need < want ? ensure_arena(ds, need) : s;
+}
 
 // Device-pointer operations (nifti layout in and out, stream-ordered).
 size_t project_workspace(const Problem& pb, bool has_act, bool has_att);

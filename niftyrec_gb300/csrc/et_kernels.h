@@ -178,9 +178,9 @@ int yg_backproject(const YgArgs& a, cudaStream_t st);
 void yg_gather(const YgArgs& a, int c0, int gcount, int first, int clamp, cudaStream_t st);
 // The reference's attenuation gradient (a.act, a.mu sampled, a.sino the camera
 // planes, a.out the gradient; with a.truncate negative results are stored as
-// zero); a.work holds yg_gradient_workspace bytes.
+// zero); a.group scratch volumes (at least 2) in a.work, yg_gradient_workspace bytes.
 int yg_gradient(const YgArgs& a, cudaStream_t st);
-size_t yg_gradient_workspace(int nx, int ny, int nz, int ncam, int group);
+size_t yg_gradient_workspace(int nx, int ny, int nz, int volumes);
 
 // ---- batches of volumes (one OSEM subset step of many plans at once) ----
 constexpr int kMaxBatch = 64;    // volumes per batched launch

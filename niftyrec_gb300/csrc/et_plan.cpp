@@ -40,6 +40,8 @@ struct Plan {
   float* mu = nullptr;     // column layout (fused) or nifti copy (general)
   float* carry = nullptr;  // [ncam][bslabs + 1][nx][cy] (fused with attenuation)
   int bslabs = 0;          // depth slabs of the spread and the carries
+  int gen_group = 1;       // general path: cameras per launch, and whether `work` holds the sources' two volumes
+  bool gen_sources = true;
   float* act_c = nullptr;  // column staging for nifti-layout calls (fused)
   float* sino_c = nullptr;
   float* out_c = nullptr;
@@ -133,12 +135,12 @@ int plan_project(Plan& p, int subset, const float* d_act, float* d_sino, int lay
   g.bg_att = pb.bg_att;
   g.truncate = truncate;
   size_t nv = static_cast<size_t>(pb.nx) * pb.ny * pb.nz;
-  g.group = general_group(nv, sizeof(float), pb.cams.n);
+  g.group = p.gen_group;
   nv *= g.group;
   g.ws_act = p.work;
   g.ws_att = p.work + nv;
   g.ws_tmp = p.work + 2 * nv;
-  g.ws_src = p.work + 3 * nv;
+  g.ws_src = p.gen_sources ? p.work + 3 * nv : nullptr;
   int s = general_project(g, st);
   return s != kOk ? s : check();
 }
@@ -200,12 +202,12 @@ int plan_backproject(Plan& p, int subset, const float* d_sino, float* d_out, int
   g.bg_att = pb.bg_att;
   g.truncate = truncate;
   size_t nv = static_cast<size_t>(pb.nx) * pb.ny * pb.nz;
-  g.group = general_group(nv, sizeof(float), pb.cams.n);
+  g.group = p.gen_group;
   nv *= g.group;
   g.ws_act = p.work;
   g.ws_att = p.work + nv;
   g.ws_tmp = p.work + 2 * nv;
-  g.ws_src = p.work + 3 * nv;
+  g.ws_src = p.gen_sources ? p.work + 3 * nv : nullptr;
   int s = general_backproject(g, st);
   return s != kOk ? s : check();
 }
@@ -317,14 +319,23 @@ int nrgb_plan_create(void** out_plan, const int* size, const float* cameras, con
                     sizeof(float) * static_cast<size_t>(ncam) * yg_carry_slabs() * nx * p->cy;
   } else {
     bytes += al(sizeof(float) * nv) * (p->has_att ? 1 : 0);
-    p->work_bytes = sizeof(float) * nv * (3 * general_group(nv, sizeof(float), ncam) + 2);
+    p->gen_group = general_group(nv, sizeof(float), ncam);
+    p->work_bytes = sizeof(float) * nv * (3 * p->gen_group + 2);
   }
-  bytes += al(p->work_bytes);
-  if (cudaMalloc(&p->mem, bytes) != cudaSuccess) {
+  cudaError_t got = cudaMalloc(&p->mem, bytes + al(p->work_bytes));
+  if (got != cudaSuccess && !p->fused) {  // the general path one camera at a time, on three volumes
+    cudaGetLastError();
+    p->gen_group = 1;
+    p->gen_sources = false;
+    p->work_bytes = sizeof(float) * nv * 3;
+    got = cudaMalloc(&p->mem, bytes + al(p->work_bytes));
+  }
+  if (got != cudaSuccess) {
     cudaGetLastError();
     delete p;
     return kErrAllocGpu;
   }
+  bytes += al(p->work_bytes);
   p->bytes = bytes;
   Carver cv(p->mem, bytes);
   p->geom_p = cv.take<CamGeom>(ncam);

@@ -313,23 +313,17 @@ int launch_weights(const YgArgs& a, int u0, int n, cudaStream_t st) {
   return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
 }
 
-// Units (or cameras) per group: their w and PSF volumes, two of each per mirror
-// unit, in three scratch slots of the backprojector.
-int grad_units(int n, int ncam, int group, bool pair) {
-  const int volumes = 3 * std::max(1, std::min(group, ncam));
-  return yg_even_group(n, std::max(1, volumes / (pair ? 4 : 2)));
-}
-
 }  // namespace
 
 int yg_gradient(const YgArgs& a_in, cudaStream_t st) {
   YgArgs a = a_in;
-  if (!a.mu || !a.act || !a.sino || !a.out || !a.work) return kErrParameters;
+  if (!a.mu || !a.act || !a.sino || !a.out || !a.work || a.group < 2) return kErrParameters;
   const int R = a.psf ? (a.psf_k - 1) / 2 : 0;
-  const bool pair = a.units && a.nunits > 0;
+  // units (or cameras) per group: w and PSF volumes, two of each per mirror unit
+  const bool pair = a.units && a.nunits > 0 && a.group >= 4;
   if (!pair) a.units = nullptr;
   const int units = pair ? a.nunits : a.ncam;
-  const int group = grad_units(units, a.ncam, a.group, pair);
+  const int group = yg_even_group(units, a.group / (pair ? 4 : 2));
   const int slots = pair ? 2 * group : group;  // volumes of a group
   a.group = group;
   for (const Window& w : call_windows(a, R)) {
@@ -361,10 +355,8 @@ int yg_gradient(const YgArgs& a_in, cudaStream_t st) {
   return cudaGetLastError() == cudaSuccess ? kOk : kErrKernel;
 }
 
-size_t yg_gradient_workspace(int nx, int ny, int nz, int ncam, int group) {
-  const size_t vol = static_cast<size_t>(nz) * nx * scratch_rows(ny);
-  // at least one unit: two volumes, and two blurred
-  return sizeof(float) * vol * std::max(4, 3 * std::max(1, std::min(group, ncam)));
+size_t yg_gradient_workspace(int nx, int ny, int nz, int volumes) {
+  return sizeof(float) * static_cast<size_t>(nz) * nx * scratch_rows(ny) * volumes;
 }
 
 }  // namespace nrgb
