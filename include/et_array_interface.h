@@ -423,11 +423,17 @@ int nrgb_get_deterministic(void);
  * fused kernels form for this camera table and volume size {nx, ny, nz};
  * *n_units = 0 when every camera runs on its own.  nrgb_row_windows: the row
  * windows {first row, rows, first valid row, end of valid rows} of ny rows for
- * a PSF of width psf_k (0: none).  Both return status 2 when the output
- * cannot hold the result (the count is still written). */
+ * a PSF of width psf_k (0: none), the last one whole.  nrgb_volume_windows: the
+ * windows that the projector and backprojector run for a volume of size {nx, ny,
+ * nz}, whose last one is split where two narrow ones are less work, with the
+ * lanes per column of each as a fifth number; PSF widths to 15 (with
+ * nrgb_set_deterministic on, backprojections and d/dmu keep the last window
+ * whole; cameras about x: the size with nx and ny exchanged).  All return status 2 when the output cannot
+ * hold the result (the count is still written). */
 int nrgb_mirror_units(const float *cameras, const int *cameras_size, const int *size, int *out_units, int max_units,
                       int *n_units);
 int nrgb_row_windows(int ny, int psf_k, int *out, int max_windows, int *n_windows);
+int nrgb_volume_windows(const int *size, int psf_k, int *out, int max_windows, int *n_windows);
 /* The batched projector's launch for volumes of up to max_nz planes, a PSF of
  * width psf_k (0: none), with or without mu, on the current device: out = {CTAs
  * per SM its kernel is built for, the kernel's static shared memory and its local

@@ -112,6 +112,7 @@ PROTOTYPES = {
     "nrgb_profile_only": (_I, [ctypes.c_char_p]),
     "nrgb_mirror_units": (_I, [_P, _PI, _PI, _PI, _I, _PI]),
     "nrgb_batch_projector_info": (_I, [_I, _I, _I, _PI]),
+    "nrgb_volume_windows": (_I, [_PI, _I, _PI, _I, _PI]),
     "nrgb_row_windows": (_I, [_I, _I, _PI, _I, _PI]),
 }
 

@@ -1380,7 +1380,7 @@ int nrgb_mirror_units(const float* cameras, const int* cameras_size, const int* 
 
 // Row windows of the fused kernels for ny rows and a PSF of width psf_k (0:
 // none), host only: {first row, rows, first valid row, end of valid rows}
-// per window (valid rows relative to the first row).
+// per window (valid rows relative to the first row), the last one whole.
 int nrgb_row_windows(int ny, int psf_k, int* out, int max_windows, int* n_windows) {
   NRGB_API("nrgb_row_windows");
   if (ny < 1 || psf_k < 0 || !n_windows || max_windows < 0 || (max_windows > 0 && !out)) return kErrParameters;
@@ -1391,6 +1391,16 @@ int nrgb_row_windows(int ny, int psf_k, int* out, int max_windows, int* n_window
   if (n > max_windows) return kErrParameters;
   std::copy(w.begin(), w.begin() + 4 * n, out);
   return kOk;
+}
+
+// The windows that a volume of size {nx, ny, nz} runs with (see the header).
+int nrgb_volume_windows(const int* size, int psf_k, int* out, int max_windows, int* n_windows) {
+  NRGB_API("nrgb_volume_windows");
+  if (!size || size[0] < 1 || size[1] < 1 || size[2] < 1 || psf_k < 0 || psf_k > 15 || (psf_k && psf_k % 2 != 1) ||
+      !n_windows || max_windows < 0 || (max_windows > 0 && !out))
+    return kErrParameters;
+  *n_windows = yg_call_windows(size[0], size[1], size[2], psf_k, out, max_windows);
+  return *n_windows <= max_windows ? kOk : kErrParameters;
 }
 
 // 1 when the last call of this thread ran the fused y-gantry kernels, 2 when

@@ -219,6 +219,10 @@ struct BatchElems {
 // -1 if more than max_windows.  nx: columns, for the split of the last window
 // (0, or where the split does not fit max_windows: unsplit).
 int yg_row_windows(int ny, int psf_k, int* out, int max_windows, int nx = 0);
+// The windows of a projection or backprojection of an nx x ny x nz volume, its PSF
+// given on the host too: 5 ints each (row0, rows, lo, hi, lanes per column), at
+// most max_windows written; returns the count.
+int yg_call_windows(int nx, int ny, int nz, int psf_k, int* out, int max_windows);
 // Lanes per column the tile kernels take for a window of `rows` rows of nx
 // columns, and the x-tiles that gives.
 void yg_window_lanes(int rows, int nx, int* lanes, int* tiles);

@@ -182,6 +182,23 @@ int yg_row_windows(int ny, int psf_k, int* out, int max_windows, int nx) {
   return static_cast<int>(w.size());
 }
 
+int yg_call_windows(int nx, int ny, int nz, int psf_k, int* out, int max_windows) {
+  YgArgs a;
+  a.nx = nx;
+  a.ny = ny;
+  a.nz = nz;
+  a.psf_k = psf_k;
+  static const float given = 0.0f;  // a PSF with its host copy
+  if (psf_k > 0) a.psf = a.psf_host = &given;
+  const std::vector<Window> wins = call_windows(a, psf_k > 0 ? (psf_k - 1) / 2 : 0);
+  for (size_t i = 0; i < wins.size() && static_cast<int>(i) < max_windows; ++i) {
+    const Window& w = wins[i];
+    const int v[5] = {w.row0, w.rows, w.lo, w.hi, windowed(a, w).lanes};
+    std::copy(v, v + 5, out + 5 * i);
+  }
+  return static_cast<int>(wins.size());
+}
+
 void yg_window_lanes(int rows, int nx, int* lanes, int* tiles) {
   *lanes = window_lanes(rows, nx);
   const int columns = 1024 / *lanes;
