@@ -6,8 +6,9 @@ projector with depth-dependent PSF and attenuation.  Its backward pass uses
 
 * d/d(activity): the library's exact-transpose backprojector (mode 1 of
   nrgb_backproject_device: transposed PSF and transposed bilinear weights);
-* d/d(mu): nrgb_attenuation_grad_device, which recomputes the depth scan of
-  every ray instead of storing per-angle transmission.
+* d/d(mu): nrgb_attenuation_grad_device, which leaves the terms of every ray
+  in scratch (4 bytes per voxel and camera of a group), sums them along the
+  ray and scatters the result.
 
 Both sum rotated-frame values into the volume with vector reductions, whose
 order varies between runs; ``set_deterministic(True)`` switches the fused

@@ -67,7 +67,7 @@ bool use_fused_x(const Problem& pb);
 // all-zero shape = default for shapes without an entry).
 int tuned_group(int nx, int ny, int nz, int ncam);
 void set_tuned_group(int nx, int ny, int nz, int ncam, int group);
-// Projector depth slabs (cluster size 2, 4 or 8) for a shape; 0 = none
+// Projector depth slabs (cluster size 2, 4, 8 or 16) for a shape; 0 = none
 // recorded (the launcher then chooses).
 int tuned_project_slabs(int nx, int ny, int nz, int ncam);
 void set_tuned_project_slabs(int nx, int ny, int nz, int ncam, int slabs);

@@ -80,7 +80,7 @@ struct YgArgs {
   int truncate = 0;
   int back_mode = kBackReference;
   int storage = kStorageF32;  // type of act and mu
-  int pslabs = 0;  // projector depth slabs = cluster size (2, 4, 8; 0: chosen by the launcher)
+  int pslabs = 0;  // projector depth slabs = cluster size (2 to 8 or 16; 0: chosen by the launcher: 2, 4, 6, 8, 16)
   // Units (device [nunits]): {camera, mirror camera or -1}; a mirror camera
   // sits at the opposite angle about the grid centre and is served from the
   // same samples by the projector and the reference-mode backprojector
@@ -118,8 +118,6 @@ struct YgArgs {
   // (yg_mu_carry) for exactly these cameras; the backprojector then skips
   // that pass and the work space holds only the scratch slot(s).
   const float* carry = nullptr;
-  // yg_backproject (reference form, deterministic transpose): the window's
-  // last gather stores max(result, 0) when a.truncate is set.
   // Gather: 1 takes the units' mirror cameras (skipping units without one).
   int mates = 0;
   // Non-zero (exact-transpose backprojector, d/dmu): deterministic form --

@@ -7,18 +7,19 @@
 // theta_x = theta_z = 0, so the resampling matrix is an exact rotation in the
 // (x, z) plane and y maps to itself.  Every detector row y then samples the
 // SAME bilinear footprint in the (x, z) plane, so the device layout puts y
-// fastest ("column layout" [z][x][cy]) and one warp handles whole columns:
-// lane l owns y = 4l..4l+3 (float4), the footprint of an (x, z) column is
-// computed once and every gather is a coalesced 16-byte-per-lane column load.
+// fastest ("column layout" [z][x][cy]) and a group of 32, 16 or 8 lanes handles
+// whole columns: lane l of the group owns y = 4l..4l+3 (float4), the footprint of
+// an (x, z) column is computed once and every gather is a coalesced
+// 16-byte-per-lane column load.
 //
 // Projector (emission-lib/_et.cpp:218-281): per camera and depth plane z,
 //   rotate (bilinear gather of activity and mu), per-plane separable PSF
 //   (row pass along x in a register sliding window over a shared tile, column
-//   pass along y through a per-warp shared row buffer), attenuated depth scan
-//   T += mu;
-//   p += v * exp(-T).  No rotated volume is written anywhere: a thread-block
-//   cluster owns (camera, 32-column x-tile), its CTAs own depth slabs and
-//   merge (T, p) through distributed shared memory.
+//   pass along y through a shared row buffer per lane group), attenuated depth
+//   scan T += mu; p += v * exp(-T).  No rotated volume is written: a thread-block
+//   cluster owns a camera, or a camera and its mirror camera, and an x-tile of 32,
+//   64 or 128 columns; its CTAs own depth slabs and merge (T, p) through
+//   distributed shared memory.
 // Backprojector, reference mode (emission-lib/_et.cpp:415-499):
 //   (1) per-slab transmission carries of the rotated mu, (2) per camera
 //   group: spread s*exp(-T) + PSF in the rotated frame into an L2-sized
@@ -171,9 +172,8 @@ __device__ __forceinline__ float4 sample4_branch(const V* __restrict__ base, con
 
 // Bilinear sample of a column.  float32: predicated loads, so that a warp has
 // the corners of several columns in flight (128^3 x 120, PSF 11: projector
-// 0.575 -> 0.537 ms, long-scoreboard stalls per issue 1.78 -> 1.31; attenuation
-// gradient 2.34 -> 2.17 ms, d/dmu 2.04 -> 1.97 ms).  bfloat16: the branch (its
-// backprojection measured 0.87 ms with the branch, 0.91 ms predicated).
+// 0.575 -> 0.537 ms, long-scoreboard stalls per issue 1.78 -> 1.31).  bfloat16: the
+// branch (its backprojection measured 0.87 ms with the branch, 0.91 ms predicated).
 __device__ __forceinline__ float4 sample4(const float* __restrict__ base, const Tap& t, int yb, bool yok) {
   return blend(load_corners(base, t, yb, yok), t);
 }
@@ -315,42 +315,8 @@ __device__ __forceinline__ float4 mask_rows(float4 v, int yb, int ny) {
 
 // Column (y) pass of the per-plane convolution for the 4 rows a lane owns:
 // out[y] = sum_k in[y+k] * kc[R-k], zero outside [0, ny) (rows >= ny are zero
-// pads, rows < 0 come from lanes below 0 and are masked).  Neighbour rows come
-// from lanes l-1, l-2 and l+1, l+2 by shuffles (the form for R = 0; larger
-// radii use yconv4s below).
-template <int R, class KC>
-__device__ __forceinline__ float4 yconv4(const float4& u, KC kc, int lane) {
-  float w[2 * R + 4];
-  w[R + 0] = u.x;
-  w[R + 1] = u.y;
-  w[R + 2] = u.z;
-  w[R + 3] = u.w;
-#pragma unroll
-  for (int t = 1; t <= R; ++t) {
-    const int dl = (t + 3) / 4;
-    const float s = __shfl_up_sync(kFull, comp(u, 4 * dl - t), dl);
-    w[R - t] = (lane >= dl) ? s : 0.0f;
-  }
-#pragma unroll
-  for (int t = 1; t <= R; ++t) {
-    const int dl = (t + 3) / 4;
-    const float s = __shfl_down_sync(kFull, comp(u, t + 3 - 4 * dl), dl);
-    w[R + 3 + t] = (lane + dl < 32) ? s : 0.0f;
-  }
-  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-  for (int k = -R; k <= R; ++k) {
-    const float kk = kc[R - k];
-    o.x = fmaf(w[R + 0 + k], kk, o.x);
-    o.y = fmaf(w[R + 1 + k], kk, o.y);
-    o.z = fmaf(w[R + 2 + k], kk, o.z);
-    o.w = fmaf(w[R + 3 + k], kk, o.w);
-  }
-  return o;
-}
-
-// Column pass through shared memory: each lane stores its 4 rows in its
-// group's row buffer and reads the neighbour rows back with 16-byte loads (one
+// pads).  Through shared memory: each lane stores its 4 rows in its group's row
+// buffer and reads the neighbour rows back with 16-byte loads (one
 // store and 2 ceil(R/4) loads in place of 2R shuffles and 2R selects).  Two
 // buffers per group alternate, so one warp barrier per call orders a store
 // after the loads of the call before the previous one.  Rows outside the
@@ -396,7 +362,7 @@ __device__ __forceinline__ void ybuf_zero_pads() {
 template <int R, int L, int YB, bool SHUF, class KC>
 __device__ __forceinline__ float4 yconv4s(const float4& u, KC kc, int lane, int b) {
   if constexpr (R == 0) {
-    return yconv4<0>(u, kc, lane);
+    return make_float4(fmaf(u.x, kc[0], 0.f), fmaf(u.y, kc[0], 0.f), fmaf(u.z, kc[0], 0.f), fmaf(u.w, kc[0], 0.f));
   } else {
     constexpr int C = (R + 3) / 4, N = R - 4 * (C - 1);
     constexpr int CL = SHUF ? C - 1 : C;  // chunks on either side read from the row buffer
@@ -563,14 +529,12 @@ struct TileShape {
   static constexpr int kTapSlots = G * kOwn;          // footprint slots per stage (see tap_slot)
   static constexpr size_t kSbBytes = sizeof(float4) * 2 * NS * L;
   static constexpr size_t kTapBytes = sizeof(Tap) * 2 * kTapSlots;
-  // Projector: 2 x steps tile buffers (steps depth planes sampled per
-  // barrier); the region also holds the slab-merge buffers after the walk (T
-  // and P per output column, and with a mirror camera its P).
-  __host__ __device__ static constexpr size_t sb_bytes(bool pair, int steps = 1) {
+  // Projector: two tile buffers; the region also holds the slab-merge buffers
+  // after the walk (T and P per output column, and with a mirror camera its P).
+  __host__ __device__ static constexpr size_t sb_bytes(bool pair) {
     return sizeof(float4) * L *
-           (2 * steps * NS > (pair ? 3 : 2) * kTX<L> ? 2 * steps * NS : (pair ? 3 : 2) * kTX<L>);
+           (2 * NS > (pair ? 3 : 2) * kTX<L> ? 2 * NS : (pair ? 3 : 2) * kTX<L>);
   }
-  __host__ __device__ static constexpr size_t tap_bytes(int steps = 1) { return sizeof(Tap) * 2 * steps * kTapSlots; }
   // Projector serving mirror cameras from bfloat16 storage: the Kahan
   // compensations of T, P and the mate's Q, one float4 per thread and output
   // column each, in shared memory ([3][kTX][L]) -- registers hold the sums.
@@ -590,16 +554,16 @@ __device__ __forceinline__ int tap_slot(int c) {
 // Tile, footprints and the separated PSF of nz planes (twice with a mirror
 // camera: its kernels are the mirrored planes, row kernels reversed).
 template <int R, int L>
-__host__ __device__ constexpr size_t tile_smem_bytes(int nz, bool pair = false, int steps = 1) {
-  return TileShape<R, L>::sb_bytes(pair, steps) + TileShape<R, L>::tap_bytes(steps) +
+__host__ __device__ constexpr size_t tile_smem_bytes(int nz, bool pair = false) {
+  return TileShape<R, L>::sb_bytes(pair) + TileShape<R, L>::kTapBytes +
          sizeof(float) * static_cast<size_t>(nz) * 2 * (2 * R + 1) * (pair ? 2 : 1);
 }
 
 // The projector's: the tile above plus, for mirror cameras from bfloat16
 // storage, the shared-memory Kahan compensations.
 template <int R, int L>
-__host__ __device__ constexpr size_t project_smem_bytes(int nz, bool pair, bool kahan, int steps = 1) {
-  return tile_smem_bytes<R, L>(nz, pair, steps) + TileShape<R, L>::comp_bytes(pair && kahan);
+__host__ __device__ constexpr size_t project_smem_bytes(int nz, bool pair, bool kahan) {
+  return tile_smem_bytes<R, L>(nz, pair) + TileShape<R, L>::comp_bytes(pair && kahan);
 }
 
 // Row pass from the shared tile: outputs i = 0..kTXW-1 of this group use tile
@@ -795,11 +759,10 @@ constexpr float kMateMaxT = 40.0f;
 // to volume a.group + a.vol0, in this camera's frame: its depth sum runs
 // towards this camera, so its S(z) is A + B * (the slab's terms up to and with z).
 //
-// STEPS: depth planes sampled per barrier (2 x STEPS tile buffers).  Two
-// planes per barrier measured no faster on GB300 (128^3 x 120: 0.676 against
-// 0.674 ms; 256^3 x 180: 11.9 against 11.2 ms), so the kernels use one.
+// One plane per barrier: two, with twice the tile buffers, measured no faster
+// (128^3 x 120: 0.676 against 0.674 ms; 256^3 x 180: 11.9 against 11.2 ms).
 template <int R, bool PSF, bool ATT, class V, bool PAIR = false, bool PTAB = false, int L = 32, int YB = L,
-          bool TERMS = false, int STEPS = 1>
+          bool TERMS = false>
 __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate, int x0, unsigned char* smem,
                                              const float* ptab = nullptr) {
   using TS = TileShape<R, L>;
@@ -810,11 +773,11 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
   const V* __restrict__ mu = reinterpret_cast<const V*>(a.mu) + a.row0;
   constexpr int NS = TS::NS;
   constexpr int K = 2 * R + 1;
-  constexpr size_t kSb = TS::sb_bytes(PAIR, STEPS);
-  float4* sb = reinterpret_cast<float4*>(smem);                    // [2 * STEPS][NS][L]
-  Tap* taps = reinterpret_cast<Tap*>(smem + kSb);                   // [2 * STEPS][kTapSlots]
-  float4* scomp = reinterpret_cast<float4*>(smem + kSb + TS::tap_bytes(STEPS));  // [3][kTX][L] (SCOMP)
-  float* s_psf = reinterpret_cast<float*>(smem + kSb + TS::tap_bytes(STEPS) + TS::comp_bytes(SCOMP));  // [nz][2K]
+  constexpr size_t kSb = TS::sb_bytes(PAIR);
+  float4* sb = reinterpret_cast<float4*>(smem);                    // [2][NS][L]
+  Tap* taps = reinterpret_cast<Tap*>(smem + kSb);                   // [2][kTapSlots]
+  float4* scomp = reinterpret_cast<float4*>(smem + kSb + TS::kTapBytes);  // [3][kTX][L] (SCOMP)
+  float* s_psf = reinterpret_cast<float*>(smem + kSb + TS::kTapBytes + TS::comp_bytes(SCOMP));  // [nz][2K]
   float* s_psf_m = s_psf + static_cast<size_t>(a.nz) * 2 * K;       // [nz][2K] (mate)
   cg::cluster_group cluster = cg::this_cluster();
   const int slab = static_cast<int>(cluster.block_rank());
@@ -1023,8 +986,8 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
     }
   };
 
-  // walk: STEPS planes per barrier; iteration j uses buffers (j & 1) * STEPS + s,
-  // rewritten at iteration j + 2 after the barrier of iteration j + 1
+  // walk: iteration k uses buffer k & 1, rewritten at iteration k + 2 after the
+  // barrier of iteration k + 1
   // carry split: planes of the slab's first half (the backprojector's slab
   // of twice the count that starts at zbeg); the slab-local transmission at
   // the middle goes straight into its carry slot, where the merge adds the
@@ -1049,17 +1012,12 @@ __device__ __forceinline__ void project_item(const YgArgs& a, int cam, int mate,
   auto walk = [&](auto mode) {
     constexpr int MODE = decltype(mode)::value;
     const int n = zend - zbeg;
-    for (int k = 0; k < n; k += STEPS) {
-      const int base = ((k / STEPS) & 1) * STEPS;
-#pragma unroll
-      for (int s = 0; s < STEPS; ++s)
-        if (k + s < n) produce(MODE == 0 ? zbeg + k + s : zend - 1 - k - s, base + s);
+    for (int k = 0; k < n; ++k) {
+      const int z = MODE == 0 ? zbeg + k : zend - 1 - k;
+      produce(z, k & 1);
       __syncthreads();
-#pragma unroll
-      for (int s = 0; s < STEPS; ++s) {
-        if (k + s < n) consume(MODE == 0 ? zbeg + k + s : zend - 1 - k - s, base + s, mode);
-        if (MODE == 0 && split && k + s + 1 == zhalf) stash_mid();
-      }
+      consume(z, k & 1, mode);
+      if (MODE == 0 && split && k + 1 == zhalf) stash_mid();
     }
     if (MODE == 0 && split && n < zhalf) stash_mid();  // the half ends past the volume
   };
@@ -1244,8 +1202,7 @@ static_assert(kTX<32> == 32 && kTX<16> == 64 && kTX<8> == 128, "1024 / L output 
 // the fewest lanes that hold the rows.
 int column_lanes(int rows) { return rows <= 32 ? 8 : rows <= 64 ? 16 : 32; }
 
-//
-// nx > 0: a last window of 65 rows or more that a 64-row and a 32-row window
+// The windows of ny rows for a halo.  nx > 0: a last window of 65 rows or more that a 64-row and a 32-row window
 // cover for fewer x-tiles is split so (192 rows with a halo of 8: 128 + 64 + 32
 // rows; 192^3 x 120 in bfloat16, PSF 15: pair 6.33 -> 6.06 ms).
 std::vector<Window> row_windows(int ny, int halo, int nx = 0) {

@@ -8,8 +8,10 @@
 namespace nrgb {
 namespace {
 
-// Row pass of a single camera: packed, but for radius 4 scalar (96^3 x 72, PSF 9:
-// 0.402 ms, packed 0.405).
+// Row pass of a single camera: packed, but scalar at radius 4, where the packed
+// form spills 16 bytes at the 80 registers of three CTAs per SM and the scalar one
+// none (111 x 93 x 111 x 72, PSF 9: backprojection 555 us, packed 559; 96^3 x 72: 402,
+// 405).  Radii 3 and 5 spill 4 and 8 bytes packed and still gain.
 template <int R, int L, class EmitFn, class KR, class KC>
 __device__ __forceinline__ void rowpass_single(const float4* __restrict__ sbuf, int base, EmitFn emit, KR kr, KC kc,
                                                int lane, int ny) {

@@ -43,7 +43,7 @@ def main(argv=None):
     ap.add_argument("--bf16", action="store_true", help="activity and mu stored in bfloat16")
     ap.add_argument("--slope", type=float, default=0.02, help="PSF sigma = 0.5 + slope * depth")
     ap.add_argument("--group", type=int, default=0, help="backprojector cameras per scratch group (0: tuned)")
-    ap.add_argument("--slabs", type=int, default=0, help="projector depth slabs 2/4/8 (0: tuned)")
+    ap.add_argument("--slabs", type=int, default=0, help="projector depth slabs 2/4/8/16 (0: tuned)")
     ap.add_argument("--no-mirror", action="store_true", help="every camera from its own matrix")
     ap.add_argument("--det", action="store_true",
                     help="deterministic exact-transpose backprojection and d/dmu (nrgb_set_deterministic)")
@@ -115,7 +115,7 @@ def main(argv=None):
                                                     psize, 0.0, 0.0, 0, vp(stream.cuda_stream))
             assert st == 0, st
         run = run_gradient
-    elif a.op == "dmu":  # d/dmu of sum(g * project(act, mu)), the fused recomputed-scan kernel
+    elif a.op == "dmu":  # d/dmu of sum(g * project(act, mu)), the fused kernels
         if a.bf16 or t_mu is None:
             raise SystemExit("dmu: float32 activity and mu required")
         g = torch.from_numpy(np.random.default_rng(3).uniform(0.5, 1.5, (a.ncam, n, n)).astype(np.float32)).to(dev)
