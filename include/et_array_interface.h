@@ -309,9 +309,10 @@ int nrgb_osem_update_device(float *d_activity, const float *d_numerator, const f
                             float epsilon, void *stream);
 
 /* Host-side fault injection (no counterpart in the reference): the next n
- * device work-space allocations that would grow the library's arena fail with
- * status 4 (allocgpu) before any CUDA call is made, so callers' error paths
- * can be tested without a GPU fault.  n = 0 clears it. */
+ * device work-space allocations that would grow the library's arena fail before
+ * any CUDA call is made, so callers' error paths can be tested without a GPU
+ * fault: a call that can run in a smaller work space tries that next, any other
+ * returns status 4 (allocgpu).  n = 0 clears it. */
 int nrgb_debug_fail_allocations(int n);
 
 /* Diagnostics: 1 if the calling thread's last call ran the fused y-gantry

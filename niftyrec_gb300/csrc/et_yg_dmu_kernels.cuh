@@ -13,7 +13,7 @@
 //     coefficients per ray and depth slab (project_item, TERMS);
 //   k_dmu_scatter_yg: the terms summed along the ray and -g S(z) scattered at
 //     each camera's own positions.
-// 128^3 x 120, PSF 11: 1.33 ms (terms 2 x 0.39, scatter 2 x 0.25), against 1.96 ms
+// 128^3 x 120, PSF 11: 1.36 ms (terms 2 x 0.40, scatter 2 x 0.27), against 1.96 ms
 // of one kernel whose second walk recomputed samples and PSF of every camera
 // alone.  The terms (4 bytes per voxel and camera, 1 GB written and read) cost
 // less than that walk.  Reading them back in the first kernel's own CTAs
